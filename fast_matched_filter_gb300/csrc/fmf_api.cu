@@ -34,6 +34,7 @@ namespace fmf {
 static thread_local int g_status = FMF_OK;
 static thread_local char g_msg[512] = "";
 static thread_local int g_launches = 0;
+static thread_local bool g_bounded_waits = false;  // this call launched a kernel with bounded waits
 
 int set_error(int status, const char *fmt, ...)
 {
@@ -55,7 +56,12 @@ static int clear_error()
 void count_launch(int n) { g_launches += n; }
 static thread_local int g_last_precision = -1;
 void set_last_precision(int precision) { g_last_precision = precision; }
-void reset_launch_count() { g_launches = 0; }
+void reset_launch_count()
+{
+    g_launches = 0;
+    g_bounded_waits = false;
+}
+void note_bounded_waits() { g_bounded_waits = true; }
 
 // ---------------------------------------------------------------- event timing
 // Opt-in (fmf_timing_begin/end): every call records CUDA events on its stream
@@ -173,7 +179,8 @@ static int cuda_status(cudaError_t e, const char *what)
 }
 
 // ---------------------------------------------------------------- kernels
-__global__ void template_range_kernel(const int *, int, int, int, int, int, int, int *, int *);
+__global__ void template_range_kernel(const int *, int, int, int, int, int, int, int *, int *, const float *,
+                                      unsigned *);
 __global__ void template_center_kernel(const float *, int, float *, float *);
 __global__ void template_energy_kernel(const float *, int, int, float *);
 __global__ void channel_centre_kernel(const float *, int, float *);
@@ -209,6 +216,12 @@ int device_error_word(unsigned **out)
 }
 
 // Reads and clears the error word after the device has finished the work.
+int collect_device_errors();
+
+// The same for the calling thread's own call: nothing to read where it launched
+// no kernel that waits.
+int collect_own_errors() { return g_bounded_waits ? collect_device_errors() : FMF_OK; }
+
 int collect_device_errors()
 {
     unsigned *w = nullptr;
@@ -272,7 +285,8 @@ int validate_args(const Args &a)
 }
 
 // ---------------------------------------------------------------- core (device pointers)
-int prepare_problem(const Args &a, Scratch &ws, cudaStream_t s, Problem *Pout, const float **data_for_tc)
+int prepare_problem(const Args &a, Scratch &ws, cudaStream_t s, Problem *Pout, const float **data_for_tc,
+                    bool want_scan)
 {
     int rc;
     const int T = (int)a.T, SC = (int)(a.S * a.C), L = (int)a.L, N = (int)a.N;
@@ -295,9 +309,13 @@ int prepare_problem(const Args &a, Scratch &ws, cudaStream_t s, Problem *Pout, c
             return rc;
     }
 
-    template_range_kernel<<<(T + 127) / 128, 128, 0, s>>>(a.mo, T, SC, L, N, (int)a.step,
-                                                            (int)a.n_corr, k_lo, k_hi);
-    count_launch();
+    unsigned *scan = nullptr;
+    if (want_scan) {
+        const size_t n = 3 * (size_t)SC + 1;
+        if ((rc = ws.get(&scan, n, "channel scan")) ||
+            (rc = cuda_status(cudaMemsetAsync(scan, 0, n * sizeof(unsigned), s), "clearing the channel scan")))
+            return rc;
+    }
     const float *sst = a.sst;
     if (!sst) {  // template energies as numpy computes them for float32 templates
         float *e = nullptr;
@@ -308,12 +326,15 @@ int prepare_problem(const Args &a, Scratch &ws, cudaStream_t s, Problem *Pout, c
         count_launch();
         sst = e;
     }
+    template_range_kernel<<<(T + 127) / 128, 128, 0, s>>>(a.mo, T, SC, L, N, (int)a.step,
+                                                            (int)a.n_corr, k_lo, k_hi, sst, scan);
+    count_launch();
     if (full) {
         template_center_kernel<<<(unsigned)((size_t)T * SC), 128, 0, s>>>(a.tpl, L, tcen, tsum);
         channel_centre_kernel<<<SC, 1024, 0, s>>>(a.data, N, mu);
         count_launch(2);
     }
-    if ((rc = launch_window_stats(a.data, N, L, SC, mu, dcen, stat_e, s)))
+    if ((rc = launch_window_stats(a.data, N, L, SC, mu, dcen, stat_e, scan, s)))
         return rc;
     if ((rc = check_launch("preprocessing kernels")))
         return rc;
@@ -343,6 +364,8 @@ int prepare_problem(const Args &a, Scratch &ws, cudaStream_t s, Problem *Pout, c
     P.pre1f = nullptr;
     P.zweight = nullptr;
     P.vp_norm = P.vp_bias = P.vp_scale = nullptr;
+    P.scan = scan;
+    P.only_if = nullptr;
 
     if (!P.network_sum) {
         size_t bytes = (size_t)T * a.n_corr * SC * sizeof(float);
@@ -398,6 +421,69 @@ int launch_plain_all(const Problem &P, cudaStream_t s)
     return FMF_OK;
 }
 
+// Templates [t0, t0 + nt) of a prepared problem.
+static Problem problem_subset(const Problem &P, int t0, int nt)
+{
+    Problem Q = P;
+    const size_t o = (size_t)t0 * P.SC;
+    Q.tpl += o * P.L;
+    Q.sst += o;
+    if (Q.tsum)
+        Q.tsum += o;
+    Q.mo += o;
+    Q.w += o;
+    Q.k_lo += t0;
+    Q.k_hi += t0;
+    Q.out += (size_t)t0 * P.n_corr * (P.network_sum ? 1 : P.SC);
+    Q.T = nt;
+    return Q;
+}
+
+// Tile of an FP32 search that may run on the tensor cores ('auto' too: it may
+// choose FP32), 0 otherwise.
+static int fp32_tile(const Args &a)
+{
+    if (a.precision != FMF_PREC_FP32 && a.precision != FMF_PREC_AUTO)
+        return 0;
+    return tc32_choose_nb(a.T, a.S * a.C, a.L, a.step, a.n_corr);
+}
+
+// An FP32 search of a prepared problem, run in parts of its templates: on the
+// tensor cores (nb != 0 and their working arrays can be had), followed by the
+// CUDA-core kernel, which runs only where the operands' flag says so; else on the
+// CUDA cores alone.
+struct Fp32Search {
+    Problem P;
+    std::vector<unsigned char> tc;
+    unsigned *err = nullptr;
+    int status = FMF_OK;
+
+    Fp32Search(const Problem &p, int nb, int group, int max_templates, Scratch &ws, cudaStream_t s) : P(p)
+    {
+        if (nb == 0 || !P.scan || (status = device_error_word(&err)))
+            return;
+        tc.resize(tc32_search_size());
+        status = tc32_begin(P, nb, group, max_templates, ws, s, search());
+        if (status == FMF_ERR_OOM) {  // the CUDA-core kernel needs no more memory
+            clear_error();
+            tc.clear();
+            status = FMF_OK;
+        }
+    }
+    Tc32Search *search() { return reinterpret_cast<Tc32Search *>(tc.data()); }
+    int run(int t0, int nt, Scratch &ws, cudaStream_t s)
+    {
+        Problem Q = problem_subset(P, t0, nt);
+        if (!tc.empty()) {
+            int rc = tc32_run(search(), t0, nt, err, ws, s);
+            if (rc)
+                return rc;
+            Q.only_if = tc32_flag(search());
+        }
+        return launch_plain_all(Q, s);
+    }
+};
+
 // Search on device pointers with its working arrays in `ws` (they stay
 // allocated, and *Pout valid, until ws goes out of scope).
 static int run_device_ws(const Args &a, cudaStream_t s, Scratch &ws, Problem *Pout)
@@ -406,7 +492,8 @@ static int run_device_ws(const Args &a, cudaStream_t s, Scratch &ws, Problem *Po
     Problem &P = *Pout;
     const float *data_for_tc = nullptr;
     cudaEvent_t ev_prep0 = mark(s);
-    if ((rc = prepare_problem(a, ws, s, &P, &data_for_tc)))
+    const int nb32 = fp32_tile(a);
+    if ((rc = prepare_problem(a, ws, s, &P, &data_for_tc, nb32 != 0)))
         return rc;
     cudaEvent_t ev_prep1 = mark(s);
     span(ev_prep0, ev_prep1, kSpanPrep);
@@ -431,7 +518,8 @@ static int run_device_ws(const Args &a, cudaStream_t s, Scratch &ws, Problem *Po
         return rc;
     }
     cudaEvent_t ev_main0 = mark(s);
-    rc = launch_plain_all(P, s);
+    Fp32Search f(P, nb32, (a.flags >> 16) & 0xff, P.T, ws, s);
+    rc = f.status ? f.status : f.run(0, P.T, ws, s);
     span(ev_main0, mark(s), kSpanKernel);
     return rc;
 }
@@ -450,24 +538,6 @@ static int run_device(const Args &a, cudaStream_t s)
 }
 
 // ---------------------------------------------------------------- host-pointer path
-// Templates [t0, t0 + nt) of a prepared problem.
-static Problem problem_subset(const Problem &P, int t0, int nt)
-{
-    Problem Q = P;
-    const size_t o = (size_t)t0 * P.SC;
-    Q.tpl += o * P.L;
-    Q.sst += o;
-    if (Q.tsum)
-        Q.tsum += o;
-    Q.mo += o;
-    Q.w += o;
-    Q.k_lo += t0;
-    Q.k_hi += t0;
-    Q.out += (size_t)t0 * P.n_corr * (P.network_sum ? 1 : P.SC);
-    Q.T = nt;
-    return Q;
-}
-
 // Device-resident search whose result is copied to `host_out` in template
 // chunks on a second stream, each chunk's copy overlapping the next chunk's
 // kernel.  Preprocessing is done once for all templates.
@@ -478,7 +548,8 @@ static int run_streamed(const Args &d, float *host_out, cudaStream_t s)
     Problem P;
     const float *data_for_tc = nullptr;
     cudaEvent_t ev_prep0 = mark(s);
-    if ((rc = prepare_problem(d, ws, s, &P, &data_for_tc)))
+    const int nb32 = fp32_tile(d);
+    if ((rc = prepare_problem(d, ws, s, &P, &data_for_tc, nb32 != 0)))
         return rc;
     cudaEvent_t ev_kern0 = mark(s);
     span(ev_prep0, ev_kern0, kSpanPrep);
@@ -503,11 +574,16 @@ static int run_streamed(const Args &d, float *host_out, cudaStream_t s)
     }
     unsigned *err = nullptr;
     std::vector<unsigned char> tcfull;
-    int split = 0;
+    int split = 0, most = 0;
     int precision = d.precision;
     if (precision == FMF_PREC_AUTO && (rc = choose_auto_precision(P, ws, s, &precision)))
         return rc;
     set_last_precision(precision);
+    for (int c = 0; c < n_chunks; c++)
+        most = bounds[c + 1] - bounds[c] > most ? bounds[c + 1] - bounds[c] : most;
+    Fp32Search fp32(P, precision == FMF_PREC_FP32 ? nb32 : 0, (d.flags >> 16) & 0xff, most, ws, s);
+    if ((rc = fp32.status))
+        return rc;
     if (precision != FMF_PREC_FP32) {
         if ((rc = device_error_word(&err)))
             return rc;
@@ -550,9 +626,9 @@ static int run_streamed(const Args &d, float *host_out, cudaStream_t s)
                     tc_subset(reinterpret_cast<const TcProb *>(tcfull.data()), t0, nt,
                               reinterpret_cast<TcProb *>(sub.data()));
                     if (!(rc = ws.get(&queue, 1, "tile queue")))
-                        rc = tc_run(reinterpret_cast<const TcProb *>(sub.data()), 1, split, queue, err, s);
+                        rc = tc_run(reinterpret_cast<const TcProb *>(sub.data()), 1, split, 0, queue, err, s);
                 } else {
-                    rc = launch_plain_all(problem_subset(P, t0, nt), s);
+                    rc = fp32.run(t0, nt, ws, s);
                 }
                 if (!rc && zc)
                     rc = launch_zero_count(d, P.out, t0, nt, zc, s);
@@ -652,13 +728,13 @@ static int run_host(const Args &a, cudaStream_t s)
     }
     if ((rc = cuda_status(cudaStreamSynchronize(s), "matched filter")))
         return rc;
-    return g_last_precision != FMF_PREC_FP32 ? collect_device_errors() : FMF_OK;
+    return collect_own_errors();
 }
 
 static int entry(const Args &a, void *stream)
 {
     clear_error();
-    g_launches = 0;
+    reset_launch_count();
     int rc = validate_args(a);
     if (rc)
         return rc;
@@ -838,7 +914,7 @@ static int search_detect_entry(const Args &a0, const DetectOut &o, cudaStream_t 
         return FMF_OK;
     if ((rc = detect_copy_back(o, a.T, dd, s)))
         return rc;
-    return g_last_precision != FMF_PREC_FP32 ? collect_device_errors() : FMF_OK;
+    return collect_device_errors();
 }
 
 }  // namespace fmf

@@ -107,7 +107,7 @@ static int batch_record(fmf_batch *b, cudaStream_t s)
                         if ((status = ws.get(&queue, 1, "tile queue")))
                             break;
                         const int m = (int)(ng - i0 < (size_t)TC_MAX_PROBS ? ng - i0 : TC_MAX_PROBS);
-                        status = tc_run(reinterpret_cast<const TcProb *>(grp.data() + psz * i0), m, split,
+                        status = tc_run(reinterpret_cast<const TcProb *>(grp.data() + psz * i0), m, split, 0,
                                         queue, err, s);
                     }
                 }

@@ -48,6 +48,13 @@ struct Problem {
     // (T) each, or null: when set, the tensor-core kernel writes
     // (tanh(x / vp_norm[t]) + vp_bias[t]) * vp_scale[t] for every output x
     const float *vp_norm, *vp_bias, *vp_scale;
+    // FP32 on the tensor cores, else null: the channel scan of prepare_problem
+    // [3 SC + 1]: the largest |x| of each data channel; its smallest window energy
+    // that can pass the threshold (bits complemented, so that zero means none); the
+    // largest template energy on it; the search's flag: the scan or the operands
+    // left it to the CUDA-core kernel
+    unsigned *scan;
+    const unsigned *only_if;  // plain kernel: run only if this word is nonzero (null: always)
 };
 
 #ifdef __CUDACC__
@@ -152,6 +159,7 @@ namespace fmf {
 int set_error(int status, const char *fmt, ...);
 void count_launch(int n = 1);
 void reset_launch_count();  // at the start of every entry point (fmf_last_launch_count)
+void note_bounded_waits();  // this call launched a kernel that may raise the device error word
 void keep_pool_cached();    // at the start of every entry point that allocates scratch
 int check_launch(const char *what);
 // The dynamic shared memory every variable-size kernel is allowed: the
@@ -217,16 +225,32 @@ int validate_args(const Args &a);
 constexpr int kStatWindows = 4096;
 size_t window_stats_smem(int L, bool full);
 int launch_window_stats(const float *data, int N, int L, int SC, const float *mu, float *dcen,
-                        float *stat_e, cudaStream_t s);
-int prepare_problem(const Args &a, Scratch &ws, cudaStream_t s, Problem *P, const float **data_for_tc);
+                        float *stat_e, unsigned *scan, cudaStream_t s);
+// scan: also make Problem::scan, for the FP32 form on the tensor cores
+int prepare_problem(const Args &a, Scratch &ws, cudaStream_t s, Problem *P, const float **data_for_tc,
+                    bool scan = false);
 
 // Tensor-core form (fmf_tc.cu).
 constexpr int TC_MAX_PROBS = 64;
+// operands of a persistent launch: one bf16 product, bf16 pairs, fp16 pairs (FP32 accuracy)
+enum { TC_FORM_BF16 = 0, TC_FORM_SPLIT = 1, TC_FORM_FP32 = 2 };
 struct TcProb;
 int tc_choose_nb(int L, int step, int split, int forced);
 int tc_prepare(const Problem &P, const float *data_for_tc, int split, int nb, int tg, Scratch &ws,
                cudaStream_t s, TcProb *out);
-int tc_run(const TcProb *probs, int n, int split, unsigned long long *queue, unsigned *err,
+
+// FP32 on the tensor cores (fmf_tc32.cu): begin a search, then run its templates in
+// parts; the search's flag word says afterwards that the CUDA cores have to run it.
+struct Tc32Search;
+size_t tc32_search_size();
+int tc32_choose_nb(size_t T, size_t SC, size_t L, size_t step, size_t n_corr);  // 0: the CUDA cores
+int tc32_begin(const Problem &P, int nb, int tg, int max_templates, Scratch &ws, cudaStream_t s,
+               Tc32Search *out);
+int tc32_run(const Tc32Search *full, int t0, int nt, unsigned *err, Scratch &ws, cudaStream_t s);
+const unsigned *tc32_flag(const Tc32Search *full);
+int tc32_prepare(const Problem &P, int nb, int tg, Scratch &ws, cudaStream_t s, TcProb *out);
+int tc_choose_parts(const TcProb *prob);
+int tc_run(const TcProb *probs, int n, int form, int parts, unsigned long long *queue, unsigned *err,
            cudaStream_t s);
 size_t tc_prob_size();
 void tc_subset(const TcProb *full, int t0, int nt, TcProb *out);

@@ -37,7 +37,8 @@
 
 namespace fmf {
 
-__global__ void template_range_kernel(const int *, int, int, int, int, int, int, int *, int *);
+__global__ void template_range_kernel(const int *, int, int, int, int, int, int, int *, int *, const float *,
+                                      unsigned *);
 __global__ void template_energy_kernel(const float *, int, int, float *);
 __global__ void template_center_kernel(const float *, int, float *, float *);
 __global__ void channel_centre_kernel(const float *, int, float *);
@@ -185,7 +186,7 @@ extern "C" int fmf_matched_filter_noalloc(const float *templates, const float *s
 
     cudaGetLastError();
     template_range_kernel<<<(T + 127) / 128, 128, 0, s>>>(moveouts, T, SC, L, N, (int)step, (int)n_corr,
-                                                            k_lo, k_hi);
+                                                            k_lo, k_hi, nullptr, nullptr);
     count_launch();
     if (energies) {  // as numpy sums float32 templates**2: bit-identical energies
         template_energy_kernel<<<(T * SC + 127) / 128, 128, 0, s>>>(templates, T * SC, L, sst);
@@ -196,7 +197,7 @@ extern "C" int fmf_matched_filter_noalloc(const float *templates, const float *s
         channel_centre_kernel<<<SC, 1024, 0, s>>>(data, N, mu);
         count_launch(2);
     }
-    if ((rc = launch_window_stats(data, N, L, SC, mu, dcen, stat_e, s)))
+    if ((rc = launch_window_stats(data, N, L, SC, mu, dcen, stat_e, nullptr, s)))
         return rc;
     cudaError_t e;
     if ((e = cudaGetLastError()) != cudaSuccess)
@@ -232,6 +233,8 @@ extern "C" int fmf_matched_filter_noalloc(const float *templates, const float *s
     P.pre1f = nullptr;
     P.zweight = nullptr;
     P.vp_norm = P.vp_bias = P.vp_scale = nullptr;
+    P.scan = nullptr;
+    P.only_if = nullptr;
     if ((rc = launch_plain_all(P, s)))
         return rc;
     return FMF_OK;

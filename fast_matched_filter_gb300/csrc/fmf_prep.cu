@@ -30,7 +30,8 @@ namespace fmf {
 
 __global__ void template_range_kernel(const int *__restrict__ mo, int T, int SC,
                                       int L, int N, int step, int n_corr,
-                                      int *__restrict__ k_lo, int *__restrict__ k_hi)
+                                      int *__restrict__ k_lo, int *__restrict__ k_hi,
+                                      const float *__restrict__ sst, unsigned *__restrict__ scan)
 {
     int t = blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= T)
@@ -41,6 +42,12 @@ __global__ void template_range_kernel(const int *__restrict__ mo, int T, int SC,
         lo = min(lo, m[ch]);
         hi = max(hi, m[ch]);
     }
+    if (scan)  // the largest template energy of each channel
+        for (int ch = 0; ch < SC; ch++) {
+            const float e = sst[(size_t)t * SC + ch];
+            if (e > 0.0f)  // NaN left out: such a channel's coefficients are all 0
+                atomicMax(scan + 2 * SC + ch, __float_as_uint(e));
+        }
     long long first = lo < 0 ? ((long long)(-lo) + step - 1) / step : 0;
     long long last = (long long)N - L - hi;
     long long a = 0, b = 0;
@@ -293,7 +300,7 @@ size_t window_stats_smem(int L, bool full) { return (size_t)StatLayout(L, full).
 template <bool FULL>
 __global__ void __launch_bounds__(kStatThreads, FULL ? 2 : 3)
 window_stats_kernel(const float *__restrict__ data, int N, int L, const float *__restrict__ mu,
-                    float *__restrict__ dcen, float *__restrict__ stat_e)
+                    float *__restrict__ dcen, float *__restrict__ stat_e, unsigned *__restrict__ scan)
 {
     extern __shared__ float4 stat_smem[];
     constexpr bool full = FULL;
@@ -314,6 +321,7 @@ window_stats_kernel(const float *__restrict__ data, int N, int L, const float *_
     const float m = full ? mu[ch] : 0.0f;
     const float *src = data + (size_t)ch * N + c0;
     constexpr int kLoads = 4;  // loads in flight per thread before their use
+    unsigned top = 0;          // bits of the largest finite |v|
     for (int i0 = threadIdx.x; i0 < span; i0 += kLoads * kStatThreads) {
         float x[kLoads];
 #pragma unroll
@@ -330,6 +338,8 @@ window_stats_kernel(const float *__restrict__ data, int N, int L, const float *_
                     dcen[(size_t)ch * N + c0 + i] = v;
                 const float sq = v * v;
                 s2[stat_pad(i)] = make_float2(sq, fmaf(v, v, -sq));  // v^2 exactly
+                const unsigned av = __float_as_uint(v) & 0x7fffffffu;
+                top = av < 0x7f800000u ? max(top, av) : top;
                 if (full)
                     s1[stat_pad(i)] = v;
             }
@@ -444,28 +454,56 @@ window_stats_kernel(const float *__restrict__ data, int N, int L, const float *_
         }
     }
     __syncthreads();
+    // energies at or below this pass no template's threshold
+    const float dead = scan ? kThreshold / __uint_as_float(scan[2 * gridDim.y + ch]) * 0.999f : 0.0f;
+    unsigned low = 0;  // the smallest energy above it, bits complemented
     for (int u = threadIdx.x; u < nwin; u += kStatThreads) {  // coalesced stores
         const size_t o = (size_t)ch * N + c0 + u;
-        if (full)
-            reinterpret_cast<float2 *>(stat_e)[o] = out2[stat_pad(u)];
-        else
-            stat_e[o] = out1[stat_pad(u)];
+        float en;
+        if (full) {
+            const float2 v = out2[stat_pad(u)];
+            reinterpret_cast<float2 *>(stat_e)[o] = v;
+            en = v.x;
+        } else {
+            en = out1[stat_pad(u)];
+            stat_e[o] = en;
+        }
+        if (en > dead)
+            low = max(low, ~__float_as_uint(en));
+    }
+    if (scan) {  // one atomic per block, and only where it changes the channel's value
+        unsigned *red = reinterpret_cast<unsigned *>(base);  // the squares are no longer read
+        top = __reduce_max_sync(0xffffffffu, top);
+        low = __reduce_max_sync(0xffffffffu, low);
+        if ((threadIdx.x & 31) == 0) {
+            red[threadIdx.x >> 5] = top;
+            red[32 + (threadIdx.x >> 5)] = low;
+        }
+        __syncthreads();
+        if (threadIdx.x < 2) {
+            unsigned v = 0;
+            for (int i = 0; i < kStatThreads / 32; i++)
+                v = max(v, red[32 * threadIdx.x + i]);
+            unsigned *word = scan + threadIdx.x * gridDim.y + ch;
+            if (v > *(volatile unsigned *)word)
+                atomicMax(word, v);
+        }
     }
 }
 
 int launch_window_stats(const float *data, int N, int L, int SC, const float *mu, float *dcen,
-                        float *stat_e, cudaStream_t s)
+                        float *stat_e, unsigned *scan, cudaStream_t s)
 {
     const bool full = mu != nullptr;
     const size_t smem = window_stats_smem(L, full);
-    void (*kern)(const float *, int, int, const float *, float *, float *) =
+    void (*kern)(const float *, int, int, const float *, float *, float *, unsigned *) =
         full ? window_stats_kernel<true> : window_stats_kernel<false>;
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxDynamicSmem);
     if (e != cudaSuccess)
         return set_error(FMF_ERR_CUDA, "window statistics shared memory (%zu bytes): %s", smem,
                          cudaGetErrorString(e));
     dim3 grid((N + kStatWindows - 1) / kStatWindows, SC);
-    kern<<<grid, kStatThreads, smem, s>>>(data, N, L, mu, dcen, stat_e);
+    kern<<<grid, kStatThreads, smem, s>>>(data, N, L, mu, dcen, stat_e, scan);
     count_launch();
     return FMF_OK;
 }

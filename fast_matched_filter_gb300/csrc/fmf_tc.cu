@@ -58,237 +58,15 @@
 #include <cuda_bf16.h>
 
 #include "fmf_common.cuh"
+#include "fmf_tc.cuh"
 
 namespace fmf {
 
-constexpr int TC_Q = 128;
-constexpr int TC_CB = TC_Q / 8;
 // Epilogue warps (2 per TMEM lane quarter; 4 per quarter for per-channel
 // template lengths, whose epilogue does more arithmetic per output and needs
 // more warps to hide its latency) + producer, 2 MMA issuers, 1 idle warp.
 constexpr int tc_epi_warps(bool var) { return var ? 16 : 8; }
 constexpr int tc_threads(bool var) { return 32 * (4 + tc_epi_warps(var)); }
-constexpr int TC_TG = 16;  // templates interleaved per group of CTAs (L2 reuse of data rows)
-constexpr unsigned long long TC_WAIT_NS = 2000000000ull;  // 2 s per wait
-
-
-// One search of a persistent launch (tile-queue items [item_begin, item_begin + n_tiles*T)).
-struct TcProb {
-    Problem P;                    // sizes, epilogue inputs, output
-    const uint16_t *g_hi, *g_lo;  // bf16 bits, data streams [SC][step][CB][rows_total][8]
-    const uint16_t *w_hi, *w_lo;  // bf16 bits, template blocks [T][SC][step][NW][64]
-    const int *mu;                // [T][SC][step] moveout of each phase in its stream
-    const int *psi;               // [T][SC][step] stream of each phase
-    long long item_begin;         // first tile-queue item of this search
-    int R;                        // data rows per stage
-    int NW;                       // 128-byte template blocks per (template, channel, phase)
-    int rows_total;               // rows per (channel, stream) in the data streams
-    int row_front;                // rows of zero padding before sample 0
-    int n_tiles;                  // output tiles of nb*128 indices
-    int tg;                       // templates interleaved per group of items
-    int nb;                       // lag blocks per tile (MMA N): 32, 64 or 128
-    int parts;                    // k >= 1: the channels of a (tile, template) in k
-                                  // ranges [j SC / k, (j + 1) SC / k) on k CTAs (items
-                                  // j = 0..k-1 adjacent); their network sums go to
-                                  // part_out[j][t][lag] and are added in order j after
-                                  // the launch (a fixed order: deterministic results)
-    float *part_out;
-};
-
-struct TcBatch {
-    TcProb prob[TC_MAX_PROBS];
-    int n_probs;
-    int split;                    // 1: hi/lo, three products; 0: single bf16 product
-    int stage_bytes;              // bytes of one pipeline stage (largest search)
-    long long total_items;
-    unsigned long long *queue;    // tile-queue head, zero before the launch
-    unsigned *err;                // device error word
-};
-
-// ------------------------------------------------------------------ PTX helpers
-__device__ __forceinline__ uint32_t smem_u32(const void *p)
-{
-    return (uint32_t)__cvta_generic_to_shared(p);
-}
-
-__device__ __forceinline__ void mbar_init(uint32_t bar, int count)
-{
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count) : "memory");
-}
-
-__device__ __forceinline__ void mbar_expect_tx(uint32_t bar, uint32_t bytes)
-{
-    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes)
-                 : "memory");
-}
-
-__device__ __forceinline__ void mbar_arrive(uint32_t bar)
-{
-    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
-}
-
-__device__ __forceinline__ bool mbar_try(uint32_t bar, uint32_t parity)
-{
-    uint32_t ok;
-    asm volatile(
-        "{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n"
-        " selp.u32 %0, 1, 0, p;\n}\n"
-        : "=r"(ok)
-        : "r"(bar), "r"(parity)
-        : "memory");
-    return ok != 0;
-}
-
-__device__ __forceinline__ unsigned long long gtimer()
-{
-    unsigned long long t;
-    asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t));
-    return t;
-}
-
-// Bounded wait on an mbarrier phase.  Returns false when the CTA aborted or
-// when this wait gave up after `limit_ns` (then it raises the error word and
-// the abort flag).
-__device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatile int *abort_flag,
-                                          unsigned *err, unsigned code,
-                                          unsigned long long limit_ns = TC_WAIT_NS)
-{
-    if (mbar_try(bar, parity))
-        return true;
-    unsigned long long t0 = gtimer();
-    for (unsigned it = 1;; it++) {
-        if (mbar_try(bar, parity))
-            return true;
-        if ((it & 63) == 0) {
-            if (*abort_flag)
-                return false;
-            if (gtimer() - t0 > limit_ns) {
-                atomicOr(err, code);
-                *abort_flag = 1;
-                return false;
-            }
-        }
-    }
-}
-
-// Warp-uniform form: lane 0 waits, the result is broadcast to the warp.
-__device__ __forceinline__ bool mbar_wait_warp(uint32_t bar, uint32_t parity, volatile int *abort_flag,
-                                               unsigned *err, unsigned code)
-{
-    int ok = 0;
-    if ((threadIdx.x & 31) == 0)
-        ok = mbar_wait(bar, parity, abort_flag, err, code) ? 1 : 0;
-    return __shfl_sync(0xffffffffu, ok, 0) != 0;
-}
-
-__device__ __forceinline__ void bulk_g2s(uint32_t dst, const void *src, uint32_t bytes, uint32_t bar)
-{
-    asm volatile(
-        "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
-            dst),
-        "l"(src), "r"(bytes), "r"(bar)
-        : "memory");
-}
-
-// Shared-memory matrix descriptor, no swizzle (layout type 0), version 1.
-__device__ __forceinline__ uint64_t sdesc(uint32_t addr, uint32_t lbo, uint32_t sbo)
-{
-    return (uint64_t)((addr & 0x3FFFFu) >> 4) | ((uint64_t)((lbo >> 4) & 0x3FFFu) << 16) |
-           ((uint64_t)((sbo >> 4) & 0x3FFFu) << 32) | (1ull << 46);
-}
-
-__device__ __forceinline__ void mma_bf16(uint32_t d_tmem, uint64_t a, uint64_t b, uint32_t idesc,
-                                         uint32_t accumulate)
-{
-    asm volatile(
-        "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n"
-        " tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}\n" ::"r"(d_tmem),
-        "l"(a), "l"(b), "r"(idesc), "r"(accumulate)
-        : "memory");
-}
-
-__device__ __forceinline__ void mma_commit(uint32_t bar)
-{
-    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
-                     bar)
-                 : "memory");
-}
-
-__device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
-__device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
-
-// 32 lanes x 32 bits, 16 consecutive columns per thread
-__device__ __forceinline__ void tmem_ld16(uint32_t taddr, float *v)
-{
-    uint32_t r[16];
-    asm volatile(
-        "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, "
-        "[%16];"
-        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]),
-          "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]),
-          "=r"(r[14]), "=r"(r[15])
-        : "r"(taddr));
-#pragma unroll
-    for (int i = 0; i < 16; i++)
-        v[i] = __uint_as_float(r[i]);
-}
-
-__device__ __forceinline__ void tmem_wait_ld() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
-
-__device__ __forceinline__ void tmem_ld8(uint32_t taddr, float *v)
-{
-    uint32_t r[8];
-    asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
-                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]),
-                   "=r"(r[7])
-                 : "r"(taddr));
-#pragma unroll
-    for (int i = 0; i < 8; i++)
-        v[i] = __uint_as_float(r[i]);
-}
-
-__device__ __forceinline__ void tmem_st16(uint32_t taddr, const float *v)
-{
-    asm volatile(
-        "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,"
-        "%16};" ::"r"(taddr),
-        "r"(__float_as_uint(v[0])), "r"(__float_as_uint(v[1])), "r"(__float_as_uint(v[2])),
-        "r"(__float_as_uint(v[3])), "r"(__float_as_uint(v[4])), "r"(__float_as_uint(v[5])),
-        "r"(__float_as_uint(v[6])), "r"(__float_as_uint(v[7])), "r"(__float_as_uint(v[8])),
-        "r"(__float_as_uint(v[9])), "r"(__float_as_uint(v[10])), "r"(__float_as_uint(v[11])),
-        "r"(__float_as_uint(v[12])), "r"(__float_as_uint(v[13])), "r"(__float_as_uint(v[14])),
-        "r"(__float_as_uint(v[15]))
-        : "memory");
-}
-
-__device__ __forceinline__ void tmem_st8(uint32_t taddr, const float *v)
-{
-    asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};" ::"r"(taddr),
-                 "r"(__float_as_uint(v[0])), "r"(__float_as_uint(v[1])), "r"(__float_as_uint(v[2])),
-                 "r"(__float_as_uint(v[3])), "r"(__float_as_uint(v[4])), "r"(__float_as_uint(v[5])),
-                 "r"(__float_as_uint(v[6])), "r"(__float_as_uint(v[7]))
-                 : "memory");
-}
-
-__device__ __forceinline__ void tmem_wait_st() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
-
-// CH consecutive accumulator columns of this warp's 32 lanes (CH = 8 or 16)
-template <int CH>
-__device__ __forceinline__ void tmem_ldc(uint32_t taddr, float *v)
-{
-    if constexpr (CH == 16)
-        tmem_ld16(taddr, v);
-    else
-        tmem_ld8(taddr, v);
-}
-template <int CH>
-__device__ __forceinline__ void tmem_stc(uint32_t taddr, const float *v)
-{
-    if constexpr (CH == 16)
-        tmem_st16(taddr, v);
-    else
-        tmem_st8(taddr, v);
-}
 
 // ------------------------------------------------------------------ preprocessing
 __device__ __forceinline__ void split_bf16(float x, uint16_t &hi, uint16_t &lo)
@@ -388,107 +166,8 @@ __global__ void tc_template_kernel(const float *__restrict__ tpl, const int *__r
 }
 
 // ------------------------------------------------------------------ persistent kernel
-// Decodes a tile-queue item: search p, output tile, template t.  Items of one
-// search are ordered so that groups of `tg` templates sweep the tiles together.
-template <bool PARTS>
-__device__ __forceinline__ void decode_item(const TcBatch &B, long long item, int &p, int &tile, int &t,
-                                            int &c_begin, int &c_end, int &part)
-{
-    int lo = 0, hi = B.n_probs - 1;
-    while (lo < hi) {
-        const int mid = (lo + hi + 1) >> 1;
-        if (B.prob[mid].item_begin <= item)
-            lo = mid;
-        else
-            hi = mid - 1;
-    }
-    p = lo;
-    const TcProb &pr = B.prob[p];
-    long long local = item - pr.item_begin;
-    c_begin = 0;
-    c_end = pr.P.SC;
-    part = 0;
-    if (PARTS) {  // the parts of a (tile, template) are adjacent items
-        const int k = pr.parts;
-        part = (int)(local % k);
-        local /= k;
-        c_begin = (int)((long long)part * pr.P.SC / k);
-        c_end = (int)((long long)(part + 1) * pr.P.SC / k);
-    }
-    const long long per_group = (long long)pr.n_tiles * pr.tg;
-    const int grp = (int)(local / per_group);
-    const long long rem = local - (long long)grp * per_group;
-    const int tg0 = grp * pr.tg;
-    const int tgn = min(pr.tg, pr.P.T - tg0);
-    tile = (int)(rem / tgn);
-    t = tg0 + (int)(rem % tgn);
-}
-
-constexpr int TC_NB_MAX = 128;  // largest tile; TMEM columns: D0 [0,128), D1 [128,256), sum [256,384)
+// TMEM columns: D0 [0,128), D1 [128,256), sum [256,384)
 constexpr int TC_NACC = 2;      // accumulator buffers
-
-// 1/sqrt(x), one approximate MUFU operation; subnormal x is flushed to zero
-// (result +inf).
-__device__ __forceinline__ float rsqrt_ftz(float x)
-{
-    float r;
-    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
-    return r;
-}
-
-// atanh(y) in FP32 for the Fisher-z network sum, at most a few ulp from the
-// exact value (the accuracy of the CUDA library's atanhf) with far fewer
-// instructions for the common small arguments:
-//  |y| <= 1/4: the Maclaurin series y + y^3/3 + ... + y^13/13 (the first
-//    omitted term is below 2^-25 of the result);
-//  1/4 < |y| < 1: atanh(a) = ln(q) / 2 with q = (1 + a) / (1 - a); q = 2^k m
-//    with m in [sqrt(1/2), sqrt(2)) and ln(m) = 2 atanh(s), s = (m - 1) / (m + 1),
-//    |s| <= 0.1716, from the same series to s^9/9;
-//  |y| = 1 gives +-inf, |y| > 1 and NaN give NaN.
-__device__ __forceinline__ float atanh_series(float y)
-{
-    const float z = y * y;
-    float p = fmaf(1.0f / 13.0f, z, 1.0f / 11.0f);
-    p = fmaf(p, z, 1.0f / 9.0f);
-    p = fmaf(p, z, 1.0f / 7.0f);
-    p = fmaf(p, z, 1.0f / 5.0f);
-    p = fmaf(p, z, 1.0f / 3.0f);
-    return fmaf(y * z, p, y);
-}
-
-__device__ __forceinline__ float atanh_reduced(float y)
-{
-    const float a = fabsf(y);
-    if (!(a < 1.0f))  // 1, above 1, NaN
-        return a == 1.0f ? copysignf(INFINITY, y) : __int_as_float(0x7fc00000);
-    const float q = __fdividef(1.0f + a, 1.0f - a);  // in (5/3, 2^25] for a > 1/4
-    const int bits = __float_as_int(q);
-    const int k = (bits - 0x3f3504f3) >> 23;  // 0x3f3504f3 = sqrt(1/2)
-    const float m = __int_as_float(bits - (k << 23));
-    const float s = __fdividef(m - 1.0f, m + 1.0f);
-    const float z = s * s;
-    float p = fmaf(1.0f / 9.0f, z, 1.0f / 7.0f);
-    p = fmaf(p, z, 1.0f / 5.0f);
-    p = fmaf(p, z, 1.0f / 3.0f);
-    float r = fmaf(s * z, p, s);                         // ln(m) / 2
-    r = fmaf((float)k, 0.5f * 0.693145751953125f, r);    // + k ln2 / 2 (ln2 in two parts)
-    r = fmaf((float)k, 0.5f * 1.4286068203094172e-06f, r);
-    return copysignf(r, y);
-}
-
-// Called by all 32 lanes of a warp together: the series on every lane, the
-// reduction only when some lane of the warp needs it (no divergent branch;
-// the common case, every |y| <= 1/4, skips it).
-__device__ __forceinline__ float fisher_atanh(float y)
-{
-    const bool big = !(fabsf(y) <= 0.25f);  // NaN included
-    float r = atanh_series(y);
-    if (__any_sync(0xffffffffu, big)) {
-        const float g = atanh_reduced(y);
-        r = big ? g : r;
-    }
-    return r;
-}
 
 // every lane of every warp takes part (the tail reads a dummy value)
 __global__ void fisher_atanh_kernel(const float *__restrict__ y, float *__restrict__ out, long long n)
@@ -703,14 +382,10 @@ __global__ void __launch_bounds__(tc_threads(VAR), 1) tc_persistent(const __grid
                         const long long meta = ((long long)t * SC + ch) * step + phi;
                         const int mu = pr.mu[meta];
                         const int sres = ((mu % TC_Q) + TC_Q) % TC_Q;
-                        int lphi = (P.L - phi + step - 1) / step;
-                        if constexpr (VAR) {  // per-channel length: the taps past it are zeros, skip them
-                            const int n = P.ntap[(size_t)t * SC + ch];
-                            const int own = n > phi ? (n - phi + step - 1) / step : 0;
-                            lphi = min(lphi, own);
-                        }
+                        // per-channel lengths: the taps past the channel's own are zeros, skip them
+                        const int taps = tc_phase_taps(P.L, step, phi, VAR ? P.ntap[(size_t)t * SC + ch] : P.L);
                         const int k_first = sres & ~15;
-                        const int k_end = (sres + lphi + TC_Q - 1 + 15) & ~15;
+                        const int k_end = tc_k_end(sres, taps);
                         const uint32_t zhi = smem_u32(smem + (size_t)s * B.stage_bytes);
                         const uint32_t whi = zhi + w_off;
                         // Descriptors advance by additions: the start-address field (bits 0-13,
@@ -1050,23 +725,6 @@ int launch_wait_selftest(unsigned *err, unsigned ms, cudaStream_t s)
 }
 
 // ------------------------------------------------------------------ host side
-struct TcShape {
-    int k_span, R, NW;
-    size_t stage;
-};
-
-static TcShape tc_shape(int L, int step, int split, int nb)
-{
-    TcShape g;
-    const int lphi = (L + step - 1) / step;
-    g.k_span = ((2 * TC_Q - 2 + lphi) + 15) & ~15;
-    g.R = nb + (g.k_span - 1) / TC_Q + 1;
-    g.NW = g.k_span / 8 + 16;
-    g.stage = (size_t)(split ? 2 : 1) * ((size_t)TC_CB * g.R * 16 + (size_t)g.NW * 128);
-    g.stage = (g.stage + 1023) & ~(size_t)1023;
-    return g;
-}
-
 constexpr size_t TC_BAR_BYTES = 256;
 
 // Largest tile (lag blocks per CTA tile) whose two pipeline stages fit in shared memory.
@@ -1089,25 +747,8 @@ int tc_prepare(const Problem &P, const float *data_for_tc, int split, int nb, in
 {
     int rc;
     const int step = P.step, L = P.L;
-    const TcShape g = tc_shape(L, step, split, nb);
     TcProb pr;
-    pr.P = P;
-    pr.R = g.R;
-    pr.NW = g.NW;
-    pr.n_tiles = (int)((P.n_corr + (long long)TC_Q * nb - 1) / ((long long)TC_Q * nb));
-    pr.tg = tg > 0 ? tg : TC_TG;
-    pr.nb = nb;
-    // Stream rows a tile can touch.  An item is processed only when its tile
-    // holds a valid output k of its template, i.e. k*step + mo >= 0 and
-    // k*step + mo + L <= N for every channel; hence its first row
-    // r0 = (I0 + mu - s)/Q lies in [-(NB + 2), (N/step + 1)/Q + 1] whatever the
-    // moveouts are, and rows [r0, r0 + R) stay inside the padded stream.
-    pr.row_front = nb + 3;
-    pr.rows_total = pr.row_front + (int)(((long long)P.N / step + 2) / TC_Q) + 2 + g.R + 1;
-    pr.item_begin = 0;
-    pr.parts = 1;
-    pr.part_out = nullptr;
-
+    const TcShape g = tc_fill_shape(P, split, nb, tg, &pr);
     const size_t g_elems = (size_t)P.SC * step * TC_CB * pr.rows_total * 8;
     const size_t w_elems = (size_t)P.T * P.SC * step * g.NW * 64;
     const size_t n_meta = (size_t)P.T * P.SC * step;
@@ -1172,7 +813,7 @@ __global__ void tc_parts_sum_kernel(const float *__restrict__ part, int k, long 
 // items: the k that minimises the busiest SM's work, ceil(k items / SMs)
 // rounds of (1/k + 0.05) item each (0.05: an item's fixed pipeline fill and
 // output write); FMF_TC_PARTS=k forces a value.
-static int tc_choose_parts(long long items, int SC)
+static int choose_parts(long long items, int SC)
 {
     const int sms = n_sms(), kmax = SC < 8 ? SC : 8;
     if (const char *env = getenv("FMF_TC_PARTS")) {
@@ -1193,23 +834,36 @@ static int tc_choose_parts(long long items, int SC)
     return best;
 }
 
+// Channel parts of a prepared search run by itself (tc_run).  A lone search with
+// fewer (tile, template) items than SMs runs each item as k channel parts
+// (network sum only; with per-channel lengths the parts add raw Fisher-z sums
+// and the transform follows the addition), k chosen to shorten the busiest
+// SM's queue.  FMF_TC_PARTS=k overrides the choice where parts are allowed.
+int tc_choose_parts(const TcProb *prob)
+{
+    const Problem &P = prob->P;
+    return P.network_sum && P.SC >= 2 ? choose_parts((long long)prob->n_tiles * P.T, P.SC) : 1;
+}
+
 // One persistent launch over the tile queue of `n` prepared searches (n <= TC_MAX_PROBS).
-// `queue` is a device counter that this call zeroes on `s` before the launch.
-int tc_run(const TcProb *probs, int n, int split, unsigned long long *queue, unsigned *err, cudaStream_t s)
+// `form`: the operands they were prepared with.  `parts`: channel parts of every
+// item (n = 1 only; 0 = tc_choose_parts).  `queue` is a device counter that this
+// call zeroes on `s` before the launch.
+int tc_run(const TcProb *probs, int n, int form, int parts, unsigned long long *queue, unsigned *err,
+           cudaStream_t s)
 {
     if (n < 1 || n > TC_MAX_PROBS)
         return set_error(FMF_ERR_ARG, "a persistent launch takes 1..%d searches", TC_MAX_PROBS);
     static thread_local TcBatch Bh;  // large; built on the host for the launch only
     TcBatch &B = Bh;
+    const int split = form != TC_FORM_BF16;  // operand pairs
     long long items = 0;
     size_t stage = 0;
-    // A lone search with fewer (tile, template) items than SMs runs each item as k
-    // channel parts (network sum only; with per-channel lengths the parts add raw
-    // Fisher-z sums and the transform follows the addition), k chosen to shorten the
-    // busiest SM's queue.  FMF_TC_PARTS=k overrides the choice where parts are allowed.
     const Problem &P0 = probs[0].P;
-    const bool can_split = n == 1 && P0.network_sum && P0.SC >= 2;
-    const int parts = can_split ? tc_choose_parts((long long)probs[0].n_tiles * P0.T, P0.SC) : 1;
+    if (n > 1)
+        parts = 1;
+    else if (parts == 0)
+        parts = tc_choose_parts(&probs[0]);
     Scratch pws(s);
     float *part_out = nullptr;
     if (parts > 1) {
@@ -1252,8 +906,14 @@ int tc_run(const TcProb *probs, int n, int split, unsigned long long *queue, uns
     for (int i = 0; i < n; i++)
         n_full += probs[i].P.normalize != 0;
     const int norm = n_full == 0 ? 0 : (n_full == n ? 1 : -1);
-    void (*kern)(const TcBatch);
-    if (n_var && norm >= 0)  // per-channel lengths: always one search, one normalisation
+    TcKernel kern;
+    int threads = tc_threads(n_var != 0);
+    if (form == TC_FORM_FP32) {
+        if (norm < 0)
+            return set_error(FMF_ERR_ARG, "a persistent FP32 launch mixes normalisations");
+        kern = tc32_kernel(n_var != 0, norm == 1);
+        threads = tc32_threads();
+    } else if (n_var && norm >= 0)  // per-channel lengths: always one search, one normalisation
         kern = parts > 1 ? (norm == 0 ? tc_persistent<true, true, 0> : tc_persistent<true, true, 1>)
                          : (norm == 0 ? tc_persistent<true, false, 0> : tc_persistent<true, false, 1>);
     else if (n_var)
@@ -1268,8 +928,9 @@ int tc_run(const TcProb *probs, int n, int split, unsigned long long *queue, uns
     if (e != cudaSuccess)
         return set_error(FMF_ERR_CUDA, "tc_persistent shared memory (%zu bytes): %s", smem,
                          cudaGetErrorString(e));
-    kern<<<grid, tc_threads(n_var != 0), smem, s>>>(B);
+    kern<<<grid, threads, smem, s>>>(B);
     count_launch();
+    note_bounded_waits();
     int rc = check_launch("tc_persistent");
     if (rc || parts == 1)
         return rc;
@@ -1314,6 +975,10 @@ void tc_subset(const TcProb *full, int t0, int nt, TcProb *out)
         q.w_lo += o * step * q.NW * 64;
     q.mu += o * step;
     q.psi += o * step;
+    if (q.t_exp) {
+        q.t_exp += o;
+        q.k_steps += o;
+    }
     *out = q;
 }
 
@@ -1333,7 +998,7 @@ int launch_tc(const Problem &P, const float *data_for_tc, int precision, unsigne
     unsigned long long *queue = nullptr;
     if ((rc = ws.get(&queue, 1, "tile queue")))
         return rc;
-    return tc_run(&pr, 1, split, queue, err, s);
+    return tc_run(&pr, 1, split ? TC_FORM_SPLIT : TC_FORM_BF16, 0, queue, err, s);
 }
 
 }  // namespace fmf

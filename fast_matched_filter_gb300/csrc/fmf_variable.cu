@@ -36,7 +36,7 @@
 namespace fmf {
 
 __global__ void channel_centre_kernel(const float *, int, float *);
-int collect_device_errors();
+int collect_own_errors();
 
 // Fisher-z weight of every (t, ch), one thread each, in the reference's mix
 // of float and double operations: z = sqrt(n - 3) * w as
@@ -202,7 +202,7 @@ constexpr int kPrefixBlock = 2048;
 // scheduling) and the unit.
 // grid (blocks, SC), 256 threads
 __global__ void channel_energy_kernel(const float *__restrict__ data, int N, const float *__restrict__ mu,
-                                      float *__restrict__ part, int nblk)
+                                      float *__restrict__ part, int nblk, unsigned *__restrict__ scan)
 {
     __shared__ float2 red[8];
     const int ch = blockIdx.y, blk = blockIdx.x;
@@ -221,6 +221,17 @@ __global__ void channel_energy_kernel(const float *__restrict__ data, int N, con
     for (int e = 0; e < per; e++) {
         const float sq = x[e] * x[e];
         pair_add(h, l, sq, fmaf(x[e], x[e], -sq));
+    }
+    if (scan) {  // Problem::scan: the channel's largest finite |d|
+        unsigned top = 0;
+#pragma unroll
+        for (int e = 0; e < per; e++) {
+            const unsigned a = __float_as_uint(x[e]) & 0x7fffffffu;
+            top = a < 0x7f800000u ? max(top, a) : top;
+        }
+        top = __reduce_max_sync(0xffffffffu, top);
+        if ((threadIdx.x & 31) == 0 && top > *(volatile unsigned *)(scan + ch))
+            atomicMax(scan + ch, top);
     }
     for (int o = 16; o > 0; o >>= 1) {
         const float yh = __shfl_down_sync(0xffffffffu, h, o), yl = __shfl_down_sync(0xffffffffu, l, o);
@@ -462,8 +473,10 @@ __global__ void prefix_write_kernel(const float *__restrict__ data, int N, const
 // out[t][k] = (tanh(out / norm_sum[t]) + bias[t]) * scale[t] for every k < n_corr
 __global__ void vp_finalize_kernel(float *__restrict__ out, int T, int n_corr,
                                    const float *__restrict__ norm_sum, const float *__restrict__ bias,
-                                   const float *__restrict__ scale)
+                                   const float *__restrict__ scale, const unsigned *__restrict__ only_if)
 {
+    if (only_if && *only_if == 0)  // the tensor cores ran this search, transform included
+        return;
     const long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (idx >= (long long)T * n_corr)
         return;
@@ -555,6 +568,18 @@ static int variable_device(const VArgs &a, int L, cudaStream_t s, float *host_ou
                  (rc = ws.get(&dcen, (size_t)SC * N, "centred data")) ||
                  (rc = ws.get(&pre1f, (size_t)SC * (N + 1), "prefix sums of d"))))
         return rc;
+    int precision = FMF_FLAG_PRECISION_OF(a.flags);
+    const bool may_fp32 = precision == FMF_PREC_FP32 || precision == FMF_PREC_AUTO;
+    const int nb32 = may_fp32 ? tc32_choose_nb(a.T, a.S * a.C, (size_t)L, a.step, a.n_corr) : 0;
+    unsigned *scan = nullptr;
+    if (nb32) {
+        const size_t n = 3 * (size_t)SC + 1;
+        if ((rc = ws.get(&scan, n, "channel scan")))
+            return rc;
+        cudaError_t e = cudaMemsetAsync(scan, 0, n * sizeof(unsigned), s);
+        if (e != cudaSuccess)
+            return set_error(FMF_ERR_CUDA, "clearing the channel scan: %s", cudaGetErrorString(e));
+    }
     int *k_hi = k_lo + T;
     float *norm_sum = consts, *bias = consts + T, *scale = consts + 2 * T;
 
@@ -566,7 +591,7 @@ static int variable_device(const VArgs &a, int L, cudaStream_t s, float *host_ou
     vp_template_kernel<<<(unsigned)((size_t)T * SC), 128, 0, s>>>(a.tpl, a.ntap, L, full ? 1 : 0, tmask, tsum);
     if (full)
         channel_centre_kernel<<<SC, 1024, 0, s>>>(a.data, N, mu);
-    channel_energy_kernel<<<dim3(nblk, SC), 256, 0, s>>>(a.data, N, mu, epart, nblk);
+    channel_energy_kernel<<<dim3(nblk, SC), 256, 0, s>>>(a.data, N, mu, epart, nblk, scan);
     channel_unit_kernel<<<SC, 32, 0, s>>>(epart, nblk, unit);
     prefix_block_kernel<<<dim3(nblk, SC), 256, 0, s>>>(a.data, N, mu, unit, bs2, bs1, nblk);
     prefix_offsets_kernel<<<(SC + 3) / 4, 128, 0, s>>>(bs2, bs1, nblk, SC);  // a warp per channel
@@ -601,7 +626,8 @@ static int variable_device(const VArgs &a, int L, cudaStream_t s, float *host_ou
     P.pre1f = pre1f;
     P.zweight = zweight;
     P.vp_norm = P.vp_bias = P.vp_scale = nullptr;
-    int precision = FMF_FLAG_PRECISION_OF(a.flags);
+    P.scan = scan;
+    P.only_if = nullptr;
     if (precision == FMF_PREC_AUTO && (rc = choose_auto_precision(P, ws, s, &precision)))
         return rc;
     set_last_precision(precision);
@@ -619,9 +645,31 @@ static int variable_device(const VArgs &a, int L, cudaStream_t s, float *host_ou
         }
         bounds[n_chunks] = T;
     }
+    int most = 0;  // templates of the largest chunk
+    for (int c = 0; c < n_chunks; c++)
+        most = bounds[c + 1] - bounds[c] > most ? bounds[c + 1] - bounds[c] : most;
     unsigned *err = nullptr;
     int split = 0;
     std::vector<unsigned char> tcfull;
+    std::vector<unsigned char> tc32;
+    if (precision == FMF_PREC_FP32 && nb32) {
+        Problem Q = P;
+        Q.vp_norm = norm_sum;
+        Q.vp_bias = bias;
+        Q.vp_scale = scale;
+        tc32.resize(tc32_search_size());
+        rc = device_error_word(&err);
+        if (!rc)
+            rc = tc32_begin(Q, nb32, 0, most, ws, s, reinterpret_cast<Tc32Search *>(tc32.data()));
+        if (rc == FMF_ERR_OOM) {  // the CUDA-core kernel needs no more memory
+            set_error(FMF_OK, "");
+            tc32.clear();
+        } else if (rc) {
+            return rc;
+        } else {
+            P.only_if = tc32_flag(reinterpret_cast<Tc32Search *>(tc32.data()));
+        }
+    }
     if (precision != FMF_PREC_FP32) {
         const int forced = ((a.flags >> 8) & 0xff) * 16;
         if (forced != 0 && forced != 32 && forced != 64 && forced != 128)
@@ -653,14 +701,18 @@ static int variable_device(const VArgs &a, int L, cudaStream_t s, float *host_ou
                 tc_subset(reinterpret_cast<const TcProb *>(tcfull.data()), t0, nt,
                           reinterpret_cast<TcProb *>(sub.data()));
                 if ((rc = ws.get(&queue, 1, "tile queue")) ||
-                    (rc = tc_run(reinterpret_cast<const TcProb *>(sub.data()), 1, split, queue, err, s)))
+                    (rc = tc_run(reinterpret_cast<const TcProb *>(sub.data()), 1, split, 0, queue, err, s)))
                     return rc;
             } else {
+                if (!tc32.empty() &&
+                    (rc = tc32_run(reinterpret_cast<const Tc32Search *>(tc32.data()), t0, nt, err, ws, s)))
+                    return rc;
                 if ((rc = launch_plain_all(var_subset(P, t0, nt), s)))
                     return rc;
                 const long long n = (long long)nt * a.n_corr;
                 vp_finalize_kernel<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(
-                    a.out + (size_t)t0 * a.n_corr, nt, (int)a.n_corr, norm_sum + t0, bias + t0, scale + t0);
+                    a.out + (size_t)t0 * a.n_corr, nt, (int)a.n_corr, norm_sum + t0, bias + t0, scale + t0,
+                    P.only_if);
                 count_launch();
                 if ((rc = check_launch("variable-length transform")))
                     return rc;
@@ -771,7 +823,7 @@ static int variable_entry(const VArgs &a, void *stream)
     cudaError_t e = cudaStreamSynchronize(s);
     if (e != cudaSuccess)
         return set_error(FMF_ERR_CUDA, "variable-length search: %s", cudaGetErrorString(e));
-    return fmf_last_precision() != FMF_PREC_FP32 ? collect_device_errors() : FMF_OK;  // the form that ran
+    return collect_own_errors();
 }
 
 }  // namespace fmf

@@ -1,0 +1,121 @@
+"""The FP32 form on the tensor cores, at the sizes where its tiles, K steps and
+chains end (needs a GB300).
+
+Tolerance, per channel of weight 1 (|cc| <= 1): a chain of at most 16 K steps
+loses up to 2^-23 of its partial sum at each (the tensor core truncates), the
+partial sums of all chains together are at most 1 (Cauchy-Schwarz), so 16 *
+2^-23; an operand pair is within 2^-23 of its value and l * l is dropped, two
+more; the additions of the chains, the window energy, the reciprocal root and
+the network sum round to nearest, 8 * 2^-24 with room.  In all 22 * 2^-23 =
+2.6e-6 for weights that sum to 1.
+"""
+import numpy as np
+import pytest
+
+import fast_matched_filter_gb300 as fmf
+from oracle import fp64
+from tests._cases import random_search
+
+pytestmark = pytest.mark.gpu
+TOL = 22 * 2.0 ** -23
+
+
+def _search(monkeypatch, tile, tp, mo, w, d, step=1, **kw):
+    monkeypatch.setenv("FMF_TC32", str(tile))
+    return fmf.matched_filter(tp, mo, w, d, step, check_zeros=False, **kw)
+
+
+def _check(got, ref):
+    assert np.array_equal(got == 0, ref == 0)
+    err = np.abs(got.astype(np.float64) - ref)
+    assert err.max() <= TOL, "max %.3g at %s" % (err.max(), np.unravel_index(err.argmax(), err.shape))
+
+
+@pytest.mark.parametrize("tile", [32, 64, 128])
+@pytest.mark.parametrize("extra", [-1, 0, 1, 129])
+def test_output_counts_around_a_tile(monkeypatch, tile, extra):
+    # n_corr one short of a tile, a tile, one more, one row and one more
+    L = 33
+    N = 128 * tile + extra + L - 1
+    tp, mo, w, d = random_search(tile + extra, 2, 2, 1, L, N, -9, 140)
+    got = _search(monkeypatch, tile, tp, mo, w, d)
+    _check(got, fp64.fp64_matched_filter(tp, mo, w, d, 1, "short", True))
+
+
+@pytest.mark.parametrize("L", [1, 15, 16, 17, 113, 128, 129, 143, 144, 145, 257, 1201])
+@pytest.mark.parametrize("normalize", ["short", "full"])
+def test_template_lengths_around_k_steps_and_chains(monkeypatch, L, normalize):
+    tp, mo, w, d = random_search(L, 2, 2, 2, L, 5000 + L, -130, 260, dc=3.0, zero_weights=1)
+    got = _search(monkeypatch, 32, tp, mo, w, d, normalize=normalize)
+    _check(got, fp64.fp64_matched_filter(tp, mo, w, d, 1, normalize, True))
+
+
+@pytest.mark.parametrize("step", [2, 3, 7, 50])
+@pytest.mark.parametrize("network_sum", [True, False])
+def test_phases_of_a_decimated_search(monkeypatch, step, network_sum):
+    tp, mo, w, d = random_search(step, 2, 2, 2, 45, 9000 + step, -40, 300, dc=1.0, zero_weights=1)
+    got = _search(monkeypatch, 32, tp, mo, w, d, step, normalize="full", network_sum=network_sum)
+    ref = fp64.fp64_matched_filter(tp, mo, w, d, step, "full", network_sum)
+    _check(got, ref.reshape(got.shape))
+
+
+@pytest.mark.parametrize("parts", [1, 2, 5])
+def test_channel_parts(monkeypatch, parts):
+    monkeypatch.setenv("FMF_TC_PARTS", str(parts))
+    tp, mo, w, d = random_search(50 + parts, 3, 3, 2, 90, 20000, 0, 200, zero_weights=4)
+    got = _search(monkeypatch, 128, tp, mo, w, d)
+    _check(got, fp64.fp64_matched_filter(tp, mo, w, d, 1, "short", True))
+
+
+@pytest.mark.parametrize("normalize", ["short", "full"])
+def test_per_channel_lengths(monkeypatch, normalize):
+    rng = np.random.default_rng(8)
+    tp, mo, w, d = random_search(9, 2, 3, 2, 150, 9000, -30, 90, dc=2.0, zero_weights=1)
+    n = rng.integers(20, 151, mo.shape).astype(np.int32)
+    n[0, 0, 0] = 150
+    for i in np.ndindex(n.shape):
+        tp[i][n[i]:] = 0.0
+    got = _search(monkeypatch, 32, tp, mo, w, d, normalize=normalize, n_samples_template=n)
+    ref = fp64.fp64_matched_filter_variable(tp, n, mo, w, d, 1, normalize)
+    # up to |cc| = 0.9 the inverse hyperbolic tangent grows an error by 1 / (1 - 0.81) < 6
+    scale = np.cumsum(w.reshape(2, -1).sum(axis=1))[:, None]
+    assert (np.abs(got - ref) / scale).max() <= 6 * TOL
+
+
+def _both(monkeypatch, tp, mo, w, d, **kw):
+    return [_search(monkeypatch, tile, tp, mo, w, d, **kw) for tile in (0, 32)]
+
+
+@pytest.mark.parametrize("normalize", ["short", "full"])
+@pytest.mark.parametrize("bad", [np.nan, np.inf, 1e30])
+def test_values_that_are_not_finite_or_huge(monkeypatch, normalize, bad):
+    """A sample that is not finite (or whose square is not) silences the windows
+    that hold it, and no others, as on the CUDA cores."""
+    tp, mo, w, d = random_search(3, 2, 2, 2, 60, 6000, 0, 50)
+    d[0, 0, 3000] = bad
+    plain, tensor = _both(monkeypatch, tp, mo, w, d, normalize=normalize, network_sum=False)
+    assert np.array_equal(np.isfinite(plain), np.isfinite(tensor))
+    assert np.array_equal(plain == 0, tensor == 0)
+    assert np.abs(plain - tensor).max() <= 2 * TOL
+
+
+@pytest.mark.parametrize("scale", [1e-14, 1e-9, 1e9, 1e18])
+def test_amplitudes_beside_one_another(monkeypatch, scale):
+    """Quiet windows far below the channel's largest value, and template and data
+    amplitudes far apart: what the operand pairs cannot hold runs on the CUDA
+    cores."""
+    tp, mo, w, d = random_search(4, 2, 2, 1, 60, 6000, 0, 50)
+    tp = (tp / np.float32(scale)).astype(np.float32)
+    d = (d * np.float32(scale)).astype(np.float32)
+    d[1, 0, :2000] *= np.float32(1e7)
+    plain, tensor = _both(monkeypatch, tp, mo, w, d)
+    assert plain.any()
+    assert np.array_equal(plain == 0, tensor == 0)
+    assert np.abs(plain - tensor).max() <= 2 * TOL
+
+
+def test_template_that_is_not_finite(monkeypatch):
+    tp, mo, w, d = random_search(5, 2, 2, 1, 60, 6000, 0, 50)
+    tp[1, 0, 0, 7] = np.inf
+    plain, tensor = _both(monkeypatch, tp, mo, w, d)
+    assert np.array_equal(plain, tensor, equal_nan=True)  # the CUDA cores ran both
