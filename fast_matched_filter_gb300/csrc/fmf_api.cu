@@ -179,10 +179,7 @@ static int cuda_status(cudaError_t e, const char *what)
 }
 
 // ---------------------------------------------------------------- kernels
-__global__ void template_range_kernel(const int *, int, int, int, int, int, int, int *, int *, const float *,
-                                      unsigned *);
 __global__ void template_center_kernel(const float *, int, float *, float *);
-__global__ void template_energy_kernel(const float *, int, int, float *);
 __global__ void channel_centre_kernel(const float *, int, float *);
 __global__ void zero_count_kernel(const float *, long long, long long, long long, unsigned long long *);
 int launch_tc(const Problem &P, const float *data_for_tc, int precision, unsigned *err, Scratch &ws,
@@ -286,7 +283,7 @@ int validate_args(const Args &a)
 
 // ---------------------------------------------------------------- core (device pointers)
 int prepare_problem(const Args &a, Scratch &ws, cudaStream_t s, Problem *Pout, const float **data_for_tc,
-                    bool want_scan)
+                    int nb32)
 {
     int rc;
     const int T = (int)a.T, SC = (int)(a.S * a.C), L = (int)a.L, N = (int)a.N;
@@ -299,8 +296,12 @@ int prepare_problem(const Args &a, Scratch &ws, cudaStream_t s, Problem *Pout, c
     if ((rc = ws.get(&k_lo, 2 * (size_t)T, "template ranges")))
         return rc;
     k_hi = k_lo + T;
-    if ((rc = ws.get(&stat_e, (size_t)SC * N * (full ? 2 : 1), "window statistics")))
+    size_t stat_elems = 0;
+    const int stat_pad = nb32 ? 128 * nb32 + 16 : 0;
+    const StatPlace place = stat_rows(SC, N, (int)a.step, stat_pad, &stat_elems);
+    if ((rc = ws.get(&stat_e, stat_elems * (full ? 2 : 1), "window statistics")))
         return rc;
+    stat_e += (size_t)stat_pad * (full ? 2 : 1);
     if (full) {
         if ((rc = ws.get(&mu, (size_t)SC, "channel centres")) ||
             (rc = ws.get(&dcen, (size_t)SC * N, "centred data")) ||
@@ -310,31 +311,24 @@ int prepare_problem(const Args &a, Scratch &ws, cudaStream_t s, Problem *Pout, c
     }
 
     unsigned *scan = nullptr;
-    if (want_scan) {
+    if (nb32) {
         const size_t n = 3 * (size_t)SC + 1;
         if ((rc = ws.get(&scan, n, "channel scan")) ||
             (rc = cuda_status(cudaMemsetAsync(scan, 0, n * sizeof(unsigned), s), "clearing the channel scan")))
             return rc;
     }
-    const float *sst = a.sst;
-    if (!sst) {  // template energies as numpy computes them for float32 templates
-        float *e = nullptr;
-        if ((rc = ws.get(&e, (size_t)T * SC, "template energies")))
-            return rc;
-        const int rows = T * SC;
-        template_energy_kernel<<<(rows + 127) / 128, 128, 0, s>>>(a.tpl, rows, L, e);
-        count_launch();
-        sst = e;
-    }
-    template_range_kernel<<<(T + 127) / 128, 128, 0, s>>>(a.mo, T, SC, L, N, (int)a.step,
-                                                            (int)a.n_corr, k_lo, k_hi, sst, scan);
-    count_launch();
+    float *energies = nullptr;  // as numpy computes them for float32 templates
+    if (!a.sst && (rc = ws.get(&energies, (size_t)T * SC, "template energies")))
+        return rc;
+    const float *sst = a.sst ? a.sst : energies;
+    launch_template_scalars(a.sst ? nullptr : a.tpl, const_cast<float *>(sst), a.sst && !scan ? 0 : T * SC, L, scan,
+                            a.mo, T, SC, N, (int)a.step, (int)a.n_corr, k_lo, k_hi, s);
     if (full) {
         template_center_kernel<<<(unsigned)((size_t)T * SC), 128, 0, s>>>(a.tpl, L, tcen, tsum);
         channel_centre_kernel<<<SC, 1024, 0, s>>>(a.data, N, mu);
         count_launch(2);
     }
-    if ((rc = launch_window_stats(a.data, N, L, SC, mu, dcen, stat_e, scan, s)))
+    if ((rc = launch_window_stats(a.data, N, L, SC, mu, dcen, stat_e, place, scan, s)))
         return rc;
     if ((rc = check_launch("preprocessing kernels")))
         return rc;
@@ -347,6 +341,9 @@ int prepare_problem(const Args &a, Scratch &ws, cudaStream_t s, Problem *Pout, c
     P.w = a.w;
     P.data = full ? dcen : a.data;
     P.stat_e = stat_e;
+    P.stat_ch = place.ch;
+    P.stat_ps = place.ps;
+    P.stat_rem = place.rem;
     P.k_lo = k_lo;
     P.k_hi = k_hi;
     P.out = a.out;
@@ -493,7 +490,7 @@ static int run_device_ws(const Args &a, cudaStream_t s, Scratch &ws, Problem *Po
     const float *data_for_tc = nullptr;
     cudaEvent_t ev_prep0 = mark(s);
     const int nb32 = fp32_tile(a);
-    if ((rc = prepare_problem(a, ws, s, &P, &data_for_tc, nb32 != 0)))
+    if ((rc = prepare_problem(a, ws, s, &P, &data_for_tc, nb32)))
         return rc;
     cudaEvent_t ev_prep1 = mark(s);
     span(ev_prep0, ev_prep1, kSpanPrep);
@@ -549,7 +546,7 @@ static int run_streamed(const Args &d, float *host_out, cudaStream_t s)
     const float *data_for_tc = nullptr;
     cudaEvent_t ev_prep0 = mark(s);
     const int nb32 = fp32_tile(d);
-    if ((rc = prepare_problem(d, ws, s, &P, &data_for_tc, nb32 != 0)))
+    if ((rc = prepare_problem(d, ws, s, &P, &data_for_tc, nb32)))
         return rc;
     cudaEvent_t ev_kern0 = mark(s);
     span(ev_prep0, ev_kern0, kSpanPrep);
@@ -1082,8 +1079,7 @@ int fmf_template_energies(const float *templates, size_t n_rows, size_t n_sample
     cudaStream_t s = (cudaStream_t)stream;
     const int rows = (int)n_rows, L = (int)n_samples_template;
     if (flags & FMF_FLAG_DEVICE_POINTERS) {
-        template_energy_kernel<<<(rows + 127) / 128, 128, 0, s>>>(templates, rows, L, out);
-        count_launch();
+        launch_template_scalars(templates, out, rows, L, nullptr, nullptr, 0, 1, 0, 1, 0, nullptr, nullptr, s);
         return check_launch("template energies");
     }
     int rc;
@@ -1095,8 +1091,7 @@ int fmf_template_energies(const float *templates, size_t n_rows, size_t n_sample
                                           cudaMemcpyHostToDevice, s),
                           "copying templates")))
         return rc;
-    template_energy_kernel<<<(rows + 127) / 128, 128, 0, s>>>(dt, rows, L, de);
-    count_launch();
+    launch_template_scalars(dt, de, rows, L, nullptr, nullptr, 0, 1, 0, 1, 0, nullptr, nullptr, s);
     if ((rc = check_launch("template energies")) ||
         (rc = cuda_status(cudaMemcpyAsync(out, de, n_rows * 4, cudaMemcpyDeviceToHost, s),
                           "copying energies")))

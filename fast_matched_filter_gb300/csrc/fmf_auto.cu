@@ -49,14 +49,14 @@ constexpr float kFisherAmp = 1.0f / (1.0f - 0.9f * 0.9f);  // 1 / (1 - cc^2) at 
 
 // grid = SC, 256 threads: D_ch - 1 of 'full' from the (centred energy, mean)
 // window statistics of the fixed-length path.
-__global__ void auto_dc_stats_kernel(const float2 *__restrict__ stat, int N, int nwin, int L,
-                                     float *__restrict__ dc)
+__global__ void auto_dc_stats_kernel(const float2 *__restrict__ stat, long long stat_ch, long long stat_ps,
+                                     int stat_rem, int step, int nwin, int L, float *__restrict__ dc)
 {
     __shared__ float red[8];
-    const float2 *row = stat + (size_t)blockIdx.x * N;
+    const float2 *row = stat + blockIdx.x * stat_ch;
     float mx = 0.0f;
     for (int u = threadIdx.x * kAutoStride; u < nwin; u += blockDim.x * kAutoStride) {
-        const float2 vm = row[u];
+        const float2 vm = row[(u % step) * stat_ps + min(u % step, stat_rem) + u / step];
         if (vm.x > 0.0f)
             mx = fmaxf(mx, (float)L * vm.y * vm.y / vm.x);
     }
@@ -188,8 +188,8 @@ int choose_auto_precision(const Problem &P, Scratch &ws, cudaStream_t s, int *pr
         if (P.pre2q)
             auto_dc_prefix_kernel<<<P.SC, 256, 0, s>>>(P.pre2q, P.unit2, P.pre1f, P.N, P.L, dc);
         else
-            auto_dc_stats_kernel<<<P.SC, 256, 0, s>>>(reinterpret_cast<const float2 *>(P.stat_e), P.N,
-                                                      P.N - P.L + 1, P.L, dc);
+            auto_dc_stats_kernel<<<P.SC, 256, 0, s>>>(reinterpret_cast<const float2 *>(P.stat_e), P.stat_ch,
+                                                      P.stat_ps, P.stat_rem, P.step, P.N - P.L + 1, P.L, dc);
         count_launch();
     }
     const double outputs = (double)P.T * P.n_corr * (P.network_sum ? 1 : P.SC);

@@ -30,8 +30,13 @@ struct Problem {
     const int *mo;        // (T, SC) moveouts
     const float *w;       // (T, SC) weights
     const float *data;    // (SC, N) data; centred per channel for "full"
-    const float *stat_e;  // short: (SC, N) window energy; full: (SC, N) float pairs (centred
-                          // energy, centred mean), one 8-byte load per lag; window starts at the index
+    // Window statistics -- short: window energies; full: float pairs (centred energy,
+    // centred mean), one 8-byte load per lag.  The window of channel ch that starts at
+    // sample step * x + psi, 0 <= psi < step, is element
+    // ch * stat_ch + psi * stat_ps + min(psi, stat_rem) + x.
+    const float *stat_e;
+    long long stat_ch, stat_ps;
+    int stat_rem;
     const int *k_lo;      // (T) first valid output index
     const int *k_hi;      // (T) one past the last valid output index (<= n_corr)
     float *out;           // (T, n_corr) or (T, n_corr, SC)
@@ -220,15 +225,30 @@ struct Args {
     long long zero_stop = 0;
 };
 int validate_args(const Args &a);
+// Template energies and valid lags (fmf_prep.cu): sst of `rows` rows from tpl (null:
+// sst is given and only scanned), lags of T templates.
+void launch_template_scalars(const float *tpl, float *sst, int rows, int L, unsigned *scan, const int *mo,
+                             int T, int SC, int N, int step, int n_corr, int *k_lo, int *k_hi, cudaStream_t s);
 // Window statistics of every channel (fmf_prep.cu): blocks of kStatWindows
 // windows; the shared memory a launch needs, and the launch itself.
 constexpr int kStatWindows = 4096;
 size_t window_stats_smem(int L, bool full);
+struct StatPlace {  // where Problem::stat_e has its rows
+    long long ch, ps;
+    int rem, step;
+};
+// One row per channel and phase of `step`, `pad` (a multiple of 4) unwritten
+// elements in front of each and at least as many behind; *elems elements in all,
+// the first of window 0 at index pad.  Rows start on 16-byte boundaries.
+StatPlace stat_rows(int SC, int N, int step, int pad, size_t *elems);
+// The same rows without padding, end to end: SC * N elements.
+StatPlace stat_rows_packed(int N, int step);
 int launch_window_stats(const float *data, int N, int L, int SC, const float *mu, float *dcen,
-                        float *stat_e, unsigned *scan, cudaStream_t s);
-// scan: also make Problem::scan, for the FP32 form on the tensor cores
+                        float *stat_e, const StatPlace &place, unsigned *scan, cudaStream_t s);
+// nb32: lag blocks per tile of the FP32 form on the tensor cores (0: not asked
+// for); it needs Problem::scan and a tile of padding round the statistics
 int prepare_problem(const Args &a, Scratch &ws, cudaStream_t s, Problem *P, const float **data_for_tc,
-                    bool scan = false);
+                    int nb32 = 0);
 
 // Tensor-core form (fmf_tc.cu).
 constexpr int TC_MAX_PROBS = 64;

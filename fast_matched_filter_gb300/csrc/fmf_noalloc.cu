@@ -37,9 +37,6 @@
 
 namespace fmf {
 
-__global__ void template_range_kernel(const int *, int, int, int, int, int, int, int *, int *, const float *,
-                                      unsigned *);
-__global__ void template_energy_kernel(const float *, int, int, float *);
 __global__ void template_center_kernel(const float *, int, float *, float *);
 __global__ void channel_centre_kernel(const float *, int, float *);
 
@@ -184,20 +181,18 @@ extern "C" int fmf_matched_filter_noalloc(const float *templates, const float *s
         tsum = cv.take<float>((size_t)T * SC);
     }
 
+    const StatPlace place = stat_rows_packed(N, (int)step);
+
     cudaGetLastError();
-    template_range_kernel<<<(T + 127) / 128, 128, 0, s>>>(moveouts, T, SC, L, N, (int)step, (int)n_corr,
-                                                            k_lo, k_hi, nullptr, nullptr);
-    count_launch();
-    if (energies) {  // as numpy sums float32 templates**2: bit-identical energies
-        template_energy_kernel<<<(T * SC + 127) / 128, 128, 0, s>>>(templates, T * SC, L, sst);
-        count_launch();
-    }
+    // energies, if asked for, as numpy sums float32 templates**2: bit-identical
+    launch_template_scalars(templates, sst, energies ? T * SC : 0, L, nullptr, moveouts, T, SC, N, (int)step,
+                            (int)n_corr, k_lo, k_hi, s);
     if (full) {
         template_center_kernel<<<(unsigned)((size_t)T * SC), 128, 0, s>>>(templates, L, tcen, tsum);
         channel_centre_kernel<<<SC, 1024, 0, s>>>(data, N, mu);
         count_launch(2);
     }
-    if ((rc = launch_window_stats(data, N, L, SC, mu, dcen, stat_e, nullptr, s)))
+    if ((rc = launch_window_stats(data, N, L, SC, mu, dcen, stat_e, place, nullptr, s)))
         return rc;
     cudaError_t e;
     if ((e = cudaGetLastError()) != cudaSuccess)
@@ -216,6 +211,9 @@ extern "C" int fmf_matched_filter_noalloc(const float *templates, const float *s
     P.w = weights;
     P.data = full ? dcen : data;
     P.stat_e = stat_e;
+    P.stat_ch = place.ch;
+    P.stat_ps = place.ps;
+    P.stat_rem = place.rem;
     P.k_lo = k_lo;
     P.k_hi = k_hi;
     P.out = cc_out;

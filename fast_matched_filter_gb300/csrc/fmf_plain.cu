@@ -95,6 +95,15 @@ __device__ __forceinline__ int next_active(const float *w, int ch, int SC)
     return ch;
 }
 
+// Element of Problem::stat_e of lag 0 of a channel with moveout mo (lag k: + k)
+__device__ __forceinline__ long long stat_offset(const Problem &P, int ch, int mo)
+{
+    if (P.step == 1)  // no division in the usual case
+        return ch * P.stat_ch + mo;
+    const int mu = mo >= 0 ? mo / P.step : -((-mo + P.step - 1) / P.step), psi = mo - P.step * mu;
+    return ch * P.stat_ch + psi * P.stat_ps + min(psi, P.stat_rem) + mu;
+}
+
 __device__ __forceinline__ void load_stage(float *buf, const Problem &P, const PlainGeom &g,
                                            int t, int ch, int phi, long long k0, int mo)
 {
@@ -116,12 +125,12 @@ __device__ __forceinline__ void load_stage(float *buf, const Problem &P, const P
         // the window energies of the tile's valid outputs (its epilogue follows this
         // phase); the others are zero-filled and never used
         float *sb = buf + g.stat_off;
-        const float *se = P.stat_e + (size_t)ch * P.N;
-        const int klo = P.k_lo[t], khi = P.k_hi[t];
+        const float *se = P.stat_e + stat_offset(P, ch, mo);
+        const int klo = P.k_lo[t], khi = P.k_hi[t], first = (int)k0;
         for (int x = threadIdx.x; x < PL_TILE; x += PL_THREADS) {
-            const long long k = k0 + x;
+            const int k = first + x;
             const bool ok = k >= klo && k < khi;
-            cp_async4(sb + padx(x), ok ? se + (k * P.step + mo) : se, ok);
+            cp_async4(sb + padx(x), ok ? se + k : P.stat_e, ok);
         }
     }
 }
@@ -275,8 +284,9 @@ plain_kernel(const Problem P, const PlainGeom g)
                 const size_t row = (size_t)t * P.SC + ch;
                 const float sst = P.sst[row], wc = w[ch];
                 const float ts = FULL ? P.tsum[row] : 0.0f;
-                const float *se = P.stat_e + (size_t)ch * P.N;
-                const float2 *sem = reinterpret_cast<const float2 *>(P.stat_e) + (size_t)ch * P.N;
+                const long long so = stat_offset(P, ch, mo[ch]);
+                const float *se = P.stat_e + so;
+                const float2 *sem = reinterpret_cast<const float2 *>(P.stat_e) + so;
                 float staged[PL_R];  // 'short': this thread's energies from the stage, if staged
                 if (!FULL && g.stat_off) {
                     const float *sb = smem + b * g.stage_floats + g.stat_off + padx(tid * PL_R);
@@ -293,14 +303,13 @@ plain_kernel(const Problem P, const PlainGeom g)
                 for (int r = 0; r < PL_R; r++) {
                     const int k = k0 + tid * PL_R + r;
                     if (k >= klo && k < khi) {
-                        const int u = k * P.step + mo[ch];  // a window inside [0, N - L]
                         float num = acc[r], energy;
                         if (FULL) {  // (centred energy, mean) pairs
-                            const float2 em = sem[u];
+                            const float2 em = sem[k];
                             num = fmaf(-em.y, ts, num);
                             energy = em.x;
                         } else {
-                            energy = g.stat_off ? staged[r] : se[u];
+                            energy = g.stat_off ? staged[r] : se[k];
                         }
                         float den = sst * energy;
                         float cc = den > kThreshold ? num * rsqrtf(den) : 0.0f;

@@ -1,19 +1,18 @@
 // fmf_prep.cu -- per-call preprocessing kernels.
 //
-//  * template_range_kernel : valid output range [k_lo, k_hi) of each template
+//  * template_scalars_kernel : valid output range [k_lo, k_hi) of each template
 //    (reference: matched_filter.c:53-76 start/stop, matched_filter.cu:302-308
-//    n_corr_t).
+//    n_corr_t), and the template energies sum(t^2) when the caller
+//    passes none, computed as the reference wrapper computes them for
+//    float32 templates (numpy.sum(templates**2, axis=-1),
+//    fast_matched_filter.py:256-261): float32 squares summed in numpy's
+//    pairwise order, so the values are bit-identical.
 //  * template_center_kernel: "full" only -- template minus its FP64 mean and
 //    the FP64 sum of the centred values.  sum(t*(d-m)) equals
 //    sum((t-tbar)*(d-m)) exactly, so centring changes no result; it removes
 //    the template's DC term from the products the numerator sums.
 //  * channel_centre_kernel : "full" only -- the constant subtracted from each
 //    data channel, the median of evenly spaced samples (robust to transients).
-//  * template_energy_kernel: the template energies sum(t^2) when the caller
-//    passes none, computed as the reference wrapper computes them for
-//    float32 templates (numpy.sum(templates**2, axis=-1),
-//    fast_matched_filter.py:256-261): float32 squares summed in numpy's
-//    pairwise order, so the values are bit-identical.
 //  * window_stats_kernel   : sliding-window statistics of every channel for
 //    windows of L samples starting at each sample index:
 //      short: E = sum d^2                      (matched_filter.c:622)
@@ -27,39 +26,6 @@
 #include "fmf_common.cuh"
 
 namespace fmf {
-
-__global__ void template_range_kernel(const int *__restrict__ mo, int T, int SC,
-                                      int L, int N, int step, int n_corr,
-                                      int *__restrict__ k_lo, int *__restrict__ k_hi,
-                                      const float *__restrict__ sst, unsigned *__restrict__ scan)
-{
-    int t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= T)
-        return;
-    int lo = 0, hi = 0;
-    const int *m = mo + (size_t)t * SC;
-    for (int ch = 0; ch < SC; ch++) {
-        lo = min(lo, m[ch]);
-        hi = max(hi, m[ch]);
-    }
-    if (scan)  // the largest template energy of each channel
-        for (int ch = 0; ch < SC; ch++) {
-            const float e = sst[(size_t)t * SC + ch];
-            if (e > 0.0f)  // NaN left out: such a channel's coefficients are all 0
-                atomicMax(scan + 2 * SC + ch, __float_as_uint(e));
-        }
-    long long first = lo < 0 ? ((long long)(-lo) + step - 1) / step : 0;
-    long long last = (long long)N - L - hi;
-    long long a = 0, b = 0;
-    if (last >= 0) {
-        b = last / step + 1;
-        if (b > n_corr)
-            b = n_corr;
-        a = first < b ? first : b;
-    }
-    k_lo[t] = (int)a;
-    k_hi[t] = (int)b;
-}
 
 __device__ __forceinline__ double block_sum_f64(double v, double *red)
 {
@@ -87,7 +53,55 @@ __device__ __forceinline__ double block_sum_f64(double v, double *red)
 // last multiple of 8 in order; more -- the sum of the two halves split at n/2
 // rounded down to a multiple of 8.  Explicit round-to-nearest operations: no
 // fused multiply-add may change a rounding.
-__device__ float pairwise_leaf_sq(const float *a, int n)
+//
+// One warp per row.  The eight partial sums of a block of up to 128 values are
+// eight lanes, combined by exchanges in the same order, so a warp sums four
+// blocks at a time; lane 0 then adds the blocks up the split tree.  (A thread
+// per row walked the whole row: 7.6 us for rows of 100 values, against 3 us.)
+constexpr int kEnergyLeaves = 256;  // blocks of one round; a block has at least 57 values
+
+// numpy's recursion over n values as a walk: the leaves in order, and after each
+// how many finished pairs to add (bits of its path).  Calls f(offset, length, adds).
+template <class F>
+__device__ __forceinline__ void pairwise_walk(int n, F f)
+{
+    int off[32], len[32];
+    bool right[32];  // frame's left half is done
+    int sp = 0;
+    off[0] = 0;
+    len[0] = n;
+    right[0] = false;
+    while (sp >= 0) {
+        if (len[sp] <= 128) {
+            int o = off[sp], m = len[sp], adds = 0;
+            sp--;
+            while (sp >= 0 && right[sp]) {  // this leaf ends the frame's right half
+                adds++;
+                sp--;
+            }
+            f(o, m, adds);
+            if (sp >= 0) {  // the frame's left half is done: its right half
+                right[sp] = true;
+                int m2 = len[sp] / 2;
+                m2 -= m2 % 8;
+                off[sp + 1] = off[sp] + m2;
+                len[sp + 1] = len[sp] - m2;
+                sp++;
+                right[sp] = false;
+            }
+        } else {
+            int m2 = len[sp] / 2;
+            m2 -= m2 % 8;
+            off[sp + 1] = off[sp];
+            len[sp + 1] = m2;
+            sp++;
+            right[sp] = false;
+        }
+    }
+}
+
+// The squares of a[0:n), n <= 128, by 8 lanes (k = 0..7) of a warp.
+__device__ __forceinline__ float pairwise_leaf_sq(const float *a, int n, int k)
 {
     if (n < 8) {
         float r = -0.0f;
@@ -95,73 +109,110 @@ __device__ float pairwise_leaf_sq(const float *a, int n)
             r = __fadd_rn(r, __fmul_rn(a[i], a[i]));
         return r;
     }
-    float r[8];
-#pragma unroll
-    for (int k = 0; k < 8; k++)
-        r[k] = __fmul_rn(a[k], a[k]);
-    int i = 8;
-    for (; i < n - (n % 8); i += 8) {
-#pragma unroll
-        for (int k = 0; k < 8; k++)
-            r[k] = __fadd_rn(r[k], __fmul_rn(a[i + k], a[i + k]));
-    }
-    float res = __fadd_rn(__fadd_rn(__fadd_rn(r[0], r[1]), __fadd_rn(r[2], r[3])),
-                          __fadd_rn(__fadd_rn(r[4], r[5]), __fadd_rn(r[6], r[7])));
-    for (; i < n; i++)
-        res = __fadd_rn(res, __fmul_rn(a[i], a[i]));
-    return res;
+    const int whole = n - (n % 8);
+    float r = __fmul_rn(a[k], a[k]);
+#pragma unroll 4
+    for (int i = 8; i < whole; i += 8)
+        r = __fadd_rn(r, __fmul_rn(a[i + k], a[i + k]));
+    const unsigned group = 0xffu << (threadIdx.x & 24);
+    for (int o = 1; o < 8; o <<= 1)  // addition commutes: every lane ends with lane 0's sum
+        r = __fadd_rn(r, __shfl_xor_sync(group, r, o));
+    for (int i = whole; i < n; i++)
+        r = __fadd_rn(r, __fmul_rn(a[i], a[i]));
+    return r;
 }
 
-__device__ float pairwise_sq(const float *a, int n)
+// One warp: the energy of row r of L values, in lane 0.
+__device__ __forceinline__ float row_energy(const float *a, int L)
 {
-    // the recursion of numpy's pairwise sum, unrolled with an explicit stack
-    // (depth <= 32 for any int n): post-order over the split tree
-    int off[32], len[32], stage[32];
-    float left[32];
+    __shared__ float leaf[4][kEnergyLeaves];
+    __shared__ int at[4][kEnergyLeaves];              // offset * 256 + length
+    __shared__ unsigned char ends[4][kEnergyLeaves];  // pairs to add after the block
+    const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    float stack[32];
     int sp = 0;
-    off[0] = 0;
-    len[0] = n;
-    stage[0] = 0;
-    float ret = 0.f;
-    while (sp >= 0) {
-        const int o = off[sp], m = len[sp];
-        if (m <= 128) {
-            ret = pairwise_leaf_sq(a + o, m);
-            sp--;
-        } else {
-            int m2 = m / 2;
-            m2 -= m2 % 8;
-            if (stage[sp] == 0) {  // descend left
-                stage[sp] = 1;
-                sp++;
-                off[sp] = o;
-                len[sp] = m2;
-                stage[sp] = 0;
-                continue;
-            }
-            if (stage[sp] == 1) {  // left done: descend right
-                left[sp] = ret;
-                stage[sp] = 2;
-                sp++;
-                off[sp] = o + m2;
-                len[sp] = m - m2;
-                stage[sp] = 0;
-                continue;
-            }
-            ret = __fadd_rn(left[sp], ret);  // both done
-            sp--;
+    for (int first = 0, total = 1; first < total; first += kEnergyLeaves) {  // a round of blocks
+        int n = 0;
+        if (lane == 0)
+            pairwise_walk(L, [&](int o, int m, int adds) {
+                const int j = n++ - first;
+                if (j >= 0 && j < kEnergyLeaves) {
+                    at[w][j] = o * 256 + m;
+                    ends[w][j] = (unsigned char)adds;
+                }
+            });
+        total = __shfl_sync(0xffffffffu, n, 0);
+        __syncwarp();
+        const int here = min(total - first, kEnergyLeaves);
+        for (int j = lane >> 3; j < here; j += 4) {
+            const float v = pairwise_leaf_sq(a + (at[w][j] >> 8), at[w][j] & 255, lane & 7);
+            if ((lane & 7) == 0)
+                leaf[w][j] = v;
         }
+        __syncwarp();
+        if (lane == 0)
+            for (int j = 0; j < here; j++) {
+                float v = leaf[w][j];
+                for (int q = ends[w][j]; q > 0; q--)
+                    v = __fadd_rn(stack[--sp], v);
+                stack[sp++] = v;
+            }
+        __syncwarp();
     }
-    return ret;
+    return stack[0];
 }
 
-// one thread per (template, channel) row
-__global__ void template_energy_kernel(const float *__restrict__ tpl, int rows, int L,
-                                       float *__restrict__ sst)
+// Everything that is made of the templates' scalars, in one launch of 128 threads per
+// block.  The first blocks, if rows > 0: a warp per row (template, channel), its
+// energy into sst (tpl set) and the largest one of each channel into scan (if
+// set).  The other blocks, if T > 0: a thread per template, its valid lags.
+__global__ void __launch_bounds__(128) template_scalars_kernel(
+    const float *__restrict__ tpl, float *__restrict__ sst, int rows, int L, unsigned *__restrict__ scan,
+    const int *__restrict__ mo, int T, int SC, int N, int step, int n_corr, int *__restrict__ k_lo,
+    int *__restrict__ k_hi)
 {
-    const int r = blockIdx.x * blockDim.x + threadIdx.x;
-    if (r < rows)
-        sst[r] = pairwise_sq(tpl + (size_t)r * L, L);
+    const int row_blocks = (int)((rows + 3ll) / 4);
+    if ((int)blockIdx.x < row_blocks) {
+        const int r = blockIdx.x * 4 + (threadIdx.x >> 5);
+        if (r >= rows)
+            return;
+        const float e = tpl ? row_energy(tpl + (size_t)r * L, L) : sst[r];
+        if ((threadIdx.x & 31) == 0) {
+            if (tpl)
+                sst[r] = e;
+            if (scan && e > 0.0f)  // NaN left out: such a channel's coefficients are all 0
+                atomicMax(scan + 2 * SC + r % SC, __float_as_uint(e));
+        }
+        return;
+    }
+    const int t = (blockIdx.x - row_blocks) * blockDim.x + threadIdx.x;
+    if (t >= T)
+        return;
+    int lo = 0, hi = 0;
+    const int *m = mo + (size_t)t * SC;
+    for (int ch = 0; ch < SC; ch++) {
+        lo = min(lo, m[ch]);
+        hi = max(hi, m[ch]);
+    }
+    long long first = lo < 0 ? ((long long)(-lo) + step - 1) / step : 0;
+    long long last = (long long)N - L - hi;
+    long long a = 0, b = 0;
+    if (last >= 0) {
+        b = last / step + 1;
+        if (b > n_corr)
+            b = n_corr;
+        a = first < b ? first : b;
+    }
+    k_lo[t] = (int)a;
+    k_hi[t] = (int)b;
+}
+
+void launch_template_scalars(const float *tpl, float *sst, int rows, int L, unsigned *scan, const int *mo,
+                             int T, int SC, int N, int step, int n_corr, int *k_lo, int *k_hi, cudaStream_t s)
+{
+    const unsigned blocks = (unsigned)((rows + 3ll) / 4 + (T + 127) / 128);
+    template_scalars_kernel<<<blocks, 128, 0, s>>>(tpl, sst, rows, L, scan, mo, T, SC, N, step, n_corr, k_lo, k_hi);
+    count_launch();
 }
 
 // check_zeros count of the reference wrapper (fast_matched_filter.py:322-361)
@@ -297,10 +348,11 @@ size_t window_stats_smem(int L, bool full) { return (size_t)StatLayout(L, full).
 // and the centred data into dcen.  Windows past N - L are not written.  One
 // instantiation per mode: the 'short' one keeps no sums of d' in registers,
 // so three blocks share an SM.
-template <bool FULL>
+template <bool FULL, bool SCAN>
 __global__ void __launch_bounds__(kStatThreads, FULL ? 2 : 3)
 window_stats_kernel(const float *__restrict__ data, int N, int L, const float *__restrict__ mu,
-                    float *__restrict__ dcen, float *__restrict__ stat_e, unsigned *__restrict__ scan)
+                    float *__restrict__ dcen, float *__restrict__ stat_e, const StatPlace place,
+                    unsigned *__restrict__ scan)
 {
     extern __shared__ float4 stat_smem[];
     constexpr bool full = FULL;
@@ -338,8 +390,10 @@ window_stats_kernel(const float *__restrict__ data, int N, int L, const float *_
                     dcen[(size_t)ch * N + c0 + i] = v;
                 const float sq = v * v;
                 s2[stat_pad(i)] = make_float2(sq, fmaf(v, v, -sq));  // v^2 exactly
-                const unsigned av = __float_as_uint(v) & 0x7fffffffu;
-                top = av < 0x7f800000u ? max(top, av) : top;
+                if (SCAN) {
+                    const unsigned av = __float_as_uint(v) & 0x7fffffffu;
+                    top = av < 0x7f800000u ? max(top, av) : top;
+                }
                 if (full)
                     s1[stat_pad(i)] = v;
             }
@@ -455,23 +509,28 @@ window_stats_kernel(const float *__restrict__ data, int N, int L, const float *_
     }
     __syncthreads();
     // energies at or below this pass no template's threshold
-    const float dead = scan ? kThreshold / __uint_as_float(scan[2 * gridDim.y + ch]) * 0.999f : 0.0f;
+    const float dead = SCAN ? kThreshold / __uint_as_float(scan[2 * gridDim.y + ch]) * 0.999f : 0.0f;
     unsigned low = 0;  // the smallest energy above it, bits complemented
+    float *row = stat_e + ch * place.ch * (full ? 2 : 1);
     for (int u = threadIdx.x; u < nwin; u += kStatThreads) {  // coalesced stores
-        const size_t o = (size_t)ch * N + c0 + u;
+        long long o = c0 + u;  // the window's first sample
+        if (place.step > 1) {
+            const int w = (int)o, x = w / place.step;
+            o = (w - x * place.step) * place.ps + min(w - x * place.step, place.rem) + x;
+        }
         float en;
         if (full) {
             const float2 v = out2[stat_pad(u)];
-            reinterpret_cast<float2 *>(stat_e)[o] = v;
+            reinterpret_cast<float2 *>(row)[o] = v;
             en = v.x;
         } else {
             en = out1[stat_pad(u)];
-            stat_e[o] = en;
+            row[o] = en;
         }
-        if (en > dead)
+        if (SCAN && en > dead)
             low = max(low, ~__float_as_uint(en));
     }
-    if (scan) {  // one atomic per block, and only where it changes the channel's value
+    if (SCAN) {  // one atomic per block, and only where it changes the channel's value
         unsigned *red = reinterpret_cast<unsigned *>(base);  // the squares are no longer read
         top = __reduce_max_sync(0xffffffffu, top);
         low = __reduce_max_sync(0xffffffffu, low);
@@ -491,19 +550,33 @@ window_stats_kernel(const float *__restrict__ data, int N, int L, const float *_
     }
 }
 
+StatPlace stat_rows(int SC, int N, int step, int pad, size_t *elems)
+{
+    StatPlace p;
+    p.step = step;
+    p.rem = 0;
+    p.ps = ((long long)(N + step - 1) / step + 2ll * pad + 3) & ~3ll;
+    p.ch = p.ps * step;
+    *elems = (size_t)SC * (size_t)p.ch;
+    return p;
+}
+
+StatPlace stat_rows_packed(int N, int step) { return StatPlace{(long long)N, N / step, N % step, step}; }
+
 int launch_window_stats(const float *data, int N, int L, int SC, const float *mu, float *dcen,
-                        float *stat_e, unsigned *scan, cudaStream_t s)
+                        float *stat_e, const StatPlace &place, unsigned *scan, cudaStream_t s)
 {
     const bool full = mu != nullptr;
     const size_t smem = window_stats_smem(L, full);
-    void (*kern)(const float *, int, int, const float *, float *, float *, unsigned *) =
-        full ? window_stats_kernel<true> : window_stats_kernel<false>;
+    void (*kern)(const float *, int, int, const float *, float *, float *, const StatPlace, unsigned *) =
+        scan ? (full ? window_stats_kernel<true, true> : window_stats_kernel<false, true>)
+             : (full ? window_stats_kernel<true, false> : window_stats_kernel<false, false>);
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxDynamicSmem);
     if (e != cudaSuccess)
         return set_error(FMF_ERR_CUDA, "window statistics shared memory (%zu bytes): %s", smem,
                          cudaGetErrorString(e));
     dim3 grid((N + kStatWindows - 1) / kStatWindows, SC);
-    kern<<<grid, kStatThreads, smem, s>>>(data, N, L, mu, dcen, stat_e, scan);
+    kern<<<grid, kStatThreads, smem, s>>>(data, N, L, mu, dcen, stat_e, place, scan);
     count_launch();
     return FMF_OK;
 }

@@ -403,11 +403,11 @@ __global__ void __launch_bounds__(tc_threads(VAR), 1) tc_persistent(const __grid
                             uint64_t bh = b0 + (((uint32_t)((k & (TC_Q - 1)) >> 3) * lbo_b +
                                                  (uint32_t)(k / TC_Q) * 16u) >> 4);
                             for (; k < blk_end; k += 16) {
-                                mma_bf16(dt, ah, bh, idesc, acc);
+                                mma_f16(dt, ah, bh, idesc, acc);
                                 acc = 1;
                                 if (split) {
-                                    mma_bf16(dt, ah, bh + b_lo, idesc, 1);
-                                    mma_bf16(dt, ah + a_lo, bh, idesc, 1);
+                                    mma_f16(dt, ah, bh + b_lo, idesc, 1);
+                                    mma_f16(dt, ah + a_lo, bh, idesc, 1);
                                 }
                                 ah += 16;
                                 bh += b_step;
@@ -473,7 +473,7 @@ __global__ void __launch_bounds__(tc_threads(VAR), 1) tc_persistent(const __grid
             const bool any = busy && a_hi > a_lo;
             // the whole warp's outputs of this item are valid (the usual case)
             const bool interior = __all_sync(0xffffffffu, a_lo <= 0 && a_hi >= NC);
-            const long long qs = (long long)TC_Q * step;
+            const long long qs = TC_Q;
             const int qs32 = TC_Q * step;
             const float *w = pr.P.w + (size_t)t * SC;
             const int *mo = pr.P.mo + (size_t)t * SC;
@@ -488,9 +488,12 @@ __global__ void __launch_bounds__(tc_threads(VAR), 1) tc_persistent(const __grid
                 const float ts = full ? tsump[row] : 0.0f;
                 const long long u0 = (kb + (long long)TC_Q * a0) * step + mo[ch];
                 // short: window energies; full: (centred energy, mean) pairs
-                const float *__restrict__ se = VAR ? nullptr : stat_e + (size_t)ch * N + u0;
-                const float2 *__restrict__ sem =
-                    VAR ? nullptr : reinterpret_cast<const float2 *>(stat_e) + (size_t)ch * N + u0;
+                const size_t meta = row * step;
+                const long long so = VAR ? 0
+                                         : ch * pr.P.stat_ch + pr.psi[meta] * pr.P.stat_ps +
+                                               min(pr.psi[meta], pr.P.stat_rem) + kb + (long long)TC_Q * a0 + pr.mu[meta];
+                const float *__restrict__ se = stat_e + so;
+                const float2 *__restrict__ sem = reinterpret_cast<const float2 *>(stat_e) + so;
                 float *oc = outp + ((size_t)t * n_corr + kb + (long long)TC_Q * a0) * SC + ch;
                 // statistics: all loads of a chunk issued together (indices clamped into the
                 // valid range) before any use; the first chunk before waiting for the accumulator
@@ -883,6 +886,11 @@ int tc_run(const TcProb *probs, int n, int form, int parts, unsigned long long *
     B.n_probs = n;
     B.split = split;
     B.stage_bytes = (int)stage;
+    B.w_bytes = B.row_bytes = 0;
+    for (int i = 0; i < n; i++) {
+        B.w_bytes = max(B.w_bytes, 2 * probs[i].NW * 128);
+        B.row_bytes = max(B.row_bytes, 8 * probs[i].R * 16);
+    }
     B.total_items = items;
     B.queue = queue;
     B.err = err;
@@ -906,13 +914,14 @@ int tc_run(const TcProb *probs, int n, int form, int parts, unsigned long long *
     for (int i = 0; i < n; i++)
         n_full += probs[i].P.normalize != 0;
     const int norm = n_full == 0 ? 0 : (n_full == n ? 1 : -1);
-    TcKernel kern;
-    int threads = tc_threads(n_var != 0);
+    void (*kern)(const TcBatch);
     if (form == TC_FORM_FP32) {
         if (norm < 0)
             return set_error(FMF_ERR_ARG, "a persistent FP32 launch mixes normalisations");
-        kern = tc32_kernel(n_var != 0, norm == 1);
-        threads = tc32_threads();
+        kern = nullptr;
+        smem = tc32_layout(&B, n_var != 0, norm == 1);
+        if (smem == 0)
+            return set_error(FMF_ERR_SMEM, "FP32 tensor-core buffers do not fit shared memory");
     } else if (n_var && norm >= 0)  // per-channel lengths: always one search, one normalisation
         kern = parts > 1 ? (norm == 0 ? tc_persistent<true, true, 0> : tc_persistent<true, true, 1>)
                          : (norm == 0 ? tc_persistent<true, false, 0> : tc_persistent<true, false, 1>);
@@ -924,14 +933,19 @@ int tc_run(const TcProb *probs, int n, int form, int parts, unsigned long long *
     else
         kern = norm == 0 ? tc_persistent<false, false, 0>
                          : (norm == 1 ? tc_persistent<false, false, 1> : tc_persistent<false, false, -1>);
-    e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxDynamicSmem);
-    if (e != cudaSuccess)
-        return set_error(FMF_ERR_CUDA, "tc_persistent shared memory (%zu bytes): %s", smem,
-                         cudaGetErrorString(e));
-    kern<<<grid, threads, smem, s>>>(B);
-    count_launch();
     note_bounded_waits();
-    int rc = check_launch("tc_persistent");
+    int rc;
+    if (form == TC_FORM_FP32) {
+        rc = tc32_launch(B, n_var != 0, norm == 1, grid, smem, s);
+    } else {
+        e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxDynamicSmem);
+        if (e != cudaSuccess)
+            return set_error(FMF_ERR_CUDA, "tc_persistent shared memory (%zu bytes): %s", smem,
+                             cudaGetErrorString(e));
+        kern<<<grid, tc_threads(n_var != 0), smem, s>>>(B);
+        count_launch();
+        rc = check_launch("tc_persistent");
+    }
     if (rc || parts == 1)
         return rc;
     const long long m = (long long)P0.T * P0.n_corr;
@@ -973,12 +987,12 @@ void tc_subset(const TcProb *full, int t0, int nt, TcProb *out)
     q.w_hi += o * step * q.NW * 64;
     if (q.w_lo)
         q.w_lo += o * step * q.NW * 64;
-    q.mu += o * step;
-    q.psi += o * step;
-    if (q.t_exp) {
-        q.t_exp += o;
-        q.k_steps += o;
+    if (q.mu) {
+        q.mu += o * step;
+        q.psi += o * step;
     }
+    if (q.t_exp)
+        q.t_exp += o;
     *out = q;
 }
 

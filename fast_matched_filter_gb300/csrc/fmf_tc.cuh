@@ -38,7 +38,7 @@ struct TcProb {
     // FP32 form (fmf_tc32.cu): operands are fp16 pairs in units of powers of two
     const int *t_exp;             // [T][SC] exponent of each channel's template
     const int *d_exp;             // [SC] exponent of each data channel
-    const int *k_steps;           // [T][SC] K steps of each channel, all phases
+    int chain_cols;               // column-block pairs of one h h chain
     const unsigned *skip;         // nonzero: the FP32 CUDA-core kernel runs this search instead
 };
 
@@ -47,6 +47,8 @@ struct TcBatch {
     int n_probs;
     int split;                    // 1: hi/lo, three products; 0: single bf16 product
     int stage_bytes;              // bytes of one pipeline stage (largest search)
+    // FP32 form: template buffers (2), data slots, statistics slots (2^stat_log2)
+    int w_bytes, n_rows, row_bytes, stat_log2, stat_bytes;
     long long total_items;
     unsigned long long *queue;    // tile-queue head, zero before the launch
     unsigned *err;                // device error word
@@ -103,6 +105,7 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatil
     if (mbar_try(bar, parity))
         return true;
     unsigned long long t0 = gtimer();
+#pragma unroll 1
     for (unsigned it = 1;; it++) {
         if (mbar_try(bar, parity))
             return true;
@@ -128,6 +131,21 @@ __device__ __forceinline__ bool mbar_wait_warp(uint32_t bar, uint32_t parity, vo
     return __shfl_sync(0xffffffffu, ok, 0) != 0;
 }
 
+// Before a slot that this thread has read goes back to the bulk copies: its reads are
+// done (an arrival alone does not wait for loads in flight, and a copy overtook
+// them while the load pipe was busy with stores).
+__device__ __forceinline__ void fence_reads_before_copy()
+{
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+}
+
+// Every lane waits; true only if all of them saw the phase complete.
+__device__ __forceinline__ bool mbar_wait_all(uint32_t bar, uint32_t parity, volatile int *abort_flag,
+                                              unsigned *err, unsigned code)
+{
+    return __all_sync(0xffffffffu, mbar_wait(bar, parity, abort_flag, err, code)) != 0;
+}
+
 __device__ __forceinline__ void bulk_g2s(uint32_t dst, const void *src, uint32_t bytes, uint32_t bar)
 {
     asm volatile(
@@ -144,7 +162,7 @@ __device__ __forceinline__ uint64_t sdesc(uint32_t addr, uint32_t lbo, uint32_t 
            ((uint64_t)((sbo >> 4) & 0x3FFFu) << 32) | (1ull << 46);
 }
 
-__device__ __forceinline__ void mma_bf16(uint32_t d_tmem, uint64_t a, uint64_t b, uint32_t idesc,
+__device__ __forceinline__ void mma_f16(uint32_t d_tmem, uint64_t a, uint64_t b, uint32_t idesc,
                                          uint32_t accumulate)
 {
     asm volatile(
@@ -154,11 +172,31 @@ __device__ __forceinline__ void mma_bf16(uint32_t d_tmem, uint64_t a, uint64_t b
         : "memory");
 }
 
+// The same with descriptors in halves: the start address is in the low word, and
+// only it moves along K, so the high words stay put.
+__device__ __forceinline__ void mma_f16(uint32_t d_tmem, uint32_t a_lo, uint32_t a_hi, uint32_t b_lo,
+                                        uint32_t b_hi, uint32_t idesc, uint32_t accumulate)
+{
+    asm volatile(
+        "{\n .reg .pred p;\n .reg .b64 a, b;\n setp.ne.b32 p, %6, 0;\n mov.b64 a, {%1, %2};\n"
+        " mov.b64 b, {%3, %4};\n tcgen05.mma.cta_group::1.kind::f16 [%0], a, b, %5, p;\n}\n" ::"r"(d_tmem),
+        "r"(a_lo), "r"(a_hi), "r"(b_lo), "r"(b_hi), "r"(idesc), "r"(accumulate)
+        : "memory");
+}
+
 __device__ __forceinline__ void mma_commit(uint32_t bar)
 {
     asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
                      bar)
                  : "memory");
+}
+
+// One lane of a converged warp.
+__device__ __forceinline__ bool elect_one()
+{
+    uint32_t one;
+    asm volatile("{\n .reg .pred p;\n elect.sync _|p, 0xffffffff;\n selp.u32 %0, 1, 0, p;\n}\n" : "=r"(one));
+    return one != 0;
 }
 
 __device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
@@ -407,8 +445,9 @@ inline TcShape tc_fill_shape(const Problem &P, int split, int nb, int tg, TcProb
     return g;
 }
 
-using TcKernel = void (*)(const TcBatch);
-TcKernel tc32_kernel(bool var, bool full);  // the FP32 form's persistent kernel (fmf_tc32.cu)
-int tc32_threads();
+// The FP32 form's persistent kernel (fmf_tc32.cu): its shared memory for the searches
+// of `B` (template buffers of w_bytes and data slots of row_bytes set), its launch.
+size_t tc32_layout(TcBatch *B, bool var, bool full);
+int tc32_launch(const TcBatch &B, bool var, bool full, unsigned grid, size_t smem, cudaStream_t s);
 
 }  // namespace fmf

@@ -42,6 +42,8 @@ namespace fmf {
 
 constexpr int T32_EPI_WARPS = 8;
 constexpr int T32_THREADS = 32 * (4 + T32_EPI_WARPS);
+constexpr int T32_MAX_ROWS = 8;     // data slots, at most
+constexpr int T32_MAX_STATS = 2;    // statistics slots, at most
 constexpr int kChain = 16;          // K steps of one h h chain
 constexpr float kLoScale = 2048.0f;  // l is kept 2^11 up
 constexpr int kTopExp = 15;          // operands are scaled to below 2^15
@@ -84,6 +86,32 @@ __device__ __forceinline__ uint4 pack8(const uint16_t *v)
     r.z = v[4] | ((uint32_t)v[5] << 16);
     r.w = v[6] | ((uint32_t)v[7] << 16);
     return r;
+}
+
+// Whether a tile of template t holds a valid output and the search runs here.
+__device__ __forceinline__ bool tc32_busy(const TcProb &pr, long long I0, int t)
+{
+    return I0 < pr.P.k_hi[t] && I0 + (long long)TC_Q * pr.nb > pr.P.k_lo[t] && !*pr.skip;
+}
+
+// Moveout of phase phi in its stream, and the stream: m = step mu + psi.
+__device__ __forceinline__ int tc32_phase(int m, int step, int &psi)
+{
+    if (step == 1) {
+        psi = 0;
+        return m;
+    }
+    const int mu = m >= 0 ? m / step : -((-m + step - 1) / step);
+    psi = m - step * mu;
+    return mu;
+}
+
+// Columns of each half tile in one statistics slot, and the bytes of that half: one
+// 16-byte group more than the columns, for windows that start between two groups.
+__host__ __device__ constexpr int tc32_stat_columns(bool full) { return full ? 16 : 32; }
+__host__ __device__ constexpr uint32_t tc32_stat_half(bool full)
+{
+    return (uint32_t)(tc32_stat_columns(full) * TC_Q * (full ? 8 : 4) + 16);
 }
 
 // ------------------------------------------------------------------ operands
@@ -135,12 +163,10 @@ __global__ void tc32_data_kernel(const float *__restrict__ data, int N, int SC, 
 
 // Template blocks as tc_template_kernel lays them out, as fp16 pairs; one block
 // per (template, channel), its taps in shared memory (read once, written 8
-// times over).  Also the phases' moveouts and streams, the channel's exponent
-// and its K steps.
+// times over).  Also the channel's exponent.
 __global__ void __launch_bounds__(256) tc32_template_kernel(
-    const float *__restrict__ tpl, const int *__restrict__ mo, const int *__restrict__ ntap, int L,
-    int step, int NW, uint16_t *__restrict__ w_hi, uint16_t *__restrict__ w_lo, int *__restrict__ mu_out,
-    int *__restrict__ psi_out, int *__restrict__ t_exp, int *__restrict__ k_steps, unsigned *skip)
+    const float *__restrict__ tpl, const int *__restrict__ mo, int L, int step, int NW,
+    uint16_t *__restrict__ w_hi, uint16_t *__restrict__ w_lo, int *__restrict__ t_exp, unsigned *skip)
 {
     extern __shared__ float taps[];
     __shared__ unsigned red[8];
@@ -175,23 +201,12 @@ __global__ void __launch_bounds__(256) tc32_template_kernel(
         if (!ok || bad)
             atomicOr(skip, 1u);
         t_exp[row] = e;
-        int steps = 0;
-        for (int phi = 0; phi < step; phi++) {
-            const int m = m0 + phi;
-            const int mu = m >= 0 ? m / step : -((-m + step - 1) / step);
-            const int s = ((mu % TC_Q) + TC_Q) % TC_Q;
-            mu_out[row * step + phi] = mu;
-            psi_out[row * step + phi] = m - step * mu;
-            steps += tc_k_end(s, tc_phase_taps(L, step, phi, ntap ? ntap[row] : L)) - (s & ~15);
-        }
-        k_steps[row] = steps >> 4;
     }
     const int per_phase = NW * 8;
     for (int i = threadIdx.x; i < step * per_phase; i += blockDim.x) {
         const int phi = i / per_phase, ne = i - phi * per_phase;
-        const int m = m0 + phi;
-        const int mu = m >= 0 ? m / step : -((-m + step - 1) / step);
-        const int s = ((mu % TC_Q) + TC_Q) % TC_Q;
+        int psi;
+        const int s = tc32_phase(m0 + phi, step, psi) & (TC_Q - 1);
         uint16_t h[8], l[8];
         const int q0 = 8 * (ne >> 3) + (ne & 7) - (TC_Q - 1 + s);
 #pragma unroll
@@ -206,35 +221,184 @@ __global__ void __launch_bounds__(256) tc32_template_kernel(
 }
 
 // ------------------------------------------------------------------ persistent kernel
+// Offsets of the barriers in the kernel's shared memory (bytes past the rings).
+struct T32Bars {
+    static constexpr uint32_t wfull = 0, wempty = 16, dfull = 32, dempty = dfull + 8 * T32_MAX_ROWS,
+                              efull = dempty + 8 * T32_MAX_ROWS, eempty = efull + 8 * T32_MAX_STATS,
+                              hfull = eempty + 8 * T32_MAX_STATS, hempty = hfull + 16, sfull = hempty + 16,
+                              sempty = sfull + 16, ifull = sempty + 16, iempty = ifull + 32,
+                              fin = iempty + 32, items = fin + 8, tmem = items + 32, abort = tmem + 4,
+                              bytes = abort + 4;
+};
+
+// One MMA issuer's walk over the items: the h h products (SMALL false; chains of
+// chain_slots data slots into H0 / H1 in turn) or the h l and l h products (into
+// S0 / S1, a channel each).
+template <bool VAR, bool SMALL>
+__device__ __forceinline__ void tc32_issue(const TcBatch &B, const long long *ring, uint32_t bar,
+                                           uint32_t w_base, uint32_t d_base, uint32_t tmem,
+                                           volatile int *abort_flag, bool one)
+{
+    const auto uniform = [](int v) { return __shfl_sync(0xffffffffu, v, 0); };
+    // the whole warp waits and keeps the books; its elected lane issues
+    const auto wait = [&](uint32_t b, uint32_t parity, unsigned code) {
+        return __all_sync(0xffffffffu, mbar_wait(b, parity, abort_flag, B.err, code)) != 0;
+    };
+    uint32_t stages = 0, slot = 0, turn = 0;
+    uint32_t acc_i = 0;  // accumulators (channels or chains) begun
+    const uint32_t n_rows = (uint32_t)B.n_rows;
+    for (uint32_t q = 0;; q++) {
+        const uint32_t is = q & 3;
+        if (!wait(bar + T32Bars::ifull + 8 * is, (q >> 2) & 1, 32u))
+            return;
+        const long long item = ring[is];
+        __syncwarp();
+        if (one)
+            mbar_arrive(bar + T32Bars::iempty + 8 * is);
+        if (item >= B.total_items)
+            return;
+        int p, tile, t, c_begin, c_end, part;
+        decode_item<true>(B, item, p, tile, t, c_begin, c_end, part);
+        p = uniform(p);
+        t = uniform(t);
+        c_end = uniform(c_end);
+        const TcProb &pr = B.prob[p];
+        const int nb = pr.nb;
+        if (!uniform(tc32_busy(pr, (long long)tile * TC_Q * nb, t)))
+            continue;
+        // kind::f16 descriptor: F32 accumulate, FP16 A and B, K-major, N = nb, M = 128
+        const uint32_t idesc = (1u << 4) | ((uint32_t)(nb >> 3) << 17) | ((uint32_t)(TC_Q >> 4) << 24);
+        const int SC = pr.P.SC, step = pr.P.step, L = pr.P.L;
+        const uint32_t chain_cols = (uint32_t)pr.chain_cols;
+        const uint32_t col_bytes = (uint32_t)pr.R * 16;
+        // 16-byte units from a high half to its low half, and of a column-block pair
+        const uint32_t a_low = (uint32_t)pr.NW * 8, b_low = 4u * (uint32_t)pr.R, b_pair = 2u * (uint32_t)pr.R;
+        const uint32_t a_hi = (uint32_t)(sdesc(0, 128, 128) >> 32);
+        const uint32_t b_hi = (uint32_t)(sdesc(0, col_bytes, 128) >> 32);
+        const uint32_t a_base = (uint32_t)sdesc(w_base, 128, 128), b_base = (uint32_t)sdesc(d_base, col_bytes, 128);
+        const uint32_t a_buf = (uint32_t)B.w_bytes >> 4, b_slot = (uint32_t)B.row_bytes >> 4;
+        const size_t row0 = (size_t)t * SC;
+        for (int g0 = uniform(c_begin); g0 < c_end; g0 += 32) {
+            // the scalars of 32 channels, one per lane
+            const int cl = min(g0 + (int)(threadIdx.x & 31), c_end - 1);
+            const int mo_l = pr.P.mo[row0 + cl], n_l = VAR ? pr.P.ntap[row0 + cl] : L;
+            uint32_t active = __ballot_sync(0xffffffffu, g0 + (int)(threadIdx.x & 31) < c_end && pr.P.w[row0 + cl] != 0.0f);
+            for (; active; active &= active - 1) {
+                const int src = __ffs(active) - 1;
+                const int mo = __shfl_sync(0xffffffffu, mo_l, src), ntap = __shfl_sync(0xffffffffu, n_l, src);
+                uint32_t left = 0;  // column-block pairs left to the accumulator
+                uint32_t dt = 0, acc = 0;
+                for (int phi = 0; phi < step; phi++, stages++) {
+                    const uint32_t wb = stages & 1;
+                    int psi;
+                    const uint32_t sres = (uint32_t)tc32_phase(mo + phi, step, psi) & (TC_Q - 1);
+                    const uint32_t k_first = sres & ~15u;
+                    const uint32_t k_end = (uint32_t)tc_k_end((int)sres, step == 1 ? ntap : tc_phase_taps(L, step, phi, ntap));
+                    if (!wait(bar + T32Bars::wfull + 8 * wb, (stages >> 1) & 1, 8u))
+                        return;
+                    const uint32_t a0 = a_base + (wb ? a_buf : 0u);
+#pragma unroll 1
+                    for (uint32_t j = 0; j < TC_CB / 2; j++) {
+                        if (left == 0) {  // the next accumulator
+                            const uint32_t empty = bar + (SMALL ? T32Bars::sempty : T32Bars::hempty) + 8 * (acc_i & 1);
+                            if (acc_i >= 2 && !wait(empty, ((acc_i >> 1) - 1) & 1, 4u))
+                                return;
+                            tc_fence_after();
+                            dt = tmem + (SMALL ? 256u : 0u) + 128u * (acc_i & 1);
+                            acc = 0;
+                            left = SMALL ? (uint32_t)step * (TC_CB / 2) : chain_cols;
+                        }
+                        // two column-block pairs per slot
+                        if ((j & 1) == 0 && !wait(bar + T32Bars::dfull + 8 * slot, turn & 1, 8u))
+                            return;
+                        // K steps k = 16 j + 128 i: A moves 16 template blocks (2 KB), B one data
+                        // row (16 bytes) per step.  The start-address field (16-byte units) of
+                        // an address below 256 KB never carries out of its 14 bits.
+                        const uint32_t late = 16 * j < k_first ? 1u : 0u;
+                        const uint32_t n = ((k_end - 16 * j + TC_Q - 1) >> 7) - late;
+                        uint32_t a = a0 + 16 * j + late * TC_Q;
+                        uint32_t b = b_base + slot * b_slot + (j & 1 ? b_pair : 0u) + late;
+#pragma unroll 1
+                        for (uint32_t i = 0; i < n; i++) {
+                            if (one) {
+                                if (SMALL) {
+                                    mma_f16(dt, a, a_hi, b + b_low, b_hi, idesc, acc);
+                                    mma_f16(dt, a + a_low, a_hi, b, b_hi, idesc, 1);
+                                } else {
+                                    mma_f16(dt, a, a_hi, b, b_hi, idesc, acc);
+                                }
+                            }
+                            acc = 1;
+                            a += TC_Q;
+                            b += 1;
+                        }
+                        const bool done = --left == 0 || (!SMALL && j == TC_CB / 2 - 1 && phi == step - 1);
+                        if (one) {
+                            if (j & 1)
+                                mma_commit(bar + T32Bars::dempty + 8 * slot);
+                            if (done)
+                                mma_commit(bar + (SMALL ? T32Bars::sfull : T32Bars::hfull) + 8 * (acc_i & 1));
+                        }
+                        if ((j & 1) && ++slot == n_rows) {
+                            slot = 0;
+                            turn++;
+                        }
+                        if (done) {
+                            acc_i++;
+                            left = 0;
+                        }
+                    }
+                    if (one)
+                        mma_commit(bar + T32Bars::wempty + 8 * wb);
+                }
+            }
+        }
+    }
+}
+
 // VAR: per-channel template lengths (Fisher-z network sum); FULL: 'full'
-// normalisation; one instantiation per mode, each with its own epilogue code.
-template <bool VAR, bool FULL>
+// normalisation; NSUM: network sum.  One instantiation per mode, each with its
+// own epilogue code only (the code of all roles shares the instruction cache).
+template <bool VAR, bool FULL, bool NSUM>
 __global__ void __launch_bounds__(T32_THREADS, 1) tc32_persistent(const __grid_constant__ TcBatch B)
 {
     extern __shared__ __align__(1024) uint8_t smem[];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    constexpr int CH = tc32_stat_columns(FULL);  // columns per slot of statistics and half tile
+    constexpr uint32_t kStatHalf = tc32_stat_half(FULL);
 
-    uint8_t *bar_base = smem + 2 * (size_t)B.stage_bytes;
-    const uint32_t full0 = smem_u32(bar_base), empty0 = full0 + 16, hfull0 = full0 + 32, hempty0 = full0 + 48,
-                   sfull0 = full0 + 64, sempty0 = full0 + 80, ifull0 = full0 + 96, iempty0 = full0 + 128,
-                   fin = full0 + 160;
-    long long *ring = reinterpret_cast<long long *>(bar_base + 168);  // 4 item slots
-    uint32_t *tmem_holder = reinterpret_cast<uint32_t *>(bar_base + 200);
-    volatile int *abort_flag = reinterpret_cast<volatile int *>(bar_base + 204);
+    // template blocks (2 buffers), data slots, statistics slots, barriers
+    const uint32_t w_base = smem_u32(smem);
+    const uint32_t d_base = w_base + 2u * B.w_bytes;
+    const uint32_t e_base = d_base + (uint32_t)B.n_rows * B.row_bytes;
+    uint8_t *bar_ptr = smem + 2u * B.w_bytes + (uint32_t)B.n_rows * B.row_bytes + ((uint32_t)B.stat_bytes << B.stat_log2);
+    const uint32_t bar = smem_u32(bar_ptr);
+    long long *ring = reinterpret_cast<long long *>(bar_ptr + T32Bars::items);  // 4 item slots
+    uint32_t *tmem_holder = reinterpret_cast<uint32_t *>(bar_ptr + T32Bars::tmem);
+    volatile int *abort_flag = reinterpret_cast<volatile int *>(bar_ptr + T32Bars::abort);
+    const int n_rows = B.n_rows, stat_log2 = B.stat_log2;
 
     if (threadIdx.x == 0) {
         for (int i = 0; i < 2; i++) {
-            mbar_init(full0 + 8 * i, 1);
-            mbar_init(empty0 + 8 * i, 2);  // one commit per MMA issuer
-            mbar_init(hfull0 + 8 * i, 1);
-            mbar_init(hempty0 + 8 * i, T32_EPI_WARPS);
-            mbar_init(sfull0 + 8 * i, 1);
-            mbar_init(sempty0 + 8 * i, T32_EPI_WARPS);
+            mbar_init(bar + T32Bars::wfull + 8 * i, 1);
+            mbar_init(bar + T32Bars::wempty + 8 * i, 2);  // one commit per MMA issuer
+            mbar_init(bar + T32Bars::hfull + 8 * i, 1);
+            mbar_init(bar + T32Bars::hempty + 8 * i, T32_EPI_WARPS);
+            mbar_init(bar + T32Bars::sfull + 8 * i, 1);
+            mbar_init(bar + T32Bars::sempty + 8 * i, T32_EPI_WARPS);
         }
-        mbar_init(fin, 2);
+        for (int i = 0; i < T32_MAX_ROWS; i++) {
+            mbar_init(bar + T32Bars::dfull + 8 * i, 1);
+            mbar_init(bar + T32Bars::dempty + 8 * i, 2);
+        }
+        for (int i = 0; i < T32_MAX_STATS; i++) {
+            mbar_init(bar + T32Bars::efull + 8 * i, 1);
+            mbar_init(bar + T32Bars::eempty + 8 * i, T32_EPI_WARPS);
+        }
+        mbar_init(bar + T32Bars::fin, 2);
         for (int i = 0; i < 4; i++) {
-            mbar_init(ifull0 + 8 * i, 1);
-            mbar_init(iempty0 + 8 * i, 2 + T32_EPI_WARPS);
+            mbar_init(bar + T32Bars::ifull + 8 * i, 1);
+            mbar_init(bar + T32Bars::iempty + 8 * i, 3 + T32_EPI_WARPS);  // issuers, warp 3, epilogue
         }
         *abort_flag = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -255,23 +419,24 @@ __global__ void __launch_bounds__(T32_THREADS, 1) tc32_persistent(const __grid_c
     const long long total = B.total_items;
 
     if (warp < 4) {
-        // registers: 384 threads x 168 at launch = 128 x 72 + 256 x 216
-        asm volatile("setmaxnreg.dec.sync.aligned.u32 72;");
+        // registers: 384 threads x 168 at launch = 128 x 88 + 256 x 208
+        asm volatile("setmaxnreg.dec.sync.aligned.u32 88;");
     }
     if (warp == 0) {
-        // ---------------------------------------------------------- producer + tile queue
-        int uses = 0;  // stages loaded so far; buffer = uses & 1
+        // ---------------------------------------------------------- tile queue, operands
+        int stages = 0;                 // (channel, phase) stages so far; template buffer = stages & 1
+        int slot = 0, turn = 0;         // data slot, times round the ring
         bool ok = true;
         for (long long q = 0; ok; q++) {
-            const int slot = (int)(q & 3);
+            const int is = (int)(q & 3);
             long long item = total;
             if (lane == 0) {
-                const bool got = q < 4 || mbar_wait(iempty0 + 8 * slot, (uint32_t)(((q >> 2) - 1) & 1),
+                const bool got = q < 4 || mbar_wait(bar + T32Bars::iempty + 8 * is, (uint32_t)(((q >> 2) - 1) & 1),
                                                     abort_flag, B.err, 1u);
                 if (got && !*abort_flag)
                     item = (long long)atomicAdd(B.queue, 1ull);
-                ring[slot] = item;
-                mbar_arrive(ifull0 + 8 * slot);
+                ring[is] = item;
+                mbar_arrive(bar + T32Bars::ifull + 8 * is);
             }
             item = __shfl_sync(0xffffffffu, item, 0);
             if (item >= total)
@@ -280,172 +445,177 @@ __global__ void __launch_bounds__(T32_THREADS, 1) tc32_persistent(const __grid_c
             decode_item<true>(B, item, p, tile, t, c_begin, c_end, part);
             const TcProb &pr = B.prob[p];
             const Problem &P = pr.P;
-            const int nb = pr.nb;
-            const long long I0 = (long long)tile * TC_Q * nb;
-            if (!(I0 < P.k_hi[t] && I0 + (long long)TC_Q * nb > P.k_lo[t]) || *pr.skip)
+            const long long I0 = (long long)tile * TC_Q * pr.nb;
+            if (!tc32_busy(pr, I0, t))
                 continue;
-            const int SC = P.SC, step = P.step, R = pr.R, NW = pr.NW;
-            const uint32_t data_bytes = (uint32_t)TC_CB * R * 16, wbytes = (uint32_t)NW * 128;
-            const float *w = P.w + (size_t)t * SC;
-            for (int ch = c_begin; ok && ch < c_end; ch++) {
-                if (w[ch] == 0.0f)
-                    continue;
-                for (int phi = 0; phi < step; phi++) {
-                    const int b = uses & 1;
-                    const long long meta = ((long long)t * SC + ch) * step + phi;
-                    const int mu = pr.mu[meta], psi = pr.psi[meta];
-                    const int sres = ((mu % TC_Q) + TC_Q) % TC_Q;
-                    const long long r0 = (I0 + mu - sres) / TC_Q + pr.row_front;
-                    if (uses >= 2 &&
-                        !mbar_wait_warp(empty0 + 8 * b, ((uses >> 1) - 1) & 1, abort_flag, B.err, 2u)) {
-                        ok = false;
-                        break;
+            const int SC = P.SC, step = P.step;
+            const uint32_t col_bytes = (uint32_t)pr.R * 16, wbytes = (uint32_t)pr.NW * 128;
+            const size_t row0 = (size_t)t * SC;
+            for (int g0 = c_begin; ok && g0 < c_end; g0 += 32) {
+                // the scalars of 32 channels, one per lane
+                const int cl = min(g0 + lane, c_end - 1);
+                const int mo_l = P.mo[row0 + cl];
+                uint32_t active = __ballot_sync(0xffffffffu, g0 + lane < c_end && P.w[row0 + cl] != 0.0f);
+                for (; ok && active; active &= active - 1) {
+                    const int from = __ffs(active) - 1, ch = g0 + from;
+                    const int mo = __shfl_sync(0xffffffffu, mo_l, from);
+                    for (int phi = 0; ok && phi < step; phi++, stages++) {
+                        const int wb = stages & 1;
+                        int psi;
+                        const int mu = tc32_phase(mo + phi, step, psi);
+                        const long long r0 = ((I0 + mu) >> 7) + pr.row_front;  // floor
+                        const uint32_t wbar = bar + T32Bars::wfull + 8 * wb;
+                        if (stages >= 2 && !mbar_wait_warp(bar + T32Bars::wempty + 8 * wb, ((stages >> 1) - 1) & 1,
+                                                           abort_flag, B.err, 2u)) {
+                            ok = false;
+                            break;
+                        }
+                        if (lane == 0)
+                            mbar_expect_tx(wbar, 2u * wbytes);
+                        __syncwarp();
+                        if (lane < 2)
+                            bulk_g2s(w_base + wb * B.w_bytes + lane * wbytes,
+                                     (lane ? pr.w_lo : pr.w_hi) + ((row0 + ch) * step + phi) * pr.NW * 64, wbytes, wbar);
+                        // data: four column blocks of the R rows, both halves, per slot; lane =
+                        // 4 * half + block
+                        const uint16_t *src =
+                            (lane & 4 ? pr.g_lo : pr.g_hi) +
+                            ((((long long)ch * step + psi) * TC_CB + (lane & 3)) * pr.rows_total + r0) * 8;
+                        const long long src_step = 4ll * pr.rows_total * 8;
+#pragma unroll 1
+                        for (int j = 0; j < TC_CB / 4; j++, src += src_step) {
+                            const uint32_t dbar = bar + T32Bars::dfull + 8 * slot;
+                            if (turn >= 1 && !mbar_wait_warp(bar + T32Bars::dempty + 8 * slot, (turn - 1) & 1,
+                                                             abort_flag, B.err, 2u)) {
+                                ok = false;
+                                break;
+                            }
+                            if (lane == 0)
+                                mbar_expect_tx(dbar, 8u * col_bytes);
+                            __syncwarp();
+                            if (lane < 8)
+                                bulk_g2s(d_base + slot * B.row_bytes + lane * col_bytes, src, col_bytes, dbar);
+                            if (++slot == n_rows) {
+                                slot = 0;
+                                turn++;
+                            }
+                        }
                     }
-                    const uint32_t st = smem_u32(smem + (size_t)b * B.stage_bytes);
-                    if (lane == 0)
-                        mbar_expect_tx(full0 + 8 * b, 2u * (data_bytes + wbytes));
-                    __syncwarp();
-                    const int cb = lane & 15, hl = lane >> 4;
-                    const uint16_t *src = (hl ? pr.g_lo : pr.g_hi) +
-                                          ((((long long)ch * step + psi) * TC_CB + cb) * pr.rows_total + r0) * 8;
-                    bulk_g2s(st + hl * data_bytes + cb * (uint32_t)R * 16, src, (uint32_t)R * 16,
-                             full0 + 8 * b);
-                    if (lane < 2) {
-                        const uint16_t *wsrc = (lane ? pr.w_lo : pr.w_hi) + meta * NW * 64;
-                        bulk_g2s(st + 2 * data_bytes + lane * wbytes, wsrc, wbytes, full0 + 8 * b);
-                    }
-                    uses++;
                 }
             }
         }
-        // do not leave with copies in flight
-        if (lane == 0)
-            for (int u = uses < 2 ? 0 : uses - 2; u < uses; u++)
-                mbar_wait(full0 + 8 * (u & 1), (u >> 1) & 1, abort_flag, B.err, 0u);
+        // do not leave with copies in flight: the last use of every buffer
+        if (lane == 0) {
+            for (int u = stages < 2 ? 0 : stages - 2; u < stages; u++)
+                mbar_wait(bar + T32Bars::wfull + 8 * (u & 1), (u >> 1) & 1, abort_flag, B.err, 0u);
+            for (int i = 0; i < n_rows; i++) {
+                const int uses = turn + (i < slot ? 1 : 0);
+                if (uses)
+                    mbar_wait(bar + T32Bars::dfull + 8 * i, (uses - 1) & 1, abort_flag, B.err, 0u);
+            }
+        }
         __syncwarp();
     } else if (warp == 1 || warp == 2) {
         // ---------------------------------------------------------- MMA issuers
-        const bool small = warp == 2;  // the h l and l h products
-        if (lane == 0) {
-            int used = 0;       // stages consumed
-            int c = 0, hc = 0;  // channels and h h chains begun
-            for (long long q = 0;; q++) {
-                const int slot = (int)(q & 3);
-                if (!mbar_wait(ifull0 + 8 * slot, (uint32_t)((q >> 2) & 1), abort_flag, B.err, 32u))
-                    goto mma_done;
-                const long long item = ring[slot];
-                mbar_arrive(iempty0 + 8 * slot);
+        // One thread each; the code of one instruction costs the tensor pipe as much time as
+        // the instruction, so each issuer has its own short loop and moves only the low
+        // words of its descriptors.
+        const bool one = elect_one();
+        if (warp == 1)
+            tc32_issue<VAR, false>(B, ring, bar, w_base, d_base, tmem, abort_flag, one);
+        else
+            tc32_issue<VAR, true>(B, ring, bar, w_base, d_base, tmem, abort_flag, one);
+        __syncwarp();
+        if (one) {
+            mma_commit(bar + T32Bars::fin);
+            mbar_wait(bar + T32Bars::fin, 0, abort_flag, B.err, 0u);
+        }
+        __syncwarp();
+    } else if (warp == 3) {
+        // ---------------------------------------------------------- window statistics
+        // Slot e: CH columns of each half of the tile (a column is 128 windows, contiguous
+        // in the statistics of the channel's stream), copied from a 16-byte boundary.
+        {
+            int ec = 0;
+            bool ok = true;
+            for (long long q = 0; ok; q++) {
+                const int is = (int)(q & 3);
+                if (!mbar_wait_warp(bar + T32Bars::ifull + 8 * is, (uint32_t)((q >> 2) & 1), abort_flag, B.err, 32u))
+                    break;
+                const long long item = ring[is];
+                __syncwarp();
+                if (lane == 0)
+                    mbar_arrive(bar + T32Bars::iempty + 8 * is);
                 if (item >= total)
                     break;
+                if (VAR)
+                    continue;
                 int p, tile, t, c_begin, c_end, part;
                 decode_item<true>(B, item, p, tile, t, c_begin, c_end, part);
                 const TcProb &pr = B.prob[p];
                 const Problem &P = pr.P;
-                const int nb = pr.nb;
-                const long long I0 = (long long)tile * TC_Q * nb;
-                if (!(I0 < P.k_hi[t] && I0 + (long long)TC_Q * nb > P.k_lo[t]) || *pr.skip)
+                const long long I0 = (long long)tile * TC_Q * pr.nb;
+                if (!tc32_busy(pr, I0, t))
                     continue;
-                // kind::f16 descriptor: F32 accumulate, FP16 A and B, K-major, N = nb, M = 128
-                const uint32_t idesc = (1u << 4) | ((uint32_t)(nb >> 3) << 17) | ((uint32_t)(TC_Q >> 4) << 24);
-                const int SC = P.SC, step = P.step;
-                const uint32_t data_bytes = (uint32_t)TC_CB * pr.R * 16, wbytes = (uint32_t)pr.NW * 128;
-                const uint32_t lbo_b = (uint32_t)pr.R * 16;
-                const uint64_t a_lo = wbytes >> 4, b_lo = data_bytes >> 4;
-                const uint64_t b_step = (2u * lbo_b) >> 4;
-                const float *w = P.w + (size_t)t * SC;
-                for (int ch = c_begin; ch < c_end; ch++) {
-                    if (w[ch] == 0.0f)
-                        continue;
-                    uint32_t acc = 0, dt = 0;
-                    int left = 0;  // K steps left in the current chain
-                    if (small) {
-                        if (c >= 2 &&
-                            !mbar_wait(sempty0 + 8 * (c & 1), ((c >> 1) - 1) & 1, abort_flag, B.err, 4u))
-                            goto mma_done;
-                        tc_fence_after();
-                        dt = tmem + 256u + 128u * (c & 1);
-                    }
-                    for (int phi = 0; phi < step; phi++, used++) {
-                        const int s = used & 1;
-                        if (!mbar_wait(full0 + 8 * s, (used >> 1) & 1, abort_flag, B.err, 8u))
-                            goto mma_done;
-                        tc_fence_after();
-                        const long long meta = ((long long)t * SC + ch) * step + phi;
-                        const int mu = pr.mu[meta];
-                        const int sres = ((mu % TC_Q) + TC_Q) % TC_Q;
-                        const int taps = tc_phase_taps(P.L, step, phi, VAR ? P.ntap[(size_t)t * SC + ch] : P.L);
-                        const int k_first = sres & ~15, k_end = tc_k_end(sres, taps);
-                        const uint32_t zhi = smem_u32(smem + (size_t)s * B.stage_bytes);
-                        const uint32_t whi = zhi + 2u * data_bytes;
-                        // descriptors advance by additions, as in fmf_tc.cu
-                        uint64_t ah = sdesc(whi + (uint32_t)(k_first >> 3) * 128u, 128, 128);
-                        const uint64_t b0 = sdesc(zhi, lbo_b, 128);
-                        int k = k_first;
-                        while (k < k_end) {
-                            const int blk_end = min(k_end, (k & ~(TC_Q - 1)) + TC_Q);
-                            uint64_t bh = b0 + (((uint32_t)((k & (TC_Q - 1)) >> 3) * lbo_b +
-                                                 (uint32_t)(k / TC_Q) * 16u) >> 4);
-                            for (; k < blk_end; k += 16) {
-                                if (small) {
-                                    mma_bf16(dt, ah, bh + b_lo, idesc, acc);
-                                    acc = 1;
-                                    mma_bf16(dt, ah + a_lo, bh, idesc, 1);
-                                } else {
-                                    if (left == 0) {  // a chain begins, in the other H accumulator
-                                        if (hc >= 2 && !mbar_wait(hempty0 + 8 * (hc & 1), ((hc >> 1) - 1) & 1,
-                                                                  abort_flag, B.err, 4u))
-                                            goto mma_done;
-                                        tc_fence_after();
-                                        dt = tmem + 128u * (hc & 1);
-                                        acc = 0;
-                                        left = kChain;
-                                    }
-                                    mma_bf16(dt, ah, bh, idesc, acc);
-                                    acc = 1;
-                                    if (--left == 0) {
-                                        mma_commit(hfull0 + 8 * (hc & 1));
-                                        hc++;
-                                    }
-                                }
-                                ah += 16;
-                                bh += b_step;
+                const int nc = pr.nb / 2;
+                const size_t row0 = (size_t)t * P.SC;
+                for (int g0 = c_begin; ok && g0 < c_end; g0 += 32) {
+                    const int cl = min(g0 + lane, c_end - 1);
+                    const int mo_l = P.mo[row0 + cl];
+                    uint32_t active = __ballot_sync(0xffffffffu, g0 + lane < c_end && P.w[row0 + cl] != 0.0f);
+                    for (; ok && active; active &= active - 1) {
+                        const int from = __ffs(active) - 1, ch = g0 + from;
+                        int psi;  // phase 0: the moveout's own stream
+                        const int mu = tc32_phase(__shfl_sync(0xffffffffu, mo_l, from), P.step, psi);
+                        constexpr int kAlign = FULL ? 1 : 3;
+                        const long long x0 = (I0 + mu) & ~(long long)kAlign;
+                        const char *src = reinterpret_cast<const char *>(P.stat_e) +
+                                          (ch * P.stat_ch + psi * P.stat_ps + x0) * (FULL ? 8 : 4);
+                        for (int c0 = 0; c0 < nc; c0 += CH, ec++) {
+                            const int es = ec & ((1 << stat_log2) - 1);
+                            const uint32_t ebar = bar + T32Bars::efull + 8 * es;
+                            if ((ec >> stat_log2) >= 1 &&
+                                !mbar_wait_warp(bar + T32Bars::eempty + 8 * es, ((ec >> stat_log2) - 1) & 1,
+                                                abort_flag, B.err, 2u)) {
+                                ok = false;
+                                break;
                             }
+                            const uint32_t bytes = min(CH, nc) * TC_Q * (FULL ? 8 : 4) + 16;
+                            if (lane == 0)
+                                mbar_expect_tx(ebar, 2u * bytes);
+                            __syncwarp();
+                            if (lane < 2)  // the two halves of the tile
+                                bulk_g2s(e_base + es * (uint32_t)B.stat_bytes + lane * kStatHalf,
+                                         src + (size_t)(lane * nc + c0) * TC_Q * (FULL ? 8 : 4), bytes, ebar);
                         }
-                        mma_commit(empty0 + 8 * s);
                     }
-                    if (small) {
-                        mma_commit(sfull0 + 8 * (c & 1));
-                    } else if (left > 0) {
-                        mma_commit(hfull0 + 8 * (hc & 1));
-                        hc++;
-                    }
-                    c++;
                 }
             }
-        mma_done:
-            mma_commit(fin);
-            mbar_wait(fin, 0, abort_flag, B.err, 0u);
+            for (int i = 0; i < (1 << stat_log2); i++) {  // the last use of every slot
+                const int uses = (ec >> stat_log2) + (i < (ec & ((1 << stat_log2) - 1)) ? 1 : 0);
+                if (uses && lane == 0)
+                    mbar_wait(bar + T32Bars::efull + 8 * i, (uses - 1) & 1, abort_flag, B.err, 0u);
+            }
         }
         __syncwarp();
-    } else if (warp >= 4) {
+    } else {
         // ---------------------------------------------------------- epilogue
         // Warp w reads TMEM lane quarter w % 4 (rows 32*(w%4) + lane) and its half of the
         // columns; numerators and network sums of its outputs live in registers.
-        asm volatile("setmaxnreg.inc.sync.aligned.u32 216;");
+        asm volatile("setmaxnreg.inc.sync.aligned.u32 208;");
         constexpr int NCM = TC_NB_MAX / 2;  // columns per thread, at most
-        constexpr int CH = 16;              // columns per batch of statistics loads
         const int quarter = warp & 3;
         const int cgroup = (warp - 4) >> 2;
         const int b = TC_Q - 1 - (32 * quarter + lane);  // phase of this thread's row
         const uint32_t lane_base = tmem + ((uint32_t)(32 * quarter) << 16);
-        int c = 0, hc = 0;  // channels and chains drained
+        int c = 0, hc = 0, ec = 0;  // channels, chains and statistics slots used
         for (long long q = 0;; q++) {
-            const int slot = (int)(q & 3);
+            const int is = (int)(q & 3);
             long long item = total;
             if (lane == 0) {
-                if (mbar_wait(ifull0 + 8 * slot, (uint32_t)((q >> 2) & 1), abort_flag, B.err, 64u)) {
-                    item = ring[slot];
-                    mbar_arrive(iempty0 + 8 * slot);
+                if (mbar_wait(bar + T32Bars::ifull + 8 * is, (uint32_t)((q >> 2) & 1), abort_flag, B.err, 64u)) {
+                    item = ring[is];
+                    mbar_arrive(bar + T32Bars::iempty + 8 * is);
                 }
             }
             item = __shfl_sync(0xffffffffu, item, 0);
@@ -459,8 +629,7 @@ __global__ void __launch_bounds__(T32_THREADS, 1) tc32_persistent(const __grid_c
             const int nb = pr.nb;
             const int NC = nb / 2;  // columns of this thread (16, 32 or 64)
             const int a0 = cgroup * NC;
-            const int SC = pr.P.SC, step = pr.P.step, n_corr = pr.P.n_corr, N = pr.P.N;
-            const bool nsum = VAR || pr.P.network_sum != 0;
+            const int SC = pr.P.SC, step = pr.P.step, n_corr = pr.P.n_corr;
             const long long I0 = (long long)tile * TC_Q * nb;
             const int klo = pr.P.k_lo[t], khi = pr.P.k_hi[t];
             const bool busy = I0 < khi && I0 + (long long)TC_Q * nb > klo;
@@ -468,113 +637,85 @@ __global__ void __launch_bounds__(T32_THREADS, 1) tc32_persistent(const __grid_c
             const long long kb = I0 + b;
             const int a_lo = (int)max(0LL, (klo - kb + TC_Q - 1) / TC_Q) - a0;
             const int a_hi = (int)min((long long)nb, (khi - kb + TC_Q - 1) / TC_Q) - a0;
-            const bool any = busy && a_hi > a_lo;
-            const bool interior = __all_sync(0xffffffffu, a_lo <= 0 && a_hi >= NC);
-            const int qs32 = TC_Q * step;
             const long long k0 = kb + (long long)TC_Q * a0;  // this thread's first output
             float sum[NCM];
 #pragma unroll
             for (int i = 0; i < NCM; i++)
                 sum[i] = 0.0f;
-            for (int ch = c_begin; busy && ch < c_end; ch++) {
-                const size_t row = (size_t)t * SC + ch;
-                const float wc = pr.P.w[row];
-                if (wc == 0.0f)
-                    continue;
-                const float sst = pr.P.sst[row];
-                const int n_chains = (pr.k_steps[row] + kChain - 1) / kChain;
+            const size_t row0 = (size_t)t * SC;
+            const int n_chains = (step * (TC_CB / 2) + pr.chain_cols - 1) / pr.chain_cols;
+            for (int g0 = c_begin; busy && g0 < c_end; g0 += 32) {
+                // the scalars of 32 channels, one per lane
+                const int cl = min(g0 + lane, c_end - 1);
+                const float w_l = g0 + lane < c_end ? pr.P.w[row0 + cl] : 0.0f, sst_l = pr.P.sst[row0 + cl];
+                const int mo_l = pr.P.mo[row0 + cl];
                 // 2^unit: the product of the operands' scales
-                const int unit_e = pr.t_exp[row] + pr.d_exp[ch] - 2 * kTopExp;
-                const float unit = exp2_int(unit_e);
-                const float ts = FULL ? pr.P.tsum[row] * exp2_int(-unit_e) : 0.0f;
-                const long long u0 = k0 * step + pr.P.mo[row];
-                const float *__restrict__ se = VAR || FULL ? nullptr : pr.P.stat_e + (size_t)ch * N + u0;
-                const float2 *__restrict__ sem =
-                    VAR || !FULL ? nullptr
-                                 : reinterpret_cast<const float2 *>(pr.P.stat_e) + (size_t)ch * N + u0;
-                float e[CH], mm[CH];
-                auto load_stats = [&](int c0) {  // indices clamped into the valid range
+                const int unit_l = pr.t_exp[row0 + cl] + pr.d_exp[cl] - 2 * kTopExp;
+                const float ts_l = FULL ? pr.P.tsum[row0 + cl] * exp2_int(-unit_l) : 0.0f;
+                uint32_t active = __ballot_sync(0xffffffffu, w_l != 0.0f);
+#pragma unroll 1
+                for (; active; active &= active - 1) {
+                    const int from = __ffs(active) - 1, ch = g0 + from;
+                    [[maybe_unused]] const size_t row = row0 + ch;
+                    const float wc = __shfl_sync(0xffffffffu, w_l, from), sst = __shfl_sync(0xffffffffu, sst_l, from);
+                    const float unit = exp2_int(__shfl_sync(0xffffffffu, unit_l, from));
+                    const float ts = FULL ? __shfl_sync(0xffffffffu, ts_l, from) : 0.0f;
+                    const int mo = __shfl_sync(0xffffffffu, mo_l, from);
+                    float num[NCM];
 #pragma unroll
-                    for (int i = 0; i < CH; i++) {
-                        const int o = (interior ? c0 + i : min(max(c0 + i, a_lo), a_hi - 1)) * qs32;
-                        if (FULL) {
-                            const float2 em = any ? __ldg(sem + o) : make_float2(0.0f, 0.0f);
-                            e[i] = em.x;
-                            mm[i] = em.y;
-                        } else {
-                            e[i] = any ? __ldg(se + o) : 0.0f;
-                        }
-                    }
-                };
-                float num[NCM];
-                for (int j = 0; j < n_chains; j++, hc++) {
-                    const uint32_t h = lane_base + 128u * (hc & 1) + a0;
-                    if (!mbar_wait_warp(hfull0 + 8 * (hc & 1), (hc >> 1) & 1, abort_flag, B.err, 16u))
-                        goto epilogue_done;
-                    tc_fence_after();
-                    float x[32];
-                    if (NC >= 32) {
+                    for (int i = 0; i < NCM; i++)
+                        num[i] = 0.0f;
+                    // numerators: the chains' sums, then S 2^-11
+#pragma unroll 1
+                    for (int j = 0; j <= n_chains; j++) {
+                        const bool last = j == n_chains;
+                        const int u = last ? c : hc;
+                        if (!mbar_wait_all(bar + (last ? T32Bars::sfull : T32Bars::hfull) + 8 * (u & 1), (u >> 1) & 1,
+                                           abort_flag, B.err, 16u))
+                            goto epilogue_done;
+                        tc_fence_after();
+                        const uint32_t h = lane_base + (last ? 256u : 0u) + 128u * (u & 1) + a0;
+                        const float f = last ? 1.0f / kLoScale : 1.0f;  // powers of two: exact products
 #pragma unroll
-                        for (int c0 = 0; c0 < NCM; c0 += 32) {
+                        for (int c0 = 0; c0 < NCM; c0 += 32) {  // a tile of 16 columns reads 16 too many
                             if (c0 < NC) {
+                                float x[32];
                                 tmem_ld32(h + c0, x);
                                 tmem_wait_ld();
 #pragma unroll
                                 for (int i = 0; i < 32; i++)
-                                    num[c0 + i] = j == 0 ? x[i] : num[c0 + i] + x[i];
+                                    num[c0 + i] = fmaf(x[i], f, num[c0 + i]);
                             }
                         }
-                    } else {
-                        tmem_ld16(h, x);
-                        tmem_wait_ld();
-#pragma unroll
-                        for (int i = 0; i < 16; i++)
-                            num[i] = j == 0 ? x[i] : num[i] + x[i];
+                        tc_fence_before();
+                        __syncwarp();
+                        if (lane == 0)
+                            mbar_arrive(bar + (last ? T32Bars::sempty : T32Bars::hempty) + 8 * (u & 1));
+                        if (!last)
+                            hc++;
                     }
-                    tc_fence_before();
-                    __syncwarp();
-                    if (lane == 0)
-                        mbar_arrive(hempty0 + 8 * (hc & 1));
-                }
-                if (!VAR)
-                    load_stats(0);
-                const uint32_t sc = lane_base + 256u + 128u * (c & 1) + a0;
-                if (!mbar_wait_warp(sfull0 + 8 * (c & 1), (c >> 1) & 1, abort_flag, B.err, 16u))
-                    goto epilogue_done;
-                tc_fence_after();
-                const float wu = wc * unit;  // a power of two: cc * wc rounds the same
-                float *oc = pr.P.out + ((size_t)t * n_corr + k0) * SC + ch;
+                    const float wu = wc * unit;  // a power of two: cc * wc rounds the same
+                    float *oc = pr.P.out + ((size_t)t * n_corr + k0) * SC + ch;
+                    if constexpr (VAR) {
+                        // window sums of the channel's own length from its running sums, the
+                        // threshold on the square root, atanh(cc - 10 eps) * z
+                        const bool any = a_hi > a_lo;
+                        const int qs32 = TC_Q * step;
+                        const long long u0 = k0 * step + mo;
+                        const int ntap = pr.P.ntap[row];
+                        const float zw = pr.P.zweight[row], u2 = pr.P.unit2[ch];
+                        const float nf = (float)ntap, inv_n = 1.0f / nf;
+                        const long long *__restrict__ pf = pr.P.pre2q + (size_t)ch * (pr.P.N + 1) + u0;
+                        const float2 *__restrict__ pg =
+                            FULL ? pr.P.pre1f + (size_t)ch * (pr.P.N + 1) + u0 : nullptr;
 #pragma unroll
-                for (int c0 = 0; c0 < NCM; c0 += CH) {
-                    if (c0 < NC) {
-                        float x[CH];
-                        tmem_ld16(sc + c0, x);
-                        tmem_wait_ld();
-#pragma unroll
-                        for (int i = 0; i < CH; i++)
-                            x[i] = fmaf(x[i], 1.0f / kLoScale, num[c0 + i]);
-                        if (c0 + CH >= NC) {
-                            tc_fence_before();
-                            __syncwarp();
-                            if (lane == 0)
-                                mbar_arrive(sempty0 + 8 * (c & 1));
-                        }
-                        if constexpr (VAR) {
-                            // window sums of the channel's own length from its running sums, the
-                            // threshold on the square root, atanh(cc - 10 eps) * z
-                            const int ntap = pr.P.ntap[row];
-                            const float zw = pr.P.zweight[row], u2 = pr.P.unit2[ch];
-                            const float nf = (float)ntap, inv_n = 1.0f / nf;
-                            const long long *__restrict__ pf = pr.P.pre2q + (size_t)ch * (N + 1) + u0;
-                            const float2 *__restrict__ pg =
-                                FULL ? pr.P.pre1f + (size_t)ch * (N + 1) + u0 : nullptr;
-#pragma unroll
-                            for (int h4 = 0; h4 < CH; h4 += 4) {  // loads of 4 values, then their use
+                        for (int h4 = 0; h4 < NCM; h4 += 4) {  // loads of 4 values, then their use
+                            if (h4 < NC) {
                                 long long lo[4], hi[4];
                                 float2 lo1[4], hi1[4];
 #pragma unroll
                                 for (int j = 0; j < 4; j++) {
-                                    const int o = min(max(c0 + h4 + j, a_lo), a_hi - 1) * qs32;
+                                    const int o = min(max(h4 + j, a_lo), a_hi - 1) * qs32;  // a valid lag
                                     lo[j] = any ? pf[o] : 0;
                                     hi[j] = any ? pf[o + ntap] : 0;
                                     if constexpr (FULL) {
@@ -584,8 +725,8 @@ __global__ void __launch_bounds__(T32_THREADS, 1) tc32_persistent(const __grid_c
                                 }
 #pragma unroll
                                 for (int j = 0; j < 4; j++) {
-                                    const int a = c0 + h4 + j;
-                                    float ssd, num1 = x[h4 + j];
+                                    const int a = h4 + j;
+                                    float ssd, num1 = num[a];
                                     if constexpr (FULL) {
                                         float mean;
                                         window_centred(lo[j], hi[j], u2, lo1[j], hi1[j], nf, inv_n, ssd, mean);
@@ -595,48 +736,67 @@ __global__ void __launch_bounds__(T32_THREADS, 1) tc32_persistent(const __grid_c
                                     }
                                     const float pe = sst * ssd, r = rsqrt_ftz(pe);
                                     const float cc = pe * r > kThreshold ? num1 * (r * unit) : 0.0f;
-                                    const float z =
-                                        fmaf(fisher_atanh(cc - 10.0f * FLT_EPSILON), zw, sum[a]);
-                                    sum[a] = (a >= a_lo && a < a_hi) ? z : sum[a];
-                                }
-                            }
-                        } else {
-                            float ec[CH], mc[CH];
-#pragma unroll
-                            for (int i = 0; i < CH; i++) {
-                                ec[i] = e[i];
-                                mc[i] = mm[i];
-                            }
-                            if (c0 + CH < NC)
-                                load_stats(c0 + CH);  // the next batch, before this one's use
-                            if (nsum && interior) {
-#pragma unroll
-                                for (int i = 0; i < CH; i++) {
-                                    const float num1 = FULL ? fmaf(-mc[i], ts, x[i]) : x[i];
-                                    const float den = sst * ec[i];
-                                    const float cc = den > kThreshold ? num1 * rsqrtf(den) : 0.0f;
-                                    sum[c0 + i] = fmaf(cc, wu, sum[c0 + i]);
-                                }
-                            } else {
-#pragma unroll
-                                for (int i = 0; i < CH; i++) {
-                                    const int a = c0 + i;
-                                    const float num1 = FULL ? fmaf(-mc[i], ts, x[i]) : x[i];
-                                    const float den = sst * ec[i];
-                                    const float cc = den > kThreshold ? num1 * rsqrtf(den) : 0.0f;
-                                    const bool valid = a >= a_lo && a < a_hi;
-                                    if (nsum)
-                                        sum[a] = valid ? fmaf(cc, wu, sum[a]) : sum[a];
-                                    else if (valid)
-                                        oc[(size_t)a * TC_Q * SC] = cc * unit;
+                                    sum[a] = fmaf(fisher_atanh(cc - 10.0f * FLT_EPSILON), zw, sum[a]);
                                 }
                             }
                         }
+                    } else {
+                        int psi;
+                        const int mu = tc32_phase(mo, step, psi);
+                        const int head = (int)((I0 + mu) & (FULL ? 1 : 3));  // past the 16-byte boundary
+#pragma unroll
+                        for (int c0 = 0; c0 < NCM; c0 += CH) {
+                            if (c0 < NC) {
+                                const int es = ec & ((1 << stat_log2) - 1);
+                                if (!mbar_wait_all(bar + T32Bars::efull + 8 * es, (ec >> stat_log2) & 1, abort_flag,
+                                                   B.err, 16u))
+                                    goto epilogue_done;
+                                const uint8_t *at = smem + (e_base - w_base) + es * (uint32_t)B.stat_bytes +
+                                                    cgroup * kStatHalf + (head + b) * (FULL ? 8 : 4);
+                                constexpr int CB = 16;  // values in flight
+#pragma unroll
+                                for (int h0 = 0; h0 < CH; h0 += CB) {
+                                    if (c0 + h0 < NC) {
+                                        float e[CB], mm[CB];
+#pragma unroll
+                                        for (int i = 0; i < CB; i++) {
+                                            if constexpr (FULL) {
+                                                const float2 v = *reinterpret_cast<const float2 *>(at + (h0 + i) * TC_Q * 8);
+                                                e[i] = v.x;
+                                                mm[i] = v.y;
+                                            } else {
+                                                e[i] = *reinterpret_cast<const float *>(at + (h0 + i) * TC_Q * 4);
+                                            }
+                                        }
+                                        if (h0 + CB >= CH || c0 + h0 + CB >= NC) {  // the slot is read
+                                            fence_reads_before_copy();
+                                            __syncwarp();
+                                            if (lane == 0)
+                                                mbar_arrive(bar + T32Bars::eempty + 8 * es);
+                                        }
+#pragma unroll
+                                        for (int i = 0; i < CB; i++) {
+                                            const int a = c0 + h0 + i;
+                                            const float num1 = FULL ? fmaf(-mm[i], ts, num[a]) : num[a];
+                                            const float den = sst * e[i];
+                                            // den is normal where it passes; outside the valid lags the
+                                            // statistics, and with them cc, are anything
+                                            const float cc = den > kThreshold ? num1 * rsqrt_ftz(den) : 0.0f;
+                                            if (NSUM)
+                                                sum[a] = fmaf(cc, wu, sum[a]);
+                                            else if (a >= a_lo && a < a_hi)
+                                                oc[(size_t)a * TC_Q * SC] = cc * unit;
+                                        }
+                                    }
+                                }
+                                ec++;
+                            }
+                        }
                     }
+                    c++;
                 }
-                c++;
             }
-            if (nsum) {
+            if (NSUM) {
                 // a channel part writes its partial sums to its own plane of part_out
                 const bool parts = pr.parts > 1;
                 float *o = (parts ? pr.part_out + (size_t)part * pr.P.T * n_corr : pr.P.out) +
@@ -651,7 +811,7 @@ __global__ void __launch_bounds__(T32_THREADS, 1) tc32_persistent(const __grid_c
 #pragma unroll
                 for (int a = 0; a < NCM; a++) {
                     if (a < NC && (long long)a * TC_Q < lim) {
-                        float v = sum[a];  // 0 outside the valid lags
+                        float v = busy && a >= a_lo && a < a_hi ? sum[a] : 0.0f;
                         if (VAR && !parts)  // the Fisher-z transform of every output
                             v = (tanhf(v / zn) + zb) * zs;
                         o[(size_t)a * TC_Q] = v;
@@ -722,7 +882,7 @@ int tc32_begin(const Problem &P, int nb, int tg, int max_templates, Scratch &ws,
     room = room < 1 ? 1 : room;
     room = room < (size_t)max_templates ? room : (size_t)max_templates;
     const size_t g_elems = (size_t)SC * step * TC_CB * pr.rows_total * 8;
-    const size_t n_rows = (size_t)P.T * SC, n_meta = n_rows * step;
+    const size_t n_rows = (size_t)P.T * SC;
     out->room = (int)room;
     out->w_elems = room * per_template;
     out->parts = tc_choose_parts(&pr);
@@ -730,17 +890,17 @@ int tc32_begin(const Problem &P, int nb, int tg, int max_templates, Scratch &ws,
     int *meta = nullptr;
     if ((rc = ws.get(&g_hi, 2 * g_elems, "fp16 data streams")) ||
         (rc = ws.get(&out->w, 2 * out->w_elems, "fp16 template blocks")) ||
-        (rc = ws.get(&meta, 2 * n_meta + 2 * n_rows + SC, "phase moveouts")))
+        (rc = ws.get(&meta, n_rows + SC, "operand exponents")))
         return rc;
     pr.g_hi = g_hi;
     pr.g_lo = g_hi + g_elems;
     pr.w_hi = out->w;
     pr.w_lo = out->w + out->w_elems;
-    pr.mu = meta;
-    pr.psi = meta + n_meta;
-    pr.t_exp = meta + 2 * n_meta;
-    pr.k_steps = pr.t_exp + n_rows;
-    pr.d_exp = pr.k_steps + n_rows;
+    pr.t_exp = meta;
+    pr.d_exp = pr.t_exp + n_rows;
+    // chains of whole column-block pairs, at most kChain K steps where a pair has no more
+    const int most = (g.k_span + TC_Q - 1) / TC_Q;  // K steps of one pair
+    pr.chain_cols = kChain / most > 1 ? kChain / most : 1;
     pr.skip = P.scan + 3 * SC;
     const long long n = (long long)SC * step * TC_CB * pr.rows_total;
     tc32_data_kernel<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(
@@ -763,9 +923,9 @@ int tc32_templates(const Tc32Search *full, int t0, int nt, cudaStream_t s, TcPro
     if (e != cudaSuccess)
         return set_error(FMF_ERR_CUDA, "tc32_template_kernel shared memory: %s", cudaGetErrorString(e));
     tc32_template_kernel<<<(unsigned)((size_t)nt * P.SC), 256, (size_t)P.L * sizeof(float), s>>>(
-        sub->P.tpl, sub->P.mo, sub->P.ntap, P.L, P.step, sub->NW, full->w, full->w + full->w_elems,
-        const_cast<int *>(sub->mu), const_cast<int *>(sub->psi), const_cast<int *>(sub->t_exp),
-        const_cast<int *>(sub->k_steps), P.scan + 3 * P.SC);
+        sub->P.tpl, sub->P.mo, P.L, P.step, sub->NW, full->w, full->w + full->w_elems,
+        const_cast<int *>(sub->t_exp),
+        P.scan + 3 * P.SC);
     count_launch();
     return check_launch("FP32 tensor-core templates");
 }
@@ -800,12 +960,47 @@ int tc32_prepare(const Problem &P, int nb, int tg, Scratch &ws, cudaStream_t s, 
     return tc32_templates(&st, 0, P.T, s, out);
 }
 
-TcKernel tc32_kernel(bool var, bool full)
+// Shared memory of one launch: two template buffers, two statistics slots (32 KB
+// each: half a channel of a full tile) and as many data slots as fit (a channel
+// has 4); long templates give up a statistics slot first.
+size_t tc32_layout(TcBatch *B, bool var, bool full)
 {
-    return var ? (full ? tc32_persistent<true, true> : tc32_persistent<true, false>)
-               : (full ? tc32_persistent<false, true> : tc32_persistent<false, false>);
+    const size_t fixed = 2 * (size_t)B->w_bytes + T32Bars::bytes;
+    B->stat_bytes = 2 * (int)tc32_stat_half(full);
+    for (int least = 3; least >= 2; least--)
+        for (int k = 1; k >= 0; k--) {
+            B->stat_log2 = var ? 0 : k;
+            const size_t stats = var ? 0 : (size_t)B->stat_bytes << B->stat_log2;
+            if (fixed + stats > (size_t)kMaxDynamicSmem)
+                continue;
+            const size_t rows = (kMaxDynamicSmem - fixed - stats) / B->row_bytes;
+            B->n_rows = rows < (size_t)T32_MAX_ROWS ? (int)rows : T32_MAX_ROWS;
+            if (B->n_rows >= least) {
+                if (var)
+                    B->stat_bytes = 0;
+                const size_t smem = fixed + stats + (size_t)B->n_rows * B->row_bytes;
+                return smem < 120 * 1024 ? 120 * 1024 : smem;  // one CTA per SM: its TMEM is all there is
+            }
+        }
+    return 0;
 }
 
-int tc32_threads() { return T32_THREADS; }
+int tc32_launch(const TcBatch &B, bool var, bool full, unsigned grid, size_t smem, cudaStream_t s)
+{
+    void (*kern)(const TcBatch);
+    if (var)
+        kern = full ? tc32_persistent<true, true, true> : tc32_persistent<true, false, true>;
+    else if (B.prob[0].P.network_sum)
+        kern = full ? tc32_persistent<false, true, true> : tc32_persistent<false, false, true>;
+    else
+        kern = full ? tc32_persistent<false, true, false> : tc32_persistent<false, false, false>;
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxDynamicSmem);
+    if (e != cudaSuccess)
+        return set_error(FMF_ERR_CUDA, "tc32_persistent shared memory (%zu bytes): %s", smem,
+                         cudaGetErrorString(e));
+    kern<<<grid, T32_THREADS, smem, s>>>(B);
+    count_launch();
+    return check_launch("tc32_persistent");
+}
 
 }  // namespace fmf

@@ -119,3 +119,12 @@ def test_template_that_is_not_finite(monkeypatch):
     tp[1, 0, 0, 7] = np.inf
     plain, tensor = _both(monkeypatch, tp, mo, w, d)
     assert np.array_equal(plain, tensor, equal_nan=True)  # the CUDA cores ran both
+
+
+def test_many_channels_written_one_by_one(monkeypatch):
+    """Per-channel outputs of full tiles: the epilogue's stores, 36 channels apart,
+    hold up its reads of the window statistics."""
+    tp, mo, w, d = random_search(11, 3, 12, 3, 100, 60000, 0, 300)
+    plain, tensor = [_search(monkeypatch, tile, tp, mo, w, d, network_sum=False) for tile in (0, 128)]
+    assert np.array_equal(plain == 0, tensor == 0)
+    assert np.abs(plain - tensor).max() <= 2 * TOL
