@@ -182,8 +182,6 @@ static int cuda_status(cudaError_t e, const char *what)
 __global__ void template_center_kernel(const float *, int, float *, float *);
 __global__ void channel_centre_kernel(const float *, int, float *);
 __global__ void zero_count_kernel(const float *, long long, long long, long long, unsigned long long *);
-int launch_tc(const Problem &P, const float *data_for_tc, int precision, unsigned *err, Scratch &ws,
-              cudaStream_t s, int forced_nb, int template_group);
 int launch_wait_selftest(unsigned *err, unsigned ms, cudaStream_t s);
 int launch_fisher_atanh(const float *y, float *out, long long n, cudaStream_t s);
 
@@ -282,8 +280,7 @@ int validate_args(const Args &a)
 }
 
 // ---------------------------------------------------------------- core (device pointers)
-int prepare_problem(const Args &a, Scratch &ws, cudaStream_t s, Problem *Pout, const float **data_for_tc,
-                    int nb32)
+int prepare_problem(const Args &a, Scratch &ws, cudaStream_t s, Problem *Pout, int stat_pad, bool want_scan)
 {
     int rc;
     const int T = (int)a.T, SC = (int)(a.S * a.C), L = (int)a.L, N = (int)a.N;
@@ -297,7 +294,6 @@ int prepare_problem(const Args &a, Scratch &ws, cudaStream_t s, Problem *Pout, c
         return rc;
     k_hi = k_lo + T;
     size_t stat_elems = 0;
-    const int stat_pad = nb32 ? 128 * nb32 + 16 : 0;
     const StatPlace place = stat_rows(SC, N, (int)a.step, stat_pad, &stat_elems);
     if ((rc = ws.get(&stat_e, stat_elems * (full ? 2 : 1), "window statistics")))
         return rc;
@@ -311,7 +307,7 @@ int prepare_problem(const Args &a, Scratch &ws, cudaStream_t s, Problem *Pout, c
     }
 
     unsigned *scan = nullptr;
-    if (nb32) {
+    if (want_scan) {
         const size_t n = 3 * (size_t)SC + 1;
         if ((rc = ws.get(&scan, n, "channel scan")) ||
             (rc = cuda_status(cudaMemsetAsync(scan, 0, n * sizeof(unsigned), s), "clearing the channel scan")))
@@ -357,6 +353,7 @@ int prepare_problem(const Args &a, Scratch &ws, cudaStream_t s, Problem *Pout, c
     P.network_sum = a.sum_mode != 0;
     P.ntap = nullptr;
     P.pre2q = nullptr;
+    P.pre_ch = P.pre_ps = 0;
     P.unit2 = nullptr;
     P.pre1f = nullptr;
     P.zweight = nullptr;
@@ -370,7 +367,6 @@ int prepare_problem(const Args &a, Scratch &ws, cudaStream_t s, Problem *Pout, c
             return rc;
     }
     *Pout = P;
-    *data_for_tc = full ? dcen : a.data;
     return FMF_OK;
 }
 
@@ -436,46 +432,72 @@ static Problem problem_subset(const Problem &P, int t0, int nt)
     return Q;
 }
 
-// Tile of an FP32 search that may run on the tensor cores ('auto' too: it may
-// choose FP32), 0 otherwise.
-static int fp32_tile(const Args &a)
-{
-    if (a.precision != FMF_PREC_FP32 && a.precision != FMF_PREC_AUTO)
-        return 0;
-    return tc32_choose_nb(a.T, a.S * a.C, a.L, a.step, a.n_corr);
-}
+// The tiles of a call: of the FP32 form (0: the CUDA cores) and of the bf16 forms,
+// each where the call may come to it ('auto' may come to both).
+struct Tiles {
+    int fp32 = 0, bf16 = 0;
+    explicit Tiles(const Args &a)
+    {
+        if (a.precision == FMF_PREC_FP32 || a.precision == FMF_PREC_AUTO)
+            fp32 = tc_fp32_nb(a.T, a.S * a.C, a.L, a.step, a.n_corr);
+        if (a.precision != FMF_PREC_FP32) {
+            const char *nb_env = getenv("FMF_TC_NB");
+            int forced = nb_env ? atoi(nb_env) : 0;
+            if (a.flags & 0xff00)
+                forced = ((a.flags >> 8) & 0xff) * 16;
+            bad = forced != 0 && forced != 32 && forced != 64 && forced != 128 ? forced : 0;
+            if (!bad)
+                bf16 = tc_choose_nb((int)a.L, (int)a.step, a.precision != FMF_PREC_BF16, forced);
+        }
+    }
+    int pad() const { return tc_pad(fp32 > bf16 ? fp32 : bf16); }
+    int bad = 0;  // a tile that does not exist
+};
 
-// An FP32 search of a prepared problem, run in parts of its templates: on the
-// tensor cores (nb != 0 and their working arrays can be had), followed by the
+// A prepared search, run in parts of its templates.  FP32: on the tensor cores
+// where it has a tile and their working arrays can be had, followed by the
 // CUDA-core kernel, which runs only where the operands' flag says so; else on the
-// CUDA cores alone.
-struct Fp32Search {
+// CUDA cores alone.  The bf16 forms: on the tensor cores.
+struct Search {
     Problem P;
     std::vector<unsigned char> tc;
     unsigned *err = nullptr;
+    bool fp32;
     int status = FMF_OK;
 
-    Fp32Search(const Problem &p, int nb, int group, int max_templates, Scratch &ws, cudaStream_t s) : P(p)
+    Search(const Problem &p, int precision, const Tiles &tiles, int flags, int max_templates, Scratch &ws,
+           cudaStream_t s)
+        : P(p), fp32(precision == FMF_PREC_FP32)
     {
-        if (nb == 0 || !P.scan || (status = device_error_word(&err)))
+        const int nb = fp32 ? tiles.fp32 : tiles.bf16;
+        if (!fp32 && tiles.bad) {
+            status = set_error(FMF_ERR_ARG, "tensor-core tile of %d lag blocks (32, 64 or 128)", tiles.bad);
             return;
-        tc.resize(tc32_search_size());
-        status = tc32_begin(P, nb, group, max_templates, ws, s, search());
-        if (status == FMF_ERR_OOM) {  // the CUDA-core kernel needs no more memory
+        }
+        if (!fp32 && nb == 0) {
+            status = set_error(FMF_ERR_SMEM, "template length %d, step %d: tensor-core tile does not fit "
+                                             "shared memory", P.L, P.step);
+            return;
+        }
+        if (nb == 0 || (status = device_error_word(&err)))
+            return;
+        tc.resize(tc_search_size());
+        status = tc_begin(P, tc_form(precision), nb, (flags >> 16) & 0xff, max_templates, ws, s, search());
+        if (fp32 && status == FMF_ERR_OOM) {  // the CUDA-core kernel needs no more memory
             clear_error();
             tc.clear();
             status = FMF_OK;
         }
     }
-    Tc32Search *search() { return reinterpret_cast<Tc32Search *>(tc.data()); }
+    TcSearch *search() { return reinterpret_cast<TcSearch *>(tc.data()); }
     int run(int t0, int nt, Scratch &ws, cudaStream_t s)
     {
         Problem Q = problem_subset(P, t0, nt);
         if (!tc.empty()) {
-            int rc = tc32_run(search(), t0, nt, err, ws, s);
-            if (rc)
+            int rc = tc_run_templates(search(), t0, nt, err, ws, s);
+            if (rc || !fp32)
                 return rc;
-            Q.only_if = tc32_flag(search());
+            Q.only_if = tc_flag(search());
         }
         return launch_plain_all(Q, s);
     }
@@ -487,10 +509,9 @@ static int run_device_ws(const Args &a, cudaStream_t s, Scratch &ws, Problem *Po
 {
     int rc;
     Problem &P = *Pout;
-    const float *data_for_tc = nullptr;
     cudaEvent_t ev_prep0 = mark(s);
-    const int nb32 = fp32_tile(a);
-    if ((rc = prepare_problem(a, ws, s, &P, &data_for_tc, nb32)))
+    const Tiles tiles(a);
+    if ((rc = prepare_problem(a, ws, s, &P, tiles.pad(), tiles.fp32 != 0)))
         return rc;
     cudaEvent_t ev_prep1 = mark(s);
     span(ev_prep0, ev_prep1, kSpanPrep);
@@ -498,24 +519,8 @@ static int run_device_ws(const Args &a, cudaStream_t s, Scratch &ws, Problem *Po
     if (precision == FMF_PREC_AUTO && (rc = choose_auto_precision(P, ws, s, &precision)))
         return rc;
     set_last_precision(precision);
-    if (precision != FMF_PREC_FP32) {
-        unsigned *err = nullptr;
-        if ((rc = device_error_word(&err)))
-            return rc;
-        const char *nb_env = getenv("FMF_TC_NB");
-        int forced = nb_env ? atoi(nb_env) : 0;
-        if (a.flags & 0xff00)
-            forced = ((a.flags >> 8) & 0xff) * 16;
-        const int group = (a.flags >> 16) & 0xff;
-        if (forced != 0 && forced != 32 && forced != 64 && forced != 128)
-            return set_error(FMF_ERR_ARG, "tensor-core tile of %d lag blocks (32, 64 or 128)", forced);
-        cudaEvent_t ev0 = mark(s);
-        rc = launch_tc(P, data_for_tc, precision, err, ws, s, forced, group);
-        span(ev0, mark(s), kSpanKernel);
-        return rc;
-    }
     cudaEvent_t ev_main0 = mark(s);
-    Fp32Search f(P, nb32, (a.flags >> 16) & 0xff, P.T, ws, s);
+    Search f(P, precision, tiles, a.flags, P.T, ws, s);
     rc = f.status ? f.status : f.run(0, P.T, ws, s);
     span(ev_main0, mark(s), kSpanKernel);
     return rc;
@@ -543,10 +548,9 @@ static int run_streamed(const Args &d, float *host_out, cudaStream_t s)
     int rc;
     Scratch ws(s);
     Problem P;
-    const float *data_for_tc = nullptr;
     cudaEvent_t ev_prep0 = mark(s);
-    const int nb32 = fp32_tile(d);
-    if ((rc = prepare_problem(d, ws, s, &P, &data_for_tc, nb32)))
+    const Tiles tiles(d);
+    if ((rc = prepare_problem(d, ws, s, &P, tiles.pad(), tiles.fp32 != 0)))
         return rc;
     cudaEvent_t ev_kern0 = mark(s);
     span(ev_prep0, ev_kern0, kSpanPrep);
@@ -569,35 +573,16 @@ static int run_streamed(const Args &d, float *host_out, cudaStream_t s)
         }
         bounds[n_chunks] = P.T;
     }
-    unsigned *err = nullptr;
-    std::vector<unsigned char> tcfull;
-    int split = 0, most = 0;
+    int most = 0;
     int precision = d.precision;
     if (precision == FMF_PREC_AUTO && (rc = choose_auto_precision(P, ws, s, &precision)))
         return rc;
     set_last_precision(precision);
     for (int c = 0; c < n_chunks; c++)
         most = bounds[c + 1] - bounds[c] > most ? bounds[c + 1] - bounds[c] : most;
-    Fp32Search fp32(P, precision == FMF_PREC_FP32 ? nb32 : 0, (d.flags >> 16) & 0xff, most, ws, s);
-    if ((rc = fp32.status))
+    Search search(P, precision, tiles, d.flags, most, ws, s);
+    if ((rc = search.status))
         return rc;
-    if (precision != FMF_PREC_FP32) {
-        if ((rc = device_error_word(&err)))
-            return rc;
-        split = precision == FMF_PREC_SPLIT_BF16;
-        const char *nb_env = getenv("FMF_TC_NB");
-        int forced = nb_env ? atoi(nb_env) : 0;
-        if (d.flags & 0xff00)
-            forced = ((d.flags >> 8) & 0xff) * 16;
-        const int nb = tc_choose_nb(P.L, P.step, split, forced);
-        if (nb == 0)
-            return set_error(FMF_ERR_SMEM, "template length %d, step %d: tensor-core tile does not fit "
-                                           "shared memory", P.L, P.step);
-        tcfull.resize(tc_prob_size());
-        if ((rc = tc_prepare(P, data_for_tc, split, nb, (d.flags >> 16) & 0xff, ws, s,
-                             reinterpret_cast<TcProb *>(tcfull.data()))))
-            return rc;
-    }
     unsigned long long *zc = nullptr;  // device zero counts, copied to d.zero_counts (host)
     if (d.zero_counts) {
         if ((rc = ws.get(&zc, (size_t)P.T, "zero counts")) ||
@@ -617,16 +602,7 @@ static int run_streamed(const Args &d, float *host_out, cudaStream_t s)
         for (int c = 0; c < n_chunks && rc == FMF_OK && e == cudaSuccess; c++, launched++) {
             const int t0 = bounds[c], nt = bounds[c + 1] - bounds[c];
             if (nt > 0) {
-                if (!tcfull.empty()) {
-                    std::vector<unsigned char> sub(tc_prob_size());
-                    unsigned long long *queue = nullptr;
-                    tc_subset(reinterpret_cast<const TcProb *>(tcfull.data()), t0, nt,
-                              reinterpret_cast<TcProb *>(sub.data()));
-                    if (!(rc = ws.get(&queue, 1, "tile queue")))
-                        rc = tc_run(reinterpret_cast<const TcProb *>(sub.data()), 1, split, 0, queue, err, s);
-                } else {
-                    rc = fp32.run(t0, nt, ws, s);
-                }
+                rc = search.run(t0, nt, ws, s);
                 if (!rc && zc)
                     rc = launch_zero_count(d, P.out, t0, nt, zc, s);
             }

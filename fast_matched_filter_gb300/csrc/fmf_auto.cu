@@ -76,18 +76,19 @@ __global__ void auto_dc_stats_kernel(const float2 *__restrict__ stat, long long 
 // of the longest length L.
 __global__ void auto_dc_prefix_kernel(const long long *__restrict__ pre2q,
                                       const float *__restrict__ unit2,
-                                      const float2 *__restrict__ pre1f, int N, int L,
-                                      float *__restrict__ dc)
+                                      const float2 *__restrict__ pre1f, long long pre_ch, long long pre_ps,
+                                      int step, int N, int L, float *__restrict__ dc)
 {
     __shared__ float red[8];
     const int ch = blockIdx.x;
-    const long long *p2 = pre2q + (size_t)ch * (N + 1);
-    const float2 *p1 = pre1f + (size_t)ch * (N + 1);
+    const long long *p2 = pre2q + ch * pre_ch;
+    const float2 *p1 = pre1f + ch * pre_ch;
+    const auto at = [=](int u) { return (u % step) * pre_ps + u / step; };
     const float q = unit2[ch], nf = (float)L, inv_n = 1.0f / nf;
     float mx = 0.0f;
     for (int u = threadIdx.x * kAutoStride; u + L <= N; u += blockDim.x * kAutoStride) {
         float v, mean;
-        window_centred(p2[u], p2[u + L], q, p1[u], p1[u + L], nf, inv_n, v, mean);
+        window_centred(p2[at(u)], p2[at(u + L)], q, p1[at(u)], p1[at(u + L)], nf, inv_n, v, mean);
         if (v > 0.0f)
             mx = fmaxf(mx, nf * mean * mean / v);
     }
@@ -186,7 +187,8 @@ int choose_auto_precision(const Problem &P, Scratch &ws, cudaStream_t s, int *pr
         if ((rc = ws.get(&dc, (size_t)P.SC, "precision estimate")))
             return rc;
         if (P.pre2q)
-            auto_dc_prefix_kernel<<<P.SC, 256, 0, s>>>(P.pre2q, P.unit2, P.pre1f, P.N, P.L, dc);
+            auto_dc_prefix_kernel<<<P.SC, 256, 0, s>>>(P.pre2q, P.unit2, P.pre1f, P.pre_ch, P.pre_ps, P.step, P.N,
+                                                       P.L, dc);
         else
             auto_dc_stats_kernel<<<P.SC, 256, 0, s>>>(reinterpret_cast<const float2 *>(P.stat_e), P.stat_ch,
                                                       P.stat_ps, P.stat_rem, P.step, P.N - P.L + 1, P.L, dc);

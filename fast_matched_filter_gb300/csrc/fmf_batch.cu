@@ -21,6 +21,9 @@
 
 namespace fmf {
 constexpr int kBatchBranches = 8;  // concurrent graph branches for the per-search work
+// A graph holds the operand blocks of all its searches at once: FP32 searches with
+// more than this stay on the CUDA cores.
+constexpr size_t kBatchTemplateBytes = (size_t)1 << 30;
 }
 
 struct fmf_batch {
@@ -60,29 +63,31 @@ static int batch_record(fmf_batch *b, cudaStream_t s)
             bws.emplace_back(new Scratch(b->branch[k]));
         const size_t n = b->searches.size();
         std::vector<Problem> P(n);
-        std::vector<const float *> dtc(n);
-        const int split = b->precision == FMF_PREC_SPLIT_BF16;
-        const bool tc = b->precision != FMF_PREC_FP32;
-        std::vector<int> nb(n);
+        const int form = tc_form(b->precision);
+        const bool fp32 = form == TC_FORM_FP32;
+        std::vector<int> nb(n, 0);  // lag blocks per tile; 0: the CUDA cores
         const size_t psz = tc_prob_size();
         std::vector<unsigned char> probs(psz * n);
         for (size_t i = 0; i < n && status == FMF_OK; i++) {
             const int k = (int)(i % kBatchBranches);
             cudaStream_t si = b->branch[k];
-            if ((status = prepare_problem(b->searches[i], *bws[k], si, &P[i], &dtc[i])))
+            const Args &a = b->searches[i];
+            nb[i] = fp32 ? tc_fp32_nb(a.T, a.S * a.C, a.L, a.step, a.n_corr)
+                         : tc_choose_nb((int)a.L, (int)a.step, form != TC_FORM_BF16, b->tile);
+            if (!fp32 && nb[i] == 0) {
+                status = set_error(FMF_ERR_SMEM, "search %zu: template length %zu with step %zu does not "
+                                                 "fit a tensor-core tile", i, a.L, a.step);
                 break;
-            if (!tc) {
+            }
+            if ((status = prepare_problem(a, *bws[k], si, &P[i], tc_pad(nb[i]), fp32 && nb[i])))
+                break;
+            if (fp32 && nb[i] && tc_template_bytes(P[i], nb[i]) > kBatchTemplateBytes)
+                nb[i] = 0;
+            if (nb[i] == 0)
                 status = launch_plain_all(P[i], si);
-                continue;
-            }
-            nb[i] = tc_choose_nb(P[i].L, P[i].step, split, b->tile);
-            if (nb[i] == 0) {
-                status = set_error(FMF_ERR_SMEM, "search %zu: template length %d with step %d does not "
-                                                 "fit a tensor-core tile", i, P[i].L, P[i].step);
-                break;
-            }
-            status = tc_prepare(P[i], dtc[i], split, nb[i], b->group, *bws[k], si,
-                                reinterpret_cast<TcProb *>(probs.data() + psz * i));
+            else
+                status = tc_prepare(P[i], form, nb[i], b->group, *bws[k], si,
+                                    reinterpret_cast<TcProb *>(probs.data() + psz * i));
         }
         // join the branches, then the persistent launches on s
         for (int k = 0; k < kBatchBranches; k++)
@@ -90,16 +95,15 @@ static int batch_record(fmf_batch *b, cudaStream_t s)
                 (e = cudaStreamWaitEvent(s, b->ev_join[k], 0)) != cudaSuccess)
                 status = status ? status : set_error(FMF_ERR_CUDA, "joining the batch capture: %s",
                                                      cudaGetErrorString(e));
-        if (status == FMF_OK && tc) {
+        if (status == FMF_OK) {
             unsigned *err = nullptr;
             if ((status = device_error_word(&err)) == FMF_OK) {
-                // one persistent launch per normalisation (each runs the epilogue
-                // instantiation of its own mode: a mixed launch carries both modes' code),
-                // 64 searches at most per launch
-                for (int norm = 0; norm < 2 && status == FMF_OK; norm++) {
+                // one persistent launch per normalisation and output layout (each runs the
+                // instantiation of its own mode), 64 searches at most per launch
+                for (int mode = 0; mode < 4 && status == FMF_OK; mode++) {
                     std::vector<unsigned char> grp;
                     for (size_t i = 0; i < n; i++)
-                        if (P[i].normalize == norm)
+                        if (nb[i] && P[i].normalize == (mode & 1) && (P[i].network_sum == 0) == (mode >> 1))
                             grp.insert(grp.end(), probs.begin() + psz * i, probs.begin() + psz * (i + 1));
                     const size_t ng = grp.size() / psz;
                     for (size_t i0 = 0; i0 < ng && status == FMF_OK; i0 += TC_MAX_PROBS) {
@@ -107,10 +111,16 @@ static int batch_record(fmf_batch *b, cudaStream_t s)
                         if ((status = ws.get(&queue, 1, "tile queue")))
                             break;
                         const int m = (int)(ng - i0 < (size_t)TC_MAX_PROBS ? ng - i0 : TC_MAX_PROBS);
-                        status = tc_run(reinterpret_cast<const TcProb *>(grp.data() + psz * i0), m, split, 0,
+                        status = tc_run(reinterpret_cast<const TcProb *>(grp.data() + psz * i0), m, form, 0,
                                         queue, err, s);
                     }
                 }
+                // FP32: the searches whose operands' flags leave them to the CUDA cores
+                for (size_t i = 0; i < n && fp32 && status == FMF_OK; i++)
+                    if (nb[i]) {
+                        P[i].only_if = P[i].scan + 3 * P[i].SC;
+                        status = launch_plain_all(P[i], s);
+                    }
             }
         }
         // the branch scratch is freed after the work on s that reads it

@@ -45,10 +45,12 @@ struct Problem {
     int network_sum;      // 1 weighted sum over channels, 0 per channel
     // Per-channel template lengths (Fisher-z network sum), else null:
     const int *ntap;      // (T, SC) taps of each channel (templates zero-padded to L)
-    const long long *pre2q; // (SC, N+1) running sums of d^2 (centred d for full), exact, in units
-                            // unit2[ch] (64-bit fixed point)
+    const long long *pre2q; // running sums of d^2 (centred d for full), exact, in units
+                            // unit2[ch] (64-bit fixed point); the sum over samples below
+                            // step * x + psi is element ch * pre_ch + psi * pre_ps + x
+    long long pre_ch, pre_ps;
     const float *unit2;     // (SC) the fixed-point unit of each channel's running sums, a power of two
-    const float2 *pre1f;    // (SC, N+1) running sums of centred d as hi + lo floats (full), else null
+    const float2 *pre1f;    // the same of centred d as hi + lo floats (full), else null
     const float *zweight; // (T, SC) Fisher-z weight of each channel
     // (T) each, or null: when set, the tensor-core kernel writes
     // (tanh(x / vp_norm[t]) + vp_bias[t]) * vp_scale[t] for every output x
@@ -245,35 +247,33 @@ StatPlace stat_rows(int SC, int N, int step, int pad, size_t *elems);
 StatPlace stat_rows_packed(int N, int step);
 int launch_window_stats(const float *data, int N, int L, int SC, const float *mu, float *dcen,
                         float *stat_e, const StatPlace &place, unsigned *scan, cudaStream_t s);
-// nb32: lag blocks per tile of the FP32 form on the tensor cores (0: not asked
-// for); it needs Problem::scan and a tile of padding round the statistics
-int prepare_problem(const Args &a, Scratch &ws, cudaStream_t s, Problem *P, const float **data_for_tc,
-                    int nb32 = 0);
+// pad: padding round the statistics' rows (tc_pad); scan: also make Problem::scan
+int prepare_problem(const Args &a, Scratch &ws, cudaStream_t s, Problem *P, int pad, bool scan);
 
-// Tensor-core form (fmf_tc.cu).
+// Tensor cores (fmf_tc.cu): begin a search, then run its templates in parts.
 constexpr int TC_MAX_PROBS = 64;
-// operands of a persistent launch: one bf16 product, bf16 pairs, fp16 pairs (FP32 accuracy)
+// operands: one bf16, bf16 pairs, fp16 pairs (FP32 accuracy)
 enum { TC_FORM_BF16 = 0, TC_FORM_SPLIT = 1, TC_FORM_FP32 = 2 };
+inline int tc_form(int precision)
+{
+    return precision == FMF_PREC_FP32 ? TC_FORM_FP32
+                                      : (precision == FMF_PREC_SPLIT_BF16 ? TC_FORM_SPLIT : TC_FORM_BF16);
+}
 struct TcProb;
-int tc_choose_nb(int L, int step, int split, int forced);
-int tc_prepare(const Problem &P, const float *data_for_tc, int split, int nb, int tg, Scratch &ws,
-               cudaStream_t s, TcProb *out);
-
-// FP32 on the tensor cores (fmf_tc32.cu): begin a search, then run its templates in
-// parts; the search's flag word says afterwards that the CUDA cores have to run it.
-struct Tc32Search;
-size_t tc32_search_size();
-int tc32_choose_nb(size_t T, size_t SC, size_t L, size_t step, size_t n_corr);  // 0: the CUDA cores
-int tc32_begin(const Problem &P, int nb, int tg, int max_templates, Scratch &ws, cudaStream_t s,
-               Tc32Search *out);
-int tc32_run(const Tc32Search *full, int t0, int nt, unsigned *err, Scratch &ws, cudaStream_t s);
-const unsigned *tc32_flag(const Tc32Search *full);
-int tc32_prepare(const Problem &P, int nb, int tg, Scratch &ws, cudaStream_t s, TcProb *out);
-int tc_choose_parts(const TcProb *prob);
+struct TcSearch;
+int tc_choose_nb(int L, int step, int pairs, int forced);  // lag blocks per tile; 0: no tile fits
+int tc_fp32_nb(size_t T, size_t SC, size_t L, size_t step, size_t n_corr);  // 0: the CUDA cores
+inline int tc_pad(int nb) { return nb ? 128 * nb + 16 : 0; }  // statistics padding of such a tile
+size_t tc_search_size();
+int tc_begin(const Problem &P, int form, int nb, int tg, int max_templates, Scratch &ws, cudaStream_t s,
+             TcSearch *out);
+int tc_run_templates(const TcSearch *full, int t0, int nt, unsigned *err, Scratch &ws, cudaStream_t s);
+const unsigned *tc_flag(const TcSearch *full);
+size_t tc_prob_size();
+size_t tc_template_bytes(const Problem &P, int nb);  // operand blocks of all templates
+int tc_prepare(const Problem &P, int form, int nb, int tg, Scratch &ws, cudaStream_t s, TcProb *out);
 int tc_run(const TcProb *probs, int n, int form, int parts, unsigned long long *queue, unsigned *err,
            cudaStream_t s);
-size_t tc_prob_size();
-void tc_subset(const TcProb *full, int t0, int nt, TcProb *out);
 int launch_plain(const Problem &P, cudaStream_t stream);
 int launch_plain_all(const Problem &P, cudaStream_t stream);
 // FMF_PREC_AUTO: the precision a prepared search runs in (fmf_auto.cu); waits on s.

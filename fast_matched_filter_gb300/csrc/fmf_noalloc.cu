@@ -227,6 +227,7 @@ extern "C" int fmf_matched_filter_noalloc(const float *templates, const float *s
     P.network_sum = sum_cc_mode != 0;
     P.ntap = nullptr;
     P.pre2q = nullptr;
+    P.pre_ch = P.pre_ps = 0;
     P.unit2 = nullptr;
     P.pre1f = nullptr;
     P.zweight = nullptr;

@@ -255,22 +255,25 @@ plain_kernel(const Problem P, const PlainGeom g)
                 const float ts = FULL ? P.tsum[row] : 0.0f;
                 const int n = P.ntap[row];
                 const float nf = (float)n, inv_n = 1.0f / nf;
-                const long long *p2 = P.pre2q + (size_t)ch * (P.N + 1);
+                // running sums at lag 0's window start (element k further for lag k) and end
+                const int mu = mo[ch] >= 0 ? mo[ch] / P.step : -((-mo[ch] + P.step - 1) / P.step);
+                const int psi = mo[ch] - P.step * mu, far = (psi + n) / P.step;
+                const long long pa = ch * P.pre_ch + psi * P.pre_ps + mu;
+                const long long pb = ch * P.pre_ch + (psi + n - far * P.step) * P.pre_ps + mu + far;
+                const long long *p2a = P.pre2q + pa, *p2b = P.pre2q + pb;
                 const float unit = P.unit2[ch];
-                const float2 *p1 = FULL ? P.pre1f + (size_t)ch * (P.N + 1) : nullptr;
+                const float2 *p1a = FULL ? P.pre1f + pa : nullptr, *p1b = FULL ? P.pre1f + pb : nullptr;
 #pragma unroll
                 for (int r = 0; r < PL_R; r++) {
                     const int k = k0 + tid * PL_R + r;
                     if (k >= klo && k < khi) {
-                        const int u = k * P.step + mo[ch];  // a window inside [0, N - n]
                         float num = acc[r], ssd;
                         if (FULL) {
                             float mean;
-                            window_centred(p2[u], p2[u + n], unit, p1[u], p1[u + n], nf, inv_n, ssd,
-                                           mean);
+                            window_centred(p2a[k], p2b[k], unit, p1a[k], p1b[k], nf, inv_n, ssd, mean);
                             num = fmaf(-mean, ts, num);
                         } else {
-                            ssd = window_energy(p2[u], p2[u + n], unit);
+                            ssd = window_energy(p2a[k], p2b[k], unit);
                         }
                         const float den = sqrtf(sst * ssd);
                         const float cc = den > kThreshold ? num / den : 0.0f;

@@ -512,11 +512,20 @@ window_stats_kernel(const float *__restrict__ data, int N, int L, const float *_
     const float dead = SCAN ? kThreshold / __uint_as_float(scan[2 * gridDim.y + ch]) * 0.999f : 0.0f;
     unsigned low = 0;  // the smallest energy above it, bits complemented
     float *row = stat_e + ch * place.ch * (full ? 2 : 1);
-    for (int u = threadIdx.x; u < nwin; u += kStatThreads) {  // coalesced stores
-        long long o = c0 + u;  // the window's first sample
-        if (place.step > 1) {
-            const int w = (int)o, x = w / place.step;
-            o = (w - x * place.step) * place.ps + min(w - x * place.step, place.rem) + x;
+    // coalesced stores: windows in order, or (step > 1) row by row, `per` of each
+    const int step = place.step, per = step == 1 ? nwin : (nwin + step - 1) / step;
+    const int head = step == 1 ? 0 : (int)(c0 % step);  // row of window 0
+    const long long x0 = step == 1 ? c0 : c0 / step;    // and its place there
+    for (int i = threadIdx.x; i < per * step; i += kStatThreads) {
+        int u = i;
+        long long o = c0 + i;
+        if (step > 1) {
+            const int r = i / per, j = i - r * per;  // the r-th row from window 0's, its j-th window
+            u = r + j * step;
+            if (u >= nwin)
+                continue;
+            const int psi = head + r < step ? head + r : head + r - step;
+            o = psi * place.ps + min(psi, place.rem) + x0 + j + (head + r < step ? 0 : 1);
         }
         float en;
         if (full) {

@@ -1,9 +1,9 @@
-// fmf_tc.cu -- tensor-core (tcgen05 / TMEM) matched filter, split-BF16 form.
+// fmf_tc.cu -- the numerators on the tensor cores (tcgen05 / TMEM): the FP32 form
+// of searches large enough for it, and the bf16 forms.
 //
-// Same outputs as the plain form (fmf_plain.cu); the numerator sum_j t[j]*d[k*step+mo+j]
-// runs on the 5th-generation tensor cores.  Every per-channel correlation is
-// a Toeplitz x Hankel product, laid out so that neither matrix is built in
-// full:
+// Same outputs as the CUDA-core kernel (fmf_plain.cu), which is bound by the
+// FP32 FMA pipe; the numerator sum_j t[j]*d[k*step+mo+j] is a Toeplitz x Hankel
+// product per channel, laid out so that neither matrix is built in full:
 //
 //   Output index i = I0 + Q*a + b of one template and channel (I0 a multiple
 //   of Q = 128, a = lag block, b = phase in [0, Q)) needs data samples
@@ -27,204 +27,485 @@
 //     offsets are 128 bytes.  W is 8/Q of the Toeplitz matrix.
 //   * step > 1: taps j = step*q + phi read the decimated stream
 //     d_psi[x] = d[step*x + psi]; each phase is a unit-step correlation with
-//     its own template taps and moveout, accumulated into the same TMEM tile.
-//   * Split-BF16: operands are bf16 hi + lo (x = hi + lo to 2^-16 relative);
-//     three MMAs per K step (hi*hi, hi*lo, lo*hi) accumulate in FP32 in TMEM.
+//     its own template taps and moveout, accumulated into the same sums.
 //
-// Persistent CTAs (one per SM) take items (one template x NB*Q consecutive
-// outputs, all channels) from a tile queue:
-//   warp 0      producer: claims items, cp.async.bulk (TMA bulk copies) of the
-//               data rows and template blocks of one (channel, phase) stage
-//               into stage buffer b (b = parity of the channel's running
-//               index), mbarrier complete_tx;
-//   warps 1, 2  MMA issuers: one thread each issues tcgen05.mma for the
-//               channels of its parity, from its stage buffer into its FP32
-//               accumulator in TMEM, and commits to the barriers (a single
-//               issuing thread cannot keep the tensor pipe busy);
-//   warp 1      also allocates the TMEM (two accumulators + the network sum);
-//   warps 4-11  epilogue: tcgen05.ld of the accumulator, normalisation by the
-//               window statistics, threshold, weighted network sum in TMEM
-//               (channel order, fused multiply-add), outputs.
-// Instantiations: tc_persistent<VAR, PARTS>.  VAR: per-channel template
-// lengths (the issuers cut each channel's K range at its own taps; 16 epilogue
-// warps, warps 4-19, form window sums from per-channel running sums and add
-// atanh(cc) * z).  PARTS: the items of a small search are split into channel
-// parts whose partial sums a second kernel adds in order.
+// Operands are pairs, high h and low l, and one K step is three MMAs: h h, h l
+// and l h (the dropped l l is the square of the pair's rounding).
+//   * split bf16: h = bf16(x), l = bf16(x - h): 2^-16 of a product at most.
+//   * FP32: x = s (h + 2^-11 l) in fp16, s a power of two (per data channel, per
+//     template channel) that brings the largest value to [2^14, 2^15), h =
+//     fp16(x / s), l = fp16(2^11 (x / s - h)).  h has 11 significant bits and l
+//     the next 11, so the pair holds x to half a unit of FP32's last place,
+//     down to 2^-50 of the channel's largest value (below that l runs out of
+//     exponent), and the dropped l l is at most 2^-24 of |t d|.
+//   * single bf16: h alone, one MMA.
+// The tensor core rounds every accumulation toward zero, so a long chain
+// drifts: one accumulator over the 38 steps of a 600-tap template was 2.3e-8
+// RMS off (FP32 FMAs: 1.8e-8), 1.2e-6 at a perfect match.  So the h h products
+// run in chains of at most kChain steps, each in a fresh accumulator that the
+// epilogue adds to its registers in FP32 (rounded to nearest); h l and l h,
+// smaller by the pair's rounding, share one accumulator per channel.
+//
+// What bounds it: the tensor pipe, and with it the power limit, from some 400
+// taps (40 templates x 60 channels x 1.08M lags x 600 taps in 6.3 ms: 1.8
+// PFLOP/s of MMAs, 1.74 is what cuBLAS sustains under the limit); the issuing
+// threads and the epilogue below (60 taps: 3.3 ms).  An issuing thread's code
+// costs as much as its MMAs: a branchy loop took 500 cycles per MMA of 64.
+//
+// Roles of a persistent CTA (12 warps, one CTA per SM), which takes items (one
+// template x NB*Q consecutive outputs, all channels or a part of them) from a
+// tile queue:
+//   warp 0      claims items; TMA bulk copies of the template blocks of a (channel,
+//               phase) stage (two buffers) and of its data, four column blocks
+//               per slot
+//   warp 1      issues the h h MMAs into H0 / H1 in turn, one chain each
+//   warp 2      issues the h l and l h MMAs into S0 / S1, one channel each (two
+//               issuers: one thread cannot issue fast enough, and neither
+//               waits for the other's accumulators)
+//   warp 3      bulk copies of the window statistics
+//   warps 4-11  epilogue: chains into registers, then per channel the
+//               normalisation and the network sum, both in registers (208 per
+//               thread; the other four warps give theirs up)
+// TMEM: H0, H1, S0, S1 of 128 columns each: all 512.
 // Every wait is bounded (globaltimer); on timeout the CTA raises an error
 // word, stops issuing, waits for its own copies/MMAs (bounded) and frees TMEM.
 #include <cfloat>
-#include <type_traits>
+#include <cstdlib>
 
 #include <cuda_bf16.h>
+#include <cuda_fp16.h>
 
-#include "fmf_common.cuh"
 #include "fmf_tc.cuh"
 
 namespace fmf {
 
-// Epilogue warps (2 per TMEM lane quarter; 4 per quarter for per-channel
-// template lengths, whose epilogue does more arithmetic per output and needs
-// more warps to hide its latency) + producer, 2 MMA issuers, 1 idle warp.
+// Epilogue warps, a quarter of them on each TMEM lane quarter: 8 with 64 columns of a
+// full tile each; 16 with 32 for per-channel lengths, whose epilogue does four
+// times the arithmetic per output and waits for it (40 templates x 60 channels x
+// 300,000 lags: 7.2 ms with 8).
 constexpr int tc_epi_warps(bool var) { return var ? 16 : 8; }
 constexpr int tc_threads(bool var) { return 32 * (4 + tc_epi_warps(var)); }
+constexpr int tc_groups(bool var) { return tc_epi_warps(var) / 4; }  // column groups of a tile
+constexpr int TC_MAX_ROWS = 8;     // data slots, at most
+constexpr int TC_MAX_STATS = 2;    // statistics slots, at most
+constexpr int kChain = 16;          // K steps of one h h chain
+constexpr float kLoScale = 2048.0f;  // l is kept 2^11 up
+constexpr int kTopExp = 15;          // operands are scaled to below 2^15
+// data and template channels whose largest value lies outside [2^-41, 2^60) go
+// to the CUDA-core kernel: the products of their scales would leave FP32
+constexpr int kMinExp = -40, kMaxExp = 60;
 
-// ------------------------------------------------------------------ preprocessing
+__device__ __forceinline__ float exp2_int(int e)  // 2^e, -126 <= e <= 127
+{
+    return __int_as_float((e + 127) << 23);
+}
+
+// exponent e with m = f 2^e, f in [1/2, 1), from the bits of a finite m >= 0; kTopExp
+// (scale 1) for 0
+__device__ __forceinline__ int max_exponent(unsigned bits, bool &ok)
+{
+    const int e = (int)(bits >> 23) - 126;
+    ok = bits == 0 || (e >= kMinExp && e <= kMaxExp);
+    return bits != 0 && ok ? e : kTopExp;
+}
+
+__device__ __forceinline__ bool finite_bits(unsigned abs_bits) { return abs_bits < 0x7f800000u; }
+
+// x / s as the pair (h, l); x that is not finite becomes 0: every window that
+// holds it has a NaN energy, and its coefficient is 0 in both kernels.
+__device__ __forceinline__ void split_fp16(float x, float inv_s, uint16_t &hi, uint16_t &lo)
+{
+    const float y = finite_bits(__float_as_uint(x) & 0x7fffffffu) ? x * inv_s : 0.0f;
+    const __half h = __float2half_rn(y);
+    const __half l = __float2half_rn((y - __half2float(h)) * kLoScale);
+    hi = __half_as_ushort(h);
+    lo = __half_as_ushort(l);
+}
+
+__device__ __forceinline__ uint4 pack8(const uint16_t *v)
+{
+    uint4 r;
+    r.x = v[0] | ((uint32_t)v[1] << 16);
+    r.y = v[2] | ((uint32_t)v[3] << 16);
+    r.z = v[4] | ((uint32_t)v[5] << 16);
+    r.w = v[6] | ((uint32_t)v[7] << 16);
+    return r;
+}
+
+// Whether the CUDA cores run this search instead.
+__device__ __forceinline__ bool tc_skipped(const TcProb &pr) { return pr.skip && *pr.skip; }
+
+// Whether the tile at I0 holds a valid output.  The range of a template without any is
+// empty, wherever it lies: its moveouts may point anywhere.
+__device__ __forceinline__ bool tc_holds(int k_lo, int k_hi, long long I0, int nb)
+{
+    return k_lo < k_hi && I0 < k_hi && I0 + (long long)TC_Q * nb > k_lo;
+}
+
+// Whether a tile of template t holds a valid output and the search runs here.
+__device__ __forceinline__ bool tc_busy(const TcProb &pr, long long I0, int t)
+{
+    return tc_holds(pr.P.k_lo[t], pr.P.k_hi[t], I0, pr.nb) && !tc_skipped(pr);
+}
+
+// Moveout of phase phi in its stream, and the stream: m = step mu + psi.
+__device__ __forceinline__ int tc_phase(int m, int step, int &psi)
+{
+    if (step == 1) {
+        psi = 0;
+        return m;
+    }
+    const int mu = m >= 0 ? m / step : -((-m + step - 1) / step);
+    psi = m - step * mu;
+    return mu;
+}
+
+// A statistics slot: `columns` lag blocks of each column group of the tile from each of
+// `streams` arrays, copied from the 16-byte boundary before the first window.
+// Fixed lengths: window energies, or (energy, mean) pairs.  Per-channel lengths:
+// running sums of d^2 at a window's start and end, for 'full' also those of d.
+struct StatSlot {
+    int columns, streams, elem, groups;
+    __host__ __device__ constexpr StatSlot(bool var, bool full)
+        : columns(var ? (full ? 2 : 4) : (full ? 16 : 32)), streams(var ? (full ? 4 : 2) : 1),
+          elem(var || full ? 8 : 4), groups(var ? 4 : 2)
+    {
+    }
+    __host__ __device__ constexpr uint32_t part() const { return (uint32_t)(columns * TC_Q * elem + 16); }
+    __host__ __device__ constexpr uint32_t bytes() const { return (uint32_t)(groups * streams) * part(); }
+    __host__ __device__ constexpr int align() const { return 16 / elem - 1; }  // mask of elements
+};
+
+// The same as a bf16 pair in the data's own units: l is bf16(x - h).
 __device__ __forceinline__ void split_bf16(float x, uint16_t &hi, uint16_t &lo)
 {
-    __nv_bfloat16 h = __float2bfloat16_rn(x);
-    __nv_bfloat16 l = __float2bfloat16_rn(x - __bfloat162float(h));
+    const float y = finite_bits(__float_as_uint(x) & 0x7fffffffu) ? x : 0.0f;
+    const __nv_bfloat16 h = __float2bfloat16_rn(y);
+    const __nv_bfloat16 l = __float2bfloat16_rn(y - __bfloat162float(h));
     hi = __bfloat16_as_ushort(h);
     lo = __bfloat16_as_ushort(l);
 }
 
-// G[ch][psi][cb][r][e] = split(d[ch][step*(Q*(r - row_front) + 8*cb + e) + psi]), zero outside [0, N).
-// One thread per 16-byte row chunk.
-__global__ void tc_data_kernel(const float *__restrict__ data, int N, int SC, int step,
-                               int rows_total, int row_front, uint16_t *__restrict__ g_hi,
-                               uint16_t *__restrict__ g_lo)
+template <bool FP32>
+__device__ __forceinline__ void split_pair(float x, float inv_s, uint16_t &hi, uint16_t &lo)
 {
-    long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    long long total = (long long)SC * step * TC_CB * rows_total;
-    if (idx >= total)
+    if constexpr (FP32)
+        split_fp16(x, inv_s, hi, lo);
+    else
+        split_bf16(x, hi, lo);
+}
+
+// ------------------------------------------------------------------ operands
+// G[ch][psi][cb][r][e] = pair of d[ch][step*(Q*(r - row_front) + 8*cb + e) + psi], zero outside [0, N);
+// one thread per 16-byte row chunk.  FP32: the first thread of a channel also
+// writes its exponent and decides whether the
+// channel's values can be held: stat is the scan of prepare_problem (largest
+// |x|; smallest window energy that can pass the threshold, complemented).
+// The error of a coefficient from the pairs is at most 2^-51 of the largest
+// value over the root of the window's energy, so windows down to 2^-42 of
+// the largest value squared keep it at 1e-9.
+template <bool FP32>
+__global__ void tc_data_kernel(const float *__restrict__ data, int N, int SC, int step, int rows_total,
+                                 int row_front, const unsigned *__restrict__ stat,
+                                 uint16_t *__restrict__ g_hi, uint16_t *__restrict__ g_lo,
+                                 int *__restrict__ d_exp, unsigned *skip)
+{
+    const long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    const long long per_ch = (long long)step * TC_CB * rows_total;
+    if (idx >= per_ch * SC)
         return;
-    int r = (int)(idx % rows_total);
-    long long rest = idx / rows_total;
-    int cb = (int)(rest % TC_CB);
-    rest /= TC_CB;
-    int psi = (int)(rest % step);
-    int ch = (int)(rest / step);
-    long long x0 = (long long)TC_Q * (r - row_front) + 8 * cb;
+    const int ch = (int)(idx / per_ch);
+    long long rest = idx - ch * per_ch;
+    float inv_s = 1.0f;
+    if constexpr (FP32) {
+        const unsigned top = stat[ch];
+        bool ok;
+        const int e = max_exponent(top, ok);
+        if (rest == 0) {
+            d_exp[ch] = e;
+            const unsigned low = ~stat[SC + ch];  // smallest energy's bits; ~0 (a NaN): none
+            const float m = __uint_as_float(top);
+            if (!ok || (low < 0x7f800000u && __uint_as_float(low) * 0x1p42f < m * m))
+                atomicOr(skip, 1u);
+        }
+        inv_s = exp2_int(kTopExp - e);
+    }
+    const int r = (int)(rest % rows_total);
+    rest /= rows_total;
+    const int cb = (int)(rest % TC_CB);
+    const int psi = (int)(rest / TC_CB);
+    const long long x0 = (long long)TC_Q * (r - row_front) + 8 * cb;
     const float *src = data + (size_t)ch * N;
     uint16_t h[8], l[8];
 #pragma unroll
-    for (int e = 0; e < 8; e++) {
-        long long pos = (long long)step * (x0 + e) + psi;
-        float v = (x0 + e >= 0 && pos < N) ? src[pos] : 0.0f;
-        split_bf16(v, h[e], l[e]);
+    for (int i = 0; i < 8; i++) {
+        const long long pos = (long long)step * (x0 + i) + psi;
+        const float v = (x0 + i >= 0 && pos < N) ? src[pos] : 0.0f;
+        split_pair<FP32>(v, inv_s, h[i], l[i]);
     }
-    uint4 hv, lv;
-    hv.x = h[0] | ((uint32_t)h[1] << 16);
-    hv.y = h[2] | ((uint32_t)h[3] << 16);
-    hv.z = h[4] | ((uint32_t)h[5] << 16);
-    hv.w = h[6] | ((uint32_t)h[7] << 16);
-    lv.x = l[0] | ((uint32_t)l[1] << 16);
-    lv.y = l[2] | ((uint32_t)l[3] << 16);
-    lv.z = l[4] | ((uint32_t)l[5] << 16);
-    lv.w = l[6] | ((uint32_t)l[7] << 16);
-    reinterpret_cast<uint4 *>(g_hi)[idx] = hv;
+    reinterpret_cast<uint4 *>(g_hi)[idx] = pack8(h);
     if (g_lo)
-        reinterpret_cast<uint4 *>(g_lo)[idx] = lv;
+        reinterpret_cast<uint4 *>(g_lo)[idx] = pack8(l);
 }
 
-// W[t][ch][phi][n][e][c] = split(tphi[8n + e + c - (Q-1+s)]), tphi[q] = tpl[step*q + phi],
-// s = mu mod Q, mu = floor((mo + phi) / step), psi = mo + phi - step*mu.
-// One thread per (block n, row e).
-__global__ void tc_template_kernel(const float *__restrict__ tpl, const int *__restrict__ mo, int T,
-                                   int SC, int L, int step, int NW, uint16_t *__restrict__ w_hi,
-                                   uint16_t *__restrict__ w_lo, int *__restrict__ mu_out,
-                                   int *__restrict__ psi_out)
+// W[t][ch][phi][n][e][c] = pair of tphi[8n + e + c - (Q-1+s)], tphi[q] = tpl[step*q + phi],
+// s = mu mod Q, mu = floor((mo + phi) / step); one block per (template,
+// channel), its taps in shared memory (read once, written 8 times over).
+// FP32: also the channel's exponent.
+template <bool FP32>
+__global__ void __launch_bounds__(256) tc_template_kernel(
+    const float *__restrict__ tpl, const int *__restrict__ mo, int L, int step, int NW,
+    uint16_t *__restrict__ w_hi, uint16_t *__restrict__ w_lo, int *__restrict__ t_exp, unsigned *skip)
 {
-    long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    long long total = (long long)T * SC * step * NW * 8;
-    if (idx >= total)
-        return;
-    int e = (int)(idx & 7);
-    long long rest = idx >> 3;
-    int n = (int)(rest % NW);
-    long long meta = rest / NW;  // (t*SC + ch)*step + phi
-    int phi = (int)(meta % step);
-    long long row = meta / step;  // t*SC + ch
-    int m = mo[row] + phi;
-    int mu = m >= 0 ? m / step : -((-m + step - 1) / step);
-    int psi = m - step * mu;
-    int s = ((mu % TC_Q) + TC_Q) % TC_Q;
-    if (n == 0 && e == 0) {
-        mu_out[meta] = mu;
-        psi_out[meta] = psi;
+    extern __shared__ float taps[];
+    const long long row = blockIdx.x;  // t*SC + ch
+    const float *src = tpl + row * L;
+    float inv_s = 1.0f;
+    if constexpr (FP32) {
+        __shared__ unsigned red[8];
+        __shared__ int bad;
+        if (threadIdx.x == 0)
+            bad = 0;
+        __syncthreads();
+        unsigned top = 0;
+        for (int j = threadIdx.x; j < L; j += blockDim.x) {
+            const float v = src[j];
+            taps[j] = v;
+            const unsigned b = __float_as_uint(v) & 0x7fffffffu;
+            if (finite_bits(b))
+                top = max(top, b);
+            else
+                bad = 1;  // the CUDA-core kernel decides what such a template gives
+        }
+        top = __reduce_max_sync(0xffffffffu, top);
+        if ((threadIdx.x & 31) == 0)
+            red[threadIdx.x >> 5] = top;
+        __syncthreads();
+        top = red[0];
+        for (int i = 1; i < (int)(blockDim.x >> 5); i++)
+            top = max(top, red[i]);
+        bool ok;
+        const int e = max_exponent(top, ok);
+        inv_s = exp2_int(kTopExp - e);
+        if (threadIdx.x == 0) {
+            if (!ok || bad)
+                atomicOr(skip, 1u);
+            t_exp[row] = e;
+        }
+    } else {
+        for (int j = threadIdx.x; j < L; j += blockDim.x)
+            taps[j] = src[j];
+        __syncthreads();
     }
-    const float *tp = tpl + row * L;
-    uint16_t h[8], l[8];
+    const int m0 = mo[row];
+    const int per_phase = NW * 8;
+    for (int i = threadIdx.x; i < step * per_phase; i += blockDim.x) {
+        const int phi = i / per_phase, ne = i - phi * per_phase;
+        int psi;
+        const int s = tc_phase(m0 + phi, step, psi) & (TC_Q - 1);
+        uint16_t h[8], l[8];
+        const int q0 = 8 * (ne >> 3) + (ne & 7) - (TC_Q - 1 + s);
 #pragma unroll
-    for (int c = 0; c < 8; c++) {
-        int q = 8 * n + e + c - (TC_Q - 1 + s);
-        int j = step * q + phi;
-        float v = (q >= 0 && j < L) ? tp[j] : 0.0f;
-        split_bf16(v, h[c], l[c]);
+        for (int c = 0; c < 8; c++) {
+            const int q = q0 + c, j = step * q + phi;
+            split_pair<FP32>(q >= 0 && j < L ? taps[j] : 0.0f, inv_s, h[c], l[c]);
+        }
+        const long long o = row * step * per_phase + i;
+        reinterpret_cast<uint4 *>(w_hi)[o] = pack8(h);
+        if (w_lo)
+            reinterpret_cast<uint4 *>(w_lo)[o] = pack8(l);
     }
-    uint4 hv, lv;
-    hv.x = h[0] | ((uint32_t)h[1] << 16);
-    hv.y = h[2] | ((uint32_t)h[3] << 16);
-    hv.z = h[4] | ((uint32_t)h[5] << 16);
-    hv.w = h[6] | ((uint32_t)h[7] << 16);
-    lv.x = l[0] | ((uint32_t)l[1] << 16);
-    lv.y = l[2] | ((uint32_t)l[3] << 16);
-    lv.z = l[4] | ((uint32_t)l[5] << 16);
-    lv.w = l[6] | ((uint32_t)l[7] << 16);
-    reinterpret_cast<uint4 *>(w_hi)[idx] = hv;
-    if (w_lo)
-        reinterpret_cast<uint4 *>(w_lo)[idx] = lv;
 }
 
 // ------------------------------------------------------------------ persistent kernel
-// TMEM columns: D0 [0,128), D1 [128,256), sum [256,384)
-constexpr int TC_NACC = 2;      // accumulator buffers
+// Offsets of the barriers in the kernel's shared memory (bytes past the rings).
+struct TcBars {
+    static constexpr uint32_t wfull = 0, wempty = 16, dfull = 32, dempty = dfull + 8 * TC_MAX_ROWS,
+                              efull = dempty + 8 * TC_MAX_ROWS, eempty = efull + 8 * TC_MAX_STATS,
+                              hfull = eempty + 8 * TC_MAX_STATS, hempty = hfull + 16, sfull = hempty + 16,
+                              sempty = sfull + 16, ifull = sempty + 16, iempty = ifull + 32,
+                              fin = iempty + 32, items = fin + 8, tmem = items + 32, abort = tmem + 4,
+                              bytes = abort + 4;
+};
 
-// every lane of every warp takes part (the tail reads a dummy value)
-__global__ void fisher_atanh_kernel(const float *__restrict__ y, float *__restrict__ out, long long n)
+// One MMA issuer's walk over the items: the h h products (SMALL false; chains of
+// chain_slots data slots into H0 / H1 in turn) or the h l and l h products (into
+// S0 / S1, a channel each).
+template <bool VAR, bool SMALL>
+__device__ __forceinline__ void tc_issue(const TcBatch &B, const long long *ring, uint32_t bar,
+                                           uint32_t w_base, uint32_t d_base, uint32_t tmem,
+                                           volatile int *abort_flag, bool one)
 {
-    const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    const float r = fisher_atanh(i < n ? y[i] : 0.0f);
-    if (i < n)
-        out[i] = r;
+    const auto uniform = [](int v) { return __shfl_sync(0xffffffffu, v, 0); };
+    // the whole warp waits and keeps the books; its elected lane issues
+    const auto wait = [&](uint32_t b, uint32_t parity, unsigned code) {
+        return __all_sync(0xffffffffu, mbar_wait(b, parity, abort_flag, B.err, code)) != 0;
+    };
+    uint32_t stages = 0, slot = 0, turn = 0;
+    uint32_t acc_i = 0;  // accumulators (channels or chains) begun
+    const uint32_t n_rows = (uint32_t)B.n_rows;
+    for (uint32_t q = 0;; q++) {
+        const uint32_t is = q & 3;
+        if (!wait(bar + TcBars::ifull + 8 * is, (q >> 2) & 1, 32u))
+            return;
+        const long long item = ring[is];
+        __syncwarp();
+        if (one)
+            mbar_arrive(bar + TcBars::iempty + 8 * is);
+        if (item >= B.total_items)
+            return;
+        int p, tile, t, c_begin, c_end, part;
+        decode_item(B, item, p, tile, t, c_begin, c_end, part);
+        p = uniform(p);
+        t = uniform(t);
+        c_end = uniform(c_end);
+        const TcProb &pr = B.prob[p];
+        const int nb = pr.nb;
+        if (!uniform(tc_busy(pr, (long long)tile * TC_Q * nb, t)))
+            continue;
+        // kind::f16 descriptor: F32 accumulate, A and B both FP16 or both BF16, K-major, N = nb, M = 128
+        const uint32_t idesc = (1u << 4) | B.mma_types | ((uint32_t)(nb >> 3) << 17) | ((uint32_t)(TC_Q >> 4) << 24);
+        const int SC = pr.P.SC, step = pr.P.step, L = pr.P.L;
+        const uint32_t chain_cols = (uint32_t)pr.chain_cols;
+        const uint32_t col_bytes = (uint32_t)pr.R * 16;
+        // 16-byte units from a high half to its low half, and of a column-block pair
+        const uint32_t a_low = (uint32_t)pr.NW * 8, b_low = 4u * (uint32_t)pr.R, b_pair = 2u * (uint32_t)pr.R;
+        const uint32_t a_hi = (uint32_t)(sdesc(0, 128, 128) >> 32);
+        const uint32_t b_hi = (uint32_t)(sdesc(0, col_bytes, 128) >> 32);
+        const uint32_t a_base = (uint32_t)sdesc(w_base, 128, 128), b_base = (uint32_t)sdesc(d_base, col_bytes, 128);
+        const uint32_t a_buf = (uint32_t)B.w_bytes >> 4, b_slot = (uint32_t)B.row_bytes >> 4;
+        const size_t row0 = (size_t)t * SC;
+        for (int g0 = uniform(c_begin); g0 < c_end; g0 += 32) {
+            // the scalars of 32 channels, one per lane
+            const int cl = min(g0 + (int)(threadIdx.x & 31), c_end - 1);
+            const int mo_l = pr.P.mo[row0 + cl], n_l = VAR ? pr.P.ntap[row0 + cl] : L;
+            uint32_t active = __ballot_sync(0xffffffffu, g0 + (int)(threadIdx.x & 31) < c_end && pr.P.w[row0 + cl] != 0.0f);
+            for (; active; active &= active - 1) {
+                const int src = __ffs(active) - 1;
+                const int mo = __shfl_sync(0xffffffffu, mo_l, src), ntap = __shfl_sync(0xffffffffu, n_l, src);
+                uint32_t left = 0;  // column-block pairs left to the accumulator
+                uint32_t dt = 0, acc = 0;
+                for (int phi = 0; phi < step; phi++, stages++) {
+                    const uint32_t wb = stages & 1;
+                    int psi;
+                    const uint32_t sres = (uint32_t)tc_phase(mo + phi, step, psi) & (TC_Q - 1);
+                    const uint32_t k_first = sres & ~15u;
+                    const uint32_t k_end = (uint32_t)tc_k_end((int)sres, step == 1 ? ntap : tc_phase_taps(L, step, phi, ntap));
+                    if (!wait(bar + TcBars::wfull + 8 * wb, (stages >> 1) & 1, 8u))
+                        return;
+                    const uint32_t a0 = a_base + (wb ? a_buf : 0u);
+#pragma unroll 1
+                    for (uint32_t j = 0; j < TC_CB / 2; j++) {
+                        if (left == 0) {  // the next accumulator
+                            const uint32_t empty = bar + (SMALL ? TcBars::sempty : TcBars::hempty) + 8 * (acc_i & 1);
+                            if (acc_i >= 2 && !wait(empty, ((acc_i >> 1) - 1) & 1, 4u))
+                                return;
+                            tc_fence_after();
+                            dt = tmem + (SMALL ? 256u : 0u) + 128u * (acc_i & 1);
+                            acc = 0;
+                            left = SMALL ? (uint32_t)step * (TC_CB / 2) : chain_cols;
+                        }
+                        // two column-block pairs per slot
+                        if ((j & 1) == 0 && !wait(bar + TcBars::dfull + 8 * slot, turn & 1, 8u))
+                            return;
+                        // K steps k = 16 j + 128 i: A moves 16 template blocks (2 KB), B one data
+                        // row (16 bytes) per step.  The start-address field (16-byte units) of
+                        // an address below 256 KB never carries out of its 14 bits.
+                        const uint32_t late = 16 * j < k_first ? 1u : 0u;
+                        const uint32_t n = ((k_end - 16 * j + TC_Q - 1) >> 7) - late;
+                        uint32_t a = a0 + 16 * j + late * TC_Q;
+                        uint32_t b = b_base + slot * b_slot + (j & 1 ? b_pair : 0u) + late;
+#pragma unroll 1
+                        for (uint32_t i = 0; i < n; i++) {
+                            if (one) {
+                                if (SMALL) {
+                                    mma_f16(dt, a, a_hi, b + b_low, b_hi, idesc, acc);
+                                    mma_f16(dt, a + a_low, a_hi, b, b_hi, idesc, 1);
+                                } else {
+                                    mma_f16(dt, a, a_hi, b, b_hi, idesc, acc);
+                                }
+                            }
+                            acc = 1;
+                            a += TC_Q;
+                            b += 1;
+                        }
+                        const bool done = --left == 0 || (!SMALL && j == TC_CB / 2 - 1 && phi == step - 1);
+                        if (one) {
+                            if (j & 1)
+                                mma_commit(bar + TcBars::dempty + 8 * slot);
+                            if (done)
+                                mma_commit(bar + (SMALL ? TcBars::sfull : TcBars::hfull) + 8 * (acc_i & 1));
+                        }
+                        if ((j & 1) && ++slot == n_rows) {
+                            slot = 0;
+                            turn++;
+                        }
+                        if (done) {
+                            acc_i++;
+                            left = 0;
+                        }
+                    }
+                    if (one)
+                        mma_commit(bar + TcBars::wempty + 8 * wb);
+                }
+            }
+        }
+    }
 }
 
-int launch_fisher_atanh(const float *y, float *out, long long n, cudaStream_t s)
-{
-    if (n <= 0)
-        return FMF_OK;
-    fisher_atanh_kernel<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(y, out, n);
-    count_launch();
-    return check_launch("fisher_atanh_kernel");
-}
-
-// VAR: per-channel template lengths (Problem::ntap set in every search of the
-// batch), a separate instantiation so that the fixed-length epilogue keeps
-// its registers.  PARTS: every search runs its items as channel parts
-// (TcProb::parts), a separate instantiation for the same reason.  NORM: 0 every
-// search 'short', 1 every search 'full', -1 each search's own (a batch mixing
-// both); the fixed modes drop the other mode's epilogue code.
-template <bool VAR, bool PARTS, int NORM>
+// VAR: per-channel template lengths (Fisher-z network sum); FULL: 'full'
+// normalisation; NSUM: network sum.  One instantiation per mode, each with its
+// own epilogue code only (the code of all roles shares the instruction cache).
+template <bool VAR, bool FULL, bool NSUM>
 __global__ void __launch_bounds__(tc_threads(VAR), 1) tc_persistent(const __grid_constant__ TcBatch B)
 {
-    constexpr int TC_EPI_WARPS = tc_epi_warps(VAR);
     extern __shared__ __align__(1024) uint8_t smem[];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int split = B.split;
+    constexpr StatSlot kStat(VAR, FULL);
+    constexpr int CH = kStat.columns;
+    constexpr uint32_t kStatPart = kStat.part();
+    constexpr int TC_EPI_WARPS = tc_epi_warps(VAR), G = tc_groups(VAR);
+    static_assert(kStat.groups == G, "statistics slots hold the epilogue's column groups");
+    const bool pairs = B.split != 0;
 
-    uint8_t *bar_base = smem + 2 * (size_t)B.stage_bytes;
-    const uint32_t full0 = smem_u32(bar_base), empty0 = full0 + 16, dfull0 = full0 + 32,
-                   dempty0 = full0 + 48, fin = full0 + 64, ifull0 = full0 + 72, iempty0 = full0 + 104;
-    long long *ring = reinterpret_cast<long long *>(bar_base + 136);  // 4 item slots
-    uint32_t *tmem_holder = reinterpret_cast<uint32_t *>(bar_base + 168);
-    volatile int *abort_flag = reinterpret_cast<volatile int *>(bar_base + 172);
+    // template blocks (2 buffers), data slots, statistics slots, barriers
+    const uint32_t w_base = smem_u32(smem);
+    const uint32_t d_base = w_base + 2u * B.w_bytes;
+    const uint32_t e_base = d_base + (uint32_t)B.n_rows * B.row_bytes;
+    uint8_t *bar_ptr = smem + 2u * B.w_bytes + (uint32_t)B.n_rows * B.row_bytes + ((uint32_t)B.stat_bytes << B.stat_log2);
+    const uint32_t bar = smem_u32(bar_ptr);
+    long long *ring = reinterpret_cast<long long *>(bar_ptr + TcBars::items);  // 4 item slots
+    uint32_t *tmem_holder = reinterpret_cast<uint32_t *>(bar_ptr + TcBars::tmem);
+    volatile int *abort_flag = reinterpret_cast<volatile int *>(bar_ptr + TcBars::abort);
+    const int n_rows = B.n_rows, stat_log2 = B.stat_log2;
 
     if (threadIdx.x == 0) {
         for (int i = 0; i < 2; i++) {
-            mbar_init(full0 + 8 * i, 1);
-            mbar_init(empty0 + 8 * i, 1);
-            mbar_init(dfull0 + 8 * i, 1);
-            mbar_init(dempty0 + 8 * i, TC_EPI_WARPS);
+            mbar_init(bar + TcBars::wfull + 8 * i, 1);
+            mbar_init(bar + TcBars::wempty + 8 * i, pairs ? 2 : 1);  // one commit per MMA issuer
+            mbar_init(bar + TcBars::hfull + 8 * i, 1);
+            mbar_init(bar + TcBars::hempty + 8 * i, TC_EPI_WARPS);
+            mbar_init(bar + TcBars::sfull + 8 * i, 1);
+            mbar_init(bar + TcBars::sempty + 8 * i, TC_EPI_WARPS);
         }
-        mbar_init(fin, 2);  // one commit per MMA issuer
+        for (int i = 0; i < TC_MAX_ROWS; i++) {
+            mbar_init(bar + TcBars::dfull + 8 * i, 1);
+            mbar_init(bar + TcBars::dempty + 8 * i, pairs ? 2 : 1);
+        }
+        for (int i = 0; i < TC_MAX_STATS; i++) {
+            mbar_init(bar + TcBars::efull + 8 * i, 1);
+            mbar_init(bar + TcBars::eempty + 8 * i, TC_EPI_WARPS);
+        }
+        mbar_init(bar + TcBars::fin, 2);
         for (int i = 0; i < 4; i++) {
-            mbar_init(ifull0 + 8 * i, 1);
-            mbar_init(iempty0 + 8 * i, 2 + TC_EPI_WARPS);  // MMA issuers + epilogue warps
+            mbar_init(bar + TcBars::ifull + 8 * i, 1);
+            mbar_init(bar + TcBars::iempty + 8 * i, (pairs ? 3 : 2) + TC_EPI_WARPS);  // issuers, warp 3, epilogue
         }
         *abort_flag = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     }
-    constexpr uint32_t TMEM_COLS = 512;  // D0, D1, sum at columns 0, 128, 256 (one CTA per SM)
+    constexpr uint32_t TMEM_COLS = 512;  // H0, H1, S0, S1 at columns 0, 128, 256, 384
     if (warp == 1) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(
                          smem_u32(tmem_holder)),
@@ -238,455 +519,432 @@ __global__ void __launch_bounds__(tc_threads(VAR), 1) tc_persistent(const __grid
     const uint32_t tmem = *tmem_holder;
     const long long total = B.total_items;
 
+    if (!VAR && warp < 4) {
+        // registers: 384 threads x 168 at launch = 128 x 88 + 256 x 208
+        asm volatile("setmaxnreg.dec.sync.aligned.u32 88;");
+    }
     if (warp == 0) {
-        // ---------------------------------------------------------- producer + tile queue
-        // Stage buffer b holds the stages of the channels whose running index g
-        // (over the active channels of all items, in order) has parity b; MMA
-        // issuer b consumes them.  uses[b] counts the stages put in buffer b.
-        int uses[2] = {0, 0};
-        long long g = 0;
+        // ---------------------------------------------------------- tile queue, operands
+        int stages = 0;                 // (channel, phase) stages so far; template buffer = stages & 1
+        int slot = 0, turn = 0;         // data slot, times round the ring
         bool ok = true;
         for (long long q = 0; ok; q++) {
-            const int slot = (int)(q & 3);
+            const int is = (int)(q & 3);
             long long item = total;
             if (lane == 0) {
-                bool got = q < 4 || mbar_wait(iempty0 + 8 * slot, (uint32_t)(((q >> 2) - 1) & 1), abort_flag,
-                                              B.err, 1u);
+                const bool got = q < 4 || mbar_wait(bar + TcBars::iempty + 8 * is, (uint32_t)(((q >> 2) - 1) & 1),
+                                                    abort_flag, B.err, 1u);
                 if (got && !*abort_flag)
                     item = (long long)atomicAdd(B.queue, 1ull);
-                ring[slot] = item;
-                mbar_arrive(ifull0 + 8 * slot);
+                ring[is] = item;
+                mbar_arrive(bar + TcBars::ifull + 8 * is);
             }
-            item = __shfl_sync(0xffffffffu, item, 0);  // warp-uniform decision
+            item = __shfl_sync(0xffffffffu, item, 0);
             if (item >= total)
                 break;
             int p, tile, t, c_begin, c_end, part;
-            decode_item<PARTS>(B, item, p, tile, t, c_begin, c_end, part);
+            decode_item(B, item, p, tile, t, c_begin, c_end, part);
             const TcProb &pr = B.prob[p];
             const Problem &P = pr.P;
-            const int nb = pr.nb;
-            const long long I0 = (long long)tile * TC_Q * nb;
-            if (!(I0 < P.k_hi[t] && I0 + (long long)TC_Q * nb > P.k_lo[t]))
+            const long long I0 = (long long)tile * TC_Q * pr.nb;
+            if (!tc_busy(pr, I0, t))
                 continue;
-            const int SC = P.SC, step = P.step, R = pr.R, NW = pr.NW;
-            const uint32_t data_bytes = (uint32_t)TC_CB * R * 16, wbytes = (uint32_t)NW * 128;
-            const uint32_t w_off = (split ? 2u : 1u) * data_bytes;
-            const float *w = P.w + (size_t)t * SC;
-            // one stage: phase phi of channel ch into buffer b
-            auto load_stage = [&](int ch, int phi, int b) -> bool {
-                if (uses[b] >= 1 &&
-                    !mbar_wait_warp(empty0 + 8 * b, (uses[b] - 1) & 1, abort_flag, B.err, 2u))
-                    return false;
-                const long long meta = ((long long)t * SC + ch) * step + phi;
-                const int mu = pr.mu[meta], psi = pr.psi[meta];
-                const int sres = ((mu % TC_Q) + TC_Q) % TC_Q;
-                const long long r0 = (I0 + mu - sres) / TC_Q + pr.row_front;
-                const uint32_t st = smem_u32(smem + (size_t)b * B.stage_bytes);
-                if (lane == 0)
-                    mbar_expect_tx(full0 + 8 * b, (split ? 2u : 1u) * (data_bytes + wbytes));
-                __syncwarp();
-                const int cb = lane & 15, hl = lane >> 4;
-                if (hl == 0 || split) {
-                    const uint16_t *src = (hl ? pr.g_lo : pr.g_hi) +
-                                          ((((long long)ch * step + psi) * TC_CB + cb) * pr.rows_total + r0) * 8;
-                    bulk_g2s(st + hl * data_bytes + cb * (uint32_t)R * 16, src, (uint32_t)R * 16,
-                             full0 + 8 * b);
+            const int SC = P.SC, step = P.step;
+            const uint32_t col_bytes = (uint32_t)pr.R * 16, wbytes = (uint32_t)pr.NW * 128;
+            const size_t row0 = (size_t)t * SC;
+            for (int g0 = c_begin; ok && g0 < c_end; g0 += 32) {
+                // the scalars of 32 channels, one per lane
+                const int cl = min(g0 + lane, c_end - 1);
+                const int mo_l = P.mo[row0 + cl];
+                uint32_t active = __ballot_sync(0xffffffffu, g0 + lane < c_end && P.w[row0 + cl] != 0.0f);
+                for (; ok && active; active &= active - 1) {
+                    const int from = __ffs(active) - 1, ch = g0 + from;
+                    const int mo = __shfl_sync(0xffffffffu, mo_l, from);
+                    for (int phi = 0; ok && phi < step; phi++, stages++) {
+                        const int wb = stages & 1;
+                        int psi;
+                        const int mu = tc_phase(mo + phi, step, psi);
+                        const long long r0 = ((I0 + mu) >> 7) + pr.row_front;  // floor
+                        const uint32_t wbar = bar + TcBars::wfull + 8 * wb;
+                        if (stages >= 2 && !mbar_wait_warp(bar + TcBars::wempty + 8 * wb, ((stages >> 1) - 1) & 1,
+                                                           abort_flag, B.err, 2u)) {
+                            ok = false;
+                            break;
+                        }
+                        if (lane == 0)
+                            mbar_expect_tx(wbar, pairs ? 2u * wbytes : wbytes);
+                        __syncwarp();
+                        if (lane < (pairs ? 2 : 1))
+                            bulk_g2s(w_base + wb * B.w_bytes + lane * wbytes,
+                                     (lane ? pr.w_lo : pr.w_hi) + ((row0 + ch) * step + phi) * pr.NW * 64, wbytes, wbar);
+                        // data: four column blocks of the R rows, both halves, per slot; lane =
+                        // 4 * half + block
+                        const uint16_t *src =
+                            (lane & 4 ? pr.g_lo : pr.g_hi) +
+                            ((((long long)ch * step + psi) * TC_CB + (lane & 3)) * pr.rows_total + r0) * 8;
+                        const long long src_step = 4ll * pr.rows_total * 8;
+#pragma unroll 1
+                        for (int j = 0; j < TC_CB / 4; j++, src += src_step) {
+                            const uint32_t dbar = bar + TcBars::dfull + 8 * slot;
+                            if (turn >= 1 && !mbar_wait_warp(bar + TcBars::dempty + 8 * slot, (turn - 1) & 1,
+                                                             abort_flag, B.err, 2u)) {
+                                ok = false;
+                                break;
+                            }
+                            if (lane == 0)
+                                mbar_expect_tx(dbar, pairs ? 8u * col_bytes : 4u * col_bytes);
+                            __syncwarp();
+                            if (lane < (pairs ? 8 : 4))
+                                bulk_g2s(d_base + slot * B.row_bytes + lane * col_bytes, src, col_bytes, dbar);
+                            if (++slot == n_rows) {
+                                slot = 0;
+                                turn++;
+                            }
+                        }
+                    }
                 }
-                if (lane < (split ? 2 : 1)) {
-                    const uint16_t *src = (lane ? pr.w_lo : pr.w_hi) + meta * NW * 64;
-                    bulk_g2s(st + w_off + lane * wbytes, src, wbytes, full0 + 8 * b);
-                }
-                uses[b]++;
-                return true;
-            };
-            auto next_active = [&](int ch) {
-                while (ch < c_end && w[ch] == 0.0f)
-                    ch++;
-                return ch;
-            };
-            // active channels in order; with step > 1 two consecutive channels
-            // have their phases interleaved, so that both buffers stay fed
-            int ch = next_active(c_begin);
-            while (ok && ch < c_end) {
-                const int ch2 = step > 1 ? next_active(ch + 1) : c_end;
-                const bool pair = ch2 < c_end;
-                const int b = (int)(g & 1);
-                for (int phi = 0; ok && phi < step; phi++) {
-                    ok = load_stage(ch, phi, b);
-                    if (ok && pair)
-                        ok = load_stage(ch2, phi, b ^ 1);
-                }
-                g += pair ? 2 : 1;
-                ch = next_active((pair ? ch2 : ch) + 1);
             }
         }
-        // do not leave with copies in flight
-        if (lane == 0)
-            for (int b = 0; b < 2; b++)
-                if (uses[b] >= 1)
-                    mbar_wait(full0 + 8 * b, (uses[b] - 1) & 1, abort_flag, B.err, 0u);
+        // do not leave with copies in flight: the last use of every buffer
+        if (lane == 0) {
+            for (int u = stages < 2 ? 0 : stages - 2; u < stages; u++)
+                mbar_wait(bar + TcBars::wfull + 8 * (u & 1), (u >> 1) & 1, abort_flag, B.err, 0u);
+            for (int i = 0; i < n_rows; i++) {
+                const int uses = turn + (i < slot ? 1 : 0);
+                if (uses)
+                    mbar_wait(bar + TcBars::dfull + 8 * i, (uses - 1) & 1, abort_flag, B.err, 0u);
+            }
+        }
         __syncwarp();
     } else if (warp == 1 || warp == 2) {
         // ---------------------------------------------------------- MMA issuers
-        // Two issuing threads (one per warp, on two SM sub-partitions): one
-        // thread cannot issue tcgen05.mma fast enough to keep the tensor pipe
-        // busy.  Issuer m takes the active channels of parity m (running index
-        // c over all items), stage buffer m and accumulator m.
-        const int m = warp - 1;
-        if (lane == 0) {
-            int used = 0;  // stages consumed from buffer m
-            long long c = 0;
-            for (long long q = 0;; q++) {
-                const int slot = (int)(q & 3);
-                if (!mbar_wait(ifull0 + 8 * slot, (uint32_t)((q >> 2) & 1), abort_flag, B.err, 32u))
-                    goto mma_done;
-                const long long item = ring[slot];
-                mbar_arrive(iempty0 + 8 * slot);
+        // One thread each; the code of one instruction costs the tensor pipe as much time as
+        // the instruction, so each issuer has its own short loop and moves only the low
+        // words of its descriptors.
+        const bool one = elect_one();
+        if (warp == 1)
+            tc_issue<VAR, false>(B, ring, bar, w_base, d_base, tmem, abort_flag, one);
+        else if (pairs)
+            tc_issue<VAR, true>(B, ring, bar, w_base, d_base, tmem, abort_flag, one);
+        __syncwarp();
+        if (one) {
+            mma_commit(bar + TcBars::fin);
+            mbar_wait(bar + TcBars::fin, 0, abort_flag, B.err, 0u);
+        }
+        __syncwarp();
+    } else if (warp == 3) {
+        // ---------------------------------------------------------- window statistics
+        // Slot e: CH columns of each half of the tile (a column is 128 windows, contiguous
+        // in the statistics of the channel's stream), copied from a 16-byte boundary.
+        {
+            int ec = 0;
+            bool ok = true;
+            for (long long q = 0; ok; q++) {
+                const int is = (int)(q & 3);
+                if (!mbar_wait_warp(bar + TcBars::ifull + 8 * is, (uint32_t)((q >> 2) & 1), abort_flag, B.err, 32u))
+                    break;
+                const long long item = ring[is];
+                __syncwarp();
+                if (lane == 0)
+                    mbar_arrive(bar + TcBars::iempty + 8 * is);
                 if (item >= total)
                     break;
                 int p, tile, t, c_begin, c_end, part;
-                decode_item<PARTS>(B, item, p, tile, t, c_begin, c_end, part);
+                decode_item(B, item, p, tile, t, c_begin, c_end, part);
                 const TcProb &pr = B.prob[p];
                 const Problem &P = pr.P;
-                const int nb = pr.nb;
-                const long long I0 = (long long)tile * TC_Q * nb;
-                if (!(I0 < P.k_hi[t] && I0 + (long long)TC_Q * nb > P.k_lo[t]))
+                const long long I0 = (long long)tile * TC_Q * pr.nb;
+                if (!tc_busy(pr, I0, t))
                     continue;
-                // kind::f16 descriptor: F32 accumulate, BF16 A and B, K-major, N = nb, M = 128
-                const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(nb >> 3) << 17) |
-                                       ((uint32_t)(TC_Q >> 4) << 24);
-                const int SC = P.SC, step = P.step;
-                const uint32_t data_bytes = (uint32_t)TC_CB * pr.R * 16, wbytes = (uint32_t)pr.NW * 128;
-                const uint32_t w_off = (split ? 2u : 1u) * data_bytes;
-                const uint32_t lbo_b = (uint32_t)pr.R * 16;
-                const float *w = P.w + (size_t)t * SC;
-                for (int ch = c_begin; ch < c_end; ch++) {
-                    if (w[ch] == 0.0f)
-                        continue;
-                    if ((c & 1) != m) {  // the other issuer's channel
-                        c++;
-                        continue;
-                    }
-                    const int d = m;  // accumulator m, reused every second channel
-                    if (c >= TC_NACC &&
-                        !mbar_wait(dempty0 + 8 * d, ((c / TC_NACC) - 1) & 1, abort_flag, B.err, 4u))
-                        goto mma_done;
-                    tc_fence_after();
-                    const uint32_t dt = tmem + (uint32_t)(d * TC_NB_MAX);
-                    uint32_t acc = 0;
-                    for (int phi = 0; phi < step; phi++, used++) {
-                        const int s = m;
-                        if (!mbar_wait(full0 + 8 * s, used & 1, abort_flag, B.err, 8u))
-                            goto mma_done;
-                        tc_fence_after();
-                        const long long meta = ((long long)t * SC + ch) * step + phi;
-                        const int mu = pr.mu[meta];
-                        const int sres = ((mu % TC_Q) + TC_Q) % TC_Q;
-                        // per-channel lengths: the taps past the channel's own are zeros, skip them
-                        const int taps = tc_phase_taps(P.L, step, phi, VAR ? P.ntap[(size_t)t * SC + ch] : P.L);
-                        const int k_first = sres & ~15;
-                        const int k_end = tc_k_end(sres, taps);
-                        const uint32_t zhi = smem_u32(smem + (size_t)s * B.stage_bytes);
-                        const uint32_t whi = zhi + w_off;
-                        // Descriptors advance by additions: the start-address field (bits 0-13,
-                        // 16-byte units) of an address below 256 KB never carries into the
-                        // next field.  A: +256 bytes per K step (two 128-byte template blocks);
-                        // B: +2 column blocks per K step inside a 128-wide K block, then the
-                        // next data row (+16 bytes) from column block 0.
-                        uint64_t ah = sdesc(whi + (uint32_t)(k_first >> 3) * 128u, 128, 128);
-                        const uint64_t a_lo = wbytes >> 4, b_lo = data_bytes >> 4;
-                        const uint64_t b0 = sdesc(zhi, lbo_b, 128);
-                        const uint64_t b_step = (2u * lbo_b) >> 4;
-                        int k = k_first;
-                        while (k < k_end) {
-                            const int blk_end = min(k_end, (k & ~(TC_Q - 1)) + TC_Q);
-                            uint64_t bh = b0 + (((uint32_t)((k & (TC_Q - 1)) >> 3) * lbo_b +
-                                                 (uint32_t)(k / TC_Q) * 16u) >> 4);
-                            for (; k < blk_end; k += 16) {
-                                mma_f16(dt, ah, bh, idesc, acc);
-                                acc = 1;
-                                if (split) {
-                                    mma_f16(dt, ah, bh + b_lo, idesc, 1);
-                                    mma_f16(dt, ah + a_lo, bh, idesc, 1);
-                                }
-                                ah += 16;
-                                bh += b_step;
-                            }
+                const int nc = pr.nb / G;
+                const size_t row0 = (size_t)t * P.SC;
+                for (int g0 = c_begin; ok && g0 < c_end; g0 += 32) {
+                    const int cl = min(g0 + lane, c_end - 1);
+                    const int mo_l = P.mo[row0 + cl], n_l = VAR ? P.ntap[row0 + cl] : 0;
+                    uint32_t active = __ballot_sync(0xffffffffu, g0 + lane < c_end && P.w[row0 + cl] != 0.0f);
+                    for (; ok && active; active &= active - 1) {
+                        const int from = __ffs(active) - 1, ch = g0 + from;
+                        int psi;  // phase 0: the moveout's own stream
+                        const int mu = tc_phase(__shfl_sync(0xffffffffu, mo_l, from), P.step, psi);
+                        // lane = G * array + column group
+                        const char *src;
+                        if constexpr (VAR) {
+                            int psi2;  // the windows' ends
+                            const int far = tc_phase(psi + __shfl_sync(0xffffffffu, n_l, from), P.step, psi2);
+                            const long long x = I0 + mu + (lane & G ? far : 0);
+                            const char *base = lane & (2 * G) ? reinterpret_cast<const char *>(P.pre1f)
+                                                        : reinterpret_cast<const char *>(P.pre2q);
+                            src = base + (ch * P.pre_ch + (lane & G ? psi2 : psi) * P.pre_ps +
+                                          (x & ~(long long)kStat.align())) * kStat.elem;
+                        } else {
+                            src = reinterpret_cast<const char *>(P.stat_e) +
+                                  (ch * P.stat_ch + psi * P.stat_ps + ((I0 + mu) & ~(long long)kStat.align())) *
+                                      kStat.elem;
                         }
-                        mma_commit(empty0 + 8 * s);
+                        src += (size_t)(lane & (G - 1)) * nc * TC_Q * kStat.elem;
+                        for (int c0 = 0; c0 < nc; c0 += CH, ec++) {
+                            const int es = ec & ((1 << stat_log2) - 1);
+                            const uint32_t ebar = bar + TcBars::efull + 8 * es;
+                            if ((ec >> stat_log2) >= 1 &&
+                                !mbar_wait_warp(bar + TcBars::eempty + 8 * es, ((ec >> stat_log2) - 1) & 1,
+                                                abort_flag, B.err, 2u)) {
+                                ok = false;
+                                break;
+                            }
+                            const uint32_t bytes = min(CH, nc) * TC_Q * kStat.elem + 16;
+                            if (lane == 0)
+                                mbar_expect_tx(ebar, (uint32_t)(G * kStat.streams) * bytes);
+                            __syncwarp();
+                            if (lane < G * kStat.streams)
+                                bulk_g2s(e_base + es * (uint32_t)B.stat_bytes + lane * kStatPart,
+                                         src + (size_t)c0 * TC_Q * kStat.elem, bytes, ebar);
+                        }
                     }
-                    mma_commit(dfull0 + 8 * d);
-                    c++;
                 }
             }
-        mma_done:
-            mma_commit(fin);
-            mbar_wait(fin, 0, abort_flag, B.err, 0u);
+            for (int i = 0; i < (1 << stat_log2); i++) {  // the last use of every slot
+                const int uses = (ec >> stat_log2) + (i < (ec & ((1 << stat_log2) - 1)) ? 1 : 0);
+                if (uses && lane == 0)
+                    mbar_wait(bar + TcBars::efull + 8 * i, (uses - 1) & 1, abort_flag, B.err, 0u);
+            }
         }
         __syncwarp();
-    } else if (warp >= 4) {
+    } else {
         // ---------------------------------------------------------- epilogue
-        // TC_EPI_WARPS warps: warp w reads TMEM lane quarter w % 4 (rows
-        // 32*(w%4) + lane) and the NC columns [a0, a0 + NC) of the accumulators;
-        // the network sum of its outputs lives in TMEM columns 2*NB + [a0, a0 + NC).
-        constexpr int CH = VAR ? 8 : 16;  // columns per TMEM access and per batch of statistics loads
+        // Warp w reads TMEM lane quarter w % 4 (rows 32*(w%4) + lane) and its half of the
+        // columns; numerators and network sums of its outputs live in registers.
+        if (!VAR)
+            asm volatile("setmaxnreg.inc.sync.aligned.u32 208;");
+        constexpr int NCM = TC_NB_MAX / G;  // columns per thread, at most
         const int quarter = warp & 3;
-        const int cgroup = (warp - 4) >> 2;  // column group of this warp
-        const int m = 32 * quarter + lane;   // accumulator row
-        const int b = TC_Q - 1 - m;          // phase of that row
+        const int cgroup = (warp - 4) >> 2;
+        const int b = TC_Q - 1 - (32 * quarter + lane);  // phase of this thread's row
         const uint32_t lane_base = tmem + ((uint32_t)(32 * quarter) << 16);
-        int c = 0;
+        int c = 0, hc = 0, ec = 0;  // channels, chains and statistics slots used
         for (long long q = 0;; q++) {
-            const int slot = (int)(q & 3);
+            const int is = (int)(q & 3);
             long long item = total;
             if (lane == 0) {
-                if (mbar_wait(ifull0 + 8 * slot, (uint32_t)((q >> 2) & 1), abort_flag, B.err, 64u)) {
-                    item = ring[slot];
-                    mbar_arrive(iempty0 + 8 * slot);
+                if (mbar_wait(bar + TcBars::ifull + 8 * is, (uint32_t)((q >> 2) & 1), abort_flag, B.err, 64u)) {
+                    item = ring[is];
+                    mbar_arrive(bar + TcBars::iempty + 8 * is);
                 }
             }
             item = __shfl_sync(0xffffffffu, item, 0);
             if (item >= total)
                 break;
             int p, tile, t, c_begin, c_end, part;
-            decode_item<PARTS>(B, item, p, tile, t, c_begin, c_end, part);
+            decode_item(B, item, p, tile, t, c_begin, c_end, part);
             const TcProb &pr = B.prob[p];
-            // per-item fields, once, into registers
+            if (tc_skipped(pr))
+                continue;
             const int nb = pr.nb;
-            const int NC = nb / (TC_EPI_WARPS / 4);  // columns of this thread (multiple of CH)
+            const int NC = nb / G;  // columns of this thread
             const int a0 = cgroup * NC;
-            const uint32_t s_cols = lane_base + (uint32_t)(TC_NACC * TC_NB_MAX + a0);
-            const int SC = pr.P.SC, step = pr.P.step, n_corr = pr.P.n_corr, N = pr.P.N;
-            const bool full = NORM >= 0 ? NORM == 1 : pr.P.normalize != 0;
-            const bool nsum = pr.P.network_sum != 0;
-            const float *__restrict__ stat_e = pr.P.stat_e;
-            const float *__restrict__ sstp = pr.P.sst;
-            const float *__restrict__ tsump = pr.P.tsum;
-            float *outp = pr.P.out;
+            const int SC = pr.P.SC, step = pr.P.step, n_corr = pr.P.n_corr;
             const long long I0 = (long long)tile * TC_Q * nb;
             const int klo = pr.P.k_lo[t], khi = pr.P.k_hi[t];
-            const bool busy = I0 < khi && I0 + (long long)TC_Q * nb > klo;
+            const bool busy = tc_holds(klo, khi, I0, nb);
             // valid lag blocks of this thread: klo <= I0 + Q*a + b < khi
             const long long kb = I0 + b;
             const int a_lo = (int)max(0LL, (klo - kb + TC_Q - 1) / TC_Q) - a0;
             const int a_hi = (int)min((long long)nb, (khi - kb + TC_Q - 1) / TC_Q) - a0;
-            const bool any = busy && a_hi > a_lo;
-            // the whole warp's outputs of this item are valid (the usual case)
-            const bool interior = __all_sync(0xffffffffu, a_lo <= 0 && a_hi >= NC);
-            const long long qs = TC_Q;
-            const int qs32 = TC_Q * step;
-            const float *w = pr.P.w + (size_t)t * SC;
-            const int *mo = pr.P.mo + (size_t)t * SC;
-            bool first = true;
-            for (int ch = c_begin; busy && ch < c_end; ch++) {
-                const float wc = w[ch];
-                if (wc == 0.0f)
-                    continue;
-                const int d = c % TC_NACC;
-                const size_t row = (size_t)t * SC + ch;
-                const float sst = sstp[row];
-                const float ts = full ? tsump[row] : 0.0f;
-                const long long u0 = (kb + (long long)TC_Q * a0) * step + mo[ch];
-                // short: window energies; full: (centred energy, mean) pairs
-                const size_t meta = row * step;
-                const long long so = VAR ? 0
-                                         : ch * pr.P.stat_ch + pr.psi[meta] * pr.P.stat_ps +
-                                               min(pr.psi[meta], pr.P.stat_rem) + kb + (long long)TC_Q * a0 + pr.mu[meta];
-                const float *__restrict__ se = stat_e + so;
-                const float2 *__restrict__ sem = reinterpret_cast<const float2 *>(stat_e) + so;
-                float *oc = outp + ((size_t)t * n_corr + kb + (long long)TC_Q * a0) * SC + ch;
-                // statistics: all loads of a chunk issued together (indices clamped into the
-                // valid range) before any use; the first chunk before waiting for the accumulator
-                float e[CH], mm[CH];
-                auto load_chunk = [&](int c0) {
+            const long long k0 = kb + (long long)TC_Q * a0;  // this thread's first output
+            float sum[NCM];
 #pragma unroll
-                    for (int i = 0; i < CH; i++) {
-                        const int ac = min(max(c0 + i, a_lo), a_hi - 1);
-                        if (full) {
-                            const float2 em = any ? __ldg(sem + ac * qs) : make_float2(0.0f, 0.0f);
-                            e[i] = em.x;
-                            mm[i] = em.y;
-                        } else {
-                            e[i] = any ? __ldg(se + ac * qs) : 0.0f;
-                            mm[i] = 0.0f;
-                        }
-                    }
-                };
-                if constexpr (!VAR)
-                    load_chunk(0);
-                // per-channel lengths: the channel's own length and Fisher-z weight, its
-                // running sums (d^2 in fixed point, and d for full) at the first window of
-                // the thread
-                [[maybe_unused]] int ntap = 0;
-                [[maybe_unused]] float zw = 0.0f, nf = 0.0f, inv_n = 0.0f, unit = 0.0f;
-                [[maybe_unused]] const long long *pf = nullptr;
-                [[maybe_unused]] const float2 *pg = nullptr;
-                if constexpr (VAR) {
-                    ntap = pr.P.ntap[row];
-                    zw = pr.P.zweight[row];
-                    unit = pr.P.unit2[ch];
-                    pf = pr.P.pre2q + (size_t)ch * (N + 1) + u0;
-                    pg = full ? pr.P.pre1f + (size_t)ch * (N + 1) + u0 : nullptr;
-                    nf = (float)ntap;
-                    inv_n = 1.0f / nf;
-                }
-                if (!mbar_wait_warp(dfull0 + 8 * d, (c / TC_NACC) & 1, abort_flag, B.err, 16u))
-                    goto epilogue_done;
-                tc_fence_after();
-                const uint32_t dcols = lane_base + (uint32_t)(d * TC_NB_MAX + a0);
+            for (int i = 0; i < NCM; i++)
+                sum[i] = 0.0f;
+            const size_t row0 = (size_t)t * SC;
+            const int n_chains = (step * (TC_CB / 2) + pr.chain_cols - 1) / pr.chain_cols;
+            const int n_sums = n_chains + (pairs ? 1 : 0);
+            for (int g0 = c_begin; busy && g0 < c_end; g0 += 32) {
+                // the scalars of 32 channels, one per lane
+                const int cl = min(g0 + lane, c_end - 1);
+                const float w_l = g0 + lane < c_end ? pr.P.w[row0 + cl] : 0.0f, sst_l = pr.P.sst[row0 + cl];
+                const int mo_l = pr.P.mo[row0 + cl];
+                // 2^unit: the product of the operands' scales
+                const int unit_l = pr.t_exp ? pr.t_exp[row0 + cl] + pr.d_exp[cl] - 2 * kTopExp : 0;
+                const int n_l = VAR ? pr.P.ntap[row0 + cl] : 0;
+                const float z_l = VAR ? pr.P.zweight[row0 + cl] : 0.0f, u2_l = VAR ? pr.P.unit2[cl] : 0.0f;
+                const float ts_l = FULL ? pr.P.tsum[row0 + cl] * exp2_int(-unit_l) : 0.0f;
+                uint32_t active = __ballot_sync(0xffffffffu, w_l != 0.0f);
 #pragma unroll 1
-                for (int c0 = 0; c0 < NC; c0 += CH) {
-                    if constexpr (!VAR) {
-                        if (c0 > 0)
-                            load_chunk(c0);
-                    }
-                    float x[CH], sv[CH];
-                    tmem_ldc<CH>(dcols + c0, x);
-                    if (nsum && !first)
-                        tmem_ldc<CH>(s_cols + c0, sv);
-                    tmem_wait_ld();
-                    if (c0 + CH >= NC) {
+                for (; active; active &= active - 1) {
+                    const int from = __ffs(active) - 1, ch = g0 + from;
+                    const float wc = __shfl_sync(0xffffffffu, w_l, from), sst = __shfl_sync(0xffffffffu, sst_l, from);
+                    const float unit = exp2_int(__shfl_sync(0xffffffffu, unit_l, from));
+                    const float ts = FULL ? __shfl_sync(0xffffffffu, ts_l, from) : 0.0f;
+                    const int mo = __shfl_sync(0xffffffffu, mo_l, from);
+                    float num[NCM];
+#pragma unroll
+                    for (int i = 0; i < NCM; i++)
+                        num[i] = 0.0f;
+                    // numerators: the chains' sums, then S (FP32: times 2^-11)
+#pragma unroll 1
+                    for (int j = 0; j < n_sums; j++) {
+                        const bool last = j == n_chains;
+                        const int u = last ? c : hc;
+                        if (!mbar_wait_all(bar + (last ? TcBars::sfull : TcBars::hfull) + 8 * (u & 1), (u >> 1) & 1,
+                                           abort_flag, B.err, 16u))
+                            goto epilogue_done;
+                        tc_fence_after();
+                        const uint32_t h = lane_base + (last ? 256u : 0u) + 128u * (u & 1) + a0;
+                        const float f = last ? B.lo_unit : 1.0f;  // powers of two: exact products
+                        constexpr int LD = VAR ? 16 : 32;  // columns per load; a small tile reads too many
+#pragma unroll
+                        for (int c0 = 0; c0 < NCM; c0 += LD) {
+                            if (c0 < NC) {
+                                float x[LD];
+                                if constexpr (VAR)
+                                    tmem_ld16(h + c0, x);
+                                else
+                                    tmem_ld32(h + c0, x);
+                                tmem_wait_ld();
+#pragma unroll
+                                for (int i = 0; i < LD; i++)
+                                    num[c0 + i] = fmaf(x[i], f, num[c0 + i]);
+                            }
+                        }
                         tc_fence_before();
                         __syncwarp();
                         if (lane == 0)
-                            mbar_arrive(dempty0 + 8 * d);
+                            mbar_arrive(bar + (last ? TcBars::sempty : TcBars::hempty) + 8 * (u & 1));
+                        if (!last)
+                            hc++;
                     }
+                    const float wu = wc * unit;  // a power of two: cc * wc rounds the same
+                    float *oc = pr.P.out + ((size_t)t * n_corr + k0) * SC + ch;
+                    int psi;
+                    const int mu = tc_phase(mo, step, psi);
+                    const int head = (int)((I0 + mu) & kStat.align());  // past the 16-byte boundary
                     if constexpr (VAR) {
-                        // window sums of the channel's own length from the running sums,
-                        // the 'precise' threshold on the square root, and
-                        // atanh(cc - 10 eps) * z into the network sum
-                        // CHECK: some output of the warp lies outside the valid lags (clamped
-                        // indices, masked sums); otherwise every one is valid
-                        auto var_chunk = [&](auto check) {
-                            constexpr bool CHECK = decltype(check)::value;
-                            auto var_value = [&](int i, float num, float ssd) {
-                                const int a = c0 + i;
-                                // the threshold on sqrt(sst * ssd), as p * rsqrt(p); p = 0 gives
-                                // NaN there, and p below the normal range (flushed) cannot pass it
-                                const float p = sst * ssd, r = rsqrt_ftz(p);
-                                const float cc = p * r > kThreshold ? num * r : 0.0f;
-                                const float prev = first ? 0.0f : sv[i];
-                                const float z = fmaf(fisher_atanh(cc - 10.0f * FLT_EPSILON), zw, prev);
-                                sv[i] = (!CHECK || (a >= a_lo && a < a_hi)) ? z : prev;
-                            };
-                            // element offsets of the windows (32-bit: at most NB * Q * step)
-                            auto off = [&](int i) {
-                                return (CHECK ? min(max(c0 + i, a_lo), a_hi - 1) : c0 + i) * qs32;
-                            };
-                            const bool ld = !CHECK || any;
-                            const float2 z2 = make_float2(0.0f, 0.0f);
-                            if (!full) {  // fixed-point running sums: an exact difference
-                                const long long *__restrict__ pf_hi = pf + ntap;
+                        // window sums of the channel's own length from its running sums, the
+                        // threshold on the square root, atanh(cc - 10 eps) * z
+                        const int ntap = __shfl_sync(0xffffffffu, n_l, from);
+                        const float zw = __shfl_sync(0xffffffffu, z_l, from), u2 = __shfl_sync(0xffffffffu, u2_l, from);
+                        const float nf = (float)ntap, inv_n = 1.0f / nf;
+                        int psi2;
+                        const int far = tc_phase(psi + ntap, step, psi2);
+                        const int head2 = (int)((I0 + mu + far) & kStat.align());
 #pragma unroll
-                                for (int h = 0; h < CH; h += 4) {  // loads of 4 values, then their use
-                                    long long lo[4], hi[4];
+                        for (int c0 = 0; c0 < NCM; c0 += CH) {
+                            if (c0 < NC) {
+                                const int es = ec & ((1 << stat_log2) - 1);
+                                if (!mbar_wait_all(bar + TcBars::efull + 8 * es, (ec >> stat_log2) & 1, abort_flag,
+                                                   B.err, 16u))
+                                    goto epilogue_done;
+                                const uint8_t *slot = smem + (e_base - w_base) + es * (uint32_t)B.stat_bytes +
+                                                      cgroup * kStatPart;
+                                const uint8_t *at = slot + (head + b) * 8, *at2 = slot + G * kStatPart + (head2 + b) * 8;
+                                long long lo[CH], hi[CH];
+                                float2 lo1[CH], hi1[CH];
 #pragma unroll
-                                    for (int j = 0; j < 4; j++) {
-                                        const int o = off(h + j);
-                                        lo[j] = ld ? pf[o] : 0;
-                                        hi[j] = ld ? pf_hi[o] : 0;
-                                    }
-#pragma unroll
-                                    for (int j = 0; j < 4; j++)
-                                        var_value(h + j, x[h + j], window_energy(lo[j], hi[j], unit));
-                                }
-                            } else {  // centred windows: double-float FP32 arithmetic
-#pragma unroll
-                                for (int h = 0; h < CH; h += 2) {
-                                    long long lo2[2], hi2[2];
-                                    float2 lo1[2], hi1[2];
-#pragma unroll
-                                    for (int j = 0; j < 2; j++) {
-                                        const int o = off(h + j);
-                                        lo2[j] = ld ? pf[o] : 0;
-                                        hi2[j] = ld ? pf[o + ntap] : 0;
-                                        lo1[j] = ld ? pg[o] : z2;
-                                        hi1[j] = ld ? pg[o + ntap] : z2;
-                                    }
-#pragma unroll
-                                    for (int j = 0; j < 2; j++) {
-                                        float v, mean;
-                                        window_centred(lo2[j], hi2[j], unit, lo1[j], hi1[j], nf, inv_n, v,
-                                                       mean);
-                                        var_value(h + j, fmaf(-mean, ts, x[h + j]), v);
+                                for (int j = 0; j < CH; j++) {
+                                    lo[j] = *reinterpret_cast<const long long *>(at + j * TC_Q * 8);
+                                    hi[j] = *reinterpret_cast<const long long *>(at2 + j * TC_Q * 8);
+                                    if constexpr (FULL) {
+                                        lo1[j] = *reinterpret_cast<const float2 *>(at + 2 * G * kStatPart + j * TC_Q * 8);
+                                        hi1[j] = *reinterpret_cast<const float2 *>(at2 + 2 * G * kStatPart + j * TC_Q * 8);
                                     }
                                 }
-                            }
-                        };
-                        if (interior)
-                            var_chunk(std::false_type{});
-                        else
-                            var_chunk(std::true_type{});
-                    } else if (nsum && interior) {
-                        // every output of the warp is valid: no per-value range test
-                        if (first) {
+                                fence_reads_before_copy();
+                                __syncwarp();
+                                if (lane == 0)
+                                    mbar_arrive(bar + TcBars::eempty + 8 * es);
+                                ec++;
+                                // (outside the valid lags the sums are anything, and are not used)
+                                float y[CH];
 #pragma unroll
-                            for (int i = 0; i < CH; i++) {
-                                const float num = full ? fmaf(-mm[i], ts, x[i]) : x[i];
-                                const float den = sst * e[i];
-                                const float cc = den > kThreshold ? num * rsqrtf(den) : 0.0f;
-                                sv[i] = fmaf(cc, wc, 0.0f);
-                            }
-                        } else {
+                                for (int j = 0; j < CH; j++) {
+                                    float ssd, num1 = num[c0 + j];
+                                    if constexpr (FULL) {
+                                        float mean;
+                                        window_centred(lo[j], hi[j], u2, lo1[j], hi1[j], nf, inv_n, ssd, mean);
+                                        num1 = fmaf(-mean, ts, num1);
+                                    } else {
+                                        ssd = window_energy(lo[j], hi[j], u2);
+                                    }
+                                    const float pe = sst * ssd, r = rsqrt_ftz(pe);
+                                    y[j] = (pe * r > kThreshold ? num1 * (r * unit) : 0.0f) - 10.0f * FLT_EPSILON;
+                                }
+                                fisher_atanh<CH>(y);
 #pragma unroll
-                            for (int i = 0; i < CH; i++) {
-                                const float num = full ? fmaf(-mm[i], ts, x[i]) : x[i];
-                                const float den = sst * e[i];
-                                const float cc = den > kThreshold ? num * rsqrtf(den) : 0.0f;
-                                sv[i] = fmaf(cc, wc, sv[i]);
+                                for (int j = 0; j < CH; j++)
+                                    sum[c0 + j] = fmaf(y[j], zw, sum[c0 + j]);
                             }
                         }
                     } else {
 #pragma unroll
-                        for (int i = 0; i < CH; i++) {
-                            const int a = c0 + i;
-                            const float num = full ? fmaf(-mm[i], ts, x[i]) : x[i];
-                            const float den = sst * e[i];
-                            float cc = den > kThreshold ? num * rsqrtf(den) : 0.0f;
-                            if (!(a >= a_lo && a < a_hi))
-                                cc = 0.0f;
-                            if (nsum)
-                                sv[i] = fmaf(cc, wc, first ? 0.0f : sv[i]);
-                            else if (a >= a_lo && a < a_hi)
-                                oc[(size_t)a * TC_Q * SC] = cc;
+                        for (int c0 = 0; c0 < NCM; c0 += CH) {
+                            if (c0 < NC) {
+                                const int es = ec & ((1 << stat_log2) - 1);
+                                if (!mbar_wait_all(bar + TcBars::efull + 8 * es, (ec >> stat_log2) & 1, abort_flag,
+                                                   B.err, 16u))
+                                    goto epilogue_done;
+                                const uint8_t *at = smem + (e_base - w_base) + es * (uint32_t)B.stat_bytes +
+                                                    cgroup * kStatPart + (head + b) * (FULL ? 8 : 4);
+                                constexpr int CB = 16;  // values in flight
+#pragma unroll
+                                for (int h0 = 0; h0 < CH; h0 += CB) {
+                                    if (c0 + h0 < NC) {
+                                        float e[CB], mm[CB];
+#pragma unroll
+                                        for (int i = 0; i < CB; i++) {
+                                            if constexpr (FULL) {
+                                                const float2 v = *reinterpret_cast<const float2 *>(at + (h0 + i) * TC_Q * 8);
+                                                e[i] = v.x;
+                                                mm[i] = v.y;
+                                            } else {
+                                                e[i] = *reinterpret_cast<const float *>(at + (h0 + i) * TC_Q * 4);
+                                            }
+                                        }
+                                        if (h0 + CB >= CH || c0 + h0 + CB >= NC) {  // the slot is read
+                                            fence_reads_before_copy();
+                                            __syncwarp();
+                                            if (lane == 0)
+                                                mbar_arrive(bar + TcBars::eempty + 8 * es);
+                                        }
+#pragma unroll
+                                        for (int i = 0; i < CB; i++) {
+                                            const int a = c0 + h0 + i;
+                                            const float num1 = FULL ? fmaf(-mm[i], ts, num[a]) : num[a];
+                                            const float den = sst * e[i];
+                                            // den is normal where it passes; outside the valid lags the
+                                            // statistics, and with them cc, are anything
+                                            const float cc = den > kThreshold ? num1 * rsqrt_ftz(den) : 0.0f;
+                                            if (NSUM)
+                                                sum[a] = fmaf(cc, wu, sum[a]);
+                                            else if (a >= a_lo && a < a_hi)
+                                                oc[(size_t)a * TC_Q * SC] = cc * unit;
+                                        }
+                                    }
+                                }
+                                ec++;
+                            }
                         }
                     }
-                    if (nsum)
-                        tmem_stc<CH>(s_cols + c0, sv);
+                    c++;
                 }
-                if (nsum)
-                    tmem_wait_st();
-                first = false;
-                c++;
             }
-            if (nsum) {
+            if (NSUM) {
                 // a channel part writes its partial sums to its own plane of part_out
-                float *o = (PARTS ? pr.part_out + (size_t)part * pr.P.T * n_corr : outp) +
-                           (size_t)t * n_corr + kb + (long long)TC_Q * a0;
-                const long long lim = n_corr - kb - (long long)TC_Q * a0;
-#pragma unroll 1
-                for (int c0 = 0; c0 < NC; c0 += CH) {
-                    float sv[CH];
-                    if (!first) {
-                        tmem_ldc<CH>(s_cols + c0, sv);
-                        tmem_wait_ld();
-                    }
-                    if constexpr (VAR && !PARTS) {  // the Fisher-z transform of every output, fused
-                        const float zn = pr.P.vp_norm[t], zb = pr.P.vp_bias[t], zs = pr.P.vp_scale[t];
+                const bool parts = pr.parts > 1;
+                float *o = (parts ? pr.part_out + (size_t)part * pr.P.T * n_corr : pr.P.out) +
+                           (size_t)t * n_corr + k0;
+                const long long lim = n_corr - k0;
+                float zn = 1.0f, zb = 0.0f, zs = 1.0f;
+                if (VAR && !parts) {
+                    zn = pr.P.vp_norm[t];
+                    zb = pr.P.vp_bias[t];
+                    zs = pr.P.vp_scale[t];
+                }
 #pragma unroll
-                        for (int i = 0; i < CH; i++) {
-                            const int a = c0 + i;
-                            const float x = (!first && a >= a_lo && a < a_hi) ? sv[i] : 0.0f;
-                            if ((long long)a * TC_Q < lim)
-                                o[(size_t)a * TC_Q] = (tanhf(x / zn) + zb) * zs;
-                        }
-                    } else {
-#pragma unroll
-                        for (int i = 0; i < CH; i++) {
-                            const int a = c0 + i;
-                            if ((long long)a * TC_Q < lim)
-                                o[(size_t)a * TC_Q] = (!first && a >= a_lo && a < a_hi) ? sv[i] : 0.0f;
-                        }
+                for (int a = 0; a < NCM; a++) {
+                    if (a < NC && (long long)a * TC_Q < lim) {
+                        float v = busy && a >= a_lo && a < a_hi ? sum[a] : 0.0f;
+                        if (VAR && !parts)  // the Fisher-z transform of every output
+                            v = (tanhf(v / zn) + zb) * zs;
+                        o[(size_t)a * TC_Q] = v;
                     }
                 }
             }
@@ -700,6 +958,26 @@ __global__ void __launch_bounds__(tc_threads(VAR), 1) tc_persistent(const __grid
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(TMEM_COLS)
                      : "memory");
     }
+}
+
+// ------------------------------------------------------------------ self-tests
+// every lane of every warp takes part (the tail reads a dummy value)
+__global__ void fisher_atanh_kernel(const float *__restrict__ y, float *__restrict__ out, long long n)
+{
+    const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    float r[1] = {i < n ? y[i] : 0.0f};
+    fisher_atanh<1>(r);
+    if (i < n)
+        out[i] = r[0];
+}
+
+int launch_fisher_atanh(const float *y, float *out, long long n, cudaStream_t s)
+{
+    if (n <= 0)
+        return FMF_OK;
+    fisher_atanh_kernel<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(y, out, n);
+    count_launch();
+    return check_launch("fisher_atanh_kernel");
 }
 
 // Self-test of the bounded waits: one CTA waits on an mbarrier that nothing
@@ -728,58 +1006,18 @@ int launch_wait_selftest(unsigned *err, unsigned ms, cudaStream_t s)
 }
 
 // ------------------------------------------------------------------ host side
-constexpr size_t TC_BAR_BYTES = 256;
-
-// Largest tile (lag blocks per CTA tile) whose two pipeline stages fit in shared memory.
-int tc_choose_nb(int L, int step, int split, int forced)
+// Largest tile (lag blocks per CTA tile) whose channel operands, twice over, fit in
+// shared memory; 0: none.
+int tc_choose_nb(int L, int step, int pairs, int forced)
 {
     const int cands[3] = {128, 64, 32};
     for (int i = 0; i < 3; i++) {
         if (forced && cands[i] != forced)
             continue;
-        if (2 * tc_shape(L, step, split, cands[i]).stage + TC_BAR_BYTES <= 227 * 1024)
+        if (2 * tc_shape(L, step, pairs, cands[i]).stage + 256 <= 227 * 1024)
             return cands[i];
     }
     return 0;
-}
-
-// Preprocessing of one search for the tensor-core kernel: bf16 hi/lo data
-// streams and template blocks, in scratch owned by `ws`.  Fills `out`.
-int tc_prepare(const Problem &P, const float *data_for_tc, int split, int nb, int tg, Scratch &ws,
-               cudaStream_t s, TcProb *out)
-{
-    int rc;
-    const int step = P.step, L = P.L;
-    TcProb pr;
-    const TcShape g = tc_fill_shape(P, split, nb, tg, &pr);
-    const size_t g_elems = (size_t)P.SC * step * TC_CB * pr.rows_total * 8;
-    const size_t w_elems = (size_t)P.T * P.SC * step * g.NW * 64;
-    const size_t n_meta = (size_t)P.T * P.SC * step;
-    uint16_t *g_hi = nullptr, *g_lo = nullptr, *w_hi = nullptr, *w_lo = nullptr;
-    int *mu = nullptr, *psi = nullptr;
-    if ((rc = ws.get(&g_hi, g_elems, "bf16 data streams")) ||
-        (split && (rc = ws.get(&g_lo, g_elems, "bf16 data streams (lo)"))) ||
-        (rc = ws.get(&w_hi, w_elems, "bf16 template blocks")) ||
-        (split && (rc = ws.get(&w_lo, w_elems, "bf16 template blocks (lo)"))) ||
-        (rc = ws.get(&mu, n_meta, "phase moveouts")) || (rc = ws.get(&psi, n_meta, "phase streams")))
-        return rc;
-    const long long n = (long long)P.SC * step * TC_CB * pr.rows_total;
-    tc_data_kernel<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(data_for_tc, P.N, P.SC, step, pr.rows_total,
-                                                               pr.row_front, g_hi, g_lo);
-    const long long m = (long long)P.T * P.SC * step * g.NW * 8;
-    tc_template_kernel<<<(unsigned)((m + 255) / 256), 256, 0, s>>>(P.tpl, P.mo, P.T, P.SC, L, step, g.NW,
-                                                                   w_hi, w_lo, mu, psi);
-    count_launch(2);
-    if ((rc = check_launch("tensor-core preprocessing")))
-        return rc;
-    pr.g_hi = g_hi;
-    pr.g_lo = g_lo;
-    pr.w_hi = w_hi;
-    pr.w_lo = w_lo;
-    pr.mu = mu;
-    pr.psi = psi;
-    *out = pr;
-    return FMF_OK;
 }
 
 static int n_sms()
@@ -837,6 +1075,34 @@ static int choose_parts(long long items, int SC)
     return best;
 }
 
+// Shared memory of one launch: two template buffers, two statistics slots (32 KB
+// each: half a channel of a full tile) and as many data slots as fit (a channel
+// has 4); long templates give up a statistics slot first.
+static size_t tc_layout(TcBatch *B, bool var, bool full)
+{
+    int nb = 0;
+    for (int i = 0; i < B->n_probs; i++)
+        nb = max(nb, B->prob[i].nb);
+    const StatSlot slot(var, full);
+    const size_t fixed = 2 * (size_t)B->w_bytes + TcBars::bytes;
+    B->stat_bytes = (int)slot.bytes();
+    if (slot.streams == 1 && nb / 2 < slot.columns)  // (the second group lies part() bytes on)
+        B->stat_bytes = (int)(slot.part() + nb / 2 * TC_Q * slot.elem + 16);
+    for (int least = 3; least >= 1; least--)
+        for (B->stat_log2 = 1; B->stat_log2 >= 0; B->stat_log2--) {
+            const size_t stats = (size_t)B->stat_bytes << B->stat_log2;
+            if (fixed + stats > (size_t)kMaxDynamicSmem)
+                continue;
+            const size_t rows = (kMaxDynamicSmem - fixed - stats) / B->row_bytes;
+            B->n_rows = rows < (size_t)TC_MAX_ROWS ? (int)rows : TC_MAX_ROWS;
+            if (B->n_rows >= least) {
+                const size_t smem = fixed + stats + (size_t)B->n_rows * B->row_bytes;
+                return smem < 120 * 1024 ? 120 * 1024 : smem;  // one CTA per SM: its TMEM is all there is
+            }
+        }
+    return 0;
+}
+
 // Channel parts of a prepared search run by itself (tc_run).  A lone search with
 // fewer (tile, template) items than SMs runs each item as k channel parts
 // (network sum only; with per-channel lengths the parts add raw Fisher-z sums
@@ -859,10 +1125,8 @@ int tc_run(const TcProb *probs, int n, int form, int parts, unsigned long long *
         return set_error(FMF_ERR_ARG, "a persistent launch takes 1..%d searches", TC_MAX_PROBS);
     static thread_local TcBatch Bh;  // large; built on the host for the launch only
     TcBatch &B = Bh;
-    const int split = form != TC_FORM_BF16;  // operand pairs
-    long long items = 0;
-    size_t stage = 0;
     const Problem &P0 = probs[0].P;
+    const bool var = P0.ntap != nullptr, full = P0.normalize != 0, nsum = P0.network_sum != 0;
     if (n > 1)
         parts = 1;
     else if (parts == 0)
@@ -874,83 +1138,55 @@ int tc_run(const TcProb *probs, int n, int form, int parts, unsigned long long *
         if (rc)
             return rc;
     }
+    B.split = form != TC_FORM_BF16;  // operand pairs
+    B.mma_types = form == TC_FORM_FP32 ? 0u : (1u << 7) | (1u << 10);
+    B.lo_unit = form == TC_FORM_FP32 ? 1.0f / kLoScale : 1.0f;
+    B.w_bytes = B.row_bytes = 0;
+    const int halves = B.split ? 2 : 1;
+    long long items = 0;
     for (int i = 0; i < n; i++) {
+        const Problem &P = probs[i].P;
+        if ((P.ntap != nullptr) != var || (P.normalize != 0) != full || (P.network_sum != 0) != nsum)
+            return set_error(FMF_ERR_ARG, "a persistent launch mixes kinds of search");
         B.prob[i] = probs[i];
         B.prob[i].item_begin = items;
         B.prob[i].parts = parts;
         B.prob[i].part_out = part_out;
-        items += (long long)probs[i].n_tiles * probs[i].P.T * parts;
-        const size_t st = tc_shape(probs[i].P.L, probs[i].P.step, split, probs[i].nb).stage;
-        stage = st > stage ? st : stage;
+        items += (long long)probs[i].n_tiles * P.T * parts;
+        B.w_bytes = max(B.w_bytes, halves * probs[i].NW * 128);
+        B.row_bytes = max(B.row_bytes, halves * 4 * probs[i].R * 16);
     }
     B.n_probs = n;
-    B.split = split;
-    B.stage_bytes = (int)stage;
-    B.w_bytes = B.row_bytes = 0;
-    for (int i = 0; i < n; i++) {
-        B.w_bytes = max(B.w_bytes, 2 * probs[i].NW * 128);
-        B.row_bytes = max(B.row_bytes, 8 * probs[i].R * 16);
-    }
     B.total_items = items;
     B.queue = queue;
     B.err = err;
-    // more than half of the SM's shared memory: one CTA per SM, so that the
-    // CTA's 512-column TMEM allocation never waits for another CTA
-    size_t smem = 2 * stage + TC_BAR_BYTES;
-    if (smem < 120 * 1024)
-        smem = 120 * 1024;
-    if (smem > 227 * 1024)
-        return set_error(FMF_ERR_SMEM, "tensor-core stages need %zu bytes of shared memory", smem);
+    const size_t smem = tc_layout(&B, var, full);
+    if (smem == 0)
+        return set_error(FMF_ERR_SMEM, "tensor-core buffers do not fit shared memory");
     cudaError_t e = cudaMemsetAsync(queue, 0, sizeof(unsigned long long), s);
     if (e != cudaSuccess)
         return set_error(FMF_ERR_CUDA, "clearing the tile queue: %s", cudaGetErrorString(e));
-    const unsigned grid = (unsigned)(items < n_sms() ? (items > 0 ? items : 1) : n_sms());
-    int n_var = 0;
-    for (int i = 0; i < n; i++)
-        n_var += probs[i].P.ntap != nullptr;
-    if (n_var != 0 && n_var != n)
-        return set_error(FMF_ERR_ARG, "a persistent launch mixes per-channel and fixed template lengths");
-    int n_full = 0;
-    for (int i = 0; i < n; i++)
-        n_full += probs[i].P.normalize != 0;
-    const int norm = n_full == 0 ? 0 : (n_full == n ? 1 : -1);
     void (*kern)(const TcBatch);
-    if (form == TC_FORM_FP32) {
-        if (norm < 0)
-            return set_error(FMF_ERR_ARG, "a persistent FP32 launch mixes normalisations");
-        kern = nullptr;
-        smem = tc32_layout(&B, n_var != 0, norm == 1);
-        if (smem == 0)
-            return set_error(FMF_ERR_SMEM, "FP32 tensor-core buffers do not fit shared memory");
-    } else if (n_var && norm >= 0)  // per-channel lengths: always one search, one normalisation
-        kern = parts > 1 ? (norm == 0 ? tc_persistent<true, true, 0> : tc_persistent<true, true, 1>)
-                         : (norm == 0 ? tc_persistent<true, false, 0> : tc_persistent<true, false, 1>);
-    else if (n_var)
-        kern = parts > 1 ? tc_persistent<true, true, -1> : tc_persistent<true, false, -1>;
-    else if (parts > 1)
-        kern = norm == 0 ? tc_persistent<false, true, 0>
-                         : (norm == 1 ? tc_persistent<false, true, 1> : tc_persistent<false, true, -1>);
+    if (var)
+        kern = full ? tc_persistent<true, true, true> : tc_persistent<true, false, true>;
+    else if (nsum)
+        kern = full ? tc_persistent<false, true, true> : tc_persistent<false, false, true>;
     else
-        kern = norm == 0 ? tc_persistent<false, false, 0>
-                         : (norm == 1 ? tc_persistent<false, false, 1> : tc_persistent<false, false, -1>);
+        kern = full ? tc_persistent<false, true, false> : tc_persistent<false, false, false>;
+    e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxDynamicSmem);
+    if (e != cudaSuccess)
+        return set_error(FMF_ERR_CUDA, "tc_persistent shared memory (%zu bytes): %s", smem,
+                         cudaGetErrorString(e));
+    const unsigned grid = (unsigned)(items < n_sms() ? (items > 0 ? items : 1) : n_sms());
+    kern<<<grid, tc_threads(var), smem, s>>>(B);
+    count_launch();
     note_bounded_waits();
-    int rc;
-    if (form == TC_FORM_FP32) {
-        rc = tc32_launch(B, n_var != 0, norm == 1, grid, smem, s);
-    } else {
-        e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxDynamicSmem);
-        if (e != cudaSuccess)
-            return set_error(FMF_ERR_CUDA, "tc_persistent shared memory (%zu bytes): %s", smem,
-                             cudaGetErrorString(e));
-        kern<<<grid, tc_threads(n_var != 0), smem, s>>>(B);
-        count_launch();
-        rc = check_launch("tc_persistent");
-    }
+    int rc = check_launch("tc_persistent");
     if (rc || parts == 1)
         return rc;
     const long long m = (long long)P0.T * P0.n_corr;
     tc_parts_sum_kernel<<<(unsigned)((m + 255) / 256), 256, 0, s>>>(part_out, parts, m, P0.n_corr,
-                                                                     P0.ntap ? P0.vp_norm : nullptr,
+                                                                     var ? P0.vp_norm : nullptr,
                                                                      P0.vp_bias, P0.vp_scale, P0.out);
     count_launch();
     return check_launch("tc_parts_sum_kernel");
@@ -958,12 +1194,12 @@ int tc_run(const TcProb *probs, int n, int form, int parts, unsigned long long *
 
 size_t tc_prob_size() { return sizeof(TcProb); }
 
-// Templates [t0, t0 + nt) of a prepared search, as a search of its own
-// (every template-indexed pointer offset; data streams shared).
-void tc_subset(const TcProb *full, int t0, int nt, TcProb *out)
+// Templates [t0, t0 + nt) of a search, as a search of its own (every
+// template-indexed pointer offset but the operand blocks; data streams shared).
+static void tc_subset(const TcProb *full, int t0, int nt, TcProb *out)
 {
     TcProb q = *full;
-    const size_t SC = q.P.SC, step = q.P.step;
+    const size_t SC = q.P.SC;
     const size_t o = (size_t)t0 * SC;
     q.P.tpl += o * q.P.L;
     q.P.sst += o;
@@ -984,35 +1220,164 @@ void tc_subset(const TcProb *full, int t0, int nt, TcProb *out)
     }
     q.P.out += (size_t)t0 * q.P.n_corr * (q.P.network_sum ? 1 : SC);
     q.P.T = nt;
-    q.w_hi += o * step * q.NW * 64;
-    if (q.w_lo)
-        q.w_lo += o * step * q.NW * 64;
-    if (q.mu) {
-        q.mu += o * step;
-        q.psi += o * step;
-    }
     if (q.t_exp)
         q.t_exp += o;
     *out = q;
 }
 
-// Single search: preprocessing + one persistent launch.
-int launch_tc(const Problem &P, const float *data_for_tc, int precision, unsigned *err, Scratch &ws,
-              cudaStream_t s, int forced_nb, int template_group)
+struct TcSearch {
+    TcProb pr;       // of all templates; the operand blocks hold `room` of them
+    int form, room, parts;
+    uint16_t *w;
+    size_t w_elems;  // of one half, all room templates
+};
+
+size_t tc_search_size() { return sizeof(TcSearch); }
+
+// Operand blocks of one part of the templates take at most this much memory.
+constexpr size_t kMaxTemplateBytes = (size_t)4 << 30;
+
+size_t tc_template_bytes(const Problem &P, int nb)
+{
+    return (size_t)P.T * P.SC * P.step * tc_shape(P.L, P.step, 1, nb).NW * 256;
+}
+
+// Lag blocks per tile of an FP32 search on the tensor cores, or 0: the CUDA cores.
+int tc_fp32_nb(size_t T, size_t SC, size_t L, size_t step, size_t n_corr)
+{
+    if (const char *env = getenv("FMF_TC32")) {  // 0: the CUDA cores; 32, 64, 128: this tile
+        if (atoi(env) == 0)
+            return 0;
+        if (atoi(env) > 1)
+            return tc_choose_nb((int)L, (int)step, 1, atoi(env));
+    }
+    // CUDA cores: microseconds of the busiest SM, a tile of 4,096 outputs at a time
+    const double taps = (double)step * (double)((((L + step - 1) / step + 19) / 20) * 20);
+    const double tiles = (double)T * (double)((n_corr + 4095) / 4096);
+    const double waves = tiles <= 304.0 ? 1.0 : tiles / 304.0;
+    const double plain_us = waves * (double)SC * (taps * 0.02 + (double)step * 0.5 + 0.5);
+    if (plain_us < 60.0)
+        return 0;
+    const int want = n_corr > 8192 ? 128 : (n_corr > 4096 ? 64 : 32);
+    for (int nb = want; nb >= 32; nb >>= 1) {
+        const int fit = tc_choose_nb((int)L, (int)step, 1, nb);
+        if (fit)
+            return fit;
+    }
+    return 0;
+}
+
+// Begins a search: data streams of `form`, and room for the operand blocks of up to
+// max_templates templates at a time.  The statistics of P (running sums, with
+// per-channel lengths) have a tile of padding round them; FP32 needs P.scan.
+int tc_begin(const Problem &P, int form, int nb, int tg, int max_templates, Scratch &ws, cudaStream_t s,
+             TcSearch *out)
 {
     int rc;
-    const int split = precision == FMF_PREC_SPLIT_BF16;
-    const int nb = tc_choose_nb(P.L, P.step, split, forced_nb);
-    if (nb == 0)
-        return set_error(FMF_ERR_SMEM, "template length %d, step %d: tensor-core tile does not fit shared memory",
-                         P.L, P.step);
-    TcProb pr;
-    if ((rc = tc_prepare(P, data_for_tc, split, nb, template_group, ws, s, &pr)))
+    const int step = P.step, SC = P.SC;
+    const bool pairs = form != TC_FORM_BF16, fp32 = form == TC_FORM_FP32;
+    const size_t halves = pairs ? 2 : 1;
+    TcProb &pr = out->pr;
+    const TcShape g = tc_fill_shape(P, pairs, nb, tg, &pr);
+    const size_t per_template = (size_t)SC * step * g.NW * 64;  // one half
+    size_t room = kMaxTemplateBytes / (2 * halves * per_template);
+    room = room < 1 ? 1 : room;
+    room = room < (size_t)max_templates ? room : (size_t)max_templates;
+    const size_t g_elems = (size_t)SC * step * TC_CB * pr.rows_total * 8;
+    const size_t n_rows = (size_t)P.T * SC;
+    out->form = form;
+    out->room = (int)room;
+    out->w_elems = room * per_template;
+    out->parts = tc_choose_parts(&pr);
+    uint16_t *g_hi = nullptr;
+    int *exps = nullptr;
+    if ((rc = ws.get(&g_hi, halves * g_elems, "tensor-core data streams")) ||
+        (rc = ws.get(&out->w, halves * out->w_elems, "tensor-core template blocks")) ||
+        (fp32 && (rc = ws.get(&exps, n_rows + SC, "operand exponents"))))
         return rc;
-    unsigned long long *queue = nullptr;
-    if ((rc = ws.get(&queue, 1, "tile queue")))
+    uint16_t *g_lo = pairs ? g_hi + g_elems : nullptr;
+    pr.g_hi = g_hi;
+    pr.g_lo = g_lo;
+    pr.w_hi = out->w;
+    pr.w_lo = pairs ? out->w + out->w_elems : nullptr;
+    if (fp32) {
+        pr.t_exp = exps;
+        pr.d_exp = exps + n_rows;
+        pr.skip = P.scan + 3 * SC;
+    }
+    // FP32: chains of whole column-block pairs, at most kChain K steps where a pair has no
+    // more; the bf16 pairs' own rounding (4.4e-6 of a product) is far above a channel-long
+    // chain's
+    const int most = (g.k_span + TC_Q - 1) / TC_Q;  // K steps of one pair
+    pr.chain_cols = fp32 ? (kChain / most > 1 ? kChain / most : 1) : step * (TC_CB / 2);
+    const long long n = (long long)SC * step * TC_CB * pr.rows_total;
+    if (fp32)
+        tc_data_kernel<true><<<(unsigned)((n + 255) / 256), 256, 0, s>>>(
+            P.data, P.N, SC, step, pr.rows_total, pr.row_front, P.scan, g_hi, g_lo, exps + n_rows, P.scan + 3 * SC);
+    else
+        tc_data_kernel<false><<<(unsigned)((n + 255) / 256), 256, 0, s>>>(
+            P.data, P.N, SC, step, pr.rows_total, pr.row_front, nullptr, g_hi, g_lo, nullptr, nullptr);
+    count_launch();
+    return check_launch("tensor-core data streams");
+}
+
+// Operand blocks of templates [t0, t0 + nt), nt <= room, into the search's
+// buffer; *sub is that part of the search.
+static int tc_templates(const TcSearch *full, int t0, int nt, cudaStream_t s, TcProb *sub)
+{
+    const Problem &P = full->pr.P;
+    tc_subset(&full->pr, t0, nt, sub);
+    const bool fp32 = full->form == TC_FORM_FP32;
+    auto kern = fp32 ? tc_template_kernel<true> : tc_template_kernel<false>;
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxDynamicSmem - 1024);
+    if (e != cudaSuccess)
+        return set_error(FMF_ERR_CUDA, "tc_template_kernel shared memory: %s", cudaGetErrorString(e));
+    kern<<<(unsigned)((size_t)nt * P.SC), 256, (size_t)P.L * sizeof(float), s>>>(
+        sub->P.tpl, sub->P.mo, P.L, P.step, sub->NW, full->w, const_cast<uint16_t *>(full->pr.w_lo),
+        const_cast<int *>(sub->t_exp), const_cast<unsigned *>(full->pr.skip));
+    count_launch();
+    return check_launch("tensor-core templates");
+}
+
+// Templates [t0, t0 + nt) of a begun search: their operand blocks and the
+// persistent launch, a roomful at a time.  The channel parts of an FP32 search are
+// those of all its templates, so that its results do not depend on how they are
+// parted (a call with host arrays runs them in parts); the bf16 forms choose them
+// for each launch, which keeps the SMs busier through the last few templates.
+int tc_run_templates(const TcSearch *full, int t0, int nt, unsigned *err, Scratch &ws, cudaStream_t s)
+{
+    int rc;
+    for (int a = t0; a < t0 + nt; a += full->room) {
+        const int n = t0 + nt - a < full->room ? t0 + nt - a : full->room;
+        TcProb sub;
+        unsigned long long *queue = nullptr;
+        if ((rc = tc_templates(full, a, n, s, &sub)) || (rc = ws.get(&queue, 1, "tile queue")) ||
+            (rc = tc_run(&sub, 1, full->form, full->form == TC_FORM_FP32 ? full->parts : 0, queue, err, s)))
+            return rc;
+    }
+    return FMF_OK;
+}
+
+// FP32: nonzero afterwards if the CUDA cores have to run the search.
+const unsigned *tc_flag(const TcSearch *full) { return full->pr.skip; }
+
+// One search of a batch: all its operands; *out is ready for a shared launch.
+int tc_prepare(const Problem &P, int form, int nb, int tg, Scratch &ws, cudaStream_t s, TcProb *out)
+{
+    TcSearch st;
+    int rc = tc_begin(P, form, nb, tg, P.T, ws, s, &st);
+    if (rc)
         return rc;
-    return tc_run(&pr, 1, split ? TC_FORM_SPLIT : TC_FORM_BF16, 0, queue, err, s);
+    if (st.room < P.T) {  // a shared launch needs them all at once
+        const size_t halves = form != TC_FORM_BF16 ? 2 : 1;
+        st.w_elems = st.w_elems / st.room * P.T;
+        st.room = P.T;
+        if ((rc = ws.get(&st.w, halves * st.w_elems, "tensor-core template blocks")))
+            return rc;
+        st.pr.w_hi = st.w;
+        st.pr.w_lo = halves == 2 ? st.w + st.w_elems : nullptr;
+    }
+    return tc_templates(&st, 0, P.T, s, out);
 }
 
 }  // namespace fmf

@@ -19,8 +19,6 @@ struct TcProb {
     Problem P;                    // sizes, epilogue inputs, output
     const uint16_t *g_hi, *g_lo;  // bf16 (FP32 form: fp16) bits, data streams [SC][step][CB][rows_total][8]
     const uint16_t *w_hi, *w_lo;  // the same, template blocks [T][SC][step][NW][64]
-    const int *mu;                // [T][SC][step] moveout of each phase in its stream
-    const int *psi;               // [T][SC][step] stream of each phase
     long long item_begin;         // first tile-queue item of this search
     int R;                        // data rows per stage
     int NW;                       // 128-byte template blocks per (template, channel, phase)
@@ -35,7 +33,7 @@ struct TcProb {
                                   // part_out[j][t][lag] and are added in order j after
                                   // the launch (a fixed order: deterministic results)
     float *part_out;
-    // FP32 form (fmf_tc32.cu): operands are fp16 pairs in units of powers of two
+    // FP32 form (fmf_tc.cu): operands are fp16 pairs in units of powers of two
     const int *t_exp;             // [T][SC] exponent of each channel's template
     const int *d_exp;             // [SC] exponent of each data channel
     int chain_cols;               // column-block pairs of one h h chain
@@ -46,8 +44,9 @@ struct TcBatch {
     TcProb prob[TC_MAX_PROBS];
     int n_probs;
     int split;                    // 1: hi/lo, three products; 0: single bf16 product
-    int stage_bytes;              // bytes of one pipeline stage (largest search)
-    // FP32 form: template buffers (2), data slots, statistics slots (2^stat_log2)
+    uint32_t mma_types;           // operand types, in their place in the MMA's instruction descriptor
+    float lo_unit;                // what a low half counts in units of the high one
+    // shared memory: template buffers (2), data slots, statistics slots (2^stat_log2)
     int w_bytes, n_rows, row_bytes, stat_log2, stat_bytes;
     long long total_items;
     unsigned long long *queue;    // tile-queue head, zero before the launch
@@ -162,18 +161,8 @@ __device__ __forceinline__ uint64_t sdesc(uint32_t addr, uint32_t lbo, uint32_t 
            ((uint64_t)((sbo >> 4) & 0x3FFFu) << 32) | (1ull << 46);
 }
 
-__device__ __forceinline__ void mma_f16(uint32_t d_tmem, uint64_t a, uint64_t b, uint32_t idesc,
-                                         uint32_t accumulate)
-{
-    asm volatile(
-        "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n"
-        " tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}\n" ::"r"(d_tmem),
-        "l"(a), "l"(b), "r"(idesc), "r"(accumulate)
-        : "memory");
-}
-
-// The same with descriptors in halves: the start address is in the low word, and
-// only it moves along K, so the high words stay put.
+// Descriptors in halves: the start address is in the low word, and only it moves
+// along K, so the high words stay put.
 __device__ __forceinline__ void mma_f16(uint32_t d_tmem, uint32_t a_lo, uint32_t a_hi, uint32_t b_lo,
                                         uint32_t b_hi, uint32_t idesc, uint32_t accumulate)
 {
@@ -202,6 +191,8 @@ __device__ __forceinline__ bool elect_one()
 __device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
 
+__device__ __forceinline__ void tmem_wait_ld() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
+
 // 32 lanes x 32 bits, 16 consecutive columns per thread
 __device__ __forceinline__ void tmem_ld16(uint32_t taddr, float *v)
 {
@@ -217,45 +208,6 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, float *v)
     for (int i = 0; i < 16; i++)
         v[i] = __uint_as_float(r[i]);
 }
-
-__device__ __forceinline__ void tmem_wait_ld() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
-
-__device__ __forceinline__ void tmem_ld8(uint32_t taddr, float *v)
-{
-    uint32_t r[8];
-    asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
-                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]),
-                   "=r"(r[7])
-                 : "r"(taddr));
-#pragma unroll
-    for (int i = 0; i < 8; i++)
-        v[i] = __uint_as_float(r[i]);
-}
-
-__device__ __forceinline__ void tmem_st16(uint32_t taddr, const float *v)
-{
-    asm volatile(
-        "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,"
-        "%16};" ::"r"(taddr),
-        "r"(__float_as_uint(v[0])), "r"(__float_as_uint(v[1])), "r"(__float_as_uint(v[2])),
-        "r"(__float_as_uint(v[3])), "r"(__float_as_uint(v[4])), "r"(__float_as_uint(v[5])),
-        "r"(__float_as_uint(v[6])), "r"(__float_as_uint(v[7])), "r"(__float_as_uint(v[8])),
-        "r"(__float_as_uint(v[9])), "r"(__float_as_uint(v[10])), "r"(__float_as_uint(v[11])),
-        "r"(__float_as_uint(v[12])), "r"(__float_as_uint(v[13])), "r"(__float_as_uint(v[14])),
-        "r"(__float_as_uint(v[15]))
-        : "memory");
-}
-
-__device__ __forceinline__ void tmem_st8(uint32_t taddr, const float *v)
-{
-    asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};" ::"r"(taddr),
-                 "r"(__float_as_uint(v[0])), "r"(__float_as_uint(v[1])), "r"(__float_as_uint(v[2])),
-                 "r"(__float_as_uint(v[3])), "r"(__float_as_uint(v[4])), "r"(__float_as_uint(v[5])),
-                 "r"(__float_as_uint(v[6])), "r"(__float_as_uint(v[7]))
-                 : "memory");
-}
-
-__device__ __forceinline__ void tmem_wait_st() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
 
 // 32 lanes x 32 bits, 32 consecutive columns per thread
 __device__ __forceinline__ void tmem_ld32(uint32_t taddr, float *v)
@@ -273,24 +225,6 @@ __device__ __forceinline__ void tmem_ld32(uint32_t taddr, float *v)
 #pragma unroll
     for (int i = 0; i < 32; i++)
         v[i] = __uint_as_float(r[i]);
-}
-
-// CH consecutive accumulator columns of this warp's 32 lanes (CH = 8 or 16)
-template <int CH>
-__device__ __forceinline__ void tmem_ldc(uint32_t taddr, float *v)
-{
-    if constexpr (CH == 16)
-        tmem_ld16(taddr, v);
-    else
-        tmem_ld8(taddr, v);
-}
-template <int CH>
-__device__ __forceinline__ void tmem_stc(uint32_t taddr, const float *v)
-{
-    if constexpr (CH == 16)
-        tmem_st16(taddr, v);
-    else
-        tmem_st8(taddr, v);
 }
 
 // ------------------------------------------------------------------ epilogue arithmetic
@@ -343,24 +277,32 @@ __device__ __forceinline__ float atanh_reduced(float y)
     return copysignf(r, y);
 }
 
-// Called by all 32 lanes of a warp together: the series on every lane, the
-// reduction only when some lane of the warp needs it (no divergent branch;
-// the common case, every |y| <= 1/4, skips it).
-__device__ __forceinline__ float fisher_atanh(float y)
+// Called by all 32 lanes of a warp together, N values each: the series on every value,
+// the reduction only when some value of the warp needs it (one vote for all; the
+// common case, every |y| <= 1/4, skips it).
+template <int N>
+__device__ __forceinline__ void fisher_atanh(float (&y)[N])
 {
-    const bool big = !(fabsf(y) <= 0.25f);  // NaN included
-    float r = atanh_series(y);
-    if (__any_sync(0xffffffffu, big)) {
-        const float g = atanh_reduced(y);
-        r = big ? g : r;
+    bool big = false;  // NaN included
+    float r[N];
+#pragma unroll
+    for (int i = 0; i < N; i++) {
+        big = big || !(fabsf(y[i]) <= 0.25f);
+        r[i] = atanh_series(y[i]);
     }
-    return r;
+    if (__any_sync(0xffffffffu, big)) {
+#pragma unroll
+        for (int i = 0; i < N; i++)
+            r[i] = fabsf(y[i]) <= 0.25f ? r[i] : atanh_reduced(y[i]);
+    }
+#pragma unroll
+    for (int i = 0; i < N; i++)
+        y[i] = r[i];
 }
 
 // ------------------------------------------------------------------ tile queue
 // Decodes a tile-queue item: search p, output tile, template t.  Items of one
 // search are ordered so that groups of `tg` templates sweep the tiles together.
-template <bool PARTS>
 __device__ __forceinline__ void decode_item(const TcBatch &B, long long item, int &p, int &tile, int &t,
                                             int &c_begin, int &c_end, int &part)
 {
@@ -378,7 +320,7 @@ __device__ __forceinline__ void decode_item(const TcBatch &B, long long item, in
     c_begin = 0;
     c_end = pr.P.SC;
     part = 0;
-    if (PARTS) {  // the parts of a (tile, template) are adjacent items
+    if (pr.parts > 1) {  // the parts of a (tile, template) are adjacent items
         const int k = pr.parts;
         part = (int)(local % k);
         local /= k;
@@ -444,10 +386,5 @@ inline TcShape tc_fill_shape(const Problem &P, int split, int nb, int tg, TcProb
     pr->parts = 1;
     return g;
 }
-
-// The FP32 form's persistent kernel (fmf_tc32.cu): its shared memory for the searches
-// of `B` (template buffers of w_bytes and data slots of row_bytes set), its launch.
-size_t tc32_layout(TcBatch *B, bool var, bool full);
-int tc32_launch(const TcBatch &B, bool var, bool full, unsigned grid, size_t smem, cudaStream_t s);
 
 }  // namespace fmf

@@ -377,12 +377,13 @@ __global__ void prefix_offsets_kernel(long long *bs2, float2 *bs1, int nblk, int
 
 // Phase 3, grid (blocks, SC), 256 threads: inclusive scan of the block plus
 // its offset -> P2[ch][i + 1] = sum_{x <= i} d'^2 in units (P2[ch][0] = 0)
-// and, for 'full', P1 of d' and the centred data.
+// and, for 'full', P1 of d' and the centred data.  Element i + 1 = step * x + psi
+// of a channel lies at psi * pre_ps + x (Problem::pre2q).
 __global__ void prefix_write_kernel(const float *__restrict__ data, int N, const float *__restrict__ mu,
                                     const float *__restrict__ unit, const long long *__restrict__ bs2,
                                     const float2 *__restrict__ bs1, int nblk,
                                     long long *__restrict__ pre2q, float2 *__restrict__ pre1f,
-                                    float *__restrict__ dcen)
+                                    long long pre_ch, long long pre_ps, int step, float *__restrict__ dcen)
 {
     __shared__ long long part2[32];
     __shared__ float2 part1[32];
@@ -449,8 +450,8 @@ __global__ void prefix_write_kernel(const float *__restrict__ data, int N, const
     const long long o2 = part2[wid] + e2;
     float oh1 = part1[wid].x, ol1 = part1[wid].y;
     pair_add(oh1, ol1, e1h, e1l);
-    long long *p2 = pre2q + (size_t)ch * (N + 1);
-    float2 *p1 = pre1f ? pre1f + (size_t)ch * (N + 1) : nullptr;
+    long long *p2 = pre2q + ch * pre_ch;
+    float2 *p1 = pre1f ? pre1f + ch * pre_ch : nullptr;
     if (blk == 0 && threadIdx.x == 0) {
         p2[0] = 0;
         if (p1)
@@ -460,11 +461,16 @@ __global__ void prefix_write_kernel(const float *__restrict__ data, int N, const
     for (int e = 0; e < per; e++) {
         const int i = i0 + threadIdx.x * per + e;
         if (i < N) {
-            p2[i + 1] = o2 + v2[e];
+            long long o = i + 1;
+            if (step > 1) {
+                const int x = (i + 1) / step;
+                o = (i + 1 - x * step) * pre_ps + x;
+            }
+            p2[o] = o2 + v2[e];
             if (p1) {
                 float c = oh1, d = ol1;
                 pair_add(c, d, v1[e].x, v1[e].y);
-                p1[i + 1] = pair_normalise(c, d);
+                p1[o] = pair_normalise(c, d);
             }
         }
     }
@@ -546,6 +552,19 @@ static int variable_device(const VArgs &a, int L, cudaStream_t s, float *host_ou
     const int T = (int)a.T, SC = (int)(a.S * a.C), N = (int)a.N;
     const bool full = a.normalize == 1;
     Scratch ws(s);
+    int precision = FMF_FLAG_PRECISION_OF(a.flags);
+    // the tiles of the FP32 form (0: the CUDA cores) and of the bf16 forms, where the call
+    // may come to them
+    int nb32 = 0, nb16 = 0;
+    const int forced = ((a.flags >> 8) & 0xff) * 16;
+    if (precision == FMF_PREC_FP32 || precision == FMF_PREC_AUTO)
+        nb32 = tc_fp32_nb(a.T, a.S * a.C, (size_t)L, a.step, a.n_corr);
+    if (precision != FMF_PREC_FP32 && (forced == 0 || forced == 32 || forced == 64 || forced == 128))
+        nb16 = tc_choose_nb(L, (int)a.step, precision != FMF_PREC_BF16, forced);
+    const long long pad = tc_pad(nb32 > nb16 ? nb32 : nb16);
+    // rows of the running sums, one per channel and phase, on 16-byte boundaries
+    const long long pre_ps = (((long long)N + a.step) / (long long)a.step + 2 * pad + 1) & ~1ll;
+    const long long pre_ch = pre_ps * (long long)a.step;
     int *k_lo = nullptr;
     float *zweight = nullptr, *consts = nullptr, *tmask = nullptr, *tsum = nullptr, *mu = nullptr,
           *dcen = nullptr;
@@ -557,7 +576,7 @@ static int variable_device(const VArgs &a, int L, cudaStream_t s, float *host_ou
         (rc = ws.get(&zweight, (size_t)T * SC, "Fisher-z weights")) ||
         (rc = ws.get(&consts, 3 * (size_t)T, "transform constants")) ||
         (rc = ws.get(&tmask, (size_t)T * SC * L, "masked templates")) ||
-        (rc = ws.get(&pre2q, (size_t)SC * (N + 1), "running sums of d^2")) ||
+        (rc = ws.get(&pre2q, (size_t)SC * pre_ch, "running sums of d^2")) ||
         (rc = ws.get(&unit, (size_t)SC, "fixed-point units")) ||
         (rc = ws.get(&epart, (size_t)SC * nblk, "block energies")) ||
         (rc = ws.get(&bs2, (size_t)SC * nblk, "block sums")) ||
@@ -566,11 +585,8 @@ static int variable_device(const VArgs &a, int L, cudaStream_t s, float *host_ou
     if (full && ((rc = ws.get(&tsum, (size_t)T * SC, "template sums")) ||
                  (rc = ws.get(&mu, (size_t)SC, "channel centres")) ||
                  (rc = ws.get(&dcen, (size_t)SC * N, "centred data")) ||
-                 (rc = ws.get(&pre1f, (size_t)SC * (N + 1), "prefix sums of d"))))
+                 (rc = ws.get(&pre1f, (size_t)SC * pre_ch, "prefix sums of d"))))
         return rc;
-    int precision = FMF_FLAG_PRECISION_OF(a.flags);
-    const bool may_fp32 = precision == FMF_PREC_FP32 || precision == FMF_PREC_AUTO;
-    const int nb32 = may_fp32 ? tc32_choose_nb(a.T, a.S * a.C, (size_t)L, a.step, a.n_corr) : 0;
     unsigned *scan = nullptr;
     if (nb32) {
         const size_t n = 3 * (size_t)SC + 1;
@@ -580,6 +596,9 @@ static int variable_device(const VArgs &a, int L, cudaStream_t s, float *host_ou
         if (e != cudaSuccess)
             return set_error(FMF_ERR_CUDA, "clearing the channel scan: %s", cudaGetErrorString(e));
     }
+    pre2q += pad;
+    if (pre1f)
+        pre1f += pad;
     int *k_hi = k_lo + T;
     float *norm_sum = consts, *bias = consts + T, *scale = consts + 2 * T;
 
@@ -596,7 +615,7 @@ static int variable_device(const VArgs &a, int L, cudaStream_t s, float *host_ou
     prefix_block_kernel<<<dim3(nblk, SC), 256, 0, s>>>(a.data, N, mu, unit, bs2, bs1, nblk);
     prefix_offsets_kernel<<<(SC + 3) / 4, 128, 0, s>>>(bs2, bs1, nblk, SC);  // a warp per channel
     prefix_write_kernel<<<dim3(nblk, SC), 256, 0, s>>>(a.data, N, mu, unit, bs2, bs1, nblk, pre2q,
-                                                        pre1f, dcen);
+                                                        pre1f, pre_ch, pre_ps, (int)a.step, dcen);
     count_launch(full ? 10 : 9);
     if ((rc = check_launch("variable-length preprocessing")))
         return rc;
@@ -624,6 +643,8 @@ static int variable_device(const VArgs &a, int L, cudaStream_t s, float *host_ou
     P.network_sum = 1;
     P.ntap = a.ntap;
     P.pre2q = pre2q;
+    P.pre_ch = pre_ch;
+    P.pre_ps = pre_ps;
     P.unit2 = unit;
     P.pre1f = pre1f;
     P.zweight = zweight;
@@ -651,44 +672,31 @@ static int variable_device(const VArgs &a, int L, cudaStream_t s, float *host_ou
     for (int c = 0; c < n_chunks; c++)
         most = bounds[c + 1] - bounds[c] > most ? bounds[c + 1] - bounds[c] : most;
     unsigned *err = nullptr;
-    int split = 0;
-    std::vector<unsigned char> tcfull;
-    std::vector<unsigned char> tc32;
-    if (precision == FMF_PREC_FP32 && nb32) {
+    std::vector<unsigned char> tc;
+    const bool fp32 = precision == FMF_PREC_FP32;
+    const int nb = fp32 ? nb32 : nb16;
+    if (!fp32 && forced != 0 && forced != 32 && forced != 64 && forced != 128)
+        return set_error(FMF_ERR_ARG, "tensor-core tile of %d lag blocks (32, 64 or 128)", forced);
+    if (!fp32 && nb == 0)
+        return set_error(FMF_ERR_SMEM, "template length %d, step %zu: tensor-core tile does not fit "
+                                       "shared memory", L, a.step);
+    if (nb) {
         Problem Q = P;
-        Q.vp_norm = norm_sum;
+        Q.vp_norm = norm_sum;  // the final transform fused into the output write
         Q.vp_bias = bias;
         Q.vp_scale = scale;
-        tc32.resize(tc32_search_size());
-        rc = device_error_word(&err);
-        if (!rc)
-            rc = tc32_begin(Q, nb32, 0, most, ws, s, reinterpret_cast<Tc32Search *>(tc32.data()));
-        if (rc == FMF_ERR_OOM) {  // the CUDA-core kernel needs no more memory
+        tc.resize(tc_search_size());
+        TcSearch *search = reinterpret_cast<TcSearch *>(tc.data());
+        if (!(rc = device_error_word(&err)))
+            rc = tc_begin(Q, tc_form(precision), nb, (a.flags >> 16) & 0xff, most, ws, s, search);
+        if (fp32 && rc == FMF_ERR_OOM) {  // the CUDA-core kernel needs no more memory
             set_error(FMF_OK, "");
-            tc32.clear();
+            tc.clear();
         } else if (rc) {
             return rc;
         } else {
-            P.only_if = tc32_flag(reinterpret_cast<Tc32Search *>(tc32.data()));
+            P.only_if = tc_flag(search);
         }
-    }
-    if (precision != FMF_PREC_FP32) {
-        const int forced = ((a.flags >> 8) & 0xff) * 16;
-        if (forced != 0 && forced != 32 && forced != 64 && forced != 128)
-            return set_error(FMF_ERR_ARG, "tensor-core tile of %d lag blocks (32, 64 or 128)", forced);
-        P.vp_norm = norm_sum;  // the final transform fused into the output write
-        P.vp_bias = bias;
-        P.vp_scale = scale;
-        split = precision == FMF_PREC_SPLIT_BF16;
-        const int nb = tc_choose_nb(L, (int)a.step, split, forced);
-        if (nb == 0)
-            return set_error(FMF_ERR_SMEM, "template length %d, step %zu: tensor-core tile does not fit "
-                                           "shared memory", L, a.step);
-        tcfull.resize(tc_prob_size());
-        if ((rc = device_error_word(&err)) ||
-            (rc = tc_prepare(P, P.data, split, nb, (a.flags >> 16) & 0xff, ws, s,
-                             reinterpret_cast<TcProb *>(tcfull.data()))))
-            return rc;
     }
     CopyStream cs;
     cudaError_t e = host_out ? cs.init(n_chunks) : cudaSuccess;
@@ -697,18 +705,10 @@ static int variable_device(const VArgs &a, int L, cudaStream_t s, float *host_ou
     for (int c = 0; c < n_chunks; c++) {
         const int t0 = bounds[c], nt = bounds[c + 1] - bounds[c];
         if (nt > 0) {
-            if (!tcfull.empty()) {
-                std::vector<unsigned char> sub(tc_prob_size());
-                unsigned long long *queue = nullptr;
-                tc_subset(reinterpret_cast<const TcProb *>(tcfull.data()), t0, nt,
-                          reinterpret_cast<TcProb *>(sub.data()));
-                if ((rc = ws.get(&queue, 1, "tile queue")) ||
-                    (rc = tc_run(reinterpret_cast<const TcProb *>(sub.data()), 1, split, 0, queue, err, s)))
-                    return rc;
-            } else {
-                if (!tc32.empty() &&
-                    (rc = tc32_run(reinterpret_cast<const Tc32Search *>(tc32.data()), t0, nt, err, ws, s)))
-                    return rc;
+            if (!tc.empty() &&
+                (rc = tc_run_templates(reinterpret_cast<const TcSearch *>(tc.data()), t0, nt, err, ws, s)))
+                return rc;
+            if (fp32) {  // after the tensor cores: only if the search's flag says so
                 if ((rc = launch_plain_all(var_subset(P, t0, nt), s)))
                     return rc;
                 const long long n = (long long)nt * a.n_corr;

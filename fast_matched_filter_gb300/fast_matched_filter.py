@@ -304,10 +304,17 @@ def _matched_filter_variable(templates, moveouts, weights, data, step, n_samples
         return None
     T, S, C = dims
     templates = templates.reshape(T, S, C, max_len)
-    pp = prepare(templates, moveouts, weights, data, step, normalize)
+    # many taps: their energies on the GPU (19 MB: 0.2 ms against 6 ms of numpy); few: the
+    # extra call costs more (60 us)
+    pp = prepare(templates, moveouts, weights, data, step, normalize,
+                 energies="device" if templates.size > 1 << 18 else "host")
     n_corr = int((pp["N"] - max_len) / pp["step"] + 1)
     nt = np.ascontiguousarray(n_samples_template.flatten(), dtype=np.int32)
     cc = _output_array(out, (T, n_corr))
+    if pp["sst"] is None:  # float32 templates: on the GPU, bit-identical to the numpy sum
+        pp["sst"] = np.empty(T * S * C, dtype=np.float32)
+        _lib.check(lib.fmf_template_energies(pp["templates"].ctypes.data, T * S * C, max_len,
+                                             pp["sst"].ctypes.data, 0, None), lib)
     st = lib.fmf_matched_filter_variable_ex(
         pp["templates"].ctypes.data, pp["sst"].ctypes.data, pp["moveouts"].ctypes.data,
         pp["data"].ctypes.data, pp["weights"].ctypes.data, pp["step"], nt.ctypes.data,
