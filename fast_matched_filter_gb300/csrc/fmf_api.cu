@@ -361,13 +361,17 @@ int prepare_problem(const Args &a, Scratch &ws, cudaStream_t s, Problem *Pout, i
     P.scan = scan;
     P.only_if = nullptr;
 
-    if (!P.network_sum) {
-        size_t bytes = (size_t)T * a.n_corr * SC * sizeof(float);
-        if ((rc = cuda_status(cudaMemsetAsync(a.out, 0, bytes, s), "clearing the output")))
-            return rc;
-    }
+    P.by_channel = nullptr;
     *Pout = P;
     return FMF_OK;
+}
+
+int clear_outputs(const Problem &P, cudaStream_t s)
+{
+    if (P.network_sum)  // every element is written
+        return FMF_OK;
+    return cuda_status(cudaMemsetAsync(P.out, 0, (size_t)P.T * P.n_corr * P.SC * sizeof(float), s),
+                       "clearing the output");
 }
 
 // check_zeros count of templates [t0, t0 + nt) of a search's output into
@@ -492,12 +496,14 @@ struct Search {
     TcSearch *search() { return reinterpret_cast<TcSearch *>(tc.data()); }
     int run(int t0, int nt, Scratch &ws, cudaStream_t s)
     {
+        int rc;
         Problem Q = problem_subset(P, t0, nt);
         if (!tc.empty()) {
-            int rc = tc_run_templates(search(), t0, nt, err, ws, s);
-            if (rc || !fp32)
+            if ((rc = tc_run_templates(search(), t0, nt, err, ws, s)) || !fp32)
                 return rc;
             Q.only_if = tc_flag(search());
+        } else if ((rc = clear_outputs(Q, s))) {
+            return rc;
         }
         return launch_plain_all(Q, s);
     }

@@ -83,6 +83,8 @@ static int batch_record(fmf_batch *b, cudaStream_t s)
                 break;
             if (fp32 && nb[i] && tc_template_bytes(P[i], nb[i]) > kBatchTemplateBytes)
                 nb[i] = 0;
+            if ((status = clear_outputs(P[i], si)))
+                break;
             if (nb[i] == 0)
                 status = launch_plain_all(P[i], si);
             else

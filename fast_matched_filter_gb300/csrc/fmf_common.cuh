@@ -40,6 +40,8 @@ struct Problem {
     const int *k_lo;      // (T) first valid output index
     const int *k_hi;      // (T) one past the last valid output index (<= n_corr)
     float *out;           // (T, n_corr) or (T, n_corr, SC)
+    float *by_channel;    // tensor cores, per-channel outputs: (T, SC, n_corr), turned into out
+                          // afterwards; null: they go to out directly
     int T, SC, L, N, step, n_corr;
     int normalize;        // 0 short, 1 full
     int network_sum;      // 1 weighted sum over channels, 0 per channel
@@ -227,6 +229,8 @@ struct Args {
     long long zero_stop = 0;
 };
 int validate_args(const Args &a);
+// Per-channel outputs of P.by_channel into P.out (fmf_prep.cu).
+int launch_channel_outputs(const Problem &P, const unsigned *flag, cudaStream_t s);
 // Template energies and valid lags (fmf_prep.cu): sst of `rows` rows from tpl (null:
 // sst is given and only scanned), lags of T templates.
 void launch_template_scalars(const float *tpl, float *sst, int rows, int L, unsigned *scan, const int *mo,
@@ -247,8 +251,10 @@ StatPlace stat_rows(int SC, int N, int step, int pad, size_t *elems);
 StatPlace stat_rows_packed(int N, int step);
 int launch_window_stats(const float *data, int N, int L, int SC, const float *mu, float *dcen,
                         float *stat_e, const StatPlace &place, unsigned *scan, cudaStream_t s);
-// pad: padding round the statistics' rows (tc_pad); scan: also make Problem::scan
+// pad: padding round the statistics' rows (tc_pad); scan: also make Problem::scan.  Does
+// not clear per-channel outputs (clear_outputs).
 int prepare_problem(const Args &a, Scratch &ws, cudaStream_t s, Problem *P, int pad, bool scan);
+int clear_outputs(const Problem &P, cudaStream_t s);  // per-channel outputs that no kernel writes
 
 // Tensor cores (fmf_tc.cu): begin a search, then run its templates in parts.
 constexpr int TC_MAX_PROBS = 64;
@@ -266,7 +272,7 @@ int tc_fp32_nb(size_t T, size_t SC, size_t L, size_t step, size_t n_corr);  // 0
 inline int tc_pad(int nb) { return nb ? 128 * nb + 16 : 0; }  // statistics padding of such a tile
 size_t tc_search_size();
 int tc_begin(const Problem &P, int form, int nb, int tg, int max_templates, Scratch &ws, cudaStream_t s,
-             TcSearch *out);
+             TcSearch *out, bool turn = true);
 int tc_run_templates(const TcSearch *full, int t0, int nt, unsigned *err, Scratch &ws, cudaStream_t s);
 const unsigned *tc_flag(const TcSearch *full);
 size_t tc_prob_size();

@@ -217,6 +217,7 @@ extern "C" int fmf_matched_filter_noalloc(const float *templates, const float *s
     P.k_lo = k_lo;
     P.k_hi = k_hi;
     P.out = cc_out;
+    P.by_channel = nullptr;
     P.T = T;
     P.SC = SC;
     P.L = L;

@@ -234,6 +234,53 @@ __global__ void zero_count_kernel(const float *__restrict__ out, long long row_l
         atomicAdd(counts + t, (unsigned long long)c);
 }
 
+// Per-channel outputs (T, n_corr, SC) from the (T, SC, n_corr) array that the tensor
+// cores' epilogue writes in runs of 32 lags: tiles of 64 lags x up to 64 channels
+// through shared memory.  Zeros outside the valid lags and on channels of weight 0; all
+// zeros if the flag leaves the search to the CUDA cores.  (Written in place, 4
+// bytes per 32-byte sector, the coefficients of 8 templates x 36 channels x
+// 119,601 lags took 712 us; now 150 us and 50 us here.)
+constexpr int kTurnLags = 64, kTurnChannels = 64;
+__global__ void __launch_bounds__(256) channel_outputs_kernel(
+    const float *__restrict__ by_channel, const float *__restrict__ w, const int *__restrict__ k_lo,
+    const int *__restrict__ k_hi, int T, int SC, int n_corr, const unsigned *__restrict__ flag,
+    float *__restrict__ out)
+{
+    __shared__ float tile[kTurnChannels][kTurnLags + 1];
+    const int c_tiles = (SC + kTurnChannels - 1) / kTurnChannels;
+    const int k0 = (int)(blockIdx.x / c_tiles) * kTurnLags, c0 = (int)(blockIdx.x % c_tiles) * kTurnChannels;
+    const int nk = min(kTurnLags, n_corr - k0), nc = min(kTurnChannels, SC - c0);
+    const bool zero = flag && *flag;
+    for (int t = blockIdx.y; t < T; t += gridDim.y) {
+        const int lo = k_lo[t] - k0, hi = k_hi[t] - k0;
+        __syncthreads();
+        for (int c = threadIdx.x >> 6; c < nc; c += 4) {
+            const int k = threadIdx.x & 63;
+            const size_t row = (size_t)t * SC + c0 + c;
+            const bool live = !zero && k >= lo && k < hi && w[row] != 0.0f;
+            tile[c][k] = live ? by_channel[row * n_corr + k0 + k] : 0.0f;
+        }
+        __syncthreads();
+        float *o = out + ((size_t)t * n_corr + k0) * SC + c0;
+        for (int i = threadIdx.x; i < nk * nc; i += 256) {
+            const int k = i / nc, c = i - k * nc;
+            o[(size_t)k * SC + c] = tile[c][k];
+        }
+    }
+}
+
+int launch_channel_outputs(const Problem &P, const unsigned *flag, cudaStream_t s)
+{
+    const long long tiles = (long long)((P.n_corr + kTurnLags - 1) / kTurnLags) *
+                            ((P.SC + kTurnChannels - 1) / kTurnChannels);
+    if (tiles > 0x7fffffffLL)
+        return set_error(FMF_ERR_ARG, "too many tiles of per-channel outputs");
+    channel_outputs_kernel<<<dim3((unsigned)tiles, (unsigned)(P.T < 65535 ? P.T : 65535)), 256, 0, s>>>(
+        P.by_channel, P.w, P.k_lo, P.k_hi, P.T, P.SC, P.n_corr, flag, P.out);
+    count_launch();
+    return check_launch("channel_outputs_kernel");
+}
+
 // grid = T*SC blocks of 128 threads
 __global__ void template_center_kernel(const float *__restrict__ tpl, int L,
                                        float *__restrict__ tcen,
@@ -268,33 +315,73 @@ __global__ void template_center_kernel(const float *__restrict__ tpl, int L,
 // sample channel's mean by ~80 times a 1e-2 noise); the median of 8192
 // evenly spaced samples stays at the level of the quiet data.  It is one of
 // the samples, so d - c is exact in FP32 wherever c/2 <= d <= 2c.
+//
+// The sample stays in registers (8 values a thread) and its median is found by
+// radix selection, 11 + 11 + 10 bits of the values' order-preserving keys; the
+// first pass's bins split a binade in four, so that few lanes of a warp meet in
+// one.  (A bitonic sort in shared memory took 70 us, whatever N.)
 constexpr int kCentreSample = 8192;
-__global__ void __launch_bounds__(1024) channel_centre_kernel(const float *__restrict__ data, int N,
-                                                              float *__restrict__ centre)
+constexpr int kCentreThreads = 1024;
+__global__ void __launch_bounds__(kCentreThreads) channel_centre_kernel(const float *__restrict__ data, int N,
+                                                                        float *__restrict__ centre)
 {
-    __shared__ float v[kCentreSample];
+    constexpr int PER = kCentreSample / kCentreThreads, BINS = 2048;
+    __shared__ unsigned hist[BINS];
+    __shared__ unsigned warp_sum[32];
+    __shared__ unsigned found[2];  // bin and the rank inside it
     const float *src = data + (size_t)blockIdx.x * N;
-    const int S = min(N, kCentreSample);
-    for (int k = threadIdx.x; k < kCentreSample; k += blockDim.x)
-        v[k] = k < S ? src[(long long)k * N / S] : INFINITY;
-    __syncthreads();
-    for (int k = 2; k <= kCentreSample; k <<= 1) {  // bitonic sort, ascending
-        for (int j = k >> 1; j > 0; j >>= 1) {
-            for (int i = threadIdx.x; i < kCentreSample; i += blockDim.x) {
-                const int p = i ^ j;
-                if (p > i) {
-                    const float a = v[i], b = v[p];
-                    if (((i & k) == 0) == (a > b)) {
-                        v[i] = b;
-                        v[p] = a;
-                    }
-                }
-            }
-            __syncthreads();
+    const int S = min(N, kCentreSample), lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    unsigned key[PER];
+#pragma unroll
+    for (int j = 0; j < PER; j++) {
+        const int k = threadIdx.x + j * kCentreThreads;
+        const unsigned u = k < S ? __float_as_uint(src[(long long)k * N / S]) : 0x7f800000u;  // padding: +inf
+        key[j] = u & 0x80000000u ? ~u : u | 0x80000000u;
+    }
+    unsigned rank = (unsigned)(S - 1) / 2, prefix = 0;
+    const int shifts[3] = {21, 10, 0}, widths[3] = {11, 11, 10};
+#pragma unroll
+    for (int pass = 0; pass < 3; pass++) {
+        const int shift = shifts[pass];
+        const unsigned mask = (1u << widths[pass]) - 1, above = pass == 0 ? 0u : ~0u << (shift + widths[pass]);
+        for (int i = threadIdx.x; i < BINS; i += kCentreThreads)
+            hist[i] = 0;
+        __syncthreads();
+#pragma unroll
+        for (int j = 0; j < PER; j++)
+            if ((key[j] & above) == (prefix & above))
+                atomicAdd(&hist[(key[j] >> shift) & mask], 1u);
+        __syncthreads();
+        // each thread two bins: exclusive scan, then the bin that holds the rank
+        const unsigned c0 = hist[2 * threadIdx.x], c1 = hist[2 * threadIdx.x + 1];
+        unsigned x = c0 + c1;
+        for (int o = 1; o < 32; o <<= 1) {
+            const unsigned y = __shfl_up_sync(0xffffffffu, x, o);
+            x += lane >= o ? y : 0;
         }
+        if (lane == 31)
+            warp_sum[wid] = x;
+        __syncthreads();
+        unsigned w = warp_sum[lane];
+        for (int o = 1; o < 32; o <<= 1) {
+            const unsigned y = __shfl_up_sync(0xffffffffu, w, o);
+            w += lane >= o ? y : 0;
+        }
+        const unsigned before_warp = __shfl_sync(0xffffffffu, w, wid) - warp_sum[wid];
+        const unsigned before = before_warp + x - (c0 + c1);
+        if (rank >= before && rank < before + c0) {
+            found[0] = 2 * threadIdx.x;
+            found[1] = rank - before;
+        } else if (rank >= before + c0 && rank < before + c0 + c1) {
+            found[0] = 2 * threadIdx.x + 1;
+            found[1] = rank - before - c0;
+        }
+        __syncthreads();
+        prefix |= found[0] << shift;
+        rank = found[1];
     }
     if (threadIdx.x == 0)
-        centre[blockIdx.x] = v[(S - 1) / 2];
+        centre[blockIdx.x] = __uint_as_float(prefix & 0x80000000u ? prefix & 0x7fffffffu : ~prefix);
 }
 
 // ---------------------------------------------------------------- window statistics

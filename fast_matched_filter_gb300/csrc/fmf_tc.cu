@@ -196,19 +196,108 @@ __device__ __forceinline__ void split_pair(float x, float inv_s, uint16_t &hi, u
 }
 
 // ------------------------------------------------------------------ operands
-// G[ch][psi][cb][r][e] = pair of d[ch][step*(Q*(r - row_front) + 8*cb + e) + psi], zero outside [0, N);
-// one thread per 16-byte row chunk.  FP32: the first thread of a channel also
-// writes its exponent and decides whether the
-// channel's values can be held: stat is the scan of prepare_problem (largest
-// |x|; smallest window energy that can pass the threshold, complemented).
-// The error of a coefficient from the pairs is at most 2^-51 of the largest
-// value over the root of the window's energy, so windows down to 2^-42 of
-// the largest value squared keep it at 1e-9.
+// FP32: the scale of a data channel from the scan of prepare_problem, stat (largest
+// |x|; smallest window energy that can pass the threshold, complemented).  The
+// caller that is `first` also writes the channel's exponent and decides whether
+// the pairs hold its values: the error of a coefficient from them is at most
+// 2^-51 of the largest value over the root of the window's energy, so windows
+// down to 2^-42 of the largest value squared keep it at 1e-9.
+__device__ __forceinline__ float tc_channel_scale(const unsigned *stat, int ch, int SC, bool first, int *d_exp,
+                                                  unsigned *skip)
+{
+    const unsigned top = stat[ch];
+    bool ok;
+    const int e = max_exponent(top, ok);
+    if (first) {
+        d_exp[ch] = e;
+        const unsigned low = ~stat[SC + ch];  // smallest energy's bits; ~0 (a NaN): none
+        const float m = __uint_as_float(top);
+        if (!ok || (low < 0x7f800000u && __uint_as_float(low) * 0x1p42f < m * m))
+            atomicOr(skip, 1u);
+    }
+    return exp2_int(kTopExp - e);
+}
+
+// G[ch][psi][cb][r][e] = pair of d[ch][step*(Q*(r - row_front) + 8*cb + e) + psi], zero outside [0, N).
+// A block turns the samples of `rows` rows of every phase through shared memory:
+// loads of consecutive samples, stores of consecutive rows of a column block (a
+// thread per 16 bytes, reading its own 8 samples, kept the L1 at 98 %: 60
+// channels x 1.08M samples 231 us).  grid: (row tiles, SC), dynamic shared memory
+// tc_turn_bytes.
+constexpr int TC_TURN_PITCH = TC_Q + 8;  // halves per row: 16-byte reads of 8 rows hit distinct banks
+constexpr int TC_TURN_STEP = 64;         // the largest step with a row of every phase
+__host__ __device__ __forceinline__ int tc_turn_rows(int step)
+{
+    int rows = 32;
+    while (rows > 1 && rows * step > TC_TURN_STEP)
+        rows >>= 1;
+    return rows;
+}
+static size_t tc_turn_bytes(int step, bool pairs)
+{
+    return (size_t)(pairs ? 2 : 1) * step * tc_turn_rows(step) * TC_TURN_PITCH * sizeof(uint16_t);
+}
+
 template <bool FP32>
-__global__ void tc_data_kernel(const float *__restrict__ data, int N, int SC, int step, int rows_total,
-                                 int row_front, const unsigned *__restrict__ stat,
-                                 uint16_t *__restrict__ g_hi, uint16_t *__restrict__ g_lo,
-                                 int *__restrict__ d_exp, unsigned *skip)
+__global__ void __launch_bounds__(256) tc_data_kernel(const float *__restrict__ data, int N, int step,
+                                                      int rows_total, int row_front,
+                                                      const unsigned *__restrict__ stat,
+                                                      uint16_t *__restrict__ g_hi, uint16_t *__restrict__ g_lo,
+                                                      int *__restrict__ d_exp, unsigned *skip)
+{
+    extern __shared__ uint4 turn_smem[];
+    const int rows = tc_turn_rows(step), ch = blockIdx.y, row0 = blockIdx.x * rows;
+    uint16_t *hi = reinterpret_cast<uint16_t *>(turn_smem), *lo = hi + step * rows * TC_TURN_PITCH;
+    float inv_s = 1.0f;
+    if constexpr (FP32)
+        inv_s = tc_channel_scale(stat, ch, (int)gridDim.y, blockIdx.x == 0 && threadIdx.x == 0, d_exp, skip);
+    const float *src = data + (size_t)ch * N;
+    const long long pos0 = (long long)step * TC_Q * (row0 - row_front);
+    const int count = step * TC_Q * rows;
+    constexpr int kLoads = 8;  // in flight per thread; count is a multiple of 128
+    for (int i0 = threadIdx.x; i0 < count; i0 += kLoads * 256) {
+        float x[kLoads];
+#pragma unroll
+        for (int j = 0; j < kLoads; j++) {
+            const int i = i0 + 256 * j;
+            const long long pos = pos0 + i;
+            x[j] = i < count && pos >= 0 && pos < N ? __ldg(src + pos) : 0.0f;
+        }
+#pragma unroll
+        for (int j = 0; j < kLoads; j++) {
+            const int i = i0 + 256 * j;
+            if (i < count) {
+                const int q = step == 1 ? i : i / step, psi = step == 1 ? 0 : i - q * step;
+                const int at = (psi * rows + (q >> 7)) * TC_TURN_PITCH + (q & (TC_Q - 1));
+                uint16_t h, l;
+                split_pair<FP32>(x[j], inv_s, h, l);
+                hi[at] = h;
+                if (g_lo)
+                    lo[at] = l;
+            }
+        }
+    }
+    __syncthreads();
+    const int n = min(rows, rows_total - row0);
+    for (int i = threadIdx.x; i < step * TC_CB * rows; i += 256) {
+        const int r = i & (rows - 1), rest = i / rows, cb = rest & (TC_CB - 1), psi = rest / TC_CB;
+        if (r < n) {
+            const int at = (psi * rows + r) * TC_TURN_PITCH + 8 * cb;
+            const size_t o = (((size_t)ch * step + psi) * TC_CB + cb) * rows_total + row0 + r;
+            reinterpret_cast<uint4 *>(g_hi)[o] = *reinterpret_cast<const uint4 *>(hi + at);
+            if (g_lo)
+                reinterpret_cast<uint4 *>(g_lo)[o] = *reinterpret_cast<const uint4 *>(lo + at);
+        }
+    }
+}
+
+// The same for larger steps, whose phases do not share a block: one thread per
+// 16-byte row chunk.
+template <bool FP32>
+__global__ void tc_data_sparse_kernel(const float *__restrict__ data, int N, int SC, int step, int rows_total,
+                                      int row_front, const unsigned *__restrict__ stat,
+                                      uint16_t *__restrict__ g_hi, uint16_t *__restrict__ g_lo,
+                                      int *__restrict__ d_exp, unsigned *skip)
 {
     const long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     const long long per_ch = (long long)step * TC_CB * rows_total;
@@ -217,19 +306,8 @@ __global__ void tc_data_kernel(const float *__restrict__ data, int N, int SC, in
     const int ch = (int)(idx / per_ch);
     long long rest = idx - ch * per_ch;
     float inv_s = 1.0f;
-    if constexpr (FP32) {
-        const unsigned top = stat[ch];
-        bool ok;
-        const int e = max_exponent(top, ok);
-        if (rest == 0) {
-            d_exp[ch] = e;
-            const unsigned low = ~stat[SC + ch];  // smallest energy's bits; ~0 (a NaN): none
-            const float m = __uint_as_float(top);
-            if (!ok || (low < 0x7f800000u && __uint_as_float(low) * 0x1p42f < m * m))
-                atomicOr(skip, 1u);
-        }
-        inv_s = exp2_int(kTopExp - e);
-    }
+    if constexpr (FP32)
+        inv_s = tc_channel_scale(stat, ch, SC, rest == 0, d_exp, skip);
     const int r = (int)(rest % rows_total);
     rest /= rows_total;
     const int cb = (int)(rest % TC_CB);
@@ -813,7 +891,10 @@ __global__ void __launch_bounds__(tc_threads(VAR), 1) tc_persistent(const __grid
                             hc++;
                     }
                     const float wu = wc * unit;  // a power of two: cc * wc rounds the same
-                    float *oc = pr.P.out + ((size_t)t * n_corr + k0) * SC + ch;
+                    // per-channel outputs: this channel's, one lag block after the other
+                    float *oc = pr.P.by_channel ? pr.P.by_channel + (row0 + ch) * n_corr + k0
+                                                : pr.P.out + ((size_t)t * n_corr + k0) * SC + ch;
+                    const size_t oc_step = (size_t)TC_Q * (pr.P.by_channel ? 1 : SC);
                     int psi;
                     const int mu = tc_phase(mo, step, psi);
                     const int head = (int)((I0 + mu) & kStat.align());  // past the 16-byte boundary
@@ -915,7 +996,7 @@ __global__ void __launch_bounds__(tc_threads(VAR), 1) tc_persistent(const __grid
                                             if (NSUM)
                                                 sum[a] = fmaf(cc, wu, sum[a]);
                                             else if (a >= a_lo && a < a_hi)
-                                                oc[(size_t)a * TC_Q * SC] = cc * unit;
+                                                oc[a * oc_step] = cc * unit;
                                         }
                                     }
                                 }
@@ -1234,8 +1315,9 @@ struct TcSearch {
 
 size_t tc_search_size() { return sizeof(TcSearch); }
 
-// Operand blocks of one part of the templates take at most this much memory.
-constexpr size_t kMaxTemplateBytes = (size_t)4 << 30;
+// Operand blocks of one part of the templates take at most this much memory, and so do
+// their per-channel outputs on the way to the caller's layout.
+constexpr size_t kMaxTemplateBytes = (size_t)4 << 30, kMaxChannelBytes = (size_t)1 << 30;
 
 size_t tc_template_bytes(const Problem &P, int nb)
 {
@@ -1269,9 +1351,10 @@ int tc_fp32_nb(size_t T, size_t SC, size_t L, size_t step, size_t n_corr)
 
 // Begins a search: data streams of `form`, and room for the operand blocks of up to
 // max_templates templates at a time.  The statistics of P (running sums, with
-// per-channel lengths) have a tile of padding round them; FP32 needs P.scan.
+// per-channel lengths) have a tile of padding round them; FP32 needs P.scan.  turn:
+// per-channel outputs go through an array of their own (channel_outputs_kernel).
 int tc_begin(const Problem &P, int form, int nb, int tg, int max_templates, Scratch &ws, cudaStream_t s,
-             TcSearch *out)
+             TcSearch *out, bool turn)
 {
     int rc;
     const int step = P.step, SC = P.SC;
@@ -1283,6 +1366,11 @@ int tc_begin(const Problem &P, int form, int nb, int tg, int max_templates, Scra
     size_t room = kMaxTemplateBytes / (2 * halves * per_template);
     room = room < 1 ? 1 : room;
     room = room < (size_t)max_templates ? room : (size_t)max_templates;
+    const size_t turned = P.network_sum || !turn ? 0 : (size_t)SC * P.n_corr;  // outputs of a template
+    if (turned) {
+        const size_t most = kMaxChannelBytes / (turned * sizeof(float));
+        room = most < 1 ? 1 : (most < room ? most : room);
+    }
     const size_t g_elems = (size_t)SC * step * TC_CB * pr.rows_total * 8;
     const size_t n_rows = (size_t)P.T * SC;
     out->form = form;
@@ -1295,6 +1383,10 @@ int tc_begin(const Problem &P, int form, int nb, int tg, int max_templates, Scra
         (rc = ws.get(&out->w, halves * out->w_elems, "tensor-core template blocks")) ||
         (fp32 && (rc = ws.get(&exps, n_rows + SC, "operand exponents"))))
         return rc;
+    if (turned && ws.get(&pr.P.by_channel, room * turned, "per-channel outputs")) {
+        set_error(FMF_OK, "");  // no room for them: written in place
+        pr.P.by_channel = nullptr;
+    }
     uint16_t *g_lo = pairs ? g_hi + g_elems : nullptr;
     pr.g_hi = g_hi;
     pr.g_lo = g_lo;
@@ -1310,13 +1402,23 @@ int tc_begin(const Problem &P, int form, int nb, int tg, int max_templates, Scra
     // chain's
     const int most = (g.k_span + TC_Q - 1) / TC_Q;  // K steps of one pair
     pr.chain_cols = fp32 ? (kChain / most > 1 ? kChain / most : 1) : step * (TC_CB / 2);
-    const long long n = (long long)SC * step * TC_CB * pr.rows_total;
-    if (fp32)
-        tc_data_kernel<true><<<(unsigned)((n + 255) / 256), 256, 0, s>>>(
-            P.data, P.N, SC, step, pr.rows_total, pr.row_front, P.scan, g_hi, g_lo, exps + n_rows, P.scan + 3 * SC);
-    else
-        tc_data_kernel<false><<<(unsigned)((n + 255) / 256), 256, 0, s>>>(
-            P.data, P.N, SC, step, pr.rows_total, pr.row_front, nullptr, g_hi, g_lo, nullptr, nullptr);
+    const unsigned *stat = fp32 ? P.scan : nullptr;
+    int *d_exp = fp32 ? exps + n_rows : nullptr;
+    unsigned *skip = fp32 ? P.scan + 3 * SC : nullptr;
+    if (step <= TC_TURN_STEP && SC <= 65535) {
+        const int rows = tc_turn_rows(step);
+        auto kern = fp32 ? tc_data_kernel<true> : tc_data_kernel<false>;
+        cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxDynamicSmem);
+        if (e != cudaSuccess)
+            return set_error(FMF_ERR_CUDA, "tc_data_kernel shared memory: %s", cudaGetErrorString(e));
+        kern<<<dim3((unsigned)((pr.rows_total + rows - 1) / rows), (unsigned)SC), 256, tc_turn_bytes(step, pairs), s>>>(
+            P.data, P.N, step, pr.rows_total, pr.row_front, stat, g_hi, g_lo, d_exp, skip);
+    } else {
+        const long long n = (long long)SC * step * TC_CB * pr.rows_total;
+        auto kern = fp32 ? tc_data_sparse_kernel<true> : tc_data_sparse_kernel<false>;
+        kern<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(P.data, P.N, SC, step, pr.rows_total, pr.row_front, stat,
+                                                         g_hi, g_lo, d_exp, skip);
+    }
     count_launch();
     return check_launch("tensor-core data streams");
 }
@@ -1352,7 +1454,9 @@ int tc_run_templates(const TcSearch *full, int t0, int nt, unsigned *err, Scratc
         TcProb sub;
         unsigned long long *queue = nullptr;
         if ((rc = tc_templates(full, a, n, s, &sub)) || (rc = ws.get(&queue, 1, "tile queue")) ||
-            (rc = tc_run(&sub, 1, full->form, full->form == TC_FORM_FP32 ? full->parts : 0, queue, err, s)))
+            (!sub.P.by_channel && (rc = clear_outputs(sub.P, s))) ||
+            (rc = tc_run(&sub, 1, full->form, full->form == TC_FORM_FP32 ? full->parts : 0, queue, err, s)) ||
+            (sub.P.by_channel && (rc = launch_channel_outputs(sub.P, sub.skip, s))))
             return rc;
     }
     return FMF_OK;
@@ -1365,7 +1469,7 @@ const unsigned *tc_flag(const TcSearch *full) { return full->pr.skip; }
 int tc_prepare(const Problem &P, int form, int nb, int tg, Scratch &ws, cudaStream_t s, TcProb *out)
 {
     TcSearch st;
-    int rc = tc_begin(P, form, nb, tg, P.T, ws, s, &st);
+    int rc = tc_begin(P, form, nb, tg, P.T, ws, s, &st, false);
     if (rc)
         return rc;
     if (st.room < P.T) {  // a shared launch needs them all at once

@@ -633,6 +633,7 @@ static int variable_device(const VArgs &a, int L, cudaStream_t s, float *host_ou
     P.k_lo = k_lo;
     P.k_hi = k_hi;
     P.out = a.out;
+    P.by_channel = nullptr;
     P.T = T;
     P.SC = SC;
     P.L = L;
