@@ -324,7 +324,11 @@ int prepare_problem(const Args &a, Scratch &ws, cudaStream_t s, Problem *Pout, i
         channel_centre_kernel<<<SC, 1024, 0, s>>>(a.data, N, mu);
         count_launch(2);
     }
-    if ((rc = launch_window_stats(a.data, N, L, SC, mu, dcen, stat_e, place, scan, s)))
+    unsigned *list = nullptr;
+    if (const size_t words = window_list_words(N, SC))
+        if ((rc = ws.get(&list, words, "window statistics")))
+            return rc;
+    if ((rc = launch_window_stats(a.data, N, L, SC, mu, dcen, stat_e, place, scan, list, s)))
         return rc;
     if ((rc = check_launch("preprocessing kernels")))
         return rc;

@@ -250,7 +250,9 @@ StatPlace stat_rows(int SC, int N, int step, int pad, size_t *elems);
 // The same rows without padding, end to end: SC * N elements.
 StatPlace stat_rows_packed(int N, int step);
 int launch_window_stats(const float *data, int N, int L, int SC, const float *mu, float *dcen,
-                        float *stat_e, const StatPlace &place, unsigned *scan, cudaStream_t s);
+                        float *stat_e, const StatPlace &place, unsigned *scan, unsigned *list, cudaStream_t s);
+// Words of `list` (scratch) with which large searches' statistics run faster; 0: none.
+size_t window_list_words(int N, int SC);
 // pad: padding round the statistics' rows (tc_pad); scan: also make Problem::scan.  Does
 // not clear per-channel outputs (clear_outputs).
 int prepare_problem(const Args &a, Scratch &ws, cudaStream_t s, Problem *P, int pad, bool scan);

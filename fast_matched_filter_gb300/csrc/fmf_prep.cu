@@ -429,17 +429,43 @@ struct StatLayout {
 
 size_t window_stats_smem(int L, bool full) { return (size_t)StatLayout(L, full).total * sizeof(float); }
 
-// grid = (ceil(N / kStatWindows), SC), kStatThreads threads, dynamic smem =
-// window_stats_smem(L, FULL).  short: stat_e[ch][u] = sum of d^2 over
+// A block's part of Problem::scan: one atomic per block, and only where it changes the
+// channel's value.  `mem`: shared memory that is not read any more after the first
+// barrier here.
+__device__ __forceinline__ void scan_block(unsigned top, unsigned low, float *mem, unsigned *scan, int ch, int SC)
+{
+    __syncthreads();
+    unsigned *red = reinterpret_cast<unsigned *>(mem);
+    const int warps = blockDim.x >> 5;
+    top = __reduce_max_sync(0xffffffffu, top);
+    low = __reduce_max_sync(0xffffffffu, low);
+    if ((threadIdx.x & 31) == 0) {
+        red[threadIdx.x >> 5] = top;
+        red[32 + (threadIdx.x >> 5)] = low;
+    }
+    __syncthreads();
+    if (threadIdx.x < 2) {
+        unsigned v = 0;
+        for (int i = 0; i < warps; i++)
+            v = max(v, red[32 * threadIdx.x + i]);
+        unsigned *word = scan + threadIdx.x * SC + ch;
+        if (v > *(volatile unsigned *)word)
+            atomicMax(word, v);
+    }
+}
+
+// Blocks of kStatWindows windows of a channel, channel by channel (any grid): all of
+// them, or those of `list` (their count, then their numbers); kStatThreads threads,
+// dynamic smem = window_stats_smem(L, FULL).  short: stat_e[ch][u] = sum of d^2 over
 // [u, u + L); FULL: (centred energy, mean) of d' = d - mu[ch] as float pairs,
 // and the centred data into dcen.  Windows past N - L are not written.  One
 // instantiation per mode: the 'short' one keeps no sums of d' in registers,
 // so three blocks share an SM.
 template <bool FULL, bool SCAN>
 __global__ void __launch_bounds__(kStatThreads, FULL ? 2 : 3)
-window_stats_kernel(const float *__restrict__ data, int N, int L, const float *__restrict__ mu,
+window_stats_kernel(const float *__restrict__ data, int N, int L, int SC, const float *__restrict__ mu,
                     float *__restrict__ dcen, float *__restrict__ stat_e, const StatPlace place,
-                    unsigned *__restrict__ scan)
+                    unsigned *__restrict__ scan, const unsigned *__restrict__ list)
 {
     extern __shared__ float4 stat_smem[];
     constexpr bool full = FULL;
@@ -452,160 +478,388 @@ window_stats_kernel(const float *__restrict__ data, int N, int L, const float *_
     float *out1 = base + lay.out;
     float2 *out2 = reinterpret_cast<float2 *>(base + lay.out);
 
-    const int ch = blockIdx.y;
+    const int per_ch = (N + kStatWindows - 1) / kStatWindows;
+    const unsigned n_blocks = list ? list[0] : (unsigned)per_ch * SC;
+    for (unsigned item = blockIdx.x; item < n_blocks; item += gridDim.x) {
+        const unsigned blk = list ? list[1 + item] : item;
+        const int ch = (int)(blk / per_ch);
+        const long long c0 = (long long)(blk % per_ch) * kStatWindows;
+        const int len = (int)min((long long)kStatWindows + L - 1, (long long)N - c0);
+        const int nwin = min(kStatWindows, len - L + 1);
+        const int span = stat_span(L), nq = span >> 5;
+        const float m = full ? mu[ch] : 0.0f;
+        const float *src = data + (size_t)ch * N + c0;
+        constexpr int kLoads = 4;  // loads in flight per thread before their use
+        unsigned top = 0;          // bits of the largest finite |v|
+        for (int i0 = threadIdx.x; i0 < span; i0 += kLoads * kStatThreads) {
+            float x[kLoads];
+#pragma unroll
+            for (int j = 0; j < kLoads; j++) {
+                const int i = i0 + j * kStatThreads;
+                x[j] = i < len ? __ldg(src + i) : 0.0f;
+            }
+#pragma unroll
+            for (int j = 0; j < kLoads; j++) {
+                const int i = i0 + j * kStatThreads;
+                if (i < span) {
+                    const float v = i < len ? x[j] - m : 0.0f;
+                    if (full && i < kStatWindows && i < len)
+                        dcen[(size_t)ch * N + c0 + i] = v;
+                    const float sq = v * v;
+                    s2[stat_pad(i)] = make_float2(sq, fmaf(v, v, -sq));  // v^2 exactly
+                    if (SCAN) {
+                        const unsigned av = __float_as_uint(v) & 0x7fffffffu;
+                        top = av < 0x7f800000u ? max(top, av) : top;
+                    }
+                    if (full)
+                        s1[stat_pad(i)] = v;
+                }
+            }
+        }
+        __syncthreads();
+        for (int k = threadIdx.x; k < nq; k += kStatThreads) {  // chunk sums
+            float h2 = 0.0f, l2 = 0.0f, h1 = 0.0f, l1 = 0.0f;
+#pragma unroll 8
+            for (int j = 0; j < 32; j++) {
+                const float2 x = s2[stat_pad(32 * k + j)];
+                pair_add(h2, l2, x.x, x.y);
+                if (full)
+                    pair_add(h1, l1, s1[stat_pad(32 * k + j)], 0.0f);
+            }
+            q2[k] = make_float2(h2, l2);
+            if (full)
+                q1[k] = make_float2(h1, l1);
+        }
+        __syncthreads();
+
+        const float Lf = (float)L, invL = 1.0f / Lf;
+        auto emit = [&](int u, float h2, float l2, float h1, float l1) {
+            if (full) {
+                float v, mean;
+                window_centred_sums(h2, l2, h1, l1, Lf, invL, v, mean);
+                out2[stat_pad(u)] = make_float2(v, mean);
+            } else {
+                out1[stat_pad(u)] = h2 + l2;
+            }
+        };
+        if (L >= 32) {
+            // windows u0 .. u0 + 15 of this thread: all start in chunk a and end
+            // past it, so suffix (in chunk a) + whole chunks + tail never overlap
+            const int u0 = threadIdx.x * kStatGroup;
+            if (u0 < nwin) {
+                const int a = u0 >> 5;
+                float sh2[kStatGroup], sl2[kStatGroup], sh1[kStatGroup], sl1[kStatGroup];
+                float h2 = 0.0f, l2 = 0.0f, h1 = 0.0f, l1 = 0.0f;
+                for (int j = u0 + kStatGroup; j < 32 * a + 32; j++) {
+                    const float2 x = s2[stat_pad(j)];
+                    pair_add(h2, l2, x.x, x.y);
+                    if (full)
+                        pair_add(h1, l1, s1[stat_pad(j)], 0.0f);
+                }
+#pragma unroll
+                for (int r = kStatGroup - 1; r >= 0; r--) {  // suffix sums, last start first
+                    const float2 x = s2[stat_pad(u0 + r)];
+                    pair_add(h2, l2, x.x, x.y);
+                    sh2[r] = h2;
+                    sl2[r] = l2;
+                    if (full) {
+                        pair_add(h1, l1, s1[stat_pad(u0 + r)], 0.0f);
+                        sh1[r] = h1;
+                        sl1[r] = l1;
+                    }
+                }
+                const int e0 = u0 + L;  // end (exclusive) of window u0
+                float mh2 = 0.0f, ml2 = 0.0f, mh1 = 0.0f, ml1 = 0.0f;  // whole chunks
+                for (int k = a + 1; k < (e0 >> 5); k++) {
+                    pair_add(mh2, ml2, q2[k].x, q2[k].y);
+                    if (full)
+                        pair_add(mh1, ml1, q1[k].x, q1[k].y);
+                }
+                float rh2 = 0.0f, rl2 = 0.0f, rh1 = 0.0f, rl1 = 0.0f;  // tail in the last chunk
+                for (int j = e0 & ~31; j < e0; j++) {
+                    const float2 x = s2[stat_pad(j)];
+                    pair_add(rh2, rl2, x.x, x.y);
+                    if (full)
+                        pair_add(rh1, rl1, s1[stat_pad(j)], 0.0f);
+                }
+#pragma unroll
+                for (int r = 0; r < kStatGroup; r++) {
+                    const int e = e0 + r;
+                    if (r > 0 && (e & 31) == 0) {  // the tail's chunk is whole: move it to the middle
+                        const int k = (e >> 5) - 1;
+                        pair_add(mh2, ml2, q2[k].x, q2[k].y);
+                        rh2 = rl2 = 0.0f;
+                        if (full) {
+                            pair_add(mh1, ml1, q1[k].x, q1[k].y);
+                            rh1 = rl1 = 0.0f;
+                        }
+                    }
+                    if (u0 + r < nwin) {
+                        float th2 = sh2[r], tl2 = sl2[r], th1 = 0.0f, tl1 = 0.0f;
+                        pair_add(th2, tl2, mh2, ml2);
+                        pair_add(th2, tl2, rh2, rl2);
+                        if (full) {
+                            th1 = sh1[r];
+                            tl1 = sl1[r];
+                            pair_add(th1, tl1, mh1, ml1);
+                            pair_add(th1, tl1, rh1, rl1);
+                        }
+                        emit(u0 + r, th2, tl2, th1, tl1);
+                    }
+                    const float2 x = s2[stat_pad(e)];
+                    pair_add(rh2, rl2, x.x, x.y);
+                    if (full)
+                        pair_add(rh1, rl1, s1[stat_pad(e)], 0.0f);
+                }
+            }
+        } else {  // windows shorter than a chunk: direct sums
+            for (int u = threadIdx.x; u < nwin; u += kStatThreads) {
+                float h2 = 0.0f, l2 = 0.0f, h1 = 0.0f, l1 = 0.0f;
+                for (int j = u; j < u + L; j++) {
+                    const float2 x = s2[stat_pad(j)];
+                    pair_add(h2, l2, x.x, x.y);
+                    if (full)
+                        pair_add(h1, l1, s1[stat_pad(j)], 0.0f);
+                }
+                emit(u, h2, l2, h1, l1);
+            }
+        }
+        __syncthreads();
+        // energies at or below this pass no template's threshold
+        const float dead = SCAN ? kThreshold / __uint_as_float(scan[2 * SC + ch]) * 0.999f : 0.0f;
+        unsigned low = 0;  // the smallest energy above it, bits complemented
+        float *row = stat_e + ch * place.ch * (full ? 2 : 1);
+        // coalesced stores: windows in order, or (step > 1) row by row, `per` of each
+        const int step = place.step, per = step == 1 ? nwin : (nwin + step - 1) / step;
+        const int head = step == 1 ? 0 : (int)(c0 % step);  // row of window 0
+        const long long x0 = step == 1 ? c0 : c0 / step;    // and its place there
+        for (int i = threadIdx.x; i < per * step; i += kStatThreads) {
+            int u = i;
+            long long o = c0 + i;
+            if (step > 1) {
+                const int r = i / per, j = i - r * per;  // the r-th row from window 0's, its j-th window
+                u = r + j * step;
+                if (u >= nwin)
+                    continue;
+                const int psi = head + r < step ? head + r : head + r - step;
+                o = psi * place.ps + min(psi, place.rem) + x0 + j + (head + r < step ? 0 : 1);
+            }
+            float en;
+            if (full) {
+                const float2 v = out2[stat_pad(u)];
+                reinterpret_cast<float2 *>(row)[o] = v;
+                en = v.x;
+            } else {
+                en = out1[stat_pad(u)];
+                row[o] = en;
+            }
+            if (SCAN && en > dead)
+                low = max(low, ~__float_as_uint(en));
+        }
+        if (SCAN)
+            scan_block(top, low, base, scan, ch, SC);
+        __syncthreads();  // shared memory is free for the next block
+    }
+}
+
+// ---------------------------------------------------------------- the usual blocks
+// The same statistics from exact running sums in fixed point, which take a third of
+// the instructions, for blocks of windows whose values lie close enough together;
+// the others go on the list for window_stats_kernel.
+//
+// A block's squares are rounded to the unit 2^(2e - 40), all its |v| below 2^e; the sums
+// of a window's squares are exact, so only the squares' own rounding remains, half
+// a unit each ('full': with the squares' exact remainders and the mean's rounding, two
+// units).  The block stays here if every window's energy is at least L 2^27 units (or,
+// for 'short', exactly zero), so that rounding is at most 2^-26 (2^-28) of it, half of
+// its float's own rounding: windows down to 1/90 of the block's largest value in
+// amplitude.  A transient on quiet noise, a value that is not finite, a level shift
+// or a window that ends in a gap send their block to the list.
+//
+// A number in units is two 20-bit digits, which magic-number additions take from
+// floats without conversion instructions (64-bit conversions run on the FP64 pipe:
+// 322 us below); the digits' running sums are 32-bit integers that wrap, and the
+// differences of one window fit them (L <= 2,048).  Chunks of 16 samples, a thread
+// each: running sums inside the chunk, then a scan of the chunks' sums.
+//
+// What bounds it: the instructions, mostly integer ones.  60 channels x 1.08M samples x
+// 600 taps: 354 us with window_stats_kernel alone, 233 us here and 3 us for the second
+// launch; 'full', 30 channels x 8.6M: 1,161 us and 903 + 3 us.
+constexpr int kFixThreads = 512;
+constexpr int kFixChunk = 16;
+constexpr int kFixBits = 40, kFixDigit = 20;
+constexpr int kFixLongest = 2048;
+// Fewer blocks than this are one or two rounds of the SMs either way, and the second
+// launch would cost more than it saves.
+constexpr int kFixLeastBlocks = 608;
+static_assert((kStatWindows + kFixLongest + kFixChunk) / kFixChunk <= kFixThreads, "a thread per chunk");
+
+struct FixLayout {  // in 4-byte words: samples, running sums of d^2 and d, chunk offsets of both
+    int chunks, padded, p2, p1, o2, o1, total;
+    __host__ __device__ FixLayout(int L, bool full)
+    {
+        chunks = (kStatWindows + L + kFixChunk) / kFixChunk;
+        padded = chunks * (kFixChunk + 1);
+        p2 = (padded + 3) & ~3;
+        p1 = p2 + 2 * padded;
+        o2 = p1 + (full ? 2 * padded : 0);
+        o1 = o2 + 2 * chunks;
+        total = o1 + (full ? 2 * chunks : 0);
+    }
+    size_t bytes() const { return (size_t)total * 4; }
+};
+
+// x in units, |x| < 2^40, as digits: adds them to hi and lo.  (1.5 * 2^23 + integer:
+// the integer, rounded to nearest, is in the low bits.)
+__device__ __forceinline__ void fix_add(float x, unsigned &hi, unsigned &lo)
+{
+    const float magic = 12582912.0f;  // 1.5 * 2^23 = 0x4b400000
+    const float t = fmaf(x, 1.0f / (1 << kFixDigit), magic);
+    const float rest = fmaf(-(t - magic), (float)(1 << kFixDigit), x);  // exact, at most 2^19
+    hi += __float_as_uint(t) - 0x4b400000u;
+    lo += __float_as_uint(rest + magic) - 0x4b400000u;
+}
+
+// hi 2^20 + lo as a float pair (hi in [-2^31, 2^31), |lo| <= 2^30): three exact parts.
+__device__ __forceinline__ void fix_pair(int hi, int lo, float &h, float &l)
+{
+    const float f1 = (float)(hi >> 8) * 268435456.0f;                       // 2^28
+    const float f2 = (float)(((hi & 255) << 12) + (lo >> 8)) * 256.0f;
+    float e;
+    h = two_diff(f1, -f2, e);
+    l = e + (float)(lo & 255);
+}
+
+// grid = (ceil(N / kStatWindows), SC), kFixThreads threads, dynamic smem FixLayout.
+template <bool FULL, bool SCAN>
+__global__ void __launch_bounds__(kFixThreads, FULL ? 2 : 3)
+window_fixed_kernel(const float *__restrict__ data, int N, int L, const float *__restrict__ mu,
+                    float *__restrict__ dcen, float *__restrict__ stat_e, const StatPlace place,
+                    unsigned *__restrict__ scan, unsigned *__restrict__ list)
+{
+    extern __shared__ float4 stat_smem[];
+    __shared__ uint2 warp_sums[2][kFixThreads / 32];
+    __shared__ unsigned shared_top;
+    __shared__ int odd;  // the block goes on the list
+    const FixLayout lay(L, FULL);
+    float *raw = reinterpret_cast<float *>(stat_smem);
+    uint2 *p2 = reinterpret_cast<uint2 *>(raw + lay.p2), *p1 = reinterpret_cast<uint2 *>(raw + lay.p1);
+    uint2 *o2 = reinterpret_cast<uint2 *>(raw + lay.o2), *o1 = reinterpret_cast<uint2 *>(raw + lay.o1);
+    const int chunks = lay.chunks, span = chunks * kFixChunk;
+    const auto pad = [](int i) { return i + (i >> 4); };
+
+    const int ch = blockIdx.y, SC = gridDim.y;
     const long long c0 = (long long)blockIdx.x * kStatWindows;
     const int len = (int)min((long long)kStatWindows + L - 1, (long long)N - c0);
     const int nwin = min(kStatWindows, len - L + 1);
-    const int span = stat_span(L), nq = span >> 5;
-    const float m = full ? mu[ch] : 0.0f;
+    const float m = FULL ? mu[ch] : 0.0f;
     const float *src = data + (size_t)ch * N + c0;
-    constexpr int kLoads = 4;  // loads in flight per thread before their use
-    unsigned top = 0;          // bits of the largest finite |v|
-    for (int i0 = threadIdx.x; i0 < span; i0 += kLoads * kStatThreads) {
+    if (threadIdx.x == 0) {
+        shared_top = 0;
+        odd = 0;
+    }
+    unsigned top = 0;   // bits of the largest |v|; of a value that is not finite, too
+    unsigned most = 0;  // bits of the largest finite one
+    float *dst = FULL ? dcen + (size_t)ch * N + c0 : nullptr;
+    constexpr int kLoads = 5;
+    for (int i0 = threadIdx.x; i0 < span; i0 += kLoads * kFixThreads) {
         float x[kLoads];
 #pragma unroll
         for (int j = 0; j < kLoads; j++) {
-            const int i = i0 + j * kStatThreads;
-            x[j] = i < len ? __ldg(src + i) : 0.0f;
+            const int i = i0 + j * kFixThreads;
+            x[j] = i < len ? __ldg(src + i) : m;
         }
 #pragma unroll
         for (int j = 0; j < kLoads; j++) {
-            const int i = i0 + j * kStatThreads;
+            const int i = i0 + j * kFixThreads;
             if (i < span) {
-                const float v = i < len ? x[j] - m : 0.0f;
-                if (full && i < kStatWindows && i < len)
-                    dcen[(size_t)ch * N + c0 + i] = v;
-                const float sq = v * v;
-                s2[stat_pad(i)] = make_float2(sq, fmaf(v, v, -sq));  // v^2 exactly
-                if (SCAN) {
-                    const unsigned av = __float_as_uint(v) & 0x7fffffffu;
-                    top = av < 0x7f800000u ? max(top, av) : top;
-                }
-                if (full)
-                    s1[stat_pad(i)] = v;
+                const float v = FULL ? x[j] - m : x[j];
+                if (FULL && i < kStatWindows && i < len)
+                    dst[i] = v;
+                const unsigned av = __float_as_uint(v) & 0x7fffffffu;
+                top = max(top, av);
+                if (SCAN)
+                    most = av < 0x7f800000u ? max(most, av) : most;
+                raw[pad(i)] = v;
             }
         }
     }
     __syncthreads();
-    for (int k = threadIdx.x; k < nq; k += kStatThreads) {  // chunk sums
-        float h2 = 0.0f, l2 = 0.0f, h1 = 0.0f, l1 = 0.0f;
-#pragma unroll 8
-        for (int j = 0; j < 32; j++) {
-            const float2 x = s2[stat_pad(32 * k + j)];
-            pair_add(h2, l2, x.x, x.y);
-            if (full)
-                pair_add(h1, l1, s1[stat_pad(32 * k + j)], 0.0f);
-        }
-        q2[k] = make_float2(h2, l2);
-        if (full)
-            q1[k] = make_float2(h1, l1);
-    }
+    top = __reduce_max_sync(0xffffffffu, top);
+    if ((threadIdx.x & 31) == 0)
+        atomicMax(&shared_top, top);
     __syncthreads();
-
+    top = shared_top;
+    const int e = top ? (int)(top >> 23) - 126 : 0;  // every |v| < 2^e
+    const bool bad = e < -38 || e > 60;              // (infinities and NaN have the largest e)
+    bool lost = false;  // some square is not zero but less than half a unit ('short')
+    const auto pow2 = [](int k) { return __int_as_float((k + 127) << 23); };
+    if (!bad) {
+        const float s = pow2(kFixBits / 2 - e);  // squares of s v are in units
+        uint2 t2 = make_uint2(0, 0), t1 = make_uint2(0, 0);
+        const int c = threadIdx.x;
+        if (c < chunks) {
+            const int at = c * (kFixChunk + 1);
+#pragma unroll
+            for (int j = 0; j < kFixChunk; j++) {
+                const float v = raw[at + j] * s, sq = v * v;
+                p2[at + j] = t2;
+                fix_add(sq, t2.x, t2.y);
+                if (FULL) {  // the square's remainder, at most 2^16 units
+                    t2.y += __float_as_uint(fmaf(v, v, -sq) + 12582912.0f) - 0x4b400000u;
+                    p1[at + j] = t1;
+                    fix_add(v * (float)(1 << kFixBits / 2), t1.x, t1.y);
+                } else {
+                    lost = lost || (sq < 0.5f && v != 0.0f);
+                }
+            }
+        }
+        // exclusive scan of the chunks' sums
+        const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+        const auto scan_chunks = [&](uint2 t, uint2 *sums, uint2 *to) {
+            uint2 y = t;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const unsigned a = __shfl_up_sync(0xffffffffu, y.x, o), b = __shfl_up_sync(0xffffffffu, y.y, o);
+                if (lane >= o) {
+                    y.x += a;
+                    y.y += b;
+                }
+            }
+            if (lane == 31)
+                sums[wid] = y;
+            __syncthreads();
+            unsigned hx = 0, lx = 0;
+            for (int i = 0; i < wid; i++) {
+                hx += sums[i].x;
+                lx += sums[i].y;
+            }
+            if (c < chunks)
+                to[c] = make_uint2(hx + y.x - t.x, lx + y.y - t.y);
+        };
+        scan_chunks(t2, warp_sums[0], o2);
+        if (FULL)
+            scan_chunks(t1, warp_sums[1], o1);
+        lost = __syncthreads_or(lost) != 0;
+    }
     const float Lf = (float)L, invL = 1.0f / Lf;
-    auto emit = [&](int u, float h2, float l2, float h1, float l1) {
-        if (full) {
-            float v, mean;
-            window_centred_sums(h2, l2, h1, l1, Lf, invL, v, mean);
-            out2[stat_pad(u)] = make_float2(v, mean);
-        } else {
-            out1[stat_pad(u)] = h2 + l2;
-        }
-    };
-    if (L >= 32) {
-        // windows u0 .. u0 + 15 of this thread: all start in chunk a and end
-        // past it, so suffix (in chunk a) + whole chunks + tail never overlap
-        const int u0 = threadIdx.x * kStatGroup;
-        if (u0 < nwin) {
-            const int a = u0 >> 5;
-            float sh2[kStatGroup], sl2[kStatGroup], sh1[kStatGroup], sl1[kStatGroup];
-            float h2 = 0.0f, l2 = 0.0f, h1 = 0.0f, l1 = 0.0f;
-            for (int j = u0 + kStatGroup; j < 32 * a + 32; j++) {
-                const float2 x = s2[stat_pad(j)];
-                pair_add(h2, l2, x.x, x.y);
-                if (full)
-                    pair_add(h1, l1, s1[stat_pad(j)], 0.0f);
-            }
-#pragma unroll
-            for (int r = kStatGroup - 1; r >= 0; r--) {  // suffix sums, last start first
-                const float2 x = s2[stat_pad(u0 + r)];
-                pair_add(h2, l2, x.x, x.y);
-                sh2[r] = h2;
-                sl2[r] = l2;
-                if (full) {
-                    pair_add(h1, l1, s1[stat_pad(u0 + r)], 0.0f);
-                    sh1[r] = h1;
-                    sl1[r] = l1;
-                }
-            }
-            const int e0 = u0 + L;  // end (exclusive) of window u0
-            float mh2 = 0.0f, ml2 = 0.0f, mh1 = 0.0f, ml1 = 0.0f;  // whole chunks
-            for (int k = a + 1; k < (e0 >> 5); k++) {
-                pair_add(mh2, ml2, q2[k].x, q2[k].y);
-                if (full)
-                    pair_add(mh1, ml1, q1[k].x, q1[k].y);
-            }
-            float rh2 = 0.0f, rl2 = 0.0f, rh1 = 0.0f, rl1 = 0.0f;  // tail in the last chunk
-            for (int j = e0 & ~31; j < e0; j++) {
-                const float2 x = s2[stat_pad(j)];
-                pair_add(rh2, rl2, x.x, x.y);
-                if (full)
-                    pair_add(rh1, rl1, s1[stat_pad(j)], 0.0f);
-            }
-#pragma unroll
-            for (int r = 0; r < kStatGroup; r++) {
-                const int e = e0 + r;
-                if (r > 0 && (e & 31) == 0) {  // the tail's chunk is whole: move it to the middle
-                    const int k = (e >> 5) - 1;
-                    pair_add(mh2, ml2, q2[k].x, q2[k].y);
-                    rh2 = rl2 = 0.0f;
-                    if (full) {
-                        pair_add(mh1, ml1, q1[k].x, q1[k].y);
-                        rh1 = rl1 = 0.0f;
-                    }
-                }
-                if (u0 + r < nwin) {
-                    float th2 = sh2[r], tl2 = sl2[r], th1 = 0.0f, tl1 = 0.0f;
-                    pair_add(th2, tl2, mh2, ml2);
-                    pair_add(th2, tl2, rh2, rl2);
-                    if (full) {
-                        th1 = sh1[r];
-                        tl1 = sl1[r];
-                        pair_add(th1, tl1, mh1, ml1);
-                        pair_add(th1, tl1, rh1, rl1);
-                    }
-                    emit(u0 + r, th2, tl2, th1, tl1);
-                }
-                const float2 x = s2[stat_pad(e)];
-                pair_add(rh2, rl2, x.x, x.y);
-                if (full)
-                    pair_add(rh1, rl1, s1[stat_pad(e)], 0.0f);
-            }
-        }
-    } else {  // windows shorter than a chunk: direct sums
-        for (int u = threadIdx.x; u < nwin; u += kStatThreads) {
-            float h2 = 0.0f, l2 = 0.0f, h1 = 0.0f, l1 = 0.0f;
-            for (int j = u; j < u + L; j++) {
-                const float2 x = s2[stat_pad(j)];
-                pair_add(h2, l2, x.x, x.y);
-                if (full)
-                    pair_add(h1, l1, s1[stat_pad(j)], 0.0f);
-            }
-            emit(u, h2, l2, h1, l1);
-        }
-    }
-    __syncthreads();
+    const float u2 = pow2(bad ? 0 : 2 * e - kFixBits), u1 = pow2(bad ? 0 : e - kFixBits);
+    const float least = Lf * 0x1p27f * u2;  // energy below which the unit is too coarse
     // energies at or below this pass no template's threshold
-    const float dead = SCAN ? kThreshold / __uint_as_float(scan[2 * gridDim.y + ch]) * 0.999f : 0.0f;
+    const float dead = SCAN ? kThreshold / __uint_as_float(scan[2 * SC + ch]) * 0.999f : 0.0f;
     unsigned low = 0;  // the smallest energy above it, bits complemented
-    float *row = stat_e + ch * place.ch * (full ? 2 : 1);
+    float *row = stat_e + ch * place.ch * (FULL ? 2 : 1);
     // coalesced stores: windows in order, or (step > 1) row by row, `per` of each
     const int step = place.step, per = step == 1 ? nwin : (nwin + step - 1) / step;
     const int head = step == 1 ? 0 : (int)(c0 % step);  // row of window 0
     const long long x0 = step == 1 ? c0 : c0 / step;    // and its place there
-    for (int i = threadIdx.x; i < per * step; i += kStatThreads) {
+    if (step == 1)
+        row += c0 * (FULL ? 2 : 1);
+    bool far = false;  // a window too quiet for the block's unit
+    const int n_items = bad ? 0 : per * step;
+    for (int i = threadIdx.x; i < n_items; i += kFixThreads) {
         int u = i;
-        long long o = c0 + i;
+        long long o = i;
         if (step > 1) {
             const int r = i / per, j = i - r * per;  // the r-th row from window 0's, its j-th window
             u = r + j * step;
@@ -614,36 +868,37 @@ window_stats_kernel(const float *__restrict__ data, int N, int L, const float *_
             const int psi = head + r < step ? head + r : head + r - step;
             o = psi * place.ps + min(psi, place.rem) + x0 + j + (head + r < step ? 0 : 1);
         }
+        const int a = pad(u), b = pad(u + L), ca = u >> 4, cb = (u + L) >> 4;
+        const uint2 pa2 = p2[a], pb2 = p2[b], qa2 = o2[ca], qb2 = o2[cb];
+        const unsigned hi2 = pb2.x + qb2.x - (pa2.x + qa2.x);
+        const int lo2 = (int)(pb2.y + qb2.y - (pa2.y + qa2.y));
         float en;
-        if (full) {
-            const float2 v = out2[stat_pad(u)];
-            reinterpret_cast<float2 *>(row)[o] = v;
-            en = v.x;
+        if constexpr (FULL) {
+            const uint2 pa1 = p1[a], pb1 = p1[b], qa1 = o1[ca], qb1 = o1[cb];
+            float h2, l2, h1, l1, mean;
+            fix_pair((int)hi2, lo2, h2, l2);
+            fix_pair((int)(pb1.x + qb1.x - (pa1.x + qa1.x)), (int)(pb1.y + qb1.y - (pa1.y + qa1.y)), h1, l1);
+            window_centred_sums(h2 * u2, l2 * u2, h1 * u1, l1 * u1, Lf, invL, en, mean);
+            far = far || !(en >= least);
+            reinterpret_cast<float2 *>(row)[o] = make_float2(en, mean);
         } else {
-            en = out1[stat_pad(u)];
+            // the top 24 bits and the rest, added with one rounding
+            const float f = fmaf((float)(hi2 >> 8), 268435456.0f, (float)((int)((hi2 & 255) << 20) + lo2));
+            en = f * u2;
+            far = far || (en < least && (en != 0.0f || lost));
             row[o] = en;
         }
         if (SCAN && en > dead)
             low = max(low, ~__float_as_uint(en));
     }
-    if (SCAN) {  // one atomic per block, and only where it changes the channel's value
-        unsigned *red = reinterpret_cast<unsigned *>(base);  // the squares are no longer read
-        top = __reduce_max_sync(0xffffffffu, top);
-        low = __reduce_max_sync(0xffffffffu, low);
-        if ((threadIdx.x & 31) == 0) {
-            red[threadIdx.x >> 5] = top;
-            red[32 + (threadIdx.x >> 5)] = low;
-        }
-        __syncthreads();
-        if (threadIdx.x < 2) {
-            unsigned v = 0;
-            for (int i = 0; i < kStatThreads / 32; i++)
-                v = max(v, red[32 * threadIdx.x + i]);
-            unsigned *word = scan + threadIdx.x * gridDim.y + ch;
-            if (v > *(volatile unsigned *)word)
-                atomicMax(word, v);
-        }
-    }
+    if (far || bad)
+        odd = 1;  // (any thread's)
+    __syncthreads();
+    if (odd && threadIdx.x == 0 && nwin > 0)
+        list[1 + atomicAdd(list, 1u)] = blockIdx.y * gridDim.x + blockIdx.x;
+    // the largest value counts in any case; the smallest energy of a listed block is made there
+    if (SCAN)
+        scan_block(most, odd ? 0u : low, raw, scan, ch, SC);
 }
 
 StatPlace stat_rows(int SC, int N, int step, int pad, size_t *elems)
@@ -659,20 +914,42 @@ StatPlace stat_rows(int SC, int N, int step, int pad, size_t *elems)
 
 StatPlace stat_rows_packed(int N, int step) { return StatPlace{(long long)N, N / step, N % step, step}; }
 
+size_t window_list_words(int N, int SC)
+{
+    const long long blocks = (long long)((N + kStatWindows - 1) / kStatWindows) * SC;
+    return blocks >= kFixLeastBlocks && blocks < 0x7fffffffLL ? (size_t)blocks + 1 : 0;
+}
+
 int launch_window_stats(const float *data, int N, int L, int SC, const float *mu, float *dcen,
-                        float *stat_e, const StatPlace &place, unsigned *scan, cudaStream_t s)
+                        float *stat_e, const StatPlace &place, unsigned *scan, unsigned *list, cudaStream_t s)
 {
     const bool full = mu != nullptr;
+    const int per_ch = (N + kStatWindows - 1) / kStatWindows;
+    unsigned grid = (unsigned)per_ch * SC;
+    cudaError_t e;
+    const size_t fixed = FixLayout(L, full).bytes();
+    if (fixed > (size_t)kMaxDynamicSmem - 1024 || L > kFixLongest || SC > 65535)
+        list = nullptr;
+    if (list) {
+        auto kern = scan ? (full ? window_fixed_kernel<true, true> : window_fixed_kernel<false, true>)
+                         : (full ? window_fixed_kernel<true, false> : window_fixed_kernel<false, false>);
+        e = cudaMemsetAsync(list, 0, sizeof(unsigned), s);
+        if (e == cudaSuccess)
+            e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxDynamicSmem - 1024);
+        if (e != cudaSuccess)
+            return set_error(FMF_ERR_CUDA, "window statistics: %s", cudaGetErrorString(e));
+        kern<<<dim3(per_ch, SC), kFixThreads, fixed, s>>>(data, N, L, mu, dcen, stat_e, place, scan, list);
+        count_launch();
+        grid = grid < 608 ? grid : 608;  // the listed blocks, few or none
+    }
+    auto kern = scan ? (full ? window_stats_kernel<true, true> : window_stats_kernel<false, true>)
+                     : (full ? window_stats_kernel<true, false> : window_stats_kernel<false, false>);
     const size_t smem = window_stats_smem(L, full);
-    void (*kern)(const float *, int, int, const float *, float *, float *, const StatPlace, unsigned *) =
-        scan ? (full ? window_stats_kernel<true, true> : window_stats_kernel<false, true>)
-             : (full ? window_stats_kernel<true, false> : window_stats_kernel<false, false>);
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxDynamicSmem);
+    e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxDynamicSmem);
     if (e != cudaSuccess)
         return set_error(FMF_ERR_CUDA, "window statistics shared memory (%zu bytes): %s", smem,
                          cudaGetErrorString(e));
-    dim3 grid((N + kStatWindows - 1) / kStatWindows, SC);
-    kern<<<grid, kStatThreads, smem, s>>>(data, N, L, mu, dcen, stat_e, place, scan);
+    kern<<<grid, kStatThreads, smem, s>>>(data, N, L, SC, mu, dcen, stat_e, place, scan, list);
     count_launch();
     return FMF_OK;
 }
