@@ -328,7 +328,12 @@ int prepare_problem(const Args &a, Scratch &ws, cudaStream_t s, Problem *Pout, i
     if (const size_t words = window_list_words(N, SC))
         if ((rc = ws.get(&list, words, "window statistics")))
             return rc;
-    if ((rc = launch_window_stats(a.data, N, L, SC, mu, dcen, stat_e, place, scan, list, s)))
+    unsigned *dc = nullptr;
+    if (full && a.precision == FMF_PREC_AUTO)
+        if ((rc = ws.get(&dc, (size_t)SC, "precision estimate")) ||
+            (rc = cuda_status(cudaMemsetAsync(dc, 0, SC * sizeof(unsigned), s), "clearing the precision estimate")))
+            return rc;
+    if ((rc = launch_window_stats(a.data, N, L, SC, mu, dcen, stat_e, place, scan, dc, list, s)))
         return rc;
     if ((rc = check_launch("preprocessing kernels")))
         return rc;
@@ -363,6 +368,7 @@ int prepare_problem(const Args &a, Scratch &ws, cudaStream_t s, Problem *Pout, i
     P.zweight = nullptr;
     P.vp_norm = P.vp_bias = P.vp_scale = nullptr;
     P.scan = scan;
+    P.dc = dc;
     P.only_if = nullptr;
 
     P.by_channel = nullptr;

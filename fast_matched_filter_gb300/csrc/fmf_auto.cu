@@ -21,7 +21,7 @@
 // over the taps that carry the energy.  D_ch = 1 for 'short'; for 'full' the
 // products are of the centred data d - c, whose window mean m adds to every
 // product's size: D_ch = 1 + max over windows of L m^2 / V (V the window's
-// centred energy), sampled every kAutoStride windows.
+// centred energy), sampled every kDcStride windows.
 //
 // Per-channel lengths sum atanh(cc_ch) * z_ch (z_ch = sqrt(n - 3) w_ch) and
 // map the sum through tanh (matched_filter.c:596-601, 405-408): an error in
@@ -44,64 +44,36 @@ namespace fmf {
 constexpr float kSplitRms = 4.4e-6f;   // RMS relative error of one split-bf16 product
 constexpr float kSplitBias = 2.8e-6f;  // bias per unit |cc| at a power-of-two copy
 constexpr float kAutoTol = 1e-5f;
-constexpr int kAutoStride = 7;
 constexpr float kFisherAmp = 1.0f / (1.0f - 0.9f * 0.9f);  // 1 / (1 - cc^2) at |cc| = 0.9
 
-// grid = SC, 256 threads: D_ch - 1 of 'full' from the (centred energy, mean)
-// window statistics of the fixed-length path.
-__global__ void auto_dc_stats_kernel(const float2 *__restrict__ stat, long long stat_ch, long long stat_ps,
-                                     int stat_rem, int step, int nwin, int L, float *__restrict__ dc)
-{
-    __shared__ float red[8];
-    const float2 *row = stat + blockIdx.x * stat_ch;
-    float mx = 0.0f;
-    for (int u = threadIdx.x * kAutoStride; u < nwin; u += blockDim.x * kAutoStride) {
-        const float2 vm = row[(u % step) * stat_ps + min(u % step, stat_rem) + u / step];
-        if (vm.x > 0.0f)
-            mx = fmaxf(mx, (float)L * vm.y * vm.y / vm.x);
-    }
-    for (int o = 16; o > 0; o >>= 1)
-        mx = fmaxf(mx, __shfl_down_sync(0xffffffffu, mx, o));
-    if ((threadIdx.x & 31) == 0)
-        red[threadIdx.x >> 5] = mx;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        for (int i = 1; i < (int)(blockDim.x >> 5); i++)
-            mx = fmaxf(mx, red[i]);
-        dc[blockIdx.x] = mx;
-    }
-}
-
-// The same from the running sums of the per-channel-length path, for windows
-// of the longest length L.
+// D_ch - 1 of 'full' from the running sums of the per-channel-length path, for
+// windows of the longest length L, as float bits (zero before the launch).  grid =
+// (parts, SC), 256 threads, a few windows each: the loads' latency bounds it (31 us for
+// 12 channels x 1M samples), so the channels are spread over all SMs.  (With a common
+// length the statistics kernels make it from the windows they hold: a pass of its own
+// with a block per channel took 882 us of a search of 30 channels x 8.6M samples, this
+// 80 us.)
 __global__ void auto_dc_prefix_kernel(const long long *__restrict__ pre2q,
                                       const float *__restrict__ unit2,
                                       const float2 *__restrict__ pre1f, long long pre_ch, long long pre_ps,
-                                      int step, int N, int L, float *__restrict__ dc)
+                                      int step, int N, int L, unsigned *__restrict__ dc)
 {
-    __shared__ float red[8];
-    const int ch = blockIdx.x;
+    const int ch = blockIdx.y;
     const long long *p2 = pre2q + ch * pre_ch;
     const float2 *p1 = pre1f + ch * pre_ch;
     const auto at = [=](int u) { return (u % step) * pre_ps + u / step; };
     const float q = unit2[ch], nf = (float)L, inv_n = 1.0f / nf;
     float mx = 0.0f;
-    for (int u = threadIdx.x * kAutoStride; u + L <= N; u += blockDim.x * kAutoStride) {
+    for (unsigned u = (blockIdx.x * blockDim.x + threadIdx.x) * kDcStride; u <= (unsigned)(N - L);
+         u += gridDim.x * blockDim.x * kDcStride) {
         float v, mean;
         window_centred(p2[at(u)], p2[at(u + L)], q, p1[at(u)], p1[at(u + L)], nf, inv_n, v, mean);
         if (v > 0.0f)
             mx = fmaxf(mx, nf * mean * mean / v);
     }
-    for (int o = 16; o > 0; o >>= 1)
-        mx = fmaxf(mx, __shfl_down_sync(0xffffffffu, mx, o));
+    const unsigned top = __reduce_max_sync(0xffffffffu, __float_as_uint(mx));
     if ((threadIdx.x & 31) == 0)
-        red[threadIdx.x >> 5] = mx;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        for (int i = 1; i < (int)(blockDim.x >> 5); i++)
-            mx = fmaxf(mx, red[i]);
-        dc[ch] = mx;
-    }
+        atomicMax(dc + ch, top);
 }
 
 // grid = T, 256 threads (8 warps, one channel per warp at a time): the
@@ -110,7 +82,7 @@ __global__ void auto_dc_prefix_kernel(const long long *__restrict__ pre2q,
 // network sum of per-channel lengths, ln_m = ln(channel windows).
 __global__ void auto_template_kernel(const float *__restrict__ tpl, const float *__restrict__ w,
                                      const int *__restrict__ ntap, int SC, int L,
-                                     const float *__restrict__ dc, int network_sum, float k,
+                                     const unsigned *__restrict__ dc, int network_sum, float k,
                                      float ln_m, unsigned *__restrict__ worst)
 {
     __shared__ float sw[8], sv[8], smax[8];
@@ -137,7 +109,7 @@ __global__ void auto_template_kernel(const float *__restrict__ tpl, const float 
             ch_max = INFINITY;  // Fisher z of a few taps: FP32
         } else if (lane == 0 && s4 > 0.0f) {
             const float leff = s2 * s2 / s4;
-            const float d = 1.0f + (dc ? dc[ch] : 0.0f);
+            const float d = 1.0f + (dc ? __uint_as_float(dc[ch]) : 0.0f);
             const float s = kSplitRms * sqrtf(d / leff);  // per-channel standard deviation
             if (ntap) {  // Fisher z: weight z = sqrt(n - 3) w, amplification A
                 const float z = sqrtf((float)(n - 3)) * wc;
@@ -177,22 +149,25 @@ int choose_auto_precision(const Problem &P, Scratch &ws, cudaStream_t s, int *pr
 {
     int rc;
     unsigned *worst = nullptr;
-    float *dc = nullptr;
+    unsigned *dc = P.dc;
     if ((rc = ws.get(&worst, 1, "precision estimate")))
         return rc;
     cudaError_t e = cudaMemsetAsync(worst, 0, sizeof(unsigned), s);
     if (e != cudaSuccess)
         return set_error(FMF_ERR_CUDA, "precision estimate: %s", cudaGetErrorString(e));
-    if (P.normalize == 1) {
+    if (P.normalize == 1 && P.pre2q) {
         if ((rc = ws.get(&dc, (size_t)P.SC, "precision estimate")))
             return rc;
-        if (P.pre2q)
-            auto_dc_prefix_kernel<<<P.SC, 256, 0, s>>>(P.pre2q, P.unit2, P.pre1f, P.pre_ch, P.pre_ps, P.step, P.N,
-                                                       P.L, dc);
-        else
-            auto_dc_stats_kernel<<<P.SC, 256, 0, s>>>(reinterpret_cast<const float2 *>(P.stat_e), P.stat_ch,
-                                                      P.stat_ps, P.stat_rem, P.step, P.N - P.L + 1, P.L, dc);
-        count_launch();
+        if ((e = cudaMemsetAsync(dc, 0, P.SC * sizeof(unsigned), s)) != cudaSuccess)
+            return set_error(FMF_ERR_CUDA, "precision estimate: %s", cudaGetErrorString(e));
+        const int rounds = 1 + P.N / (kDcStride * 2048);  // eight windows a thread
+        for (int c0 = 0; c0 < P.SC; c0 += 65535) {
+            const int nc = P.SC - c0 < 65535 ? P.SC - c0 : 65535;
+            auto_dc_prefix_kernel<<<dim3(rounds, nc), 256, 0, s>>>(P.pre2q + c0 * P.pre_ch, P.unit2 + c0,
+                                                                   P.pre1f + c0 * P.pre_ch, P.pre_ch, P.pre_ps,
+                                                                   P.step, P.N, P.L, dc + c0);
+            count_launch();
+        }
     }
     const double outputs = (double)P.T * P.n_corr * (P.network_sum ? 1 : P.SC);
     const float k = (float)(std::sqrt(2.0 * std::log(outputs > 2.0 ? outputs : 2.0)) + 3.0);

@@ -63,6 +63,9 @@ struct Problem {
     // largest template energy on it; the search's flag: the scan or the operands
     // left it to the CUDA-core kernel
     unsigned *scan;
+    // FMF_PREC_AUTO of 'full' with a common length, else null: the largest D - 1 of the
+    // window of channel ch over every kDcStride-th window, as float bits [SC]
+    unsigned *dc;
     const unsigned *only_if;  // plain kernel: run only if this word is nonzero (null: always)
 };
 
@@ -249,8 +252,10 @@ struct StatPlace {  // where Problem::stat_e has its rows
 StatPlace stat_rows(int SC, int N, int step, int pad, size_t *elems);
 // The same rows without padding, end to end: SC * N elements.
 StatPlace stat_rows_packed(int N, int step);
+constexpr int kDcStride = 7;  // windows of the precision estimate
 int launch_window_stats(const float *data, int N, int L, int SC, const float *mu, float *dcen,
-                        float *stat_e, const StatPlace &place, unsigned *scan, unsigned *list, cudaStream_t s);
+                        float *stat_e, const StatPlace &place, unsigned *scan, unsigned *dc, unsigned *list,
+                        cudaStream_t s);
 // Words of `list` (scratch) with which large searches' statistics run faster; 0: none.
 size_t window_list_words(int N, int SC);
 // pad: padding round the statistics' rows (tc_pad); scan: also make Problem::scan.  Does

@@ -192,7 +192,7 @@ extern "C" int fmf_matched_filter_noalloc(const float *templates, const float *s
         channel_centre_kernel<<<SC, 1024, 0, s>>>(data, N, mu);
         count_launch(2);
     }
-    if ((rc = launch_window_stats(data, N, L, SC, mu, dcen, stat_e, place, nullptr, nullptr, s)))
+    if ((rc = launch_window_stats(data, N, L, SC, mu, dcen, stat_e, place, nullptr, nullptr, nullptr, s)))
         return rc;
     cudaError_t e;
     if ((e = cudaGetLastError()) != cudaSuccess)
@@ -234,6 +234,7 @@ extern "C" int fmf_matched_filter_noalloc(const float *templates, const float *s
     P.zweight = nullptr;
     P.vp_norm = P.vp_bias = P.vp_scale = nullptr;
     P.scan = nullptr;
+    P.dc = nullptr;
     P.only_if = nullptr;
     if ((rc = launch_plain_all(P, s)))
         return rc;

@@ -429,6 +429,19 @@ struct StatLayout {
 
 size_t window_stats_smem(int L, bool full) { return (size_t)StatLayout(L, full).total * sizeof(float); }
 
+// Problem::dc of a window (u-th of its channel): every kDcStride-th one counts.
+__device__ __forceinline__ float window_dc(float mx, unsigned u, float Lf, float en, float mean)
+{
+    return u % kDcStride == 0 && en > 0.0f ? fmaxf(mx, Lf * mean * mean / en) : mx;
+}
+
+__device__ __forceinline__ void block_dc(float mx, unsigned *word)
+{
+    const unsigned top = __reduce_max_sync(0xffffffffu, __float_as_uint(mx));
+    if ((threadIdx.x & 31) == 0 && top > *(volatile unsigned *)word)
+        atomicMax(word, top);
+}
+
 // A block's part of Problem::scan: one atomic per block, and only where it changes the
 // channel's value.  `mem`: shared memory that is not read any more after the first
 // barrier here.
@@ -465,7 +478,7 @@ template <bool FULL, bool SCAN>
 __global__ void __launch_bounds__(kStatThreads, FULL ? 2 : 3)
 window_stats_kernel(const float *__restrict__ data, int N, int L, int SC, const float *__restrict__ mu,
                     float *__restrict__ dcen, float *__restrict__ stat_e, const StatPlace place,
-                    unsigned *__restrict__ scan, const unsigned *__restrict__ list)
+                    unsigned *__restrict__ scan, unsigned *__restrict__ dc, const unsigned *__restrict__ list)
 {
     extern __shared__ float4 stat_smem[];
     constexpr bool full = FULL;
@@ -628,6 +641,7 @@ window_stats_kernel(const float *__restrict__ data, int N, int L, int SC, const 
         // energies at or below this pass no template's threshold
         const float dead = SCAN ? kThreshold / __uint_as_float(scan[2 * SC + ch]) * 0.999f : 0.0f;
         unsigned low = 0;  // the smallest energy above it, bits complemented
+        float mx = 0.0f;
         float *row = stat_e + ch * place.ch * (full ? 2 : 1);
         // coalesced stores: windows in order, or (step > 1) row by row, `per` of each
         const int step = place.step, per = step == 1 ? nwin : (nwin + step - 1) / step;
@@ -649,6 +663,8 @@ window_stats_kernel(const float *__restrict__ data, int N, int L, int SC, const 
                 const float2 v = out2[stat_pad(u)];
                 reinterpret_cast<float2 *>(row)[o] = v;
                 en = v.x;
+                if (dc)
+                    mx = window_dc(mx, (unsigned)c0 + u, Lf, v.x, v.y);
             } else {
                 en = out1[stat_pad(u)];
                 row[o] = en;
@@ -656,6 +672,8 @@ window_stats_kernel(const float *__restrict__ data, int N, int L, int SC, const 
             if (SCAN && en > dead)
                 low = max(low, ~__float_as_uint(en));
         }
+        if (full && dc)
+            block_dc(mx, dc + ch);
         if (SCAN)
             scan_block(top, low, base, scan, ch, SC);
         __syncthreads();  // shared memory is free for the next block
@@ -735,7 +753,7 @@ template <bool FULL, bool SCAN>
 __global__ void __launch_bounds__(kFixThreads, FULL ? 2 : 3)
 window_fixed_kernel(const float *__restrict__ data, int N, int L, const float *__restrict__ mu,
                     float *__restrict__ dcen, float *__restrict__ stat_e, const StatPlace place,
-                    unsigned *__restrict__ scan, unsigned *__restrict__ list)
+                    unsigned *__restrict__ scan, unsigned *__restrict__ dc, unsigned *__restrict__ list)
 {
     extern __shared__ float4 stat_smem[];
     __shared__ uint2 warp_sums[2][kFixThreads / 32];
@@ -848,6 +866,7 @@ window_fixed_kernel(const float *__restrict__ data, int N, int L, const float *_
     // energies at or below this pass no template's threshold
     const float dead = SCAN ? kThreshold / __uint_as_float(scan[2 * SC + ch]) * 0.999f : 0.0f;
     unsigned low = 0;  // the smallest energy above it, bits complemented
+    float mx = 0.0f;
     float *row = stat_e + ch * place.ch * (FULL ? 2 : 1);
     // coalesced stores: windows in order, or (step > 1) row by row, `per` of each
     const int step = place.step, per = step == 1 ? nwin : (nwin + step - 1) / step;
@@ -881,6 +900,8 @@ window_fixed_kernel(const float *__restrict__ data, int N, int L, const float *_
             window_centred_sums(h2 * u2, l2 * u2, h1 * u1, l1 * u1, Lf, invL, en, mean);
             far = far || !(en >= least);
             reinterpret_cast<float2 *>(row)[o] = make_float2(en, mean);
+            if (dc)
+                mx = window_dc(mx, (unsigned)c0 + u, Lf, en, mean);
         } else {
             // the top 24 bits and the rest, added with one rounding
             const float f = fmaf((float)(hi2 >> 8), 268435456.0f, (float)((int)((hi2 & 255) << 20) + lo2));
@@ -896,6 +917,8 @@ window_fixed_kernel(const float *__restrict__ data, int N, int L, const float *_
     __syncthreads();
     if (odd && threadIdx.x == 0 && nwin > 0)
         list[1 + atomicAdd(list, 1u)] = blockIdx.y * gridDim.x + blockIdx.x;
+    if (FULL && dc && !odd)
+        block_dc(mx, dc + ch);
     // the largest value counts in any case; the smallest energy of a listed block is made there
     if (SCAN)
         scan_block(most, odd ? 0u : low, raw, scan, ch, SC);
@@ -921,7 +944,8 @@ size_t window_list_words(int N, int SC)
 }
 
 int launch_window_stats(const float *data, int N, int L, int SC, const float *mu, float *dcen,
-                        float *stat_e, const StatPlace &place, unsigned *scan, unsigned *list, cudaStream_t s)
+                        float *stat_e, const StatPlace &place, unsigned *scan, unsigned *dc, unsigned *list,
+                        cudaStream_t s)
 {
     const bool full = mu != nullptr;
     const int per_ch = (N + kStatWindows - 1) / kStatWindows;
@@ -938,7 +962,7 @@ int launch_window_stats(const float *data, int N, int L, int SC, const float *mu
             e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxDynamicSmem - 1024);
         if (e != cudaSuccess)
             return set_error(FMF_ERR_CUDA, "window statistics: %s", cudaGetErrorString(e));
-        kern<<<dim3(per_ch, SC), kFixThreads, fixed, s>>>(data, N, L, mu, dcen, stat_e, place, scan, list);
+        kern<<<dim3(per_ch, SC), kFixThreads, fixed, s>>>(data, N, L, mu, dcen, stat_e, place, scan, dc, list);
         count_launch();
         grid = grid < 608 ? grid : 608;  // the listed blocks, few or none
     }
@@ -949,7 +973,7 @@ int launch_window_stats(const float *data, int N, int L, int SC, const float *mu
     if (e != cudaSuccess)
         return set_error(FMF_ERR_CUDA, "window statistics shared memory (%zu bytes): %s", smem,
                          cudaGetErrorString(e));
-    kern<<<grid, kStatThreads, smem, s>>>(data, N, L, SC, mu, dcen, stat_e, place, scan, list);
+    kern<<<grid, kStatThreads, smem, s>>>(data, N, L, SC, mu, dcen, stat_e, place, scan, dc, list);
     count_launch();
     return FMF_OK;
 }

@@ -651,6 +651,7 @@ static int variable_device(const VArgs &a, int L, cudaStream_t s, float *host_ou
     P.zweight = zweight;
     P.vp_norm = P.vp_bias = P.vp_scale = nullptr;
     P.scan = scan;
+    P.dc = nullptr;
     P.only_if = nullptr;
     if (precision == FMF_PREC_AUTO && (rc = choose_auto_precision(P, ws, s, &precision)))
         return rc;
