@@ -439,10 +439,14 @@ __device__ __forceinline__ void tc_issue(const TcBatch &B, const long long *ring
         c_end = uniform(c_end);
         const TcProb &pr = B.prob[p];
         const int nb = pr.nb;
-        if (!uniform(tc_busy(pr, (long long)tile * TC_Q * nb, t)))
+        const long long I0 = (long long)tile * TC_Q * nb;
+        if (!uniform(tc_busy(pr, I0, t)))
             continue;
-        // kind::f16 descriptor: F32 accumulate, A and B both FP16 or both BF16, K-major, N = nb, M = 128
-        const uint32_t idesc = (1u << 4) | B.mma_types | ((uint32_t)(nb >> 3) << 17) | ((uint32_t)(TC_Q >> 4) << 24);
+        // the template's lag blocks in this tile, in steps of 16: the other accumulator
+        // columns stay as they are, and their outputs are not used
+        const int cols = uniform((int)min((long long)nb, (pr.P.k_hi[t] - I0 + 16 * TC_Q - 1) / (16 * TC_Q) * 16));
+        // kind::f16 descriptor: F32 accumulate, A and B both FP16 or both BF16, K-major, N = cols, M = 128
+        const uint32_t idesc = (1u << 4) | B.mma_types | ((uint32_t)(cols >> 3) << 17) | ((uint32_t)(TC_Q >> 4) << 24);
         const int SC = pr.P.SC, step = pr.P.step, L = pr.P.L;
         const uint32_t chain_cols = (uint32_t)pr.chain_cols;
         const uint32_t col_bytes = (uint32_t)pr.R * 16;
