@@ -71,13 +71,19 @@ constexpr int kDetChunk = 1024;           // templates per round of scratch
 constexpr int kDetCap = 16384;            // candidate peaks per template row
 constexpr int kDetSample = 16384;         // sampled keys per row (sample-select)
 constexpr int kDetBlocks = 152 * 8 * 8;   // blocks of a row pass: 8 waves of 8 per SM
-constexpr int kSpill = 16;                // rows past a column's capacity (one step's appends)
+constexpr int kStep = 8;                  // values per lane and step of the counting pass; entries per sector
+constexpr int kRing = 2 * kStep;          // staged entries per column
+constexpr int kDetPickBlocks = 152 * 8;   // blocks of the pass over the candidates
+constexpr int kCandBins = 1024;           // bins of the candidates' window
+constexpr int kPickCap = 2048;            // candidates that share the middle ranks' bins
 constexpr int kDetRowBlocks = 152 * 4;    // the fixed grid of the passes over rows that fell back
 
 // source of a row's radix selection
 constexpr int kSrcRow = 0;   // the row itself (fallback)
-constexpr int kSrcCand = 1;  // the candidate keys gathered by det_count_kernel
-constexpr int kSrcDone = 2;  // already exact (the row was sorted whole)
+constexpr int kSrcCand = 1;  // the candidates gathered by det_count_kernel, by their bins
+constexpr int kSrcDone = 2;  // already exact
+constexpr int kSrcPick = 3;  // the few of them in the middle ranks' bins
+constexpr int kSrcKeys = 4;  // all of them, by the bits of their keys (those bins hold too many)
 
 struct DetState {
     int begin, end;        // lag window of the row
@@ -92,6 +98,8 @@ struct DetState {
     int src;               // kSrcRow / kSrcCand / kSrcDone
     unsigned klo, khi;     // key window of the current selection
     int n_lt, n_in;        // keys below klo, keys inside [klo, khi]
+    int bin0, bin1;        // bins (cand_bin) of the middle ranks
+    int n_list;            // candidates in them
     // the MAD classes of the counting pass (one_read = 1): the median lies in
     // [m_lo, m_hi] and the MAD in [a_lo, a_hi] when both windows hold
     int one_read;
@@ -105,14 +113,12 @@ struct DetState {
 
 // The lists of a row are written in columns, one per thread of the counting
 // pass, so that appending takes no scan and no shared counter: thread l of
-// warp w of block b puts its k-th entry at list + t * cap + ((b * 8 + w) *
-// (C + kSpill) + k) * 32 + (l & 31), up to C entries (rows C.. of the warp's
-// region take a step's overflow, unread), and its count at
-// cnt[(t * S + b) * 256 + l] (more than C: overflowed).  Equal counts across a
-// warp make coalesced stores and loads.
+// warp w of block b has C entries from list + t * cap + (b * 8 + w) * C * 32, the k-th
+// of them at ((k / 8) * 32 + l % 32) * 8 + k % 8 -- eight in a row, a sector of its
+// own -- and its count at cnt[(t * S + b) * 256 + l] (more than C: overflowed).
 struct Lanes {
     int S;                 // counting blocks per row
-    int Ck, Ca;            // column capacity: candidates of a selection / undecided values
+    int Ck, Ca;            // column capacity: candidates of a selection / undecided values (multiples of 8)
     int *cnt_k, *cnt_a;    // entries per column (may exceed the capacity)
 };
 
@@ -191,6 +197,7 @@ __global__ void det_init_kernel(DetState *__restrict__ st, int T, int n_corr,
     s.src = kSrcRow;
     s.klo = s.khi = 0u;
     s.n_lt = s.n_in = 0;
+    s.bin0 = s.bin1 = s.n_list = 0;
     s.one_read = 0;
     s.m_lo = s.m_hi = s.a_lo = s.a_hi = 0.0f;
     s.has_below = 0;
@@ -293,6 +300,14 @@ __device__ void block_select2(const unsigned *sk, int P, int r0, int r1, unsigne
     }
     k0 = pre[0];
     k1 = pre[1];
+}
+
+// A candidate's bin, of kCandBins over its window [lo, hi]: never falls as x rises (nor
+// do a float difference and product), so bins are ranges of ranks.
+__device__ __forceinline__ float bin_scale(float lo, float hi) { return __fdiv_rn((float)kCandBins, __fsub_rn(hi, lo)); }
+__device__ __forceinline__ int cand_bin(float x, float lo, float scale)
+{
+    return min(max((int)__fmul_rn(__fsub_rn(x, lo), scale), 0), kCandBins - 1);
 }
 
 // |x - m| in float32, as numpy computes the MAD's deviations.
@@ -559,20 +574,100 @@ __device__ __forceinline__ void note_hot(DetState *st, int t, long long o, int *
 // are compared as floats (rows are free of NaN; -0 compares as +0, and the
 // readers key a candidate x as x + 0).  The per-value work is predicated, with
 // no branch: the pass stays at the rate of the row's read.
+//
+// The entries of a column wait in shared memory, a ring of kRing rows per warp (a
+// lane's bank is its own, so appending never conflicts), and go out a sector of eight
+// at a time.  Stored as they came, each 4-byte value cost a 32-byte sector, and these
+// sectors bounded the pass (COUNTMEASURED).  What bounds it now: its instructions,
+// about 20 per value.
+struct Column {
+    unsigned in, out;  // entries begun and stored, times 128 (bytes of a ring row)
+    // a sector, if there is one (at most one: fewer than 8 entries waited before a step
+    // of 8); `ring`: the lane's word of row 0, `column`: its first sector
+    __device__ __forceinline__ void store(const char *ring, char *column, unsigned cap, bool rest)
+    {
+        if (in - out >= kStep * 128u || (rest && in != out)) {
+            const float *r = reinterpret_cast<const float *>(ring + (out & (kStep * 128u)));
+            if (out < cap) {
+                float4 *o = reinterpret_cast<float4 *>(column + out);
+                o[0] = make_float4(r[0], r[32], r[64], r[96]);
+                o[1] = make_float4(r[128], r[160], r[192], r[224]);
+            }
+            out += kStep * 128u;
+        }
+    }
+};
+
+// Eight entries of a column from the k-th on (k a multiple of 8).
+__device__ __forceinline__ void load_sector(const float *column, int k, float (&x)[8])
+{
+    const float4 *p = reinterpret_cast<const float4 *>(column + (size_t)k * 32);
+    const float4 a = p[0], b = p[1];
+    x[0] = a.x, x[1] = a.y, x[2] = a.z, x[3] = a.w;
+    x[4] = b.x, x[5] = b.y, x[6] = b.z, x[7] = b.w;
+}
+
+// x < lo counted in lt; x in [lo, hi] appended to the ring at k_ring (its shared
+// address, the lane's word).  NaN does neither.
+__device__ __forceinline__ void take_candidate(float x, float lo, float hi, unsigned &lt, unsigned &in, unsigned k_ring)
+{
+    asm volatile("{\n\t.reg .pred p, q;\n\t.reg .u32 a;\n\t"
+                 "setp.lt.f32 p, %2, %3;\n\t"
+                 "setp.le.and.f32 q, %2, %4, !p;\n\t"
+                 "@p add.u32 %0, %0, 1;\n\t"
+                 "and.b32 a, %1, %6;\n\t"
+                 "or.b32 a, a, %5;\n\t"
+                 "@q st.shared.f32 [a], %2;\n\t"
+                 "@q add.u32 %1, %1, 128;\n\t}"
+                 : "+r"(lt), "+r"(in)
+                 : "f"(x), "f"(lo), "f"(hi), "r"(k_ring), "n"(kRing * 128 - 1)
+                 : "memory");
+}
+
+// x in [b_lo, b_hi] counted in nb; else, in [n_lo, n_hi], appended.
+__device__ __forceinline__ void take_undecided(float x, float b_lo, float b_hi, float n_lo, float n_hi, unsigned &nb,
+                                               unsigned &in, unsigned a_ring)
+{
+    asm volatile("{\n\t.reg .pred p, q;\n\t.reg .u32 a;\n\t"
+                 "setp.ge.f32 p, %2, %3;\n\t"
+                 "setp.le.and.f32 p, %2, %4, p;\n\t"
+                 "setp.ge.and.f32 q, %2, %5, !p;\n\t"
+                 "setp.le.and.f32 q, %2, %6, q;\n\t"
+                 "@p add.u32 %0, %0, 1;\n\t"
+                 "and.b32 a, %1, %8;\n\t"
+                 "or.b32 a, a, %7;\n\t"
+                 "@q st.shared.f32 [a], %2;\n\t"
+                 "@q add.u32 %1, %1, 128;\n\t}"
+                 : "+r"(nb), "+r"(in)
+                 : "f"(x), "f"(b_lo), "f"(b_hi), "f"(n_lo), "f"(n_hi), "r"(a_ring), "n"(kRing * 128 - 1)
+                 : "memory");
+}
+constexpr int kRingBytes = kDetThreads / 32 * 2 * kRing * 128;
+constexpr size_t kCountSmem = kRing * 128 + kRingBytes + kCandBins * sizeof(unsigned);  // (aligned rings, bins)
+
 template <bool ROW>
-__global__ void __launch_bounds__(kDetThreads, 3)  // 24 warps per SM, 16 values per lane in flight
+__global__ void __launch_bounds__(kDetThreads, 4)  // 32 warps per SM, 16 values per lane in flight
 det_count_kernel(const float *__restrict__ cc, size_t ld, DetState *__restrict__ st,
                  float *__restrict__ cand, long long cap, float *__restrict__ amb, long long amb_cap,
-                 Lanes g, int *__restrict__ hot, int hcap)
+                 Lanes g, unsigned *__restrict__ bins, int *__restrict__ hot, int hcap)
 {
     const int t = blockIdx.y;
     if (st[t].src != kSrcCand)
         return;  // uniform over the block
+    extern __shared__ float4 count_smem[];
+    // a ring on a multiple of its size: an entry's address is an OR away
+    char *const rings = reinterpret_cast<char *>(count_smem) +
+                        (-(unsigned)__cvta_generic_to_shared(count_smem) & (kRing * 128u - 1u));
+    unsigned *const bin = reinterpret_cast<unsigned *>(rings + kRingBytes);
+    for (int i = threadIdx.x; i < kCandBins; i += kDetThreads)
+        bin[i] = 0u;
+    __syncthreads();
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const size_t col = ((size_t)t * g.S + blockIdx.x) * kDetThreads + threadIdx.x;
     const size_t region = (size_t)blockIdx.x * (kDetThreads / 32) + warp;
-    float *kc = cand + (size_t)t * cap + region * (size_t)(g.Ck + kSpill) * 32 + lane;
-    float *ac = amb + (size_t)t * amb_cap + region * (size_t)(g.Ca + kSpill) * 32 + lane;
+    float *kc = cand + (size_t)t * cap + region * (size_t)g.Ck * 32 + 8 * lane;
+    float *ac = amb + (size_t)t * amb_cap + region * (size_t)g.Ca * 32 + 8 * lane;
+    char *const kring = rings + warp * (2 * kRing * 128) + 4 * lane, *const aring = kring + kRing * 128;
     const float lo = key_value(st[t].klo), hi = key_value(st[t].khi);
     const float med = st[t].med;
     // the MAD classes as float intervals, empty (x >= +inf never holds) where the
@@ -586,34 +681,21 @@ det_count_kernel(const float *__restrict__ cc, size_t ld, DetState *__restrict__
     const bool peaks = ROW && st[t].peaks_ready;
     const float thr_lo = st[t].thr_lo;
     unsigned lt = 0, nb = 0;
-    // offsets (floats) of the next entry of this thread's columns; a step's appends
-    // past the capacity land in the spill rows, and the offset is clamped after it
-    unsigned ko = 0, ao = 0;
-    const unsigned kmax = (unsigned)g.Ck * 32u, amax = (unsigned)g.Ca * 32u;
-    bool ovk = false, ova = false;
-    auto take = [&](float x, bool ok) {
-        lt += (unsigned)(ok & (x < lo));
-        const bool in = ok & (x >= lo) & (x <= hi);
-        if (in)
-            kc[ko] = x;
-        ko += in ? 32u : 0u;
-        if constexpr (ROW) {
-            const bool below = ok & (x >= b_lo) & (x <= b_hi);
-            nb += (unsigned)below;
-            const bool un = ok & !below & (x >= n_lo) & (x <= n_hi);
-            if (un)
-                ac[ao] = x;
-            ao += un ? 32u : 0u;
-        }
+    Column kcol{0, 0}, acol{0, 0};
+    const unsigned kmax = (unsigned)g.Ck * 128u, amax = (unsigned)g.Ca * 128u;
+    const unsigned k_ring = (unsigned)__cvta_generic_to_shared(kring);
+    const unsigned a_ring = (unsigned)__cvta_generic_to_shared(aring);
+    auto take = [&](float x) {
+        take_candidate(x, lo, hi, lt, kcol.in, k_ring);
+        if constexpr (ROW)
+            take_undecided(x, b_lo, b_hi, n_lo, n_hi, nb, acol.in, a_ring);
     };
-    auto clamp = [&]() {  // after at most kSpill appends per column
-        ovk |= ko > kmax;
-        ko = min(ko, kmax);
-        if constexpr (ROW) {
-            ova |= ao > amax;
-            ao = min(ao, amax);
-        }
+    auto step_done = [&](bool rest) {  // after at most kStep appends per column
+        kcol.store(kring, reinterpret_cast<char *>(kc), kmax, rest);
+        if constexpr (ROW)
+            acol.store(aring, reinterpret_cast<char *>(ac), amax, rest);
     };
+    const float none = __int_as_float(0x7fc00000);  // NaN: no value
     if constexpr (ROW) {
         const float *row = cc + (size_t)t * ld + st[t].begin;
         const long long n = st[t].end - st[t].begin;
@@ -621,99 +703,103 @@ det_count_kernel(const float *__restrict__ cc, size_t ld, DetState *__restrict__
         if (blockIdx.x == 0 && warp == 0) {  // the unaligned ends, at most 3 + 3 values
             const long long i = lane < rs.head ? lane : rs.head + 4 * rs.nvec + (lane - rs.head);
             const bool ok = lane < rs.head + rs.tail;
-            const float x = ok ? row[i] : 0.0f;
-            if (peaks && ok && x >= thr_lo)
+            const float x = ok ? row[i] : none;
+            if (peaks && x >= thr_lo)
                 note_hot(st, t, i, hot, hcap);
-            take(x, ok);
-            clamp();
+            take(x);
+            step_done(false);
         }
         // a warp step: 32 float4s from each quarter of the row, so that a lane's four
         // float4s lie far apart (on a smooth row, neighbouring values share their
         // class: a lane's appends then come in runs of at most 4)
-        const float4 *vrow = reinterpret_cast<const float4 *>(row + rs.head);
-        const long long quarter = (rs.nvec + 3) / 4;
-        const long long steps = (quarter + 31) / 32;
-        const long long cstride = (long long)gridDim.x * (kDetThreads / 32);
-        auto load4 = [&](long long c, float4 (&v)[4]) {
-#pragma unroll
-            for (int u = 0; u < 4; u++) {
-                const long long q = c * 32 + lane, i = u * quarter + q;
-                v[u] = (c < steps && q < quarter && i < rs.nvec) ? vrow[i] : make_float4(0.f, 0.f, 0.f, 0.f);
-            }
-        };
-        float4 nv[4];
-        long long c = (long long)blockIdx.x * (kDetThreads / 32) + warp;
-        load4(c, nv);
-        for (; c < steps; c += cstride) {
-            float4 v[4];
+        const float4 *vrow = reinterpret_cast<const float4 *>(row + rs.head) + lane;
+        const int nvec = (int)rs.nvec, quarter = (nvec + 3) / 4;
+        const int steps = (quarter + 31) / 32, cstride = (int)gridDim.x * (kDetThreads / 32);
+        const int whole = max(nvec - 3 * quarter, 0) / 32;  // steps without a value missing
+        auto load = [&](int c, float4 (&v)[4]) {
 #pragma unroll
             for (int u = 0; u < 4; u++)
-                v[u] = nv[u];
-            load4(c + cstride, nv);  // the next step's values are in flight while this one is counted
+                v[u] = vrow[u * quarter + 32 * c];
+        };
+        auto count = [&](const float4 (&v)[4], int c) {
             // values at or above thr_lo (rare): one vote per step on the lanes' largest
-            // values (the zeros loaded past the row's end can only cost the slow path)
-            float mx = -INFINITY;
+            // values
+            float mx = none;
 #pragma unroll
             for (int u = 0; u < 4; u++)
                 mx = fmaxf(mx, fmaxf(fmaxf(v[u].x, v[u].y), fmaxf(v[u].z, v[u].w)));
             if (peaks && __any_sync(0xffffffffu, mx >= thr_lo)) {
 #pragma unroll
                 for (int u = 0; u < 4; u++) {
-                    const long long q = c * 32 + lane, i = u * quarter + q;
-                    const float m4 = fmaxf(fmaxf(v[u].x, v[u].y), fmaxf(v[u].z, v[u].w));
-                    if (q < quarter && i < rs.nvec && m4 >= thr_lo) {
-                        const long long o = rs.head + 4 * i;
-                        if (v[u].x >= thr_lo)
-                            note_hot(st, t, o, hot, hcap);
-                        if (v[u].y >= thr_lo)
-                            note_hot(st, t, o + 1, hot, hcap);
-                        if (v[u].z >= thr_lo)
-                            note_hot(st, t, o + 2, hot, hcap);
-                        if (v[u].w >= thr_lo)
-                            note_hot(st, t, o + 3, hot, hcap);
-                    }
+                    const long long o = rs.head + 4ll * (u * quarter + 32 * c + lane);
+                    if (v[u].x >= thr_lo)
+                        note_hot(st, t, o, hot, hcap);
+                    if (v[u].y >= thr_lo)
+                        note_hot(st, t, o + 1, hot, hcap);
+                    if (v[u].z >= thr_lo)
+                        note_hot(st, t, o + 2, hot, hcap);
+                    if (v[u].w >= thr_lo)
+                        note_hot(st, t, o + 3, hot, hcap);
                 }
             }
-            if (c * 32 + 32 <= quarter && 3 * quarter + c * 32 + 32 <= rs.nvec) {  // a whole step (warp-uniform)
 #pragma unroll
-                for (int u = 0; u < 4; u++) {
-                    take(v[u].x, true);
-                    take(v[u].y, true);
-                    take(v[u].z, true);
-                    take(v[u].w, true);
-                }
-            } else {
-#pragma unroll
-                for (int u = 0; u < 4; u++) {
-                    const long long q = c * 32 + lane;
-                    const bool ok = q < quarter && u * quarter + q < rs.nvec;
-                    take(v[u].x, ok);
-                    take(v[u].y, ok);
-                    take(v[u].z, ok);
-                    take(v[u].w, ok);
-                }
+            for (int u = 0; u < 4; u++) {
+                take(v[u].x);
+                take(v[u].y);
+                take(v[u].z);
+                take(v[u].w);
+                if (u & 1)
+                    step_done(false);
             }
-            clamp();
+        };
+        int c = (int)blockIdx.x * (kDetThreads / 32) + warp;
+        float4 v[4], w[4];  // one is counted while the other is in flight
+        if (c < whole) {
+            load(c, v);
+            for (;;) {
+                c += cstride;
+                if (c < whole)
+                    load(c, w);
+                count(v, c - cstride);
+                if (c >= whole)
+                    break;
+                c += cstride;
+                if (c < whole)
+                    load(c, v);
+                count(w, c - cstride);
+                if (c >= whole)
+                    break;
+            }
+        }
+        for (; c < steps; c += cstride) {
+#pragma unroll
+            for (int u = 0; u < 4; u++) {
+                const int q = 32 * c + lane;
+                v[u] = q < quarter && u * quarter + q < nvec ? vrow[u * quarter + 32 * c]
+                                                             : make_float4(none, none, none, none);
+            }
+            count(v, c);
         }
     } else {
-        // this thread's own column of undecided values, eight loads in flight
+        // this thread's own column of undecided values
         const int m = min(g.cnt_a[col], g.Ca);
         const int mw = __reduce_max_sync(0xffffffffu, m);
         for (int k = 0; k < mw; k += 8) {
-            float x[8];
+            float x[8] = {};
+            if (k < m)
+                load_sector(ac, k, x);
 #pragma unroll
             for (int j = 0; j < 8; j++)
-                x[j] = k + j < m ? ac[(size_t)(k + j) * 32] : 0.0f;
-#pragma unroll
-            for (int j = 0; j < 8; j++)
-                take(dev(x[j], med), k + j < m);
-            clamp();
+                take(k + j < m ? dev(x[j], med) : none);
+            step_done(false);
         }
     }
-    const int nk = ovk ? g.Ck + 1 : (int)(ko / 32u);  // past the capacity: overflowed
+    step_done(true);
+    const bool ovk = kcol.in > kmax, ova = acol.in > amax;
+    const int nk = ovk ? g.Ck + 1 : (int)(kcol.in / 128u);  // past the capacity: overflowed
     g.cnt_k[col] = nk;
     if (ROW)
-        g.cnt_a[col] = ova ? g.Ca + 1 : (int)(ao / 32u);
+        g.cnt_a[col] = ova ? g.Ca + 1 : (int)(acol.in / 128u);
     const bool over_k = __any_sync(0xffffffffu, ovk);
     const bool over_a = ROW && __any_sync(0xffffffffu, ova);
     const int sum_k = __reduce_add_sync(0xffffffffu, (unsigned)nk);
@@ -733,20 +819,37 @@ det_count_kernel(const float *__restrict__ cc, size_t ld, DetState *__restrict__
         if (over_a)
             atomicOr(&st[t].over_a, 1);
     }
+    // the candidates' bins, from the column this thread wrote
+    const float scale = bin_scale(lo, hi);
+    for (int k = 0; k < min(nk, g.Ck); k += 8) {
+        float x[8];
+        load_sector(kc, k, x);
+#pragma unroll
+        for (int j = 0; j < 8; j++)
+            if (k + j < nk)
+                atomicAdd(&bin[cand_bin(x[j], lo, scale)], 1u);
+    }
+    __syncthreads();
+    unsigned *gb = bins + (size_t)t * kCandBins;
+    for (int i = threadIdx.x; i < kCandBins; i += kDetThreads)
+        if (bin[i])
+            atomicAdd(gb + i, bin[i]);
 }
 
-// Step 3 (and 4): does the window hold both middle ranks?  Then select among
-// the candidates, over the key bits they do not share; else fall back to the
-// whole row -- for the median that also gives up the MAD classes of the
-// counting pass (they assume the median inside [m_lo, m_hi]) and its hot
-// values; for the MAD, the hot values (the superset may miss some, or have
-// overflowed its list).
-__global__ void det_check_kernel(DetState *__restrict__ st, int T, int mode, int pcap, float n_mad)
+// Step 3 (and 4): does the window hold both middle ranks?  Then find their bins, and
+// select among the candidates there, or, if these are too many (ties), over the key
+// bits that the window's keys do not share; else fall back to the whole row -- for
+// the median that also gives up the MAD classes of the counting pass (they assume the
+// median inside [m_lo, m_hi]) and its hot values; for the MAD, the hot values (the
+// superset may miss some, or have overflowed its list).  One warp per row.
+__global__ void det_pick_kernel(DetState *__restrict__ st, const unsigned *__restrict__ bins, int mode, int pcap,
+                                float n_mad)
 {
-    const int t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= T || st[t].src != kSrcCand)
+    const int t = blockIdx.x, lane = threadIdx.x;
+    if (st[t].src != kSrcCand)
         return;
     DetState s = st[t];
+    __syncwarp();
     const long long n = s.end - s.begin;
     const long long a = (n - 1) / 2, b = n / 2;
     if (!s.over_k && s.n_lt <= a && b < (long long)s.n_lt + s.n_in) {
@@ -758,6 +861,43 @@ __global__ void det_check_kernel(DetState *__restrict__ st, int T, int mode, int
         if (s.top == 0) {  // every candidate has the key klo
             finish_select(s, mode, middle_value(s.klo, s.klo, (int)n), n_mad);
             s.src = kSrcDone;
+        } else {
+            constexpr int per = kCandBins / 32;
+            const unsigned *h = bins + (size_t)t * kCandBins + lane * per;
+            unsigned sum = 0;
+            for (int i = 0; i < per; i++)
+                sum += h[i];
+            unsigned inc = sum;
+            for (int o = 1; o < 32; o <<= 1) {
+                const unsigned y = __shfl_up_sync(0xffffffffu, inc, o);
+                if (lane >= o)
+                    inc += y;
+            }
+            int at[2];
+            unsigned before[2], size[2];
+            for (int r = 0; r < 2; r++) {
+                const unsigned rk = (unsigned)s.rank[r];
+                const unsigned found = __ballot_sync(0xffffffffu, rk < inc);
+                const int src = found ? __ffs(found) - 1 : 31;
+                unsigned c = inc - sum;
+                int i = 0;
+                if (lane == src)
+                    for (; i < per - 1 && rk >= c + h[i]; i++)
+                        c += h[i];
+                at[r] = __shfl_sync(0xffffffffu, lane * per + i, src);
+                before[r] = __shfl_sync(0xffffffffu, c, src);
+                size[r] = __shfl_sync(0xffffffffu, h[i], src);
+            }
+            s.bin0 = at[0];
+            s.bin1 = at[1];
+            s.n_list = 0;
+            if (size[0] + (at[1] != at[0] ? size[1] : 0u) <= (unsigned)kPickCap) {
+                s.src = kSrcPick;
+                s.rank[0] -= (int)before[0];
+                s.rank[1] -= (int)before[0];
+            } else {
+                s.src = kSrcKeys;
+            }
         }
     } else {
         s.src = kSrcRow;
@@ -773,7 +913,66 @@ __global__ void det_check_kernel(DetState *__restrict__ st, int T, int mode, int
         s.peaks_ready = 0;
     if (!s.peaks_ready)
         s.n_cand = 0;
-    st[t] = s;
+    if (lane == 0)
+        st[t] = s;
+}
+
+// The candidates in the middle ranks' bins, into the row's list (a few dozen of a
+// hundred thousand).  Grid: (blocks per row, templates); a block takes every
+// gridDim.x-th of the counting pass's blocks.
+__global__ void __launch_bounds__(kDetThreads)
+det_gather_kernel(DetState *__restrict__ st, const float *__restrict__ cand, long long cap, Lanes g,
+                  unsigned *__restrict__ list)
+{
+    const int t = blockIdx.y;
+    if (st[t].src != kSrcPick)
+        return;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    constexpr int kWarps = kDetThreads / 32;
+    const float lo = key_value(st[t].klo), scale = bin_scale(lo, key_value(st[t].khi));
+    const int bin0 = st[t].bin0, bin1 = st[t].bin1;
+    for (int blk = blockIdx.x; blk < g.S; blk += gridDim.x) {
+        const size_t col = ((size_t)t * g.S + blk) * kDetThreads + threadIdx.x;
+        const float *kc = cand + (size_t)t * cap + ((size_t)blk * kWarps + warp) * (size_t)g.Ck * 32 + 8 * lane;
+        const int m = g.cnt_k[col];  // <= Ck: no column overflowed
+        for (int k = 0; k < m; k += 8) {
+            float x[8];
+            load_sector(kc, k, x);
+#pragma unroll
+            for (int j = 0; j < 8; j++) {
+                const int b = cand_bin(x[j], lo, scale);
+                if (k + j < m && b >= bin0 && b <= bin1) {  // (the bins between them are empty)
+                    const int at = atomicAdd(&st[t].n_list, 1);
+                    if (at < kPickCap)
+                        list[(size_t)t * kPickCap + at] = order_key(__fadd_rn(x[j], 0.0f));
+                }
+            }
+        }
+    }
+}
+
+// The middle keys of the list: one block per row.
+__global__ void __launch_bounds__(kDetThreads)
+det_finish_kernel(DetState *__restrict__ st, const unsigned *__restrict__ list, int mode, float n_mad)
+{
+    __shared__ unsigned sk[kPickCap];
+    __shared__ unsigned hist[2 * kDetBins];
+    __shared__ int pick[4];
+    const int t = blockIdx.x;
+    if (st[t].src != kSrcPick)
+        return;
+    const int n = min(st[t].n_list, kPickCap), r0 = st[t].rank[0], r1 = st[t].rank[1];
+    for (int i = threadIdx.x; i < n; i += kDetThreads)
+        sk[i] = list[(size_t)t * kPickCap + i];
+    __syncthreads();
+    unsigned k0, k1;
+    block_select2(sk, n, r0, r1, hist, pick, k0, k1);
+    if (threadIdx.x == 0) {
+        DetState s = st[t];
+        finish_select(s, mode, middle_value(k0, k1, s.end - s.begin), n_mad);
+        s.src = kSrcDone;
+        st[t] = s;
+    }
 }
 
 // Histogram update: every lane of the warp calls it (lanes whose value does
@@ -812,62 +1011,8 @@ __device__ __forceinline__ void hist_add(unsigned *h, float v, bool ok, int mode
     }
 }
 
-// One selection pass over the candidates: histogram of the current digit over
-// the candidates whose higher key bits equal a rank's prefix, each thread
-// reading its own column as the counting pass wrote it.  Grid: (blocks per
-// row, templates), as the counting pass.
-__global__ void __launch_bounds__(kDetThreads)
-det_hist_kernel(const DetState *__restrict__ st, unsigned *__restrict__ hist,
-                const float *__restrict__ cand, long long cap, Lanes g, int pass)
-{
-    __shared__ unsigned h[2 * kDetBins];
-    const int t = blockIdx.y;
-    const DetState s = st[t];
-    if (s.src != kSrcCand || s.end - s.begin <= 0)
-        return;  // uniform over the block, before any barrier (rows that fell back:
-                 // det_hist_row_kernel)
-    if (pass > 0 && s.top <= 11 * pass)
-        return;  // the key is complete
-    for (int i = threadIdx.x; i < 2 * kDetBins; i += kDetThreads)
-        h[i] = 0u;
-    __syncthreads();
-    int shift, width;
-    pass_digit(s.top, pass, shift, width);
-    const unsigned dmask = (1u << width) - 1u;
-    const unsigned high = above_mask(shift + width);
-    const unsigned p0 = s.prefix[0], p1 = s.prefix[1];
-    const bool two = p0 != p1;  // the two middle ranks sit in different buckets
-    const float med = s.med;
-    const int lane = threadIdx.x & 31;
-    const int warp = threadIdx.x >> 5;
-    constexpr int kWarps = kDetThreads / 32;
-    {
-        const size_t col = ((size_t)t * g.S + blockIdx.x) * kDetThreads + threadIdx.x;
-        const size_t region = (size_t)blockIdx.x * kWarps + warp;
-        const float *kc = cand + (size_t)t * cap + region * (size_t)(g.Ck + kSpill) * 32 + lane;
-        const int m = g.cnt_k[col];  // <= Ck: no column overflowed
-        const int mw = __reduce_max_sync(0xffffffffu, m);
-        for (int k = 0; k < mw; k += 8) {  // eight loads in flight
-            float x[8];
-#pragma unroll
-            for (int j = 0; j < 8; j++)
-                x[j] = k + j < m ? kc[(size_t)(k + j) * 32] : 0.0f;
-#pragma unroll
-            for (int j = 0; j < 8; j++)
-                hist_add(h, x[j], k + j < m, 2, med, shift, dmask, high, p0, p1, two, lane, false);
-        }
-    }
-    __syncthreads();
-    unsigned *gh = hist + (size_t)t * 2 * kDetBins;
-    for (int i = threadIdx.x; i < (two ? 2 : 1) * kDetBins; i += kDetThreads) {
-        const unsigned c = h[i];
-        if (c)
-            atomicAdd(gh + i, c);
-    }
-}
-
-// The rows that need a pass over the whole row, compacted into list[0..*count)
-// (one block): kind 0 those selecting over the whole row, kind 1 those whose
+// The rows that need more passes, compacted into list[0..*count) (one block):
+// kind 0 those selecting over key bits, kind 1 those whose
 // peaks were not gathered by the counting pass (at least 3 lags).
 __global__ void __launch_bounds__(1024)
 det_collect_kernel(const DetState *__restrict__ st, int T, int kind, int *__restrict__ list,
@@ -878,7 +1023,7 @@ det_collect_kernel(const DetState *__restrict__ st, int T, int kind, int *__rest
         n = 0;
     __syncthreads();
     for (int t = threadIdx.x; t < T; t += blockDim.x) {
-        const bool need = kind == 0 ? st[t].src == kSrcRow && st[t].end > st[t].begin
+        const bool need = kind == 0 ? (st[t].src == kSrcRow || st[t].src == kSrcKeys) && st[t].end > st[t].begin
                                     : !st[t].peaks_ready && st[t].end - st[t].begin >= 3;
         if (need)
             list[atomicAdd(&n, 1)] = t;
@@ -888,16 +1033,19 @@ det_collect_kernel(const DetState *__restrict__ st, int T, int kind, int *__rest
         *count = n;
 }
 
-// The same pass for the rows that fell back to selection over the whole row
-// (a sample window that missed, a column that overflowed): every block of a
-// fixed grid takes a slice of each such row in turn, so a row that fell back
-// is read at the rate of the whole GPU, not of its own few blocks.  mode 0
-// keys the values, mode 1 |x - median|; equal digits are aggregated per warp
-// in the first pass (a row's keys share their high digits).
+// One selection pass by key bits: histogram of the current digit over the keys whose
+// higher bits equal a rank's prefix, for the rows that fell back to selection over the
+// whole row (a sample window that missed, a column that overflowed) and those with too
+// many candidates in one bin (each thread then reads columns as the counting pass
+// wrote them).  Every block of a fixed grid takes a slice of each such row in turn, so
+// a row that fell back is read at the rate of the whole GPU, not of its own few
+// blocks.  mode 0 keys the values, mode 1 |x - median|; equal digits are aggregated
+// per warp in the first pass over a row (its keys share their high digits).
 __global__ void __launch_bounds__(kDetThreads)
 det_hist_row_kernel(const float *__restrict__ cc, size_t ld, const DetState *__restrict__ st,
                     const int *__restrict__ list, const int *__restrict__ count,
-                    unsigned *__restrict__ hist, int pass, int mode)
+                    unsigned *__restrict__ hist, const float *__restrict__ cand, long long cap, Lanes g,
+                    int pass, int mode)
 {
     __shared__ unsigned h[2 * kDetBins];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -921,32 +1069,43 @@ det_hist_row_kernel(const float *__restrict__ cc, size_t ld, const DetState *__r
         for (int i = threadIdx.x; i < 2 * kDetBins; i += kDetThreads)
             h[i] = 0u;
         __syncthreads();
-        const float *row = cc + (size_t)t * ld + s.begin;
-        const RowSplit rs = split_row(row, n);
-        if (blockIdx.x == 0 && warp == 0) {  // the unaligned ends, at most 3 + 3 values
-            const long long i = lane < rs.head ? lane : rs.head + 4 * rs.nvec + (lane - rs.head);
-            const bool ok = lane < rs.head + rs.tail;
-            const float v = ok ? row[i] : 0.f;
-            hist_add(h, v, ok, mode, s.med, shift, dmask, high, p0, p1, two, lane, agg);
-        }
-        const float4 *vrow = reinterpret_cast<const float4 *>(row + rs.head);
-        const long long steps = (rs.nvec + 63) / 64;  // 64 float4s per warp step
-        for (long long c = (long long)blockIdx.x * kWarps + warp; c < steps;
-             c += (long long)gridDim.x * kWarps) {
-            float4 v[2];
-            bool ok[2];
-#pragma unroll
-            for (int u = 0; u < 2; u++) {
-                const long long i = c * 64 + u * 32 + lane;
-                ok[u] = i < rs.nvec;
-                v[u] = ok[u] ? vrow[i] : make_float4(0.f, 0.f, 0.f, 0.f);
+        if (s.src == kSrcKeys) {
+            for (int r = (int)blockIdx.x * kWarps + warp; r < g.S * kWarps; r += (int)gridDim.x * kWarps) {
+                const float *kc = cand + (size_t)t * cap + (size_t)r * g.Ck * 32 + 8 * lane;
+                const int m = g.cnt_k[((size_t)t * g.S * kWarps + r) * 32 + lane];  // <= Ck: no column overflowed
+                const int mw = __reduce_max_sync(0xffffffffu, m);
+                for (int j = 0; j < mw; j++)
+                    hist_add(h, j < m ? kc[(j & ~7) * 32 + (j & 7)] : 0.0f, j < m, 2, s.med, shift, dmask, high, p0, p1, two,
+                             lane, true);
             }
+        } else {
+            const float *row = cc + (size_t)t * ld + s.begin;
+            const RowSplit rs = split_row(row, n);
+            if (blockIdx.x == 0 && warp == 0) {  // the unaligned ends, at most 3 + 3 values
+                const long long i = lane < rs.head ? lane : rs.head + 4 * rs.nvec + (lane - rs.head);
+                const bool ok = lane < rs.head + rs.tail;
+                const float v = ok ? row[i] : 0.f;
+                hist_add(h, v, ok, mode, s.med, shift, dmask, high, p0, p1, two, lane, agg);
+            }
+            const float4 *vrow = reinterpret_cast<const float4 *>(row + rs.head);
+            const long long steps = (rs.nvec + 63) / 64;  // 64 float4s per warp step
+            for (long long c = (long long)blockIdx.x * kWarps + warp; c < steps;
+                 c += (long long)gridDim.x * kWarps) {
+                float4 v[2];
+                bool ok[2];
 #pragma unroll
-            for (int u = 0; u < 2; u++) {
-                hist_add(h, v[u].x, ok[u], mode, s.med, shift, dmask, high, p0, p1, two, lane, agg);
-                hist_add(h, v[u].y, ok[u], mode, s.med, shift, dmask, high, p0, p1, two, lane, agg);
-                hist_add(h, v[u].z, ok[u], mode, s.med, shift, dmask, high, p0, p1, two, lane, agg);
-                hist_add(h, v[u].w, ok[u], mode, s.med, shift, dmask, high, p0, p1, two, lane, agg);
+                for (int u = 0; u < 2; u++) {
+                    const long long i = c * 64 + u * 32 + lane;
+                    ok[u] = i < rs.nvec;
+                    v[u] = ok[u] ? vrow[i] : make_float4(0.f, 0.f, 0.f, 0.f);
+                }
+#pragma unroll
+                for (int u = 0; u < 2; u++) {
+                    hist_add(h, v[u].x, ok[u], mode, s.med, shift, dmask, high, p0, p1, two, lane, agg);
+                    hist_add(h, v[u].y, ok[u], mode, s.med, shift, dmask, high, p0, p1, two, lane, agg);
+                    hist_add(h, v[u].z, ok[u], mode, s.med, shift, dmask, high, p0, p1, two, lane, agg);
+                    hist_add(h, v[u].w, ok[u], mode, s.med, shift, dmask, high, p0, p1, two, lane, agg);
+                }
             }
         }
         __syncthreads();
@@ -1253,14 +1412,16 @@ int detect_device(const float *cc, int T, int n_corr, size_t ld, const int *begi
     unsigned *hist = nullptr;
     int2 *cand = nullptr;
     int *hot = nullptr, *col_cnt = nullptr, *row_list = nullptr;
+    unsigned *bins = nullptr, *list = nullptr;
     float *saved = nullptr, *amb = nullptr, *keys = nullptr;
     // candidates per row: a sample window holds about 2.5 % of a row; the values whose
-    // MAD class waits for the median, about 7 % of a Gaussian row
-    // (at least 2 * kSpill rows of every thread's columns, so a row's columns always fit)
-    const long long key_cap = std::max(2LL * kSpill * kDetThreads,
-                                       n_corr < 65536 ? n_corr : std::max(65536LL, (long long)n_corr / 8));
-    const long long amb_cap = std::max(2LL * kSpill * kDetThreads,
-                                       n_corr < 65536 ? n_corr : std::max(65536LL, (long long)n_corr / 4));
+    // MAD class waits for the median, about 7 % of a Gaussian row (at least two sectors
+    // of each of a block's columns; whole sectors)
+    const auto list_cap = [&](int part) {
+        const long long n = n_corr < 65536 ? n_corr : std::max(65536, n_corr / part);
+        return (std::max(2LL * kStep * kDetThreads, n) + 7) & ~7LL;
+    };
+    const long long key_cap = list_cap(8), amb_cap = list_cap(4);
     if ((rc = ws.get(&st, (size_t)chunk, "detection state")) ||
         (rc = ws.get(&hist, (size_t)chunk * 2 * kDetBins, "detection histograms")) ||
         (rc = ws.get(&keys, (size_t)chunk * key_cap, "candidate keys")) ||
@@ -1269,6 +1430,8 @@ int detect_device(const float *cc, int T, int n_corr, size_t ld, const int *begi
         (rc = ws.get(&hot, (size_t)chunk * kDetCap, "values above the threshold bound")) ||
         (rc = ws.get(&saved, (size_t)chunk * kDetSample, "sampled values")) ||
         (rc = ws.get(&col_cnt, 2 * ((size_t)kDetBlocks + chunk) * kDetThreads, "list column counts")) ||
+        (rc = ws.get(&bins, (size_t)chunk * kCandBins, "candidate bins")) ||
+        (rc = ws.get(&list, (size_t)chunk * kPickCap, "picked candidates")) ||
         (rc = ws.get(&row_list, (size_t)chunk + 1, "rows of whole-row passes")))
         return rc;
     cudaError_t e = cudaFuncSetAttribute(det_select_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -1276,6 +1439,10 @@ int detect_device(const float *cc, int T, int n_corr, size_t ld, const int *begi
     if (e == cudaSuccess)
         e = cudaFuncSetAttribute(det_sample_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  (int)(kDetSample * sizeof(unsigned)));
+    if (e == cudaSuccess)
+        e = cudaFuncSetAttribute(det_count_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kCountSmem);
+    if (e == cudaSuccess)
+        e = cudaFuncSetAttribute(det_count_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kCountSmem);
     if (e != cudaSuccess)
         return set_error(FMF_ERR_CUDA, "detection shared memory: %s", cudaGetErrorString(e));
     if ((e = cudaMemsetAsync(hist, 0, (size_t)chunk * 2 * kDetBins * sizeof(unsigned), s)) != cudaSuccess)
@@ -1293,41 +1460,34 @@ int detect_device(const float *cc, int T, int n_corr, size_t ld, const int *begi
         if (per_row < 1)
             per_row = 1;
         const dim3 grid((unsigned)per_row, (unsigned)nt);
-        // one column per counting thread (nt * per_row <= kDetBlocks + nt blocks); rows
-        // C .. C + kSpill - 1 of each warp's region take a step's overflow
+        // one column per counting thread (nt * per_row <= kDetBlocks + nt blocks)
         Lanes g;
         g.S = (int)per_row;
-        g.Ck = (int)(key_cap / (per_row * kDetThreads) - kSpill);
-        g.Ca = (int)(amb_cap / (per_row * kDetThreads) - kSpill);
+        g.Ck = (int)(key_cap / (per_row * kDetThreads)) & ~7;
+        g.Ca = (int)(amb_cap / (per_row * kDetThreads)) & ~7;
+        const dim3 pick_grid((unsigned)std::min(per_row, ((long long)kDetPickBlocks + nt - 1) / nt), (unsigned)nt);
         g.cnt_k = col_cnt;
         g.cnt_a = col_cnt + ((size_t)kDetBlocks + chunk) * kDetThreads;
-        const int check_blocks = (nt + 127) / 128;
         det_init_kernel<<<(nt + 127) / 128, 128, 0, s>>>(st, nt, n_corr, begin ? begin + t0 : nullptr,
                                                          end ? end + t0 : nullptr);
-        // the median: sample, the one read of the rows, selection over the candidates
-        det_sample_kernel<<<nt, 1024, kDetSample * sizeof(unsigned), s>>>(rows, ld, st, 0, n_mad, saved);
-        det_count_kernel<true><<<grid, kDetThreads, 0, s>>>(rows, ld, st, keys, key_cap, amb, amb_cap, g, hot,
-                                                            kDetCap);
-        det_check_kernel<<<check_blocks, 128, 0, s>>>(st, nt, 0, kDetCap, n_mad);
         int *const rcount = row_list + chunk;
-        det_collect_kernel<<<1, 1024, 0, s>>>(st, nt, 0, row_list, rcount);
-        for (int pass = 0; pass < 3; pass++) {
-            det_hist_kernel<<<grid, kDetThreads, 0, s>>>(st, hist, keys, key_cap, g, pass);
-            det_hist_row_kernel<<<kDetRowBlocks, kDetThreads, 0, s>>>(rows, ld, st, row_list, rcount, hist,
-                                                                      pass, 0);
-            det_resolve_kernel<<<nt, 32, 0, s>>>(st, hist, pass, 0, n_mad);
-        }
-        // the MAD: the sample about the exact median, the listed values, selection
-        det_sample_kernel<<<nt, 1024, kDetSample * sizeof(unsigned), s>>>(rows, ld, st, 1, n_mad, saved);
-        det_count_kernel<false><<<grid, kDetThreads, 0, s>>>(rows, ld, st, keys, key_cap, amb, amb_cap, g, hot,
-                                                             kDetCap);
-        det_check_kernel<<<check_blocks, 128, 0, s>>>(st, nt, 1, kDetCap, n_mad);
-        det_collect_kernel<<<1, 1024, 0, s>>>(st, nt, 0, row_list, rcount);
-        for (int pass = 0; pass < 3; pass++) {
-            det_hist_kernel<<<grid, kDetThreads, 0, s>>>(st, hist, keys, key_cap, g, pass);
-            det_hist_row_kernel<<<kDetRowBlocks, kDetThreads, 0, s>>>(rows, ld, st, row_list, rcount, hist,
-                                                                      pass, 1);
-            det_resolve_kernel<<<nt, 32, 0, s>>>(st, hist, pass, 1, n_mad);
+        // mode 0, the median: sample, the one read of the rows, selection over the candidates;
+        // mode 1, the MAD: the sample about the exact median, the listed values, selection
+        for (int mode = 0; mode < 2; mode++) {
+            det_sample_kernel<<<nt, 1024, kDetSample * sizeof(unsigned), s>>>(rows, ld, st, mode, n_mad, saved);
+            if ((e = cudaMemsetAsync(bins, 0, (size_t)nt * kCandBins * sizeof(unsigned), s)) != cudaSuccess)
+                return set_error(FMF_ERR_CUDA, "clearing the candidate bins: %s", cudaGetErrorString(e));
+            (mode ? det_count_kernel<false> : det_count_kernel<true>)<<<grid, kDetThreads, kCountSmem, s>>>(
+                rows, ld, st, keys, key_cap, amb, amb_cap, g, bins, hot, kDetCap);
+            det_pick_kernel<<<nt, 32, 0, s>>>(st, bins, mode, kDetCap, n_mad);
+            det_gather_kernel<<<pick_grid, kDetThreads, 0, s>>>(st, keys, key_cap, g, list);
+            det_finish_kernel<<<nt, kDetThreads, 0, s>>>(st, list, mode, n_mad);
+            det_collect_kernel<<<1, 1024, 0, s>>>(st, nt, 0, row_list, rcount);
+            for (int pass = 0; pass < 3; pass++) {
+                det_hist_row_kernel<<<kDetRowBlocks, kDetThreads, 0, s>>>(rows, ld, st, row_list, rcount, hist, keys,
+                                                                          key_cap, g, pass, mode);
+                det_resolve_kernel<<<nt, 32, 0, s>>>(st, hist, pass, mode, n_mad);
+            }
         }
         det_hot_kernel<<<nt, kDetThreads, 0, s>>>(rows, ld, st, hot, kDetCap, cand, kDetCap);
         det_collect_kernel<<<1, 1024, 0, s>>>(st, nt, 1, row_list, rcount);
@@ -1336,7 +1496,7 @@ int detect_device(const float *cc, int T, int n_corr, size_t ld, const int *begi
             st, cand, kDetCap, min_sep, max_det, med_out ? med_out + t0 : nullptr,
             mad_out ? mad_out + t0 : nullptr, thr_out ? thr_out + t0 : nullptr, count_out + t0,
             lag_out + (size_t)t0 * max_det, val_out + (size_t)t0 * max_det);
-        count_launch(31);
+        count_launch(29);
         if ((rc = check_launch("detection kernels")))
             return rc;
     }

@@ -196,3 +196,17 @@ def test_detect_ties_and_constant_rows():
         x[t, rng.choice(n - 200, 3, replace=False) + 100] += 5.0
     det = fmf.detect(x, n_mad=30.0, min_separation=1000, max_detections=256)
     assert_matches(det, x, 30.0, 1000, 256)
+
+
+@pytest.mark.parametrize("share", [0.0002, 0.004, 0.02, 0.3])
+@pytest.mark.parametrize("n", [20011, 70000, 300000])
+def test_detect_equal_values_at_the_median(n, share):
+    """A gap's zeros at the middle of a row: few of them are picked out of the middle
+    ranks' bins, more are selected among by key bits, many overflow the candidates'
+    columns and take passes over the row."""
+    rng = np.random.default_rng(n)
+    cc = (rng.standard_normal((3, n)) * 0.01).astype(np.float32)
+    cc[:, rng.permutation(n)[: int(n * share)]] = 0.0
+    cc[1] += np.float32(0.25)
+    cc[2, ::1000] = np.float32(3.0)
+    assert_matches(fmf.detect(cc, n_mad=8.0, min_separation=25, max_detections=512), cc, 8.0, 25, 512)
