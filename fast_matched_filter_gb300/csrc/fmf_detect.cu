@@ -22,7 +22,7 @@
 //
 // The order statistics are exact, from one read of each row in the usual
 // case (a sample-select):
-//   1. one block per row sorts a strided sample of the row: the key window
+//   1. one block per row takes a strided sample of the row: the key window
 //      [klo, khi] around the two middle ranks (three binomial standard
 //      deviations wide), so the median lies in [m_lo, m_hi], the values of
 //      those keys; and from the sample's |x - m| about the window's middle, a
@@ -35,19 +35,21 @@
 //      either (listed: about 7 % of a Gaussian row); the same read notes the
 //      values at or above a lower bound of the threshold
 //      (m_lo + n_mad * a_lo: thr = med + n_mad * mad is monotone in both);
-//   3. the median: if the window holds both middle ranks, a radix selection
-//      over the candidates (passes of up to 11 bits over the key bits the
-//      window's keys do not share, each a shared-memory histogram of the keys
-//      that match the bits chosen so far); if not -- a window that missed
-//      (about one row in 800), heavy ties, an adversarial row -- the same
-//      selection over the whole row, by a fixed grid of blocks over the list
-//      of such rows, so that the row is read at the rate of the whole GPU;
+//   3. the median: if the window holds both middle ranks, the candidates' bins
+//      (counted as the pass ended) give the one or two that hold them; a read of the
+//      candidates gathers those bins' few values, and a block per row selects among
+//      them.  If a bin holds too many (ties), a radix selection over the candidates
+//      (passes of up to 11 bits over the key bits the window's keys do not share);
+//      if the window does not hold -- one that missed (about one row in 800), heavy
+//      ties, an adversarial row -- the same selection over the whole row.  A fixed
+//      grid of blocks takes these passes over the list of such rows, so that a row is
+//      read at the rate of the whole GPU;
 //   4. the MAD: the sample keyed by |x - med| narrows [a_lo, a_hi]; the listed
 //      values keyed by |x - med| are counted below the window or gathered in
 //      it, and selected as in 3.  A row whose median or MAD window missed, or
 //      whose list overflowed, selects its MAD over the whole row and takes its
-//      peaks in a pass of its own.  Rows no longer than the sample are sorted
-//      whole.
+//      peaks in a pass of its own.  Rows no longer than the sample are selected
+//      in step 1.
 // The values noted in step 2 are examined by a small kernel for the local
 // maximum and plateau rules: a superset of the peaks, gathered into a list
 // per template (capacity kDetCap) and filtered by one thread block per
@@ -66,6 +68,7 @@ namespace {
 
 constexpr int kDetBins = 2048;            // histogram bins of the 11-bit passes
 constexpr int kDetThreads = 256;          // histogram / peak kernels
+constexpr int kDetSampleThreads = 512;    // two sample blocks per SM
 constexpr int kDetSelectThreads = 1024;   // per-template filter kernel
 constexpr int kDetChunk = 1024;           // templates per round of scratch
 constexpr int kDetCap = 16384;            // candidate peaks per template row
@@ -95,7 +98,7 @@ struct DetState {
     float thr_lo;          // a lower bound of thr known before the counting pass
     int peaks_ready;       // 1: the counting pass noted the values >= thr_lo
     int n_hot;             // values >= thr_lo noted (may exceed the capacity)
-    int src;               // kSrcRow / kSrcCand / kSrcDone
+    int src;               // kSrc...
     unsigned klo, khi;     // key window of the current selection
     int n_lt, n_in;        // keys below klo, keys inside [klo, khi]
     int bin0, bin1;        // bins (cand_bin) of the middle ranks
@@ -230,6 +233,46 @@ __device__ __forceinline__ void finish_select(DetState &s, int mode, float v, fl
     }
 }
 
+// A value's bin, of B over the window [lo, hi]: never falls as x rises (nor do a float
+// difference and product), so bins are ranges of ranks.
+template <int B>
+__device__ __forceinline__ float bin_scale(float lo, float hi)
+{
+    return __fdiv_rn((float)B, __fsub_rn(hi, lo));
+}
+template <int B>
+__device__ __forceinline__ int value_bin(float x, float lo, float scale)
+{
+    return min(max((int)__fmul_rn(__fsub_rn(x, lo), scale), 0), B - 1);
+}
+
+// The bin of h[kDetBins] that holds rank rk, and the count before it (one warp).
+__device__ void find_rank(const unsigned *h, unsigned rk, int lane, int *pick)
+{
+    const int per = kDetBins / 32;
+    unsigned sum = 0;
+    for (int i = 0; i < per; i++)
+        sum += h[lane * per + i];
+    unsigned inc = sum;
+    for (int o = 1; o < 32; o <<= 1) {
+        const unsigned y = __shfl_up_sync(0xffffffffu, inc, o);
+        if (lane >= o)
+            inc += y;
+    }
+    const unsigned exc = inc - sum;
+    if (rk >= exc && rk < inc) {
+        unsigned c = exc;
+        int i = 0;
+        for (; i < per - 1; i++) {
+            if (rk < c + h[lane * per + i])
+                break;
+            c += h[lane * per + i];
+        }
+        pick[0] = lane * per + i;
+        pick[1] = (int)c;
+    }
+}
+
 // The keys of ranks r0 <= r1 (0-based, ascending) among the first P keys of
 // sk, by the block: three radix passes (11, 11 and 10 bits), each a
 // shared-memory histogram per rank of the keys that match that rank's bits so
@@ -267,29 +310,7 @@ __device__ void block_select2(const unsigned *sk, int P, int r0, int r1, unsigne
         }
         __syncthreads();
         if (warp < 2) {
-            const unsigned *h = hist + (two ? warp : 0) * kDetBins;
-            const int per = kDetBins / 32;
-            unsigned sum = 0;
-            for (int i = 0; i < per; i++)
-                sum += h[lane * per + i];
-            unsigned inc = sum;
-            for (int o = 1; o < 32; o <<= 1) {
-                const unsigned y = __shfl_up_sync(0xffffffffu, inc, o);
-                if (lane >= o)
-                    inc += y;
-            }
-            const unsigned exc = inc - sum, rk = (unsigned)(warp == 0 ? r[0] : r[1]);
-            if (rk >= exc && rk < inc) {
-                unsigned c = exc;
-                int i = 0;
-                for (; i < per - 1; i++) {
-                    if (rk < c + h[lane * per + i])
-                        break;
-                    c += h[lane * per + i];
-                }
-                pick[2 * warp] = lane * per + i;
-                pick[2 * warp + 1] = (int)c;
-            }
+            find_rank(hist + (two ? warp : 0) * kDetBins, (unsigned)r[warp], lane, pick + 2 * warp);
         }
         __syncthreads();
         for (int q = 0; q < 2; q++) {
@@ -302,12 +323,79 @@ __device__ void block_select2(const unsigned *sk, int P, int r0, int r1, unsigne
     k1 = pre[1];
 }
 
-// A candidate's bin, of kCandBins over its window [lo, hi]: never falls as x rises (nor
-// do a float difference and product), so bins are ranges of ranks.
-__device__ __forceinline__ float bin_scale(float lo, float hi) { return __fdiv_rn((float)kCandBins, __fsub_rn(hi, lo)); }
-__device__ __forceinline__ int cand_bin(float x, float lo, float scale)
+// The same ranks through bins of the values between the smallest and the largest key:
+// one pass, then each rank among the few keys of its bin (a few hundred of 16,384
+// beside peaks of 100 standard deviations).  The radix passes where a bin holds more
+// than kSampleBin keys or the values' range is not finite.
+constexpr int kSampleBin = kDetBins / 2;
+__device__ void block_select2_bins(const unsigned *sk, int n, int r0, int r1, unsigned *hist, int *pick,
+                                   unsigned *range, unsigned &k0, unsigned &k1)
 {
-    return min(max((int)__fmul_rn(__fsub_rn(x, lo), scale), 0), kCandBins - 1);
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    if (threadIdx.x == 0) {
+        range[0] = 0xffffffffu;
+        range[1] = 0u;
+        range[2] = range[3] = 0u;  // keys of either bin
+    }
+    for (int i = threadIdx.x; i < kDetBins; i += blockDim.x)
+        hist[i] = 0u;
+    __syncthreads();
+    unsigned least = 0xffffffffu, most = 0u;
+    for (int i = threadIdx.x; i < n; i += blockDim.x) {
+        least = min(least, sk[i]);
+        most = max(most, sk[i]);
+    }
+    least = __reduce_min_sync(0xffffffffu, least);
+    most = __reduce_max_sync(0xffffffffu, most);
+    if (lane == 0) {
+        atomicMin(&range[0], least);
+        atomicMax(&range[1], most);
+    }
+    __syncthreads();
+    const float lo = key_value(range[0]), scale = bin_scale<kDetBins>(lo, key_value(range[1]));
+    if (!(scale > 0.0f && scale < INFINITY)) {
+        block_select2(sk, n, r0, r1, hist, pick, k0, k1);
+        return;
+    }
+    for (int i = threadIdx.x; i < n; i += blockDim.x)
+        atomicAdd(&hist[value_bin<kDetBins>(key_value(sk[i]), lo, scale)], 1u);
+    __syncthreads();
+    if (warp < 2)
+        find_rank(hist, (unsigned)(warp == 0 ? r0 : r1), lane, pick + 2 * warp);
+    __syncthreads();
+    const int bin[2] = {pick[0], pick[2]}, rank[2] = {r0 - pick[1], r1 - pick[3]};
+    if (hist[bin[0]] > (unsigned)kSampleBin || hist[bin[1]] > (unsigned)kSampleBin) {
+        __syncthreads();
+        block_select2(sk, n, r0, r1, hist, pick, k0, k1);
+        return;
+    }
+    unsigned *const list = hist + kDetBins;  // kSampleBin keys each
+    for (int i = threadIdx.x; i < n; i += blockDim.x) {
+        const unsigned k = sk[i];
+        const int b = value_bin<kDetBins>(key_value(k), lo, scale);
+        for (int q = 0; q < 2; q++)
+            if (b == bin[q])
+                list[q * kSampleBin + atomicAdd(&range[2 + q], 1u)] = k;
+    }
+    __syncthreads();
+    for (int q = 0; q < 2; q++) {
+        const unsigned *l = list + q * kSampleBin;
+        const int m = (int)range[2 + q];
+        for (int i = threadIdx.x; i < m; i += blockDim.x) {
+            const unsigned k = l[i];
+            int below = 0, equal = 0;
+            for (int j = 0; j < m; j++) {
+                below += l[j] < k;
+                equal += l[j] == k;
+            }
+            if (below <= rank[q] && rank[q] < below + equal)
+                pick[q] = (int)k;
+        }
+    }
+    __syncthreads();
+    k0 = (unsigned)pick[0];
+    k1 = (unsigned)pick[1];
+    __syncthreads();
 }
 
 // |x - m| in float32, as numpy computes the MAD's deviations.
@@ -361,7 +449,7 @@ __device__ unsigned last_key(unsigned c, F pred)
 }
 
 // Step 1 and 4 of the sample-select (one block per row).  Mode 0: a strided
-// sample of the row (kept in `saved`), sorted: the exact median and MAD for a
+// sample of the row (kept in `saved`), selected among: the exact median and MAD for a
 // row no longer than the sample; else the median's key window, the MAD's
 // window about the median window's middle, and the MAD classes of the
 // counting pass.  Mode 1 (the median now exact): the sample keyed by
@@ -372,7 +460,7 @@ __device__ unsigned last_key(unsigned c, F pred)
 // over the whole row, a few reads of it at the rate of the whole GPU
 constexpr int kPad = 3 * 64 + 16;
 
-__global__ void __launch_bounds__(1024)
+__global__ void __launch_bounds__(kDetSampleThreads, 2)
 det_sample_kernel(const float *__restrict__ cc, size_t ld, DetState *__restrict__ st, int mode,
                   float n_mad, float *__restrict__ saved)
 {
@@ -380,6 +468,7 @@ det_sample_kernel(const float *__restrict__ cc, size_t ld, DetState *__restrict_
     unsigned *sk = reinterpret_cast<unsigned *>(sample_smem);  // kDetSample keys
     __shared__ unsigned hist[2 * kDetBins];
     __shared__ int pick[4];
+    __shared__ unsigned range[4];
     const int t = blockIdx.x;
     const int begin = st[t].begin;
     const long long n = st[t].end - begin;
@@ -387,9 +476,6 @@ det_sample_kernel(const float *__restrict__ cc, size_t ld, DetState *__restrict_
         return;
     const float *row = cc + (size_t)t * ld + begin;
     const int m = n < kDetSample ? (int)n : kDetSample;
-    int P = 1;
-    while (P < m)
-        P <<= 1;
     const long long a = (n - 1) / 2, b = n / 2;
     float *sv = saved + (size_t)t * kDetSample;
     const float med = st[t].med;  // mode 1: exact
@@ -406,7 +492,7 @@ det_sample_kernel(const float *__restrict__ cc, size_t ld, DetState *__restrict_
         st[t] = s;
     };
     if (mode == 1) {
-        const bool whole = m == n;  // sorted whole by the median's sample
+        const bool whole = m == n;  // selected whole by the median's sample
         const bool list = !whole && st[t].one_read && !st[t].over_a && med >= st[t].m_lo &&
                           med <= st[t].m_hi;
         if (!whole && !list) {
@@ -417,31 +503,33 @@ det_sample_kernel(const float *__restrict__ cc, size_t ld, DetState *__restrict_
     }
     // sample positions floor(i * n / m) from a fixed-point step (no 64-bit division
     // per sample); any spread of positions serves, the selection is exact
-    // (blockDim.x = 1024, P <= kDetSample: kPer slots per thread, all loads issued
-    // before the first store, so the scattered reads are in flight together)
+    // (kPer loads per thread issued before the first store, so the scattered reads are
+    // in flight together)
     const unsigned long long stepq = ((unsigned long long)n << 20) / (unsigned long long)m;
-    constexpr int kPer = kDetSample / 1024;
-    float v[kPer];
+    constexpr int kPer = 16;
+    for (int i0 = threadIdx.x; i0 < m; i0 += kPer * kDetSampleThreads) {
+        float v[kPer];
 #pragma unroll
-    for (int j = 0; j < kPer; j++) {
-        const int i = threadIdx.x + j * 1024;
-        v[j] = 0.0f;
-        if (i < m) {
-            if (mode == 0) {
-                const long long pos = (long long)(((unsigned long long)i * stepq) >> 20);
-                v[j] = row[pos < n ? pos : n - 1];
-            } else {
-                v[j] = sv[i];
+        for (int j = 0; j < kPer; j++) {
+            const int i = i0 + j * kDetSampleThreads;
+            v[j] = 0.0f;
+            if (i < m) {
+                if (mode == 0) {
+                    const long long pos = (long long)(((unsigned long long)i * stepq) >> 20);
+                    v[j] = row[pos < n ? pos : n - 1];
+                } else {
+                    v[j] = sv[i];
+                }
             }
         }
-    }
 #pragma unroll
-    for (int j = 0; j < kPer; j++) {
-        const int i = threadIdx.x + j * 1024;
-        if (i < P) {
-            if (mode == 0 && i < m)
-                sv[i] = v[j];
-            sk[i] = i < m ? order_key(mode == 0 ? v[j] : dev(v[j], med)) : 0xffffffffu;  // padding ranks last
+        for (int j = 0; j < kPer; j++) {
+            const int i = i0 + j * kDetSampleThreads;
+            if (i < m) {
+                if (mode == 0)
+                    sv[i] = v[j];
+                sk[i] = order_key(mode == 0 ? v[j] : dev(v[j], med));
+            }
         }
     }
     __syncthreads();
@@ -451,7 +539,7 @@ det_sample_kernel(const float *__restrict__ cc, size_t ld, DetState *__restrict_
     const int r0 = m == n ? (int)a : (int)(pa - kPad > 0 ? pa - kPad : 0);
     const int r1 = m == n ? (int)b : (int)(pb + kPad < m - 1 ? pb + kPad : m - 1);
     unsigned k0, k1;
-    block_select2(sk, P, r0, r1, hist, pick, k0, k1);
+    block_select2_bins(sk, m, r0, r1, hist, pick, range, k0, k1);
     if (m == n) {  // the whole row: exact
         if (threadIdx.x == 0) {
             DetState s = st[t];
@@ -489,11 +577,11 @@ det_sample_kernel(const float *__restrict__ cc, size_t ld, DetState *__restrict_
     const float m_lo = __fadd_rn(key_value(k0), 0.0f), m_hi = __fadd_rn(key_value(k1), 0.0f);
     const float mid = __fadd_rn(__fmul_rn(0.5f, m_lo), __fmul_rn(0.5f, m_hi));
     __syncthreads();  // every thread is past its last read of the value keys
-    for (int i = threadIdx.x; i < P; i += blockDim.x)
-        sk[i] = i < m ? order_key(dev(sv[i], mid)) : 0xffffffffu;
+    for (int i = threadIdx.x; i < m; i += blockDim.x)
+        sk[i] = order_key(dev(sv[i], mid));
     __syncthreads();
     unsigned ka0, ka1;
-    block_select2(sk, P, r0, r1, hist, pick, ka0, ka1);
+    block_select2_bins(sk, m, r0, r1, hist, pick, range, ka0, ka1);
     if (threadIdx.x != 0)
         return;
     DetState s = st[t];
@@ -578,8 +666,9 @@ __device__ __forceinline__ void note_hot(DetState *st, int t, long long o, int *
 // The entries of a column wait in shared memory, a ring of kRing rows per warp (a
 // lane's bank is its own, so appending never conflicts), and go out a sector of eight
 // at a time.  Stored as they came, each 4-byte value cost a 32-byte sector, and these
-// sectors bounded the pass (COUNTMEASURED).  What bounds it now: its instructions,
-// about 20 per value.
+// sectors bounded the pass (500 rows of 4.3M values: 2.23 ms, of 1.28 ms for the
+// rows' bytes; 1.64 ms here).  What bounds it now: the rows' and the lists' bytes
+// (1.2 per row byte) and its instructions, about 20 per value, to about the same part.
 struct Column {
     unsigned in, out;  // entries begun and stored, times 128 (bytes of a ring row)
     // a sector, if there is one (at most one: fewer than 8 entries waited before a step
@@ -820,14 +909,14 @@ det_count_kernel(const float *__restrict__ cc, size_t ld, DetState *__restrict__
             atomicOr(&st[t].over_a, 1);
     }
     // the candidates' bins, from the column this thread wrote
-    const float scale = bin_scale(lo, hi);
+    const float scale = bin_scale<kCandBins>(lo, hi);
     for (int k = 0; k < min(nk, g.Ck); k += 8) {
         float x[8];
         load_sector(kc, k, x);
 #pragma unroll
         for (int j = 0; j < 8; j++)
             if (k + j < nk)
-                atomicAdd(&bin[cand_bin(x[j], lo, scale)], 1u);
+                atomicAdd(&bin[value_bin<kCandBins>(x[j], lo, scale)], 1u);
     }
     __syncthreads();
     unsigned *gb = bins + (size_t)t * kCandBins;
@@ -929,7 +1018,7 @@ det_gather_kernel(DetState *__restrict__ st, const float *__restrict__ cand, lon
         return;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     constexpr int kWarps = kDetThreads / 32;
-    const float lo = key_value(st[t].klo), scale = bin_scale(lo, key_value(st[t].khi));
+    const float lo = key_value(st[t].klo), scale = bin_scale<kCandBins>(lo, key_value(st[t].khi));
     const int bin0 = st[t].bin0, bin1 = st[t].bin1;
     for (int blk = blockIdx.x; blk < g.S; blk += gridDim.x) {
         const size_t col = ((size_t)t * g.S + blk) * kDetThreads + threadIdx.x;
@@ -940,7 +1029,7 @@ det_gather_kernel(DetState *__restrict__ st, const float *__restrict__ cand, lon
             load_sector(kc, k, x);
 #pragma unroll
             for (int j = 0; j < 8; j++) {
-                const int b = cand_bin(x[j], lo, scale);
+                const int b = value_bin<kCandBins>(x[j], lo, scale);
                 if (k + j < m && b >= bin0 && b <= bin1) {  // (the bins between them are empty)
                     const int at = atomicAdd(&st[t].n_list, 1);
                     if (at < kPickCap)
@@ -1208,7 +1297,7 @@ det_hot_kernel(const float *__restrict__ cc, size_t ld, DetState *__restrict__ s
 
 // Local maxima at or above the threshold, appended (unordered) to the
 // template's candidate list, for the rows whose counting pass did not gather
-// them (rows sorted whole by the sample, windows that missed, supersets that
+// them (rows selected whole by the sample, windows that missed, supersets that
 // overflowed): every block of a fixed grid takes a slice of each such row in
 // turn.  Samples are read with 16-byte loads; the rare sample at or above the
 // threshold is examined with scalar loads.
@@ -1474,7 +1563,7 @@ int detect_device(const float *cc, int T, int n_corr, size_t ld, const int *begi
         // mode 0, the median: sample, the one read of the rows, selection over the candidates;
         // mode 1, the MAD: the sample about the exact median, the listed values, selection
         for (int mode = 0; mode < 2; mode++) {
-            det_sample_kernel<<<nt, 1024, kDetSample * sizeof(unsigned), s>>>(rows, ld, st, mode, n_mad, saved);
+            det_sample_kernel<<<nt, kDetSampleThreads, kDetSample * sizeof(unsigned), s>>>(rows, ld, st, mode, n_mad, saved);
             if ((e = cudaMemsetAsync(bins, 0, (size_t)nt * kCandBins * sizeof(unsigned), s)) != cudaSuccess)
                 return set_error(FMF_ERR_CUDA, "clearing the candidate bins: %s", cudaGetErrorString(e));
             (mode ? det_count_kernel<false> : det_count_kernel<true>)<<<grid, kDetThreads, kCountSmem, s>>>(
