@@ -12,6 +12,9 @@
 #include <cstring>
 #include <cstdlib>
 #include <climits>
+#include <algorithm>
+#include <condition_variable>
+#include <memory>
 #include <mutex>
 #include <thread>
 #include <vector>
@@ -106,52 +109,120 @@ static void span(cudaEvent_t a, cudaEvent_t b, int kind)
     }
 }
 
-// Maps the host pages of [p, p + bytes) for writing, on several threads, so
-// that the device-to-host copy of a result into them does not fault every page
-// in on its way: a fresh output array -- the reference's front-end allocates
-// one per call, fast_matched_filter.py:269-274 -- is untouched memory, and a
-// copy into it ran at 29 GB/s against 190 GB/s into mapped pages (8.6 GB for
-// the full-day search).  Mapped pages cost a page-table walk; where the
-// kernel refuses the advice (older kernels, page-locked mappings) nothing
-// is done.
-void populate_host(void *p, size_t bytes)
-{
-#if defined(__linux__)
-    const long page = sysconf(_SC_PAGESIZE);
-    if (!p || bytes == 0 || page <= 0)
-        return;
-    const uintptr_t a = (uintptr_t)p & ~(uintptr_t)(page - 1);
-    const uintptr_t b = ((uintptr_t)p + bytes + page - 1) & ~(uintptr_t)(page - 1);
-    const size_t pages = (b - a) / page;
-    const size_t min_part = ((size_t)32 << 20) / page;  // at least 32 MB per thread
-    unsigned nt = std::thread::hardware_concurrency();
-    nt = nt == 0 ? 1 : (nt > 16 ? 16 : nt);
-    if (pages / min_part < nt)
-        nt = (unsigned)(pages / min_part > 0 ? pages / min_part : 1);
-    auto part = [&](unsigned i) {
-        const size_t p0 = pages * i / nt, p1 = pages * (i + 1) / nt;
-        if (p1 > p0)
-            madvise((void *)(a + p0 * page), (p1 - p0) * page, MADV_POPULATE_WRITE);
-    };
-    if (nt == 1) {
-        part(0);
-        return;
-    }
+static bool host_is_pinned(const void *p);
+
+// A fresh output array -- the reference's front-end allocates one per call,
+// fast_matched_filter.py:269-274 -- is untouched memory, and a copy into it runs at
+// 27 GB/s against 190 GB/s into mapped pages.  So its pages are mapped first: an output
+// copied in one piece while the inputs travel and the kernels run (from 16 MB on: one
+// channel of a day at 100 Hz, 35 MB out, 2.00 -> 1.18 ms; less is mapped while the
+// kernels run), one copied in pieces before each piece, behind the kernels of the
+// others (started with the inputs, 432 MB held up their copies: 25.9 -> 26.2 ms).  Two
+// threads map 73 GB/s, four 80 to 86, eight 53 to 69 (they wait for one another in the
+// system).  Mapped pages cost a page-table walk; where the system refuses the advice
+// (older kernels) nothing is done.
+struct HostPages::State {
+    static constexpr size_t kBlock = (size_t)2 << 20;
+    static constexpr int kMaxThreads = 4;
+    uintptr_t begin, end;  // whole pages
+    size_t n_blocks, next = 0;
+    std::vector<unsigned char> done;
+    std::mutex m;
+    std::condition_variable cv;
     std::vector<std::thread> pool;
-    for (unsigned i = 1; i < nt; i++)
-        pool.emplace_back(part, i);
-    part(0);
-    for (auto &t : pool)
-        t.join();
-#else
-    (void)p;
-    (void)bytes;
+
+    // Maps the next block below `need`; false if there is none.
+    bool map_one(size_t need)
+    {
+        size_t i;
+        {
+            std::lock_guard<std::mutex> lock(m);
+            if (next >= need)
+                return false;
+            i = next++;
+        }
+        const uintptr_t p = begin + i * kBlock;
+#if defined(__linux__) && defined(MADV_POPULATE_WRITE)
+        madvise((void *)p, end - p < kBlock ? end - p : kBlock, MADV_POPULATE_WRITE);
 #endif
+        {
+            std::lock_guard<std::mutex> lock(m);
+            done[i] = 1;
+        }
+        cv.notify_all();
+        return true;
+    }
+    void start(size_t need, int threads)
+    {
+        for (int i = 0; i < threads; i++)
+            pool.emplace_back([this, need] {
+                while (map_one(need)) {
+                }
+            });
+    }
+    void join()
+    {
+        for (auto &t : pool)
+            t.join();
+        pool.clear();
+    }
+};
+
+constexpr size_t kAheadBytes = (size_t)16 << 20;
+
+HostPages::HostPages(void *p, size_t bytes) : st(nullptr)
+{
+    const long page = sysconf(_SC_PAGESIZE);
+    if (!p || bytes == 0 || page <= 0 || host_is_pinned(p))
+        return;
+    try {
+        std::unique_ptr<State> q(new State);
+        q->begin = (uintptr_t)p & ~(uintptr_t)(page - 1);
+        q->end = ((uintptr_t)p + bytes + page - 1) & ~(uintptr_t)(page - 1);
+        q->n_blocks = (q->end - q->begin + State::kBlock - 1) / State::kBlock;
+        q->done.resize(q->n_blocks);
+        st = q.release();
+        if (bytes >= kAheadBytes && bytes < kPieceBytes)
+            st->start(st->n_blocks, (int)std::min<size_t>(State::kMaxThreads, bytes / (4 * State::kBlock)));
+    } catch (...) {  // no memory or no threads: wait() maps what is left
+    }
 }
 
-// Page-locked (or registered) host memory is mapped already: populate_host
-// would only walk its page tables.
-bool host_is_pinned(const void *p)
+HostPages::~HostPages()
+{
+    if (!st)
+        return;
+    {
+        std::lock_guard<std::mutex> lock(st->m);
+        st->next = st->n_blocks;
+    }
+    st->join();
+    delete st;
+}
+
+void HostPages::wait(size_t bytes)
+{
+    if (!st)
+        return;
+    const size_t need = std::min(st->n_blocks, bytes / State::kBlock + 2);  // (begin may lie below p)
+    if (st->pool.empty() && need - std::min(st->next, need) >= 8) {
+        try {
+            st->start(need, State::kMaxThreads - 1);
+        } catch (...) {  // no threads: this one maps all
+        }
+        while (st->map_one(need)) {
+        }
+        st->join();
+        return;
+    }
+    while (st->map_one(need)) {
+    }
+    std::unique_lock<std::mutex> lock(st->m);
+    st->cv.wait(lock, [&] { return std::all_of(st->done.begin(), st->done.begin() + need, [](unsigned char d) { return d; }); });
+}
+
+// Page-locked (or registered) host memory is mapped already.
+static bool host_is_pinned(const void *p)
 {
     cudaPointerAttributes at;
     if (cudaPointerGetAttributes(&at, p) != cudaSuccess) {
@@ -559,7 +630,7 @@ static int run_device(const Args &a, cudaStream_t s)
 // Device-resident search whose result is copied to `host_out` in template
 // chunks on a second stream, each chunk's copy overlapping the next chunk's
 // kernel.  Preprocessing is done once for all templates.
-static int run_streamed(const Args &d, float *host_out, cudaStream_t s)
+static int run_streamed(const Args &d, float *host_out, HostPages &pages, cudaStream_t s)
 {
     int rc;
     Scratch ws(s);
@@ -572,7 +643,7 @@ static int run_streamed(const Args &d, float *host_out, cudaStream_t s)
     span(ev_prep0, ev_kern0, kSpanPrep);
     const size_t row = (size_t)P.n_corr * (P.network_sum ? 1 : P.SC);  // floats per template
     const size_t out_bytes = (size_t)P.T * row * sizeof(float);
-    const int n_chunks = out_bytes < ((size_t)64 << 20) ? 1 : (P.T < 8 ? P.T : 8);
+    const int n_chunks = out_bytes < kPieceBytes ? 1 : (P.T < 8 ? P.T : 8);
     // Template chunks of tapering size (weights 8,8,8,8,4,2,1,1 of 40 when there
     // are enough templates): each chunk's copy overlaps the next chunk's kernel,
     // and the last copy, which nothing overlaps, is small.
@@ -628,7 +699,6 @@ static int run_streamed(const Args &d, float *host_out, cudaStream_t s)
         // end of the last correlation kernel (twice: each span owns its events)
         cudaEvent_t ev_kern1 = mark(s), ev_kern1b = mark(s), ev_out0 = nullptr;
         span(ev_kern0, ev_kern1, kSpanKernel);
-        const bool pinned = host_is_pinned(host_out);
         for (int c = 0; c < launched && rc == FMF_OK && e == cudaSuccess; c++) {
             const int t0 = bounds[c], nt = bounds[c + 1] - bounds[c];
             if (nt <= 0)
@@ -638,8 +708,7 @@ static int run_streamed(const Args &d, float *host_out, cudaStream_t s)
                 break;
             if (!ev_out0)
                 ev_out0 = mark(s2);
-            if (!pinned)
-                populate_host(host_out + off, n);  // while the kernels run
+            pages.wait(off * sizeof(float) + n);
             if ((e = cudaMemcpyAsync(host_out + off, P.out + off, n, cudaMemcpyDeviceToHost, s2)) !=
                 cudaSuccess)
                 break;
@@ -703,6 +772,7 @@ static int run_host(const Args &a, cudaStream_t s)
 {
     int rc;
     const size_t out_n = a.T * a.n_corr * (a.sum_mode ? 1 : a.S * a.C);
+    HostPages pages(a.out, out_n * sizeof(float));
     {
         Scratch io(s);  // device copies of the arguments, freed in stream order
         Args d;
@@ -712,7 +782,7 @@ static int run_host(const Args &a, cudaStream_t s)
             return rc;
         span(ev_in0, mark(s), kSpanInput);
         d.out = out;
-        if ((rc = run_streamed(d, a.out, s)))
+        if ((rc = run_streamed(d, a.out, pages, s)))
             return rc;
     }
     if ((rc = cuda_status(cudaStreamSynchronize(s), "matched filter")))

@@ -181,8 +181,23 @@ int check_launch(const char *what);
 constexpr int kMaxDynamicSmem = 227 * 1024;
 // Maps the host pages of a result buffer for writing before a copy into it
 // (parallel; a no-op where the kernel refuses).
-void populate_host(void *p, size_t bytes);
-bool host_is_pinned(const void *p);  // page-locked or registered host memory
+// Host outputs of this size are copied in pieces, each behind the next one's kernels.
+constexpr size_t kPieceBytes = (size_t)64 << 20;
+// Maps the pages of a host output, of a medium size on threads of its own from
+// construction on; wait() returns once the first `bytes` of it are mapped.  Page-locked
+// memory is left alone.
+class HostPages {
+public:
+    HostPages(void *p, size_t bytes);
+    ~HostPages();
+    HostPages(const HostPages &) = delete;
+    HostPages &operator=(const HostPages &) = delete;
+    void wait(size_t bytes);
+
+private:
+    struct State;
+    State *st;
+};
 
 // Stream-ordered scratch allocations (cudaMallocAsync from the device's
 // default pool).  The pool keeps freed blocks for reuse by later calls;

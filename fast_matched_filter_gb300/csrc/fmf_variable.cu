@@ -546,7 +546,7 @@ struct CopyStream {
 // tapering size (8,8,8,8,4,2,1,1 of 40 parts), each chunk's copy on a second
 // stream overlapping the later chunks' kernels (all of which are queued before
 // the first copy, which blocks the host when host_out is pageable).
-static int variable_device(const VArgs &a, int L, cudaStream_t s, float *host_out = nullptr)
+static int variable_device(const VArgs &a, int L, cudaStream_t s, float *host_out = nullptr, HostPages *pages = nullptr)
 {
     int rc;
     const int T = (int)a.T, SC = (int)(a.S * a.C), N = (int)a.N;
@@ -657,7 +657,7 @@ static int variable_device(const VArgs &a, int L, cudaStream_t s, float *host_ou
         return rc;
     set_last_precision(precision);
     const size_t row_bytes = a.n_corr * sizeof(float);
-    const int n_chunks = (!host_out || (size_t)T * row_bytes < ((size_t)64 << 20)) ? 1 : (T < 8 ? T : 8);
+    const int n_chunks = (!host_out || (size_t)T * row_bytes < kPieceBytes) ? 1 : (T < 8 ? T : 8);
     int bounds[9];
     {
         static const int wts[8] = {8, 8, 8, 8, 4, 2, 1, 1};
@@ -727,13 +727,11 @@ static int variable_device(const VArgs &a, int L, cudaStream_t s, float *host_ou
     }
     if (!host_out)
         return FMF_OK;
-    const bool out_pinned = host_is_pinned(host_out);
     for (int c = 0; c < n_chunks; c++) {
         const int t0 = bounds[c], nt = bounds[c + 1] - bounds[c];
         if (nt <= 0)
             continue;
-        if (!out_pinned)
-            populate_host(host_out + (size_t)t0 * a.n_corr, (size_t)nt * row_bytes);  // while kernels run
+        pages->wait((size_t)(t0 + nt) * row_bytes);
         if ((e = cudaStreamWaitEvent(cs.s2, cs.ev[c], 0)) != cudaSuccess ||
             (e = cudaMemcpyAsync(host_out + (size_t)t0 * a.n_corr, a.out + (size_t)t0 * a.n_corr,
                                  (size_t)nt * row_bytes, cudaMemcpyDeviceToHost, cs.s2)) != cudaSuccess)
@@ -802,6 +800,7 @@ static int variable_entry(const VArgs &a, void *stream)
     const size_t SC = a.S * a.C;
     const size_t cnt[7] = {a.T * SC * L, a.T * SC, a.T * SC, SC * a.N, a.T * SC, a.T * SC, a.T * a.n_corr};
     float *buf[7];
+    HostPages pages(a.out, cnt[6] * sizeof(float));
     {
         Scratch io(s);
         for (int i = 0; i < 7; i++)
@@ -821,7 +820,7 @@ static int variable_entry(const VArgs &a, void *stream)
         d.w = buf[4];
         d.ntap = reinterpret_cast<const int *>(buf[5]);
         d.out = buf[6];
-        if ((rc = variable_device(d, L, s, a.out)))
+        if ((rc = variable_device(d, L, s, a.out, &pages)))
             return rc;
     }
     cudaError_t e = cudaStreamSynchronize(s);

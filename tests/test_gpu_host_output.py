@@ -1,0 +1,30 @@
+"""Results in fresh host memory, around the sizes at which its pages are mapped ahead
+of the copy and in pieces (needs a GB300): equal to those left on the device."""
+import numpy as np
+import pytest
+
+import fast_matched_filter_gb300 as fmf
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("megabytes", [0.01, 1, 15.9, 16.1, 63.9, 64.1])
+@pytest.mark.parametrize("T", [1, 9])
+def test_host_output_equals_device_output(megabytes, T):
+    import torch
+
+    L = 16
+    n_corr = int(megabytes * 2 ** 20 / (4 * T)) + 1
+    rng = np.random.default_rng(T)
+    tp = rng.standard_normal((T, 1, 1, L)).astype(np.float32)
+    d = rng.standard_normal((1, 1, n_corr + L - 1)).astype(np.float32)
+    mo, w = np.zeros((T, 1, 1), np.int32), np.ones((T, 1, 1), np.float32)
+    got = fmf.matched_filter(tp, mo, w, d, 1, check_zeros=False)
+    out = torch.empty((T, n_corr), device="cuda")
+    fmf.matched_filter_device(torch.tensor(tp).cuda(), None, torch.tensor(mo).cuda(), torch.tensor(w).cuda(),
+                              torch.tensor(d).cuda(), 1, out)
+    torch.cuda.synchronize()
+    assert np.array_equal(got, out.cpu().numpy())
+    given = np.empty(T * n_corr + 1, np.float32)[1:].reshape(T, n_corr)  # not on a page
+    fmf.matched_filter(tp, mo, w, d, 1, check_zeros=False, out=given)
+    assert np.array_equal(given, got)
