@@ -251,20 +251,37 @@ __global__ void __launch_bounds__(256) channel_outputs_kernel(
     const int k0 = (int)(blockIdx.x / c_tiles) * kTurnLags, c0 = (int)(blockIdx.x % c_tiles) * kTurnChannels;
     const int nk = min(kTurnLags, n_corr - k0), nc = min(kTurnChannels, SC - c0);
     const bool zero = flag && *flag;
+    const int dk = 256 / nc, dc = 256 % nc;  // from one of a thread's elements to the next
     for (int t = blockIdx.y; t < T; t += gridDim.y) {
         const int lo = k_lo[t] - k0, hi = k_hi[t] - k0;
         __syncthreads();
-        for (int c = threadIdx.x >> 6; c < nc; c += 4) {
-            const int k = threadIdx.x & 63;
-            const size_t row = (size_t)t * SC + c0 + c;
-            const bool live = !zero && k >= lo && k < hi && w[row] != 0.0f;
-            tile[c][k] = live ? by_channel[row * n_corr + k0 + k] : 0.0f;
+        const int k = threadIdx.x & 63;
+        const bool lag = !zero && k >= lo && k < hi;
+        const float *src = by_channel + ((size_t)t * SC + c0) * n_corr + k0 + k;
+        constexpr int kLoads = 8;  // in flight
+        for (int b = threadIdx.x >> 6; b < nc; b += 4 * kLoads) {
+            float x[kLoads];
+#pragma unroll
+            for (int j = 0; j < kLoads; j++) {
+                const int c = b + 4 * j;
+                x[j] = lag && c < nc && w[(size_t)t * SC + c0 + c] != 0.0f ? src[(size_t)c * n_corr] : 0.0f;
+            }
+#pragma unroll
+            for (int j = 0; j < kLoads; j++)
+                if (b + 4 * j < nc)
+                    tile[b + 4 * j][k] = x[j];
         }
         __syncthreads();
         float *o = out + ((size_t)t * n_corr + k0) * SC + c0;
+        int kk = threadIdx.x / nc, cc = threadIdx.x % nc;
         for (int i = threadIdx.x; i < nk * nc; i += 256) {
-            const int k = i / nc, c = i - k * nc;
-            o[(size_t)k * SC + c] = tile[c][k];
+            o[(size_t)kk * SC + cc] = tile[cc][kk];
+            kk += dk;
+            cc += dc;
+            if (cc >= nc) {
+                cc -= nc;
+                kk++;
+            }
         }
     }
 }

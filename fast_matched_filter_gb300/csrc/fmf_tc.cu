@@ -1196,7 +1196,7 @@ static size_t tc_layout(TcBatch *B, bool var, bool full)
 int tc_choose_parts(const TcProb *prob)
 {
     const Problem &P = prob->P;
-    return P.network_sum && P.SC >= 2 ? choose_parts((long long)prob->n_tiles * P.T, P.SC) : 1;
+    return P.SC >= 2 ? choose_parts((long long)prob->n_tiles * P.T, P.SC) : 1;
 }
 
 // One persistent launch over the tile queue of `n` prepared searches (n <= TC_MAX_PROBS).
@@ -1218,7 +1218,7 @@ int tc_run(const TcProb *probs, int n, int form, int parts, unsigned long long *
         parts = tc_choose_parts(&probs[0]);
     Scratch pws(s);
     float *part_out = nullptr;
-    if (parts > 1) {
+    if (parts > 1 && nsum) {
         int rc = pws.get(&part_out, (size_t)parts * P0.T * P0.n_corr, "channel-part sums");
         if (rc)
             return rc;
@@ -1267,7 +1267,7 @@ int tc_run(const TcProb *probs, int n, int form, int parts, unsigned long long *
     count_launch();
     note_bounded_waits();
     int rc = check_launch("tc_persistent");
-    if (rc || parts == 1)
+    if (rc || !part_out)
         return rc;
     const long long m = (long long)P0.T * P0.n_corr;
     tc_parts_sum_kernel<<<(unsigned)((m + 255) / 256), 256, 0, s>>>(part_out, parts, m, P0.n_corr,
