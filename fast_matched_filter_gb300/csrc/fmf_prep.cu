@@ -446,6 +446,58 @@ struct StatLayout {
 
 size_t window_stats_smem(int L, bool full) { return (size_t)StatLayout(L, full).total * sizeof(float); }
 
+// A thread's windows of a block's for coalesced stores where step > 1: row by row, the
+// r-th row from window 0's, its j-th window, with one division at the start instead of
+// one per window.
+struct WindowWalk {
+    const StatPlace place;
+    int per, rows, head, x0, r, j, dr, dj;
+    __device__ WindowWalk(const StatPlace &p, int c0, int nwin) : place(p)
+    {
+        const int n = (int)blockDim.x, i = (int)threadIdx.x;
+        per = nwin > 0 ? (nwin - 1) / p.step + 1 : 1;  // windows of a row
+        rows = min(p.step, nwin);
+        head = c0 % p.step;                          // row of window 0
+        x0 = c0 / p.step;                            // and its place there
+        r = i / per;
+        j = i - r * per;
+        dr = n / per;
+        dj = n - dr * per;
+    }
+    __device__ bool in() const { return r < rows; }
+    __device__ int window() const { return r + j * place.step; }
+    __device__ long long at() const
+    {
+        const int wrap = head + r >= place.step, psi = head + r - (wrap ? place.step : 0);
+        return psi * place.ps + min(psi, place.rem) + x0 + j + wrap;
+    }
+    __device__ void next()
+    {
+        r += dr;
+        j += dj;
+        if (j >= per) {
+            j -= per;
+            r++;
+        }
+    }
+};
+
+// f(u, o) for this thread's windows u of the block's nwin; o: its place in the channel
+// past first_place().
+__device__ __forceinline__ long long first_place(const StatPlace &place, long long c0) { return place.step == 1 ? c0 : 0; }
+template <int THREADS, class F>
+__device__ __forceinline__ void each_window(const StatPlace &place, long long c0, int nwin, F f)
+{
+    if (place.step == 1) {
+        for (int u = threadIdx.x; u < nwin; u += THREADS)
+            f(u, (long long)u);
+    } else {
+        for (WindowWalk at(place, (int)c0, nwin); at.in(); at.next())
+            if (at.window() < nwin)
+                f(at.window(), at.at());
+    }
+}
+
 // Problem::dc of a window (u-th of its channel): every kDcStride-th one counts.
 __device__ __forceinline__ float window_dc(float mx, unsigned u, float Lf, float en, float mean)
 {
@@ -659,22 +711,8 @@ window_stats_kernel(const float *__restrict__ data, int N, int L, int SC, const 
         const float dead = SCAN ? kThreshold / __uint_as_float(scan[2 * SC + ch]) * 0.999f : 0.0f;
         unsigned low = 0;  // the smallest energy above it, bits complemented
         float mx = 0.0f;
-        float *row = stat_e + ch * place.ch * (full ? 2 : 1);
-        // coalesced stores: windows in order, or (step > 1) row by row, `per` of each
-        const int step = place.step, per = step == 1 ? nwin : (nwin + step - 1) / step;
-        const int head = step == 1 ? 0 : (int)(c0 % step);  // row of window 0
-        const long long x0 = step == 1 ? c0 : c0 / step;    // and its place there
-        for (int i = threadIdx.x; i < per * step; i += kStatThreads) {
-            int u = i;
-            long long o = c0 + i;
-            if (step > 1) {
-                const int r = i / per, j = i - r * per;  // the r-th row from window 0's, its j-th window
-                u = r + j * step;
-                if (u >= nwin)
-                    continue;
-                const int psi = head + r < step ? head + r : head + r - step;
-                o = psi * place.ps + min(psi, place.rem) + x0 + j + (head + r < step ? 0 : 1);
-            }
+        float *row = stat_e + (ch * place.ch + first_place(place, c0)) * (full ? 2 : 1);
+        each_window<kStatThreads>(place, c0, nwin, [&](int u, long long o) {
             float en;
             if (full) {
                 const float2 v = out2[stat_pad(u)];
@@ -688,7 +726,7 @@ window_stats_kernel(const float *__restrict__ data, int N, int L, int SC, const 
             }
             if (SCAN && en > dead)
                 low = max(low, ~__float_as_uint(en));
-        }
+        });
         if (full && dc)
             block_dc(mx, dc + ch);
         if (SCAN)
@@ -884,26 +922,9 @@ window_fixed_kernel(const float *__restrict__ data, int N, int L, const float *_
     const float dead = SCAN ? kThreshold / __uint_as_float(scan[2 * SC + ch]) * 0.999f : 0.0f;
     unsigned low = 0;  // the smallest energy above it, bits complemented
     float mx = 0.0f;
-    float *row = stat_e + ch * place.ch * (FULL ? 2 : 1);
-    // coalesced stores: windows in order, or (step > 1) row by row, `per` of each
-    const int step = place.step, per = step == 1 ? nwin : (nwin + step - 1) / step;
-    const int head = step == 1 ? 0 : (int)(c0 % step);  // row of window 0
-    const long long x0 = step == 1 ? c0 : c0 / step;    // and its place there
-    if (step == 1)
-        row += c0 * (FULL ? 2 : 1);
+    float *row = stat_e + (ch * place.ch + first_place(place, c0)) * (FULL ? 2 : 1);
     bool far = false;  // a window too quiet for the block's unit
-    const int n_items = bad ? 0 : per * step;
-    for (int i = threadIdx.x; i < n_items; i += kFixThreads) {
-        int u = i;
-        long long o = i;
-        if (step > 1) {
-            const int r = i / per, j = i - r * per;  // the r-th row from window 0's, its j-th window
-            u = r + j * step;
-            if (u >= nwin)
-                continue;
-            const int psi = head + r < step ? head + r : head + r - step;
-            o = psi * place.ps + min(psi, place.rem) + x0 + j + (head + r < step ? 0 : 1);
-        }
+    each_window<kFixThreads>(place, c0, bad ? 0 : nwin, [&](int u, long long o) {
         const int a = pad(u), b = pad(u + L), ca = u >> 4, cb = (u + L) >> 4;
         const uint2 pa2 = p2[a], pb2 = p2[b], qa2 = o2[ca], qb2 = o2[cb];
         const unsigned hi2 = pb2.x + qb2.x - (pa2.x + qa2.x);
@@ -928,7 +949,7 @@ window_fixed_kernel(const float *__restrict__ data, int N, int L, const float *_
         }
         if (SCAN && en > dead)
             low = max(low, ~__float_as_uint(en));
-    }
+    });
     if (far || bad)
         odd = 1;  // (any thread's)
     __syncthreads();
