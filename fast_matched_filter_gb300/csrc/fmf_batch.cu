@@ -126,8 +126,12 @@ static int batch_record(fmf_batch *b, cudaStream_t s)
                         unsigned long long *queue = nullptr;
                         if ((status = bws[mode]->get(&queue, 1, "tile queue")))
                             break;
+                        if ((e = cudaMemsetAsync(queue, 0, sizeof(*queue), sm)) != cudaSuccess) {
+                            status = set_error(FMF_ERR_CUDA, "clearing the tile queue: %s", cudaGetErrorString(e));
+                            break;
+                        }
                         const int m = (int)(ng - i0 < (size_t)TC_MAX_PROBS ? ng - i0 : TC_MAX_PROBS);
-                        status = tc_run(reinterpret_cast<const TcProb *>(grp.data() + psz * i0), m, form, 0,
+                        status = tc_run(reinterpret_cast<const TcProb *>(grp.data() + psz * i0), m, form, 1,
                                         queue, err, sm);
                     }
                     if (ng && ((e = cudaEventRecord(b->ev_join[mode], sm)) != cudaSuccess ||

@@ -224,10 +224,19 @@ __global__ void zero_count_kernel(const float *__restrict__ out, long long row_l
     const int t = blockIdx.y;
     const float *row = out + (size_t)t * row_len;
     const long long span = last_axis == row_len ? stop : row_len;  // network sum: lags < stop
+    const bool all = last_axis == row_len;
+    const long long stride = (long long)gridDim.x * blockDim.x;
     unsigned c = 0;
-    for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < span;
-         i += (long long)gridDim.x * blockDim.x)
-        c += (row[i] == 0.0f && i % last_axis < stop) ? 1u : 0u;
+    constexpr int kLoads = 8;  // in flight (one at a time: 1 TB/s)
+    for (long long i0 = (long long)blockIdx.x * blockDim.x + threadIdx.x; i0 < span; i0 += kLoads * stride) {
+        float x[kLoads];
+#pragma unroll
+        for (int j = 0; j < kLoads; j++)
+            x[j] = i0 + j * stride < span ? __ldg(row + i0 + j * stride) : 1.0f;
+#pragma unroll
+        for (int j = 0; j < kLoads; j++)
+            c += x[j] == 0.0f && (all || (i0 + j * stride) % last_axis < stop) ? 1u : 0u;
+    }
     for (int o = 16; o > 0; o >>= 1)
         c += __shfl_down_sync(0xffffffffu, c, o);
     if ((threadIdx.x & 31) == 0 && c)

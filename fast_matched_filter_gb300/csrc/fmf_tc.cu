@@ -87,6 +87,7 @@ constexpr int tc_epi_warps(bool var) { return var ? 16 : 8; }
 constexpr int tc_threads(bool var) { return 32 * (4 + tc_epi_warps(var)); }
 constexpr int tc_groups(bool var) { return tc_epi_warps(var) / 4; }  // column groups of a tile
 constexpr int TC_MAX_ROWS = 8;     // data slots, at most
+constexpr int TC_MAX_PARTS = 8;    // channel parts of an item, at most
 constexpr int TC_MAX_STATS = 2;    // statistics slots, at most
 constexpr int kChain = 16;          // K steps of one h h chain
 constexpr float kLoScale = 2048.0f;  // l is kept 2^11 up
@@ -255,6 +256,10 @@ __global__ void __launch_bounds__(256) tc_data_kernel(const float *__restrict__ 
     const long long pos0 = (long long)step * TC_Q * (row0 - row_front);
     const int count = step * TC_Q * rows;
     constexpr int kLoads = 8;  // in flight per thread; count is a multiple of 128
+    // sample i is sample q of phase psi; a thread's next one, without a division, 256 on
+    const int dq = 256 / step, dpsi = 256 - dq * step;
+    int q = (int)threadIdx.x / step, psi = (int)threadIdx.x - q * step;
+    const bool one = step == 1;
     for (int i0 = threadIdx.x; i0 < count; i0 += kLoads * 256) {
         float x[kLoads];
 #pragma unroll
@@ -267,20 +272,28 @@ __global__ void __launch_bounds__(256) tc_data_kernel(const float *__restrict__ 
         for (int j = 0; j < kLoads; j++) {
             const int i = i0 + 256 * j;
             if (i < count) {
-                const int q = step == 1 ? i : i / step, psi = step == 1 ? 0 : i - q * step;
-                const int at = (psi * rows + (q >> 7)) * TC_TURN_PITCH + (q & (TC_Q - 1));
+                const int at = one ? (i >> 7) * TC_TURN_PITCH + (i & (TC_Q - 1))
+                                   : (psi * rows + (q >> 7)) * TC_TURN_PITCH + (q & (TC_Q - 1));
                 uint16_t h, l;
                 split_pair<FP32>(x[j], inv_s, h, l);
                 hi[at] = h;
                 if (g_lo)
                     lo[at] = l;
             }
+            if (!one) {
+                q += dq;
+                psi += dpsi;
+                if (psi >= step) {
+                    psi -= step;
+                    q++;
+                }
+            }
         }
     }
     __syncthreads();
-    const int n = min(rows, rows_total - row0);
+    const int n = min(rows, rows_total - row0), rows_log2 = 31 - __clz(rows);
     for (int i = threadIdx.x; i < step * TC_CB * rows; i += 256) {
-        const int r = i & (rows - 1), rest = i / rows, cb = rest & (TC_CB - 1), psi = rest / TC_CB;
+        const int r = i & (rows - 1), rest = i >> rows_log2, cb = rest & (TC_CB - 1), psi = rest / TC_CB;
         if (r < n) {
             const int at = (psi * rows + r) * TC_TURN_PITCH + 8 * cb;
             const size_t o = (((size_t)ch * step + psi) * TC_CB + cb) * rows_total + row0 + r;
@@ -329,14 +342,18 @@ __global__ void tc_data_sparse_kernel(const float *__restrict__ data, int N, int
 // W[t][ch][phi][n][e][c] = pair of tphi[8n + e + c - (Q-1+s)], tphi[q] = tpl[step*q + phi],
 // s = mu mod Q, mu = floor((mo + phi) / step); one block per (template,
 // channel), its taps in shared memory (read once, written 8 times over).
-// FP32: also the channel's exponent.
+// FP32: also the channel's exponent.  queue: the tile queue of the persistent launch
+// that follows, cleared here (a memset costs 2 us).
 template <bool FP32>
 __global__ void __launch_bounds__(256) tc_template_kernel(
     const float *__restrict__ tpl, const int *__restrict__ mo, int L, int step, int NW,
-    uint16_t *__restrict__ w_hi, uint16_t *__restrict__ w_lo, int *__restrict__ t_exp, unsigned *skip)
+    uint16_t *__restrict__ w_hi, uint16_t *__restrict__ w_lo, int *__restrict__ t_exp, unsigned *skip,
+    unsigned long long *queue)
 {
     extern __shared__ float taps[];
     const long long row = blockIdx.x;  // t*SC + ch
+    if (queue && row == 0 && threadIdx.x == 0)
+        *queue = 0;
     const float *src = tpl + row * L;
     float inv_s = 1.0f;
     if constexpr (FP32) {
@@ -1117,7 +1134,10 @@ static int n_sms()
 
 // out[i] = sum over parts j = 0..k-1 of part[j][i], in that order; with
 // per-channel lengths (norm set) the Fisher-z transform of that sum,
-// (tanh(v / norm[t]) + bias[t]) * scale[t] for row t = i / n_corr.
+// (tanh(v / norm[t]) + bias[t]) * scale[t] for row t = i / n_corr.  Bound by the loads'
+// latency: all parts' values are in flight (one after the other: 12 us for 13 x 115,115
+// outputs, 8 us here).  Added by whichever part came last in the
+// persistent kernel itself, they held up its end instead: 0.27 -> 0.39 ms of the search.
 __global__ void tc_parts_sum_kernel(const float *__restrict__ part, int k, long long m, int n_corr,
                                     const float *__restrict__ norm, const float *__restrict__ bias,
                                     const float *__restrict__ scale, float *__restrict__ out)
@@ -1125,9 +1145,16 @@ __global__ void tc_parts_sum_kernel(const float *__restrict__ part, int k, long 
     const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= m)
         return;
-    float v = part[i];
-    for (int j = 1; j < k; j++)
-        v += part[(size_t)j * m + i];
+    float x[TC_MAX_PARTS];
+#pragma unroll
+    for (int j = 0; j < TC_MAX_PARTS; j++)
+        if (j < k)
+            x[j] = __ldg(part + (size_t)j * m + i);
+    float v = x[0];
+#pragma unroll
+    for (int j = 1; j < TC_MAX_PARTS; j++)
+        if (j < k)
+            v += x[j];
     if (norm) {
         const int t = (int)(i / n_corr);
         v = (tanhf(v / norm[t]) + bias[t]) * scale[t];
@@ -1141,7 +1168,7 @@ __global__ void tc_parts_sum_kernel(const float *__restrict__ part, int k, long 
 // output write); FMF_TC_PARTS=k forces a value.
 static int choose_parts(long long items, int SC)
 {
-    const int sms = n_sms(), kmax = SC < 8 ? SC : 8;
+    const int sms = n_sms(), kmax = SC < TC_MAX_PARTS ? SC : TC_MAX_PARTS;
     if (const char *env = getenv("FMF_TC_PARTS")) {
         const int k = atoi(env);
         if (k >= 1)
@@ -1200,9 +1227,8 @@ int tc_choose_parts(const TcProb *prob)
 }
 
 // One persistent launch over the tile queue of `n` prepared searches (n <= TC_MAX_PROBS).
-// `form`: the operands they were prepared with.  `parts`: channel parts of every
-// item (n = 1 only; 0 = tc_choose_parts).  `queue` is a device counter that this
-// call zeroes on `s` before the launch.
+// `form`: the operands they were prepared with.  `queue`: a device counter, zero before
+// the launch.  `parts`: channel parts of every item (n = 1 only).
 int tc_run(const TcProb *probs, int n, int form, int parts, unsigned long long *queue, unsigned *err,
            cudaStream_t s)
 {
@@ -1212,10 +1238,6 @@ int tc_run(const TcProb *probs, int n, int form, int parts, unsigned long long *
     TcBatch &B = Bh;
     const Problem &P0 = probs[0].P;
     const bool var = P0.ntap != nullptr, full = P0.normalize != 0, nsum = P0.network_sum != 0;
-    if (n > 1)
-        parts = 1;
-    else if (parts == 0)
-        parts = tc_choose_parts(&probs[0]);
     Scratch pws(s);
     float *part_out = nullptr;
     if (parts > 1 && nsum) {
@@ -1248,9 +1270,6 @@ int tc_run(const TcProb *probs, int n, int form, int parts, unsigned long long *
     const size_t smem = tc_layout(&B, var, full);
     if (smem == 0)
         return set_error(FMF_ERR_SMEM, "tensor-core buffers do not fit shared memory");
-    cudaError_t e = cudaMemsetAsync(queue, 0, sizeof(unsigned long long), s);
-    if (e != cudaSuccess)
-        return set_error(FMF_ERR_CUDA, "clearing the tile queue: %s", cudaGetErrorString(e));
     void (*kern)(const TcBatch);
     if (var)
         kern = full ? tc_persistent<true, true, true> : tc_persistent<true, false, true>;
@@ -1258,7 +1277,7 @@ int tc_run(const TcProb *probs, int n, int form, int parts, unsigned long long *
         kern = full ? tc_persistent<false, true, true> : tc_persistent<false, false, true>;
     else
         kern = full ? tc_persistent<false, true, false> : tc_persistent<false, false, false>;
-    e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxDynamicSmem);
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxDynamicSmem);
     if (e != cudaSuccess)
         return set_error(FMF_ERR_CUDA, "tc_persistent shared memory (%zu bytes): %s", smem,
                          cudaGetErrorString(e));
@@ -1429,7 +1448,8 @@ int tc_begin(const Problem &P, int form, int nb, int tg, int max_templates, Scra
 
 // Operand blocks of templates [t0, t0 + nt), nt <= room, into the search's
 // buffer; *sub is that part of the search.
-static int tc_templates(const TcSearch *full, int t0, int nt, cudaStream_t s, TcProb *sub)
+static int tc_templates(const TcSearch *full, int t0, int nt, unsigned long long *queue, cudaStream_t s,
+                        TcProb *sub)
 {
     const Problem &P = full->pr.P;
     tc_subset(&full->pr, t0, nt, sub);
@@ -1440,7 +1460,7 @@ static int tc_templates(const TcSearch *full, int t0, int nt, cudaStream_t s, Tc
         return set_error(FMF_ERR_CUDA, "tc_template_kernel shared memory: %s", cudaGetErrorString(e));
     kern<<<(unsigned)((size_t)nt * P.SC), 256, (size_t)P.L * sizeof(float), s>>>(
         sub->P.tpl, sub->P.mo, P.L, P.step, sub->NW, full->w, const_cast<uint16_t *>(full->pr.w_lo),
-        const_cast<int *>(sub->t_exp), const_cast<unsigned *>(full->pr.skip));
+        const_cast<int *>(sub->t_exp), const_cast<unsigned *>(full->pr.skip), queue);
     count_launch();
     return check_launch("tensor-core templates");
 }
@@ -1457,9 +1477,10 @@ int tc_run_templates(const TcSearch *full, int t0, int nt, unsigned *err, Scratc
         const int n = t0 + nt - a < full->room ? t0 + nt - a : full->room;
         TcProb sub;
         unsigned long long *queue = nullptr;
-        if ((rc = tc_templates(full, a, n, s, &sub)) || (rc = ws.get(&queue, 1, "tile queue")) ||
+        if ((rc = ws.get(&queue, 1, "tile queue")) || (rc = tc_templates(full, a, n, queue, s, &sub)) ||
             (!sub.P.by_channel && (rc = clear_outputs(sub.P, s))) ||
-            (rc = tc_run(&sub, 1, full->form, full->form == TC_FORM_FP32 ? full->parts : 0, queue, err, s)) ||
+            (rc = tc_run(&sub, 1, full->form, full->form == TC_FORM_FP32 ? full->parts : tc_choose_parts(&sub), queue,
+                         err, s)) ||
             (sub.P.by_channel && (rc = launch_channel_outputs(sub.P, sub.skip, s))))
             return rc;
     }
@@ -1485,7 +1506,7 @@ int tc_prepare(const Problem &P, int form, int nb, int tg, Scratch &ws, cudaStre
         st.pr.w_hi = st.w;
         st.pr.w_lo = halves == 2 ? st.w + st.w_elems : nullptr;
     }
-    return tc_templates(&st, 0, P.T, s, out);
+    return tc_templates(&st, 0, P.T, nullptr, s, out);
 }
 
 }  // namespace fmf
