@@ -223,8 +223,8 @@ __device__ __forceinline__ float tc_channel_scale(const unsigned *stat, int ch, 
 // A block turns the samples of `rows` rows of every phase through shared memory:
 // loads of consecutive samples, stores of consecutive rows of a column block (a
 // thread per 16 bytes, reading its own 8 samples, kept the L1 at 98 %: 60
-// channels x 1.08M samples 231 us).  grid: (row tiles, SC), dynamic shared memory
-// tc_turn_bytes.
+// channels x 1.08M samples 231 us, 93 us here).  A block of `tiles` per channel, 256
+// threads, dynamic shared memory tc_turn_bytes.
 constexpr int TC_TURN_PITCH = TC_Q + 8;  // halves per row: 16-byte reads of 8 rows hit distinct banks
 constexpr int TC_TURN_STEP = 64;         // the largest step with a row of every phase
 __host__ __device__ __forceinline__ int tc_turn_rows(int step)
@@ -239,19 +239,26 @@ static size_t tc_turn_bytes(int step, bool pairs)
     return (size_t)(pairs ? 2 : 1) * step * tc_turn_rows(step) * TC_TURN_PITCH * sizeof(uint16_t);
 }
 
+struct TcDataWork {
+    const float *data;
+    int N, SC, step, tiles, rows_total, row_front;
+    const unsigned *stat;
+    uint16_t *g_hi, *g_lo;
+    int *d_exp;
+    unsigned *skip;
+};
+
 template <bool FP32>
-__global__ void __launch_bounds__(256) tc_data_kernel(const float *__restrict__ data, int N, int step,
-                                                      int rows_total, int row_front,
-                                                      const unsigned *__restrict__ stat,
-                                                      uint16_t *__restrict__ g_hi, uint16_t *__restrict__ g_lo,
-                                                      int *__restrict__ d_exp, unsigned *skip)
+__device__ __forceinline__ void tc_data_block(const TcDataWork &d, int block, uint4 *turn_smem)
 {
-    extern __shared__ uint4 turn_smem[];
-    const int rows = tc_turn_rows(step), ch = blockIdx.y, row0 = blockIdx.x * rows;
+    const int step = d.step, N = d.N, rows_total = d.rows_total, row_front = d.row_front;
+    const float *__restrict__ data = d.data;
+    uint16_t *__restrict__ g_hi = d.g_hi, *__restrict__ g_lo = d.g_lo;
+    const int rows = tc_turn_rows(step), ch = block / d.tiles, tile = block - ch * d.tiles, row0 = tile * rows;
     uint16_t *hi = reinterpret_cast<uint16_t *>(turn_smem), *lo = hi + step * rows * TC_TURN_PITCH;
     float inv_s = 1.0f;
     if constexpr (FP32)
-        inv_s = tc_channel_scale(stat, ch, (int)gridDim.y, blockIdx.x == 0 && threadIdx.x == 0, d_exp, skip);
+        inv_s = tc_channel_scale(d.stat, ch, d.SC, tile == 0 && threadIdx.x == 0, d.d_exp, d.skip);
     const float *src = data + (size_t)ch * N;
     const long long pos0 = (long long)step * TC_Q * (row0 - row_front);
     const int count = step * TC_Q * rows;
@@ -344,16 +351,26 @@ __global__ void tc_data_sparse_kernel(const float *__restrict__ data, int N, int
 // channel), its taps in shared memory (read once, written 8 times over).
 // FP32: also the channel's exponent.  queue: the tile queue of the persistent launch
 // that follows, cleared here (a memset costs 2 us).
+struct TcTemplateWork {
+    const float *tpl;
+    const int *mo;
+    int L, step, NW;
+    uint16_t *w_hi, *w_lo;
+    int *t_exp;
+    unsigned *skip;
+    unsigned long long *queue;
+};
+
 template <bool FP32>
-__global__ void __launch_bounds__(256) tc_template_kernel(
-    const float *__restrict__ tpl, const int *__restrict__ mo, int L, int step, int NW,
-    uint16_t *__restrict__ w_hi, uint16_t *__restrict__ w_lo, int *__restrict__ t_exp, unsigned *skip,
-    unsigned long long *queue)
+__device__ __forceinline__ void tc_template_block(const TcTemplateWork &w, long long row /* t*SC + ch */, float *taps)
 {
-    extern __shared__ float taps[];
-    const long long row = blockIdx.x;  // t*SC + ch
-    if (queue && row == 0 && threadIdx.x == 0)
-        *queue = 0;
+    const float *__restrict__ tpl = w.tpl;
+    uint16_t *__restrict__ w_hi = w.w_hi, *__restrict__ w_lo = w.w_lo;
+    const int L = w.L, step = w.step, NW = w.NW;
+    int *t_exp = w.t_exp;
+    unsigned *skip = w.skip;
+    if (w.queue && row == 0 && threadIdx.x == 0)
+        *w.queue = 0;
     const float *src = tpl + row * L;
     float inv_s = 1.0f;
     if constexpr (FP32) {
@@ -392,7 +409,7 @@ __global__ void __launch_bounds__(256) tc_template_kernel(
             taps[j] = src[j];
         __syncthreads();
     }
-    const int m0 = mo[row];
+    const int m0 = w.mo[row];
     const int per_phase = NW * 8;
     for (int i = threadIdx.x; i < step * per_phase; i += blockDim.x) {
         const int phi = i / per_phase, ne = i - phi * per_phase;
@@ -410,6 +427,17 @@ __global__ void __launch_bounds__(256) tc_template_kernel(
         if (w_lo)
             reinterpret_cast<uint4 *>(w_lo)[o] = pack8(l);
     }
+}
+
+// Both in one launch: blocks [0, n_data) turn data, the others make template blocks.
+template <bool FP32>
+__global__ void __launch_bounds__(256) tc_operand_kernel(const TcDataWork d, unsigned n_data, const TcTemplateWork w)
+{
+    extern __shared__ uint4 operand_smem[];
+    if (blockIdx.x < n_data)
+        tc_data_block<FP32>(d, (int)blockIdx.x, operand_smem);
+    else
+        tc_template_block<FP32>(w, (long long)(blockIdx.x - n_data), reinterpret_cast<float *>(operand_smem));
 }
 
 // ------------------------------------------------------------------ persistent kernel
@@ -1332,9 +1360,13 @@ static void tc_subset(const TcProb *full, int t0, int nt, TcProb *out)
 struct TcSearch {
     TcProb pr;       // of all templates; the operand blocks hold `room` of them
     int form, room, parts;
+    TcDataWork data;
+    bool data_due;   // the data streams are made with the first templates
     uint16_t *w;
     size_t w_elems;  // of one half, all room templates
 };
+
+constexpr size_t kOneLaunchTaps = 24 * 1024;  // bytes: 8 blocks of 256 threads per SM
 
 size_t tc_search_size() { return sizeof(TcSearch); }
 
@@ -1425,44 +1457,50 @@ int tc_begin(const Problem &P, int form, int nb, int tg, int max_templates, Scra
     // chain's
     const int most = (g.k_span + TC_Q - 1) / TC_Q;  // K steps of one pair
     pr.chain_cols = fp32 ? (kChain / most > 1 ? kChain / most : 1) : step * (TC_CB / 2);
-    const unsigned *stat = fp32 ? P.scan : nullptr;
-    int *d_exp = fp32 ? exps + n_rows : nullptr;
-    unsigned *skip = fp32 ? P.scan + 3 * SC : nullptr;
-    if (step <= TC_TURN_STEP && SC <= 65535) {
-        const int rows = tc_turn_rows(step);
-        auto kern = fp32 ? tc_data_kernel<true> : tc_data_kernel<false>;
-        cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxDynamicSmem);
-        if (e != cudaSuccess)
-            return set_error(FMF_ERR_CUDA, "tc_data_kernel shared memory: %s", cudaGetErrorString(e));
-        kern<<<dim3((unsigned)((pr.rows_total + rows - 1) / rows), (unsigned)SC), 256, tc_turn_bytes(step, pairs), s>>>(
-            P.data, P.N, step, pr.rows_total, pr.row_front, stat, g_hi, g_lo, d_exp, skip);
-    } else {
-        const long long n = (long long)SC * step * TC_CB * pr.rows_total;
-        auto kern = fp32 ? tc_data_sparse_kernel<true> : tc_data_sparse_kernel<false>;
-        kern<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(P.data, P.N, SC, step, pr.rows_total, pr.row_front, stat,
-                                                         g_hi, g_lo, d_exp, skip);
-    }
+    TcDataWork &d = out->data;
+    d = TcDataWork{P.data, P.N, SC, step, 0, pr.rows_total, pr.row_front, fp32 ? P.scan : nullptr, g_hi, g_lo,
+                   fp32 ? exps + n_rows : nullptr, fp32 ? P.scan + 3 * SC : nullptr};
+    const int rows = tc_turn_rows(step);
+    d.tiles = (pr.rows_total + rows - 1) / rows;
+    out->data_due = step <= TC_TURN_STEP && (long long)d.tiles * SC < (1ll << 30);
+    if (out->data_due)  // with the first templates
+        return FMF_OK;
+    const long long n = (long long)SC * step * TC_CB * pr.rows_total;
+    auto kern = fp32 ? tc_data_sparse_kernel<true> : tc_data_sparse_kernel<false>;
+    kern<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(P.data, P.N, SC, step, pr.rows_total, pr.row_front, d.stat,
+                                                     g_hi, g_lo, d.d_exp, d.skip);
     count_launch();
     return check_launch("tensor-core data streams");
 }
 
 // Operand blocks of templates [t0, t0 + nt), nt <= room, into the search's
 // buffer; *sub is that part of the search.
-static int tc_templates(const TcSearch *full, int t0, int nt, unsigned long long *queue, cudaStream_t s,
-                        TcProb *sub)
+static int tc_templates(TcSearch *full, int t0, int nt, unsigned long long *queue, cudaStream_t s, TcProb *sub)
 {
     const Problem &P = full->pr.P;
     tc_subset(&full->pr, t0, nt, sub);
     const bool fp32 = full->form == TC_FORM_FP32;
-    auto kern = fp32 ? tc_template_kernel<true> : tc_template_kernel<false>;
+    auto kern = fp32 ? tc_operand_kernel<true> : tc_operand_kernel<false>;
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxDynamicSmem - 1024);
     if (e != cudaSuccess)
-        return set_error(FMF_ERR_CUDA, "tc_template_kernel shared memory: %s", cudaGetErrorString(e));
-    kern<<<(unsigned)((size_t)nt * P.SC), 256, (size_t)P.L * sizeof(float), s>>>(
-        sub->P.tpl, sub->P.mo, P.L, P.step, sub->NW, full->w, const_cast<uint16_t *>(full->pr.w_lo),
-        const_cast<int *>(sub->t_exp), const_cast<unsigned *>(full->pr.skip), queue);
+        return set_error(FMF_ERR_CUDA, "tc_operand_kernel shared memory: %s", cudaGetErrorString(e));
+    const TcTemplateWork w{sub->P.tpl, sub->P.mo, P.L, P.step, sub->NW, full->w,
+                           const_cast<uint16_t *>(full->pr.w_lo), const_cast<int *>(sub->t_exp),
+                           const_cast<unsigned *>(full->pr.skip), queue};
+    unsigned n_data = full->data_due ? (unsigned)full->data.tiles * full->data.SC : 0;
+    const unsigned n_templates = (unsigned)((size_t)nt * P.SC);
+    const size_t turn = tc_turn_bytes(P.step, full->pr.g_lo != nullptr), taps = (size_t)P.L * sizeof(float);
+    // one launch (4 us less than two in a search of 50 us), unless the templates' shared
+    // memory would leave room for fewer of the data's blocks
+    if (n_data && (taps > kOneLaunchTaps || n_templates > (1u << 30))) {
+        kern<<<n_data, 256, turn, s>>>(full->data, n_data, w);
+        count_launch();
+        n_data = 0;
+    }
+    kern<<<n_data + n_templates, 256, n_data && turn > taps ? turn : taps, s>>>(full->data, n_data, w);
+    full->data_due = false;
     count_launch();
-    return check_launch("tensor-core templates");
+    return check_launch("tensor-core operands");
 }
 
 // Templates [t0, t0 + nt) of a begun search: their operand blocks and the
@@ -1470,7 +1508,7 @@ static int tc_templates(const TcSearch *full, int t0, int nt, unsigned long long
 // those of all its templates, so that its results do not depend on how they are
 // parted (a call with host arrays runs them in parts); the bf16 forms choose them
 // for each launch, which keeps the SMs busier through the last few templates.
-int tc_run_templates(const TcSearch *full, int t0, int nt, unsigned *err, Scratch &ws, cudaStream_t s)
+int tc_run_templates(TcSearch *full, int t0, int nt, unsigned *err, Scratch &ws, cudaStream_t s)
 {
     int rc;
     for (int a = t0; a < t0 + nt; a += full->room) {

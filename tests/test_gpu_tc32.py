@@ -128,3 +128,60 @@ def test_many_channels_written_one_by_one(monkeypatch):
     plain, tensor = [_search(monkeypatch, tile, tp, mo, w, d, network_sum=False) for tile in (0, 128)]
     assert np.array_equal(plain == 0, tensor == 0)
     assert np.abs(plain - tensor).max() <= 2 * TOL
+
+
+@pytest.mark.parametrize("step,L", [(32, 100), (33, 100), (64, 200), (65, 200), (8, 6144), (8, 6145)])
+@pytest.mark.parametrize("normalize", ["short", "full"])
+def test_operands_of_large_steps_and_long_templates(monkeypatch, step, L, normalize):
+    """Where a block turns two rows of every phase, one, and none (a kernel of its own);
+    and where the templates' shared memory gives them a launch of their own."""
+    tp, mo, w, d = random_search(step + L, 2, 2, 2, L, 150 * step + L + 4000, -200, 300, dc=1.0, zero_weights=1)
+    got = _search(monkeypatch, 32, tp, mo, w, d, step, normalize=normalize)
+    _check(got, fp64.fp64_matched_filter(tp, mo, w, d, step, normalize, True))
+
+
+@pytest.mark.parametrize("channels", [2, 64, 65, 130])
+def test_channels_written_one_by_one_around_a_tile(monkeypatch, channels):
+    """Per-channel outputs are turned 64 channels at a time."""
+    tp, mo, w, d = random_search(channels, 2, channels, 1, 40, 4200, -20, 60, zero_weights=1)
+    plain, tensor = [_search(monkeypatch, tile, tp, mo, w, d, network_sum=False) for tile in (0, 32)]
+    assert np.array_equal(plain == 0, tensor == 0)
+    assert np.abs(plain - tensor).max() <= 2 * TOL
+
+
+@pytest.mark.parametrize("step", [1, 3])
+@pytest.mark.parametrize("normalize", ["short", "full"])
+def test_per_channel_lengths_of_a_decimated_search(monkeypatch, step, normalize):
+    rng = np.random.default_rng(step)
+    tp, mo, w, d = random_search(21, 2, 3, 2, 150, 9000, -30, 90, dc=2.0)
+    n = rng.integers(20, 151, mo.shape).astype(np.int32)
+    n[0, 0, 0] = 150
+    for i in np.ndindex(n.shape):
+        tp[i][n[i]:] = 0.0
+    got = _search(monkeypatch, 32, tp, mo, w, d, step, normalize=normalize, n_samples_template=n)
+    ref = fp64.fp64_matched_filter_variable(tp, n, mo, w, d, step, normalize)
+    scale = np.cumsum(w.reshape(2, -1).sum(axis=1))[:, None]
+    assert (np.abs(got - ref) / scale).max() <= 6 * TOL  # as in test_per_channel_lengths
+
+
+@pytest.mark.parametrize("small", [True, False])
+def test_batch_of_fp32_searches(small):
+    """Searches of a batch on the tensor cores and, the small ones, on the CUDA cores;
+    both normalisations and output layouts."""
+    import torch
+
+    b = fmf.Batch("fp32")
+    want = []
+    for i in range(6):
+        T, N = (1, 900) if small and i % 2 else (12, 14000)
+        tp, mo, w, d = random_search(60 + i, T, 3, 2, 100, N, 0, 120, dc=1.0)
+        normalize, network_sum = ("full", "short")[i % 2], i < 4
+        n_corr = N - 100 + 1
+        out = torch.zeros((T, n_corr) if network_sum else (T, n_corr, 3, 2), device="cuda")
+        dev = [torch.tensor(x).cuda() for x in (tp, (tp * tp).sum(axis=-1), mo, w, d)]
+        b.add(*dev, 1, out, normalize=normalize, network_sum=network_sum)
+        want.append((out, dev, fp64.fp64_matched_filter(tp, mo, w, d, 1, normalize, network_sum)))
+    b.run()
+    torch.cuda.synchronize()
+    for out, _, ref in want:
+        _check(out.cpu().numpy(), ref.reshape(tuple(out.shape)))
