@@ -290,6 +290,7 @@ inline int tc_form(int precision)
 struct TcProb;
 struct TcSearch;
 int tc_choose_nb(int L, int step, int pairs, int forced);  // lag blocks per tile; 0: no tile fits
+constexpr size_t kFp32LeastTaps = 56;  // of FP32 templates on the tensor cores
 int tc_fp32_nb(size_t T, size_t SC, size_t L, size_t step, size_t n_corr);  // 0: the CUDA cores
 inline int tc_pad(int nb) { return nb ? 128 * nb + 16 : 0; }  // statistics padding of such a tile
 size_t tc_search_size();

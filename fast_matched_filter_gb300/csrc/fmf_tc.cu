@@ -1380,6 +1380,21 @@ size_t tc_template_bytes(const Problem &P, int nb)
 }
 
 // Lag blocks per tile of an FP32 search on the tensor cores, or 0: the CUDA cores.
+// The latter take 21 us and what plain_us says (10 % off, over 288 searches of 1 to 64
+// templates, 1 to 15 channels, 50 to 800 taps, 2,000 to 120,000 samples, step 1 and 3);
+// the tensor cores' further kernels take 40 to 50 us however small the search.  They
+// cross near 25 (16 templates x 1 channel x 200 taps x 30,000 samples: 30 us here, 39 us
+// there) and the line is at 50, where the tensor cores are up to 1.5 times faster (16
+// templates x 15 channels x 50 taps x 8,000: 89 us and 48 us; 64 templates: 230 us and
+// 85 us): searches below it run the very kernels of the entry point without
+// allocations, and launch as many.  Taken by this rule the 288 are within 2 % of the
+// faster side on average.  The tile: one of 64 or
+// 32 where the outputs would leave most of a larger one empty (4 templates x 15
+// channels x 50 taps, 651 outputs: 55, 56, 58 us with 32, 64, 128; 39,984 outputs: 86,
+// 75, 70 us).
+//
+// Below kFp32LeastTaps the pairs' 22 bits show: the error against 64 bits is 1.4 of the
+// FMAs' at 10 taps, 1.08 at 40, 1.00 at 44 to 52 and falls to 0.6 at 300.
 int tc_fp32_nb(size_t T, size_t SC, size_t L, size_t step, size_t n_corr)
 {
     if (const char *env = getenv("FMF_TC32")) {  // 0: the CUDA cores; 32, 64, 128: this tile
@@ -1388,12 +1403,14 @@ int tc_fp32_nb(size_t T, size_t SC, size_t L, size_t step, size_t n_corr)
         if (atoi(env) > 1)
             return tc_choose_nb((int)L, (int)step, 1, atoi(env));
     }
-    // CUDA cores: microseconds of the busiest SM, a tile of 4,096 outputs at a time
+    if (L < kFp32LeastTaps)
+        return 0;
+    // a tile of 4,096 outputs per block, two blocks per SM, groups of 20 taps per phase
     const double taps = (double)step * (double)((((L + step - 1) / step + 19) / 20) * 20);
-    const double tiles = (double)T * (double)((n_corr + 4095) / 4096);
-    const double waves = tiles <= 304.0 ? 1.0 : tiles / 304.0;
-    const double plain_us = waves * (double)SC * (taps * 0.02 + (double)step * 0.5 + 0.5);
-    if (plain_us < 60.0)
+    const double tiles = (double)T * (double)((n_corr + 4095) / 4096) / 304.0;
+    const double plain_us = (double)SC * ((taps * 0.0165 + (double)step * 1.45 + 1.9) * (tiles < 1.0 ? 1.0 : tiles) +
+                                          taps * 0.03 * tiles);
+    if (plain_us < 50.0)
         return 0;
     const int want = n_corr > 8192 ? 128 : (n_corr > 4096 ? 64 : 32);
     for (int nb = want; nb >= 32; nb >>= 1) {

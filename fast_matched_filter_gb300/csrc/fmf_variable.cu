@@ -557,7 +557,8 @@ static int variable_device(const VArgs &a, int L, cudaStream_t s, float *host_ou
     // may come to them
     int nb32 = 0, nb16 = 0;
     const int forced = ((a.flags >> 8) & 0xff) * 16;
-    if (precision == FMF_PREC_FP32 || precision == FMF_PREC_AUTO)
+    // (channels down to half the longest length are usual)
+    if ((precision == FMF_PREC_FP32 || precision == FMF_PREC_AUTO) && (size_t)L >= 2 * kFp32LeastTaps)
         nb32 = tc_fp32_nb(a.T, a.S * a.C, (size_t)L, a.step, a.n_corr);
     if (precision != FMF_PREC_FP32 && (forced == 0 || forced == 32 || forced == 64 || forced == 128))
         nb16 = tc_choose_nb(L, (int)a.step, precision != FMF_PREC_BF16, forced);
