@@ -583,7 +583,10 @@ __device__ __forceinline__ void tc_issue(const TcBatch &B, const long long *ring
 // VAR: per-channel template lengths (Fisher-z network sum); FULL: 'full'
 // normalisation; NSUM: network sum.  One instantiation per mode, each with its
 // own epilogue code only (the code of all roles shares the instruction cache).
-template <bool VAR, bool FULL, bool NSUM>
+// ONE (per-channel lengths): every channel is one chain (the bf16 forms), whose
+// numerators go from the accumulators to the sums without a stop in registers; with
+// that stop 16 epilogue warps spill.
+template <bool VAR, bool FULL, bool NSUM, bool ONE>
 __global__ void __launch_bounds__(tc_threads(VAR), 1) tc_persistent(const __grid_constant__ TcBatch B)
 {
     extern __shared__ __align__(1024) uint8_t smem[];
@@ -902,13 +905,21 @@ __global__ void __launch_bounds__(tc_threads(VAR), 1) tc_persistent(const __grid
                     const float unit = exp2_int(__shfl_sync(0xffffffffu, unit_l, from));
                     const float ts = FULL ? __shfl_sync(0xffffffffu, ts_l, from) : 0.0f;
                     const int mo = __shfl_sync(0xffffffffu, mo_l, from);
-                    float num[NCM];
+                    float num[ONE ? 1 : NCM];
 #pragma unroll
                     for (int i = 0; i < NCM; i++)
-                        num[i] = 0.0f;
+                        if constexpr (!ONE)
+                            num[i] = 0.0f;
+                    if constexpr (ONE) {  // both sums are awaited here and read below
+                        if (!mbar_wait_all(bar + TcBars::hfull + 8 * (hc & 1), (hc >> 1) & 1, abort_flag, B.err, 16u) ||
+                            (pairs && !mbar_wait_all(bar + TcBars::sfull + 8 * (c & 1), (c >> 1) & 1, abort_flag,
+                                                     B.err, 16u)))
+                            goto epilogue_done;
+                        tc_fence_after();
+                    }
                     // numerators: the chains' sums, then S (FP32: times 2^-11)
 #pragma unroll 1
-                    for (int j = 0; j < n_sums; j++) {
+                    for (int j = 0; !ONE && j < n_sums; j++) {
                         const bool last = j == n_chains;
                         const int u = last ? c : hc;
                         if (!mbar_wait_all(bar + (last ? TcBars::sfull : TcBars::hfull) + 8 * (u & 1), (u >> 1) & 1,
@@ -929,7 +940,8 @@ __global__ void __launch_bounds__(tc_threads(VAR), 1) tc_persistent(const __grid
                                 tmem_wait_ld();
 #pragma unroll
                                 for (int i = 0; i < LD; i++)
-                                    num[c0 + i] = fmaf(x[i], f, num[c0 + i]);
+                                    if constexpr (!ONE)
+                                        num[c0 + i] = fmaf(x[i], f, num[c0 + i]);
                             }
                         }
                         tc_fence_before();
@@ -956,9 +968,33 @@ __global__ void __launch_bounds__(tc_threads(VAR), 1) tc_persistent(const __grid
                         int psi2;
                         const int far = tc_phase(psi + ntap, step, psi2);
                         const int head2 = (int)((I0 + mu + far) & kStat.align());
+                        float x[16];  // ONE: the numerators of 16 columns
 #pragma unroll
                         for (int c0 = 0; c0 < NCM; c0 += CH) {
                             if (c0 < NC) {
+                                if constexpr (ONE) {
+                                    if (c0 % 16 == 0) {  // (a tile of 32 lag blocks reads 8 columns too many)
+                                        tmem_ld16(lane_base + 128u * (hc & 1) + a0 + c0, x);
+                                        float small[16];
+                                        if (pairs)
+                                            tmem_ld16(lane_base + 256u + 128u * (c & 1) + a0 + c0, small);
+                                        tmem_wait_ld();
+                                        if (pairs) {
+#pragma unroll
+                                            for (int i = 0; i < 16; i++)
+                                                x[i] = fmaf(small[i], B.lo_unit, x[i]);
+                                        }
+                                        if (c0 + 16 >= NC) {  // the accumulators are read
+                                            tc_fence_before();
+                                            __syncwarp();
+                                            if (lane == 0) {
+                                                mbar_arrive(bar + TcBars::hempty + 8 * (hc & 1));
+                                                if (pairs)
+                                                    mbar_arrive(bar + TcBars::sempty + 8 * (c & 1));
+                                            }
+                                        }
+                                    }
+                                }
                                 const int es = ec & ((1 << stat_log2) - 1);
                                 if (!mbar_wait_all(bar + TcBars::efull + 8 * es, (ec >> stat_log2) & 1, abort_flag,
                                                    B.err, 16u))
@@ -986,7 +1022,11 @@ __global__ void __launch_bounds__(tc_threads(VAR), 1) tc_persistent(const __grid
                                 float y[CH];
 #pragma unroll
                                 for (int j = 0; j < CH; j++) {
-                                    float ssd, num1 = num[c0 + j];
+                                    float ssd, num1;
+                                    if constexpr (ONE)
+                                        num1 = x[(c0 + j) % 16];
+                                    else
+                                        num1 = num[c0 + j];
                                     if constexpr (FULL) {
                                         float mean;
                                         window_centred(lo[j], hi[j], u2, lo1[j], hi1[j], nf, inv_n, ssd, mean);
@@ -1053,6 +1093,8 @@ __global__ void __launch_bounds__(tc_threads(VAR), 1) tc_persistent(const __grid
                             }
                         }
                     }
+                    if (ONE)
+                        hc++;
                     c++;
                 }
             }
@@ -1299,12 +1341,14 @@ int tc_run(const TcProb *probs, int n, int form, int parts, unsigned long long *
     if (smem == 0)
         return set_error(FMF_ERR_SMEM, "tensor-core buffers do not fit shared memory");
     void (*kern)(const TcBatch);
-    if (var)
-        kern = full ? tc_persistent<true, true, true> : tc_persistent<true, false, true>;
+    if (var && form == TC_FORM_FP32)
+        kern = full ? tc_persistent<true, true, true, false> : tc_persistent<true, false, true, false>;
+    else if (var)
+        kern = full ? tc_persistent<true, true, true, true> : tc_persistent<true, false, true, true>;
     else if (nsum)
-        kern = full ? tc_persistent<false, true, true> : tc_persistent<false, false, true>;
+        kern = full ? tc_persistent<false, true, true, false> : tc_persistent<false, false, true, false>;
     else
-        kern = full ? tc_persistent<false, true, false> : tc_persistent<false, false, false>;
+        kern = full ? tc_persistent<false, true, false, false> : tc_persistent<false, false, false, false>;
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxDynamicSmem);
     if (e != cudaSuccess)
         return set_error(FMF_ERR_CUDA, "tc_persistent shared memory (%zu bytes): %s", smem,
