@@ -117,7 +117,8 @@ static bool host_is_pinned(const void *p);
 // copied in one piece while the inputs travel and the kernels run (from 16 MB on: one
 // channel of a day at 100 Hz, 35 MB out, 2.00 -> 1.18 ms; less is mapped while the
 // kernels run), one copied in pieces before each piece, behind the kernels of the
-// others (started with the inputs, 432 MB held up their copies: 25.9 -> 26.2 ms).  Two
+// others (started with the inputs, 432 MB held up their copies: 25.9 -> 26.2 ms; so it
+// does not start with inputs of more than twice its size either).  Two
 // threads map 73 GB/s, four 80 to 86, eight 53 to 69 (they wait for one another in the
 // system).  Mapped pages cost a page-table walk; where the system refuses the advice
 // (older kernels) nothing is done.
@@ -170,7 +171,7 @@ struct HostPages::State {
 
 constexpr size_t kAheadBytes = (size_t)16 << 20;
 
-HostPages::HostPages(void *p, size_t bytes) : st(nullptr)
+HostPages::HostPages(void *p, size_t bytes, size_t inputs) : st(nullptr)
 {
     const long page = sysconf(_SC_PAGESIZE);
     if (!p || bytes == 0 || page <= 0 || host_is_pinned(p))
@@ -182,7 +183,7 @@ HostPages::HostPages(void *p, size_t bytes) : st(nullptr)
         q->n_blocks = (q->end - q->begin + State::kBlock - 1) / State::kBlock;
         q->done.resize(q->n_blocks);
         st = q.release();
-        if (bytes >= kAheadBytes && bytes < kPieceBytes)
+        if (bytes >= kAheadBytes && bytes < kPieceBytes && inputs <= 2 * bytes)
             st->start(st->n_blocks, (int)std::min<size_t>(State::kMaxThreads, bytes / (4 * State::kBlock)));
     } catch (...) {  // no memory or no threads: wait() maps what is left
     }
@@ -772,7 +773,7 @@ static int run_host(const Args &a, cudaStream_t s)
 {
     int rc;
     const size_t out_n = a.T * a.n_corr * (a.sum_mode ? 1 : a.S * a.C);
-    HostPages pages(a.out, out_n * sizeof(float));
+    HostPages pages(a.out, out_n * sizeof(float), (a.T * a.L + a.N) * a.S * a.C * sizeof(float));
     {
         Scratch io(s);  // device copies of the arguments, freed in stream order
         Args d;

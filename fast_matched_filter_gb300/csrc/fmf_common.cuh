@@ -184,11 +184,11 @@ constexpr int kMaxDynamicSmem = 227 * 1024;
 // Host outputs of this size are copied in pieces, each behind the next one's kernels.
 constexpr size_t kPieceBytes = (size_t)64 << 20;
 // Maps the pages of a host output, of a medium size on threads of its own from
-// construction on; wait() returns once the first `bytes` of it are mapped.  Page-locked
-// memory is left alone.
+// construction on unless `inputs` bytes to be copied meanwhile are many more; wait()
+// returns once the first `bytes` of it are mapped.  Page-locked memory is left alone.
 class HostPages {
 public:
-    HostPages(void *p, size_t bytes);
+    HostPages(void *p, size_t bytes, size_t inputs);
     ~HostPages();
     HostPages(const HostPages &) = delete;
     HostPages &operator=(const HostPages &) = delete;

@@ -164,11 +164,12 @@ __device__ __forceinline__ int tc_phase(int m, int step, int &psi)
 // A statistics slot: `columns` lag blocks of each column group of the tile from each of
 // `streams` arrays, copied from the 16-byte boundary before the first window.
 // Fixed lengths: window energies, or (energy, mean) pairs.  Per-channel lengths:
-// running sums of d^2 at a window's start and end, for 'full' also those of d.
+// running sums of d^2 at a window's start and end; for 'full' there are no slots (the
+// epilogue reads those, and those of d, itself).
 struct StatSlot {
     int columns, streams, elem, groups;
     __host__ __device__ constexpr StatSlot(bool var, bool full)
-        : columns(var ? (full ? 2 : 4) : (full ? 16 : 32)), streams(var ? (full ? 4 : 2) : 1),
+        : columns(var ? 4 : (full ? 16 : 32)), streams(var ? (full ? 0 : 2) : 1),
           elem(var || full ? 8 : 4), groups(var ? 4 : 2)
     {
     }
@@ -649,9 +650,13 @@ __global__ void __launch_bounds__(tc_threads(VAR), 1) tc_persistent(const __grid
     const uint32_t tmem = *tmem_holder;
     const long long total = B.total_items;
 
-    if (!VAR && warp < 4) {
-        // registers: 384 threads x 168 at launch = 128 x 88 + 256 x 208
-        asm volatile("setmaxnreg.dec.sync.aligned.u32 88;");
+    if (warp < 4) {
+        // registers: 384 threads x 168 at launch = 128 x 88 + 256 x 208; 640 x 96 =
+        // 128 x 64 + 512 x 104 ('full' only: 1,432 -> 1,375 us below, 'short' 757 -> 830 us)
+        if (VAR && FULL)
+            asm volatile("setmaxnreg.dec.sync.aligned.u32 64;");
+        else if (!VAR)
+            asm volatile("setmaxnreg.dec.sync.aligned.u32 88;");
     }
     if (warp == 0) {
         // ---------------------------------------------------------- tile queue, operands
@@ -784,7 +789,7 @@ __global__ void __launch_bounds__(tc_threads(VAR), 1) tc_persistent(const __grid
                 const TcProb &pr = B.prob[p];
                 const Problem &P = pr.P;
                 const long long I0 = (long long)tile * TC_Q * pr.nb;
-                if (!tc_busy(pr, I0, t))
+                if (kStat.streams == 0 || !tc_busy(pr, I0, t))
                     continue;
                 const int nc = pr.nb / G;
                 const size_t row0 = (size_t)t * P.SC;
@@ -802,9 +807,7 @@ __global__ void __launch_bounds__(tc_threads(VAR), 1) tc_persistent(const __grid
                             int psi2;  // the windows' ends
                             const int far = tc_phase(psi + __shfl_sync(0xffffffffu, n_l, from), P.step, psi2);
                             const long long x = I0 + mu + (lane & G ? far : 0);
-                            const char *base = lane & (2 * G) ? reinterpret_cast<const char *>(P.pre1f)
-                                                        : reinterpret_cast<const char *>(P.pre2q);
-                            src = base + (ch * P.pre_ch + (lane & G ? psi2 : psi) * P.pre_ps +
+                            src = reinterpret_cast<const char *>(P.pre2q) + (ch * P.pre_ch + (lane & G ? psi2 : psi) * P.pre_ps +
                                           (x & ~(long long)kStat.align())) * kStat.elem;
                         } else {
                             src = reinterpret_cast<const char *>(P.stat_e) +
@@ -843,7 +846,9 @@ __global__ void __launch_bounds__(tc_threads(VAR), 1) tc_persistent(const __grid
         // ---------------------------------------------------------- epilogue
         // Warp w reads TMEM lane quarter w % 4 (rows 32*(w%4) + lane) and its half of the
         // columns; numerators and network sums of its outputs live in registers.
-        if (!VAR)
+        if (VAR && FULL)
+            asm volatile("setmaxnreg.inc.sync.aligned.u32 104;");
+        else if (!VAR)
             asm volatile("setmaxnreg.inc.sync.aligned.u32 208;");
         constexpr int NCM = TC_NB_MAX / G;  // columns per thread, at most
         const int quarter = warp & 3;
@@ -968,6 +973,11 @@ __global__ void __launch_bounds__(tc_threads(VAR), 1) tc_persistent(const __grid
                         int psi2;
                         const int far = tc_phase(psi + ntap, step, psi2);
                         const int head2 = (int)((I0 + mu + far) & kStat.align());
+                        // 'full' reads its four running sums per output, 32 bytes, from global memory
+                        // (L2): in slots of two columns they took 16 waits a channel (12 stations x
+                        // 3 channels x 598 taps x 7 templates x 959,372 samples: 1,651 us, 1,375 here)
+                        const long long g1 = ch * pr.P.pre_ch + (long long)psi * pr.P.pre_ps + k0 + mu;
+                        const long long g2 = ch * pr.P.pre_ch + (long long)psi2 * pr.P.pre_ps + k0 + mu + far;
                         float x[16];  // ONE: the numerators of 16 columns
 #pragma unroll
                         for (int c0 = 0; c0 < NCM; c0 += CH) {
@@ -995,29 +1005,36 @@ __global__ void __launch_bounds__(tc_threads(VAR), 1) tc_persistent(const __grid
                                         }
                                     }
                                 }
-                                const int es = ec & ((1 << stat_log2) - 1);
-                                if (!mbar_wait_all(bar + TcBars::efull + 8 * es, (ec >> stat_log2) & 1, abort_flag,
-                                                   B.err, 16u))
-                                    goto epilogue_done;
-                                const uint8_t *slot = smem + (e_base - w_base) + es * (uint32_t)B.stat_bytes +
-                                                      cgroup * kStatPart;
-                                const uint8_t *at = slot + (head + b) * 8, *at2 = slot + G * kStatPart + (head2 + b) * 8;
                                 long long lo[CH], hi[CH];
                                 float2 lo1[CH], hi1[CH];
+                                if constexpr (FULL) {
 #pragma unroll
-                                for (int j = 0; j < CH; j++) {
-                                    lo[j] = *reinterpret_cast<const long long *>(at + j * TC_Q * 8);
-                                    hi[j] = *reinterpret_cast<const long long *>(at2 + j * TC_Q * 8);
-                                    if constexpr (FULL) {
-                                        lo1[j] = *reinterpret_cast<const float2 *>(at + 2 * G * kStatPart + j * TC_Q * 8);
-                                        hi1[j] = *reinterpret_cast<const float2 *>(at2 + 2 * G * kStatPart + j * TC_Q * 8);
+                                    for (int j = 0; j < CH; j++) {
+                                        lo[j] = __ldg(pr.P.pre2q + g1 + (c0 + j) * TC_Q);
+                                        hi[j] = __ldg(pr.P.pre2q + g2 + (c0 + j) * TC_Q);
+                                        lo1[j] = __ldg(pr.P.pre1f + g1 + (c0 + j) * TC_Q);
+                                        hi1[j] = __ldg(pr.P.pre1f + g2 + (c0 + j) * TC_Q);
                                     }
+                                } else {
+                                    const int es = ec & ((1 << stat_log2) - 1);
+                                    if (!mbar_wait_all(bar + TcBars::efull + 8 * es, (ec >> stat_log2) & 1,
+                                                       abort_flag, B.err, 16u))
+                                        goto epilogue_done;
+                                    const uint8_t *slot = smem + (e_base - w_base) + es * (uint32_t)B.stat_bytes +
+                                                          cgroup * kStatPart;
+                                    const uint8_t *at = slot + (head + b) * 8,
+                                                  *at2 = slot + G * kStatPart + (head2 + b) * 8;
+#pragma unroll
+                                    for (int j = 0; j < CH; j++) {
+                                        lo[j] = *reinterpret_cast<const long long *>(at + j * TC_Q * 8);
+                                        hi[j] = *reinterpret_cast<const long long *>(at2 + j * TC_Q * 8);
+                                    }
+                                    fence_reads_before_copy();
+                                    __syncwarp();
+                                    if (lane == 0)
+                                        mbar_arrive(bar + TcBars::eempty + 8 * es);
+                                    ec++;
                                 }
-                                fence_reads_before_copy();
-                                __syncwarp();
-                                if (lane == 0)
-                                    mbar_arrive(bar + TcBars::eempty + 8 * es);
-                                ec++;
                                 // (outside the valid lags the sums are anything, and are not used)
                                 float y[CH];
 #pragma unroll

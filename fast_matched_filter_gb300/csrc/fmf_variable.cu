@@ -205,6 +205,7 @@ __global__ void channel_energy_kernel(const float *__restrict__ data, int N, con
                                       float *__restrict__ part, int nblk, unsigned *__restrict__ scan)
 {
     __shared__ float2 red[8];
+    __shared__ unsigned tops[8];
     const int ch = blockIdx.y, blk = blockIdx.x;
     const float m = mu ? mu[ch] : 0.0f;
     const float *src = data + (size_t)ch * N;
@@ -230,8 +231,8 @@ __global__ void channel_energy_kernel(const float *__restrict__ data, int N, con
             top = a < 0x7f800000u ? max(top, a) : top;
         }
         top = __reduce_max_sync(0xffffffffu, top);
-        if ((threadIdx.x & 31) == 0 && top > *(volatile unsigned *)(scan + ch))
-            atomicMax(scan + ch, top);
+        if ((threadIdx.x & 31) == 0)
+            tops[threadIdx.x >> 5] = top;
     }
     for (int o = 16; o > 0; o >>= 1) {
         const float yh = __shfl_down_sync(0xffffffffu, h, o), yl = __shfl_down_sync(0xffffffffu, l, o);
@@ -245,6 +246,15 @@ __global__ void channel_energy_kernel(const float *__restrict__ data, int N, con
         for (int i = 0; i < 8; i++)
             pair_add(th, tl, red[i].x, red[i].y);
         part[(size_t)ch * nblk + blk] = th + tl;
+    }
+    // one atomic per block, and only where it changes the value (one per warp: 196 us for
+    // 36 channels x 959,372 samples, of 34 us without the scan)
+    if (scan && threadIdx.x == 32) {
+        unsigned top = 0;
+        for (int i = 0; i < 8; i++)
+            top = max(top, tops[i]);
+        if (top > *(volatile unsigned *)(scan + ch))
+            atomicMax(scan + ch, top);
     }
 }
 
@@ -801,7 +811,7 @@ static int variable_entry(const VArgs &a, void *stream)
     const size_t SC = a.S * a.C;
     const size_t cnt[7] = {a.T * SC * L, a.T * SC, a.T * SC, SC * a.N, a.T * SC, a.T * SC, a.T * a.n_corr};
     float *buf[7];
-    HostPages pages(a.out, cnt[6] * sizeof(float));
+    HostPages pages(a.out, cnt[6] * sizeof(float), (cnt[0] + cnt[3]) * sizeof(float));
     {
         Scratch io(s);
         for (int i = 0; i < 7; i++)
