@@ -455,8 +455,8 @@ struct TcBars {
 // One MMA issuer's walk over the items: the h h products (SMALL false; chains of
 // chain_slots data slots into H0 / H1 in turn) or the h l and l h products (into
 // S0 / S1, a channel each).
-template <bool VAR, bool SMALL>
-__device__ __forceinline__ void tc_issue(const TcBatch &B, const long long *ring, uint32_t bar,
+template <bool VAR, bool SMALL, int N>
+__device__ __forceinline__ void tc_issue(const TcBatch<N> &B, const long long *ring, uint32_t bar,
                                            uint32_t w_base, uint32_t d_base, uint32_t tmem,
                                            volatile int *abort_flag, bool one)
 {
@@ -587,8 +587,8 @@ __device__ __forceinline__ void tc_issue(const TcBatch &B, const long long *ring
 // ONE (per-channel lengths): every channel is one chain (the bf16 forms), whose
 // numerators go from the accumulators to the sums without a stop in registers; with
 // that stop 16 epilogue warps spill.
-template <bool VAR, bool FULL, bool NSUM, bool ONE>
-__global__ void __launch_bounds__(tc_threads(VAR), 1) tc_persistent(const __grid_constant__ TcBatch B)
+template <bool VAR, bool FULL, bool NSUM, bool ONE, int N>
+__global__ void __launch_bounds__(tc_threads(VAR), 1) tc_persistent(const __grid_constant__ TcBatch<N> B)
 {
     extern __shared__ __align__(1024) uint8_t smem[];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -1277,11 +1277,8 @@ static int choose_parts(long long items, int SC)
 // Shared memory of one launch: two template buffers, two statistics slots (32 KB
 // each: half a channel of a full tile) and as many data slots as fit (a channel
 // has 4); long templates give up a statistics slot first.
-static size_t tc_layout(TcBatch *B, bool var, bool full)
+static size_t tc_layout(TcLaunch *B, int nb, bool var, bool full)
 {
-    int nb = 0;
-    for (int i = 0; i < B->n_probs; i++)
-        nb = max(nb, B->prob[i].nb);
     const StatSlot slot(var, full);
     const size_t fixed = 2 * (size_t)B->w_bytes + TcBars::bytes;
     B->stat_bytes = (int)slot.bytes();
@@ -1313,16 +1310,29 @@ int tc_choose_parts(const TcProb *prob)
     return P.SC >= 2 ? choose_parts((long long)prob->n_tiles * P.T, P.SC) : 1;
 }
 
-// One persistent launch over the tile queue of `n` prepared searches (n <= TC_MAX_PROBS).
+template <int N>
+static void (*tc_kernel(int form, bool var, bool full, bool nsum))(const TcBatch<N>)
+{
+    if constexpr (N == 1) {  // (no batch holds searches of per-channel lengths)
+        if (var && form == TC_FORM_FP32)
+            return full ? tc_persistent<true, true, true, false, 1> : tc_persistent<true, false, true, false, 1>;
+        if (var)
+            return full ? tc_persistent<true, true, true, true, 1> : tc_persistent<true, false, true, true, 1>;
+    }
+    if (nsum)
+        return full ? tc_persistent<false, true, true, false, N> : tc_persistent<false, false, true, false, N>;
+    return full ? tc_persistent<false, true, false, false, N> : tc_persistent<false, false, false, false, N>;
+}
+
+// One persistent launch over the tile queue of `n` prepared searches (n <= N).
 // `form`: the operands they were prepared with.  `queue`: a device counter, zero before
 // the launch.  `parts`: channel parts of every item (n = 1 only).
-int tc_run(const TcProb *probs, int n, int form, int parts, unsigned long long *queue, unsigned *err,
-           cudaStream_t s)
+template <int N>
+static int tc_run_n(const TcProb *probs, int n, int form, int parts, unsigned long long *queue, unsigned *err,
+                    cudaStream_t s)
 {
-    if (n < 1 || n > TC_MAX_PROBS)
-        return set_error(FMF_ERR_ARG, "a persistent launch takes 1..%d searches", TC_MAX_PROBS);
-    static thread_local TcBatch Bh;  // large; built on the host for the launch only
-    TcBatch &B = Bh;
+    static thread_local TcBatch<N> Bh;  // large; built on the host for the launch only
+    TcBatch<N> &B = Bh;
     const Problem &P0 = probs[0].P;
     const bool var = P0.ntap != nullptr, full = P0.normalize != 0, nsum = P0.network_sum != 0;
     Scratch pws(s);
@@ -1336,6 +1346,7 @@ int tc_run(const TcProb *probs, int n, int form, int parts, unsigned long long *
     B.mma_types = form == TC_FORM_FP32 ? 0u : (1u << 7) | (1u << 10);
     B.lo_unit = form == TC_FORM_FP32 ? 1.0f / kLoScale : 1.0f;
     B.w_bytes = B.row_bytes = 0;
+    int nb = 0;
     const int halves = B.split ? 2 : 1;
     long long items = 0;
     for (int i = 0; i < n; i++) {
@@ -1349,23 +1360,18 @@ int tc_run(const TcProb *probs, int n, int form, int parts, unsigned long long *
         items += (long long)probs[i].n_tiles * P.T * parts;
         B.w_bytes = max(B.w_bytes, halves * probs[i].NW * 128);
         B.row_bytes = max(B.row_bytes, halves * 4 * probs[i].R * 16);
+        nb = max(nb, probs[i].nb);
     }
     B.n_probs = n;
     B.total_items = items;
     B.queue = queue;
     B.err = err;
-    const size_t smem = tc_layout(&B, var, full);
+    const size_t smem = tc_layout(&B, nb, var, full);
     if (smem == 0)
         return set_error(FMF_ERR_SMEM, "tensor-core buffers do not fit shared memory");
-    void (*kern)(const TcBatch);
-    if (var && form == TC_FORM_FP32)
-        kern = full ? tc_persistent<true, true, true, false> : tc_persistent<true, false, true, false>;
-    else if (var)
-        kern = full ? tc_persistent<true, true, true, true> : tc_persistent<true, false, true, true>;
-    else if (nsum)
-        kern = full ? tc_persistent<false, true, true, false> : tc_persistent<false, false, true, false>;
-    else
-        kern = full ? tc_persistent<false, true, false, false> : tc_persistent<false, false, false, false>;
+    if (N > 1 && var)
+        return set_error(FMF_ERR_ARG, "a batch of searches of per-channel lengths");
+    void (*kern)(const TcBatch<N>) = tc_kernel<N>(form, var, full, nsum);
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxDynamicSmem);
     if (e != cudaSuccess)
         return set_error(FMF_ERR_CUDA, "tc_persistent shared memory (%zu bytes): %s", smem,
@@ -1383,6 +1389,14 @@ int tc_run(const TcProb *probs, int n, int form, int parts, unsigned long long *
                                                                      P0.vp_bias, P0.vp_scale, P0.out);
     count_launch();
     return check_launch("tc_parts_sum_kernel");
+}
+
+int tc_run(const TcProb *probs, int n, int form, int parts, unsigned long long *queue, unsigned *err, cudaStream_t s)
+{
+    if (n < 1 || n > TC_MAX_PROBS)
+        return set_error(FMF_ERR_ARG, "a persistent launch takes 1..%d searches", TC_MAX_PROBS);
+    return n == 1 ? tc_run_n<1>(probs, n, form, parts, queue, err, s)
+                  : tc_run_n<TC_MAX_PROBS>(probs, n, form, parts, queue, err, s);
 }
 
 size_t tc_prob_size() { return sizeof(TcProb); }

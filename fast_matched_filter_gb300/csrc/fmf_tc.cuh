@@ -40,8 +40,7 @@ struct TcProb {
     const unsigned *skip;         // nonzero: the FP32 CUDA-core kernel runs this search instead
 };
 
-struct TcBatch {
-    TcProb prob[TC_MAX_PROBS];
+struct TcLaunch {
     int n_probs;
     int split;                    // 1: hi/lo, three products; 0: single bf16 product
     uint32_t mma_types;           // operand types, in their place in the MMA's instruction descriptor
@@ -51,6 +50,13 @@ struct TcBatch {
     long long total_items;
     unsigned long long *queue;    // tile-queue head, zero before the launch
     unsigned *err;                // device error word
+};
+
+// The kernel's parameter: a lone search's is a 64th of a batch's (27 KB, which cost the
+// caller 4 us more a launch).
+template <int N>
+struct TcBatch : TcLaunch {
+    TcProb prob[N];
 };
 
 // ------------------------------------------------------------------ PTX helpers
@@ -303,10 +309,11 @@ __device__ __forceinline__ void fisher_atanh(float (&y)[N])
 // ------------------------------------------------------------------ tile queue
 // Decodes a tile-queue item: search p, output tile, template t.  Items of one
 // search are ordered so that groups of `tg` templates sweep the tiles together.
-__device__ __forceinline__ void decode_item(const TcBatch &B, long long item, int &p, int &tile, int &t,
+template <int N>
+__device__ __forceinline__ void decode_item(const TcBatch<N> &B, long long item, int &p, int &tile, int &t,
                                             int &c_begin, int &c_end, int &part)
 {
-    int lo = 0, hi = B.n_probs - 1;
+    int lo = 0, hi = N == 1 ? 0 : B.n_probs - 1;
     while (lo < hi) {
         const int mid = (lo + hi + 1) >> 1;
         if (B.prob[mid].item_begin <= item)
