@@ -87,7 +87,7 @@ constexpr int tc_epi_warps(bool var) { return var ? 16 : 8; }
 constexpr int tc_threads(bool var) { return 32 * (4 + tc_epi_warps(var)); }
 constexpr int tc_groups(bool var) { return tc_epi_warps(var) / 4; }  // column groups of a tile
 constexpr int TC_MAX_ROWS = 8;     // data slots, at most
-constexpr int TC_MAX_PARTS = 8;    // channel parts of an item, at most
+constexpr int TC_MAX_PARTS = 32;   // channel parts of an item, at most
 constexpr int TC_MAX_STATS = 2;    // statistics slots, at most
 constexpr int kChain = 16;          // K steps of one h h chain
 constexpr float kLoScale = 2048.0f;  // l is kept 2^11 up
@@ -1222,9 +1222,9 @@ static int n_sms()
 // out[i] = sum over parts j = 0..k-1 of part[j][i], in that order; with
 // per-channel lengths (norm set) the Fisher-z transform of that sum,
 // (tanh(v / norm[t]) + bias[t]) * scale[t] for row t = i / n_corr.  Bound by the loads'
-// latency: all parts' values are in flight (one after the other: 12 us for 13 x 115,115
-// outputs, 8 us here).  Added by whichever part came last in the
-// persistent kernel itself, they held up its end instead: 0.27 -> 0.39 ms of the search.
+// latency: eight parts' values are in flight (one after the other: 12 us for 13 x 115,115
+// outputs, 8 us here).  Added by whichever part came last in the persistent kernel
+// itself, they held up its end instead: 0.27 -> 0.39 ms of the search.
 __global__ void tc_parts_sum_kernel(const float *__restrict__ part, int k, long long m, int n_corr,
                                     const float *__restrict__ norm, const float *__restrict__ bias,
                                     const float *__restrict__ scale, float *__restrict__ out)
@@ -1232,16 +1232,19 @@ __global__ void tc_parts_sum_kernel(const float *__restrict__ part, int k, long 
     const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= m)
         return;
-    float x[TC_MAX_PARTS];
+    constexpr int kLoads = 8;
+    float v = 0.0f;
+    for (int j0 = 0; j0 < k; j0 += kLoads) {
+        float x[kLoads];
 #pragma unroll
-    for (int j = 0; j < TC_MAX_PARTS; j++)
-        if (j < k)
-            x[j] = __ldg(part + (size_t)j * m + i);
-    float v = x[0];
+        for (int j = 0; j < kLoads; j++)
+            if (j0 + j < k)
+                x[j] = __ldg(part + (size_t)(j0 + j) * m + i);
 #pragma unroll
-    for (int j = 1; j < TC_MAX_PARTS; j++)
-        if (j < k)
-            v += x[j];
+        for (int j = 0; j < kLoads; j++)
+            if (j0 + j < k)
+                v = j0 + j == 0 ? x[j] : v + x[j];
+    }
     if (norm) {
         const int t = (int)(i / n_corr);
         v = (tanhf(v / norm[t]) + bias[t]) * scale[t];
@@ -1249,10 +1252,12 @@ __global__ void tc_parts_sum_kernel(const float *__restrict__ part, int k, long 
     out[i] = v;
 }
 
-// Channel parts k (1..8, at most SC) for a search of `items` (tile, template)
+// Channel parts k (1..32, at most SC) for a search of `items` (tile, template)
 // items: the k that minimises the busiest SM's work, ceil(k items / SMs)
 // rounds of (1/k + 0.05) item each (0.05: an item's fixed pipeline fill and
-// output write); FMF_TC_PARTS=k forces a value.
+// output write), within 5 % of the best k in thirteen searches of 6 to 400 items.  (One
+// template x 60 channels x 300 taps x 3,000 samples: 70 us in 8 parts, 56 in 16, 50 in
+// 32.)  FMF_TC_PARTS=k forces a value.
 static int choose_parts(long long items, int SC)
 {
     const int sms = n_sms(), kmax = SC < TC_MAX_PARTS ? SC : TC_MAX_PARTS;
