@@ -65,7 +65,7 @@ def parse_args(argv=None):
     p.add_argument("--no-e2e", action="store_true")
     p.add_argument("--no-cpu-baseline", action="store_true")
     p.add_argument("--no-compare", action="store_true",
-                   help="skip the plain FP32 comparison run")
+                   help="skip the FP32 comparison run")
     p.add_argument("--no-precision-report", action="store_true",
                    help="skip the FP64 error report on a subset")
     p.add_argument("--no-detect", action="store_true",
@@ -389,14 +389,14 @@ def run_ours(args):
                                      else "single GPU"}),
             "roofline": roof, "gpu_launches": main["launches"], "clocks": main["clocks"]}
     if precision != "fp32" and not args.no_compare:
-        plain = timed("fp32", max(1, min(args.steps, 2)), 1, False)
-        line["plain_fp32"] = {"value": plain["value"], "unit": UNIT,
-                              "ms_per_step": plain["ms_per_step"],
-                              "kernel_ms_avg": plain["kernel_ms_avg"],
-                              "speedup_of_headline": value / plain["value"],
-                              "roofline": roofline(cfg, "fp32", plain["kernel_ms_avg"],
-                                                   plain["prep_ms_avg"],
-                                                   fp32_measured=measured_fp32_tflops(lib))}
+        f32 = timed("fp32", max(1, min(args.steps, 2)), 1, False)
+        line["fp32"] = {"value": f32["value"], "unit": UNIT,
+                        "ms_per_step": f32["ms_per_step"],
+                        "kernel_ms_avg": f32["kernel_ms_avg"],
+                        "speedup_of_headline": value / f32["value"],
+                        "roofline": roofline(cfg, "fp32", f32["kernel_ms_avg"],
+                                             f32["prep_ms_avg"],
+                                             fp32_measured=measured_fp32_tflops(lib))}
 
     if rank == 0 and not args.no_precision_report:
         line["precision_vs_fp64"] = precision_report(cfg)
@@ -515,28 +515,25 @@ def fp32_peak(measured):
 def roofline(cfg, precision, kern_ms, prep_ms, fp32_measured=None):
     peaks, src = load_peaks()
     algo_tflops = 2.0 * cfg["macs"] / (kern_ms / 1e3) / 1e12
-    if precision == "fp32":
-        peak, nominal, psrc = fp32_peak(fp32_measured)
-        roof = {"bound": "fp32_fma", "achieved": algo_tflops, "peak": peak, "unit": "TFLOP/s",
-                "frac": algo_tflops / peak, "nominal_peak": nominal, "nominal_frac": algo_tflops / nominal,
-                "traffic": None, "kernel": "plain_kernel", "peak_source": psrc}
-    else:
-        bf16 = float(peaks.get("bf16_tflops_sustained", peaks["bf16_tflops"]))
-        products = 3 if precision == "split_bf16" else 1
-        # the bound in algorithmic FLOP/s: each multiply-accumulate costs `products`
-        # bf16 tensor-core products
-        peak = bf16 / products
-        ex, nb = tc_executed_macs(cfg)
-        executed = 2.0 * ex * products / (kern_ms / 1e3) / 1e12
-        traffic, tsrc = profiled_traffic("tc_persistent", cfg)
-        roof = {"bound": "tensor", "achieved": algo_tflops, "peak": peak, "unit": "TFLOP/s",
-                "frac": algo_tflops / peak, "traffic": traffic, "traffic_source": tsrc,
-                "kernel": "tc_persistent (nb=%d)" % nb,
-                "peak_source": "%s bf16_tflops_sustained (cuBLAS bf16 GEMM, seconds-long loop) "
-                               "/ %d bf16 products per multiply-accumulate" % (src, products),
-                "bf16_peak": bf16,
-                "executed_tflops": executed, "executed_frac": executed / bf16,
-                "executed_over_algorithmic": ex * products / cfg["macs"]}
+    bf16 = float(peaks.get("bf16_tflops_sustained", peaks["bf16_tflops"]))
+    products = 1 if precision == "bf16" else 3  # fp32: fp16 pairs at the bf16 rate
+    # the bound in algorithmic FLOP/s: each multiply-accumulate costs `products`
+    # half-precision tensor-core products
+    peak = bf16 / products
+    ex, nb = tc_executed_macs(cfg)
+    executed = 2.0 * ex * products / (kern_ms / 1e3) / 1e12
+    traffic, tsrc = profiled_traffic("tc_persistent", cfg)
+    roof = {"bound": "tensor", "achieved": algo_tflops, "peak": peak, "unit": "TFLOP/s",
+            "frac": algo_tflops / peak, "traffic": traffic, "traffic_source": tsrc,
+            "kernel": "tc_persistent (nb=%d, %s)" % (nb, precision),
+            "peak_source": "%s bf16_tflops_sustained (cuBLAS bf16 GEMM, seconds-long loop) "
+                           "/ %d half-precision products per multiply-accumulate" % (src, products),
+            "bf16_peak": bf16,
+            "executed_tflops": executed, "executed_frac": executed / bf16,
+            "executed_over_algorithmic": ex * products / cfg["macs"]}
+    if precision == "fp32":  # against the FMA units, which it ran on before the tensor cores
+        fma, _, fma_src = fp32_peak(fp32_measured)
+        roof.update({"fp32_fma_peak": fma, "fp32_fma_frac": algo_tflops / fma, "fp32_fma_source": fma_src})
     roof["kernel_ms_avg"] = kern_ms
     roof["prep_ms_avg"] = prep_ms
     return roof
@@ -708,7 +705,7 @@ def run_detection(cfg, dev_out, world, steps=3, warmup=1):
                                            "launches per row byte, scaled to these rows",
                          "peak_source": "%s hbm_gbs (copy)" % peak_kind,
                          "kernel": "fmf_detect (det_sample x2, det_count x2: one read of each "
-                                   "row; det_hist x6 over the candidates, det_resolve x6, "
+                                   "row; det_pick, det_gather and det_finish x2 over the candidates, "
                                    "det_select)"}}
 
 
@@ -773,7 +770,7 @@ def run_variable(args):
     """Per-channel template lengths (Fisher-z network sum) through
     fmf_matched_filter_variable_ex: device-resident inputs (value) and host
     inputs (e2e).  MACs count each channel's own length.  --precision auto
-    runs the tensor-core numerators (split bf16), with the plain FP32 form
+    runs the tensor-core numerators (split bf16), with the FP32 form
     timed beside them."""
     import torch
     from fast_matched_filter_gb300 import _lib
@@ -821,31 +818,18 @@ def run_variable(args):
         return ms, launches, (clocks.summary() if sample_clocks else None)
 
     peaks, kind = load_peaks()
-    fma_peak, fma_nominal, fma_src = fp32_peak(measured_fp32_tflops(lib))  # TFLOP/s
-
-    def plain_roofline(ms):
-        # the kernel runs each channel over its own taps rounded up to its 20-tap unroll
-        executed = int(n_corr) * int(((nt.astype(np.int64) + 19) // 20 * 20).sum())
-        achieved = 2 * cfg["macs"] / (ms / 1e3) / 1e12
-        return {"bound": "fp32_fma", "achieved": achieved, "peak": fma_peak, "unit": "TFLOP/s",
-                "frac": achieved / fma_peak, "nominal_peak": fma_nominal,
-                "nominal_frac": achieved / fma_nominal,
-                "executed_frac": 2 * executed / (ms / 1e3) / 1e12 / fma_peak,
-                "traffic": None, "kernel": "plain_kernel (per-channel lengths)",
-                "peak_source": fma_src}
-
-    def tc_roofline(ms):
+    def tc_roofline(ms, precision=precision):
         bf16 = peaks.get("bf16_tflops_sustained", FALLBACK_PEAKS["bf16_tflops_sustained"])
         achieved = 2 * cfg["macs"] / (ms / 1e3) / 1e12
         executed, nb = tc_executed_macs(cfg)
-        n_prod = 3 if precision == "split_bf16" else 1
-        peak = bf16 / n_prod  # algorithmic FLOP/s bound: n_prod bf16 products per MAC
+        n_prod = 1 if precision == "bf16" else 3
+        peak = bf16 / n_prod  # algorithmic FLOP/s bound: n_prod half-precision products per MAC
         ex = 2 * executed * n_prod / (ms / 1e3) / 1e12
         return {"bound": "tensor", "achieved": achieved, "peak": peak, "unit": "TFLOP/s",
                 "frac": achieved / peak, "traffic": None,
-                "kernel": "tc_persistent (nb=%d, per-channel K ranges)" % nb,
+                "kernel": "tc_persistent (nb=%d, per-channel K ranges, %s)" % (nb, precision),
                 "peak_source": "%s bf16_tflops_sustained (cuBLAS bf16 GEMM, seconds-long loop) "
-                               "/ %d bf16 products per multiply-accumulate" % (kind, n_prod),
+                               "/ %d half-precision products per multiply-accumulate" % (kind, n_prod),
                 "bf16_peak": bf16, "executed_tflops": ex, "executed_frac": ex / bf16,
                 "executed_over_algorithmic": executed * n_prod / cfg["macs"]}
 
@@ -859,13 +843,13 @@ def run_variable(args):
             "config": describe(cfg, {"precision": precision,
                                      "template_lengths": "400-800 per channel",
                                      "parallelism": "single GPU"}),
-            "roofline": plain_roofline(ms) if precision == "fp32" else tc_roofline(ms),
+            "roofline": tc_roofline(ms),
             "gpu_launches": launches, "clocks": clocks}
     if precision != "fp32" and not args.no_compare:
         pms, _, _ = timed("fp32", max(1, min(args.steps, 2)), 1, False)
         pv = cfg["macs"] / (pms / 1e3) / 1e12
-        line["plain_fp32"] = {"value": pv, "unit": UNIT, "ms_per_step": pms,
-                              "speedup_of_headline": value / pv, "roofline": plain_roofline(pms)}
+        line["fp32"] = {"value": pv, "unit": UNIT, "ms_per_step": pms,
+                        "speedup_of_headline": value / pv, "roofline": tc_roofline(pms, "fp32")}
     # end to end: host inputs, synchronous entry point (inputs copied in, cc copied out)
     cc = np.zeros((T, n_corr), dtype=np.float32)
 
@@ -894,7 +878,7 @@ def run_variable(args):
 
 def run_batch(args):
     """Batched uneven searches: one graph (preprocessing + persistent tile-queue
-    launch) vs the same searches as sequential plain FP32 calls and as
+    launch) vs the same searches as sequential FP32 calls and as
     sequential tensor-core calls."""
     import torch
 
@@ -939,7 +923,7 @@ def run_batch(args):
         ms_batch = timeit(batch.run, args.steps, max(args.warmup, 1))
     launches = batch.run()
     ms_seq_tc = timeit(lambda: sequential("split_bf16"), max(1, args.steps // 2), 1)
-    ms_seq_plain = timeit(lambda: sequential("fp32"), max(1, args.steps // 2), 1)
+    ms_seq_fp32 = timeit(lambda: sequential("fp32"), max(1, args.steps // 2), 1)
     lib = fmf.fast_matched_filter._require_lib()
     from fast_matched_filter_gb300 import _lib
     _lib.check(lib.fmf_device_errors(), lib)
@@ -956,9 +940,9 @@ def run_batch(args):
             "gpu_launches": launches * args.steps, "clocks": clocks.summary(),
             "sequential_split_bf16": {"value": total_macs / (ms_seq_tc / 1e3) / 1e12,
                                       "ms_per_step": ms_seq_tc},
-            "sequential_plain_fp32": {"value": total_macs / (ms_seq_plain / 1e3) / 1e12,
-                                      "ms_per_step": ms_seq_plain,
-                                      "batched_speedup": ms_seq_plain / ms_batch}}
+            "sequential_fp32": {"value": total_macs / (ms_seq_fp32 / 1e3) / 1e12,
+                                      "ms_per_step": ms_seq_fp32,
+                                      "batched_speedup": ms_seq_fp32 / ms_batch}}
     batch.close()
     print(json.dumps(line))
     return 0

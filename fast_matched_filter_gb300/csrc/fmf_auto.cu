@@ -1,14 +1,15 @@
 // fmf_auto.cu -- the numerator precision FMF_PREC_AUTO chooses for a search.
 //
 // The split-bf16 tensor-core form (x = hi + lo, three bf16 products, FP32
-// accumulation) is ~8x faster than the plain FP32 form, but each of its
+// accumulation) is up to 5 % faster than the FP32 form on the tensor cores (8x on
+// the CUDA cores), but each of its
 // products t*d carries a relative error of 4.4e-6 RMS (2.7e-5 at most): a
 // coefficient over L taps errs by about 4.4e-6 / sqrt(L) (measured on random
 // operands, FP64 reference), and a template copied into the data at a
 // power-of-two scale adds a bias of up to 2.8e-6 * |cc| (the dropped lo*lo
 // products then all have one sign).  AUTO runs the split form when this
 // model puts the largest error of the whole search at or below 1e-5 (relative
-// to max(1, sum |w|) for network sums), and the plain FP32 form otherwise:
+// to max(1, sum |w|) for network sums), and the FP32 form otherwise:
 //
 //   per channel   s_ch = 4.4e-6 * sqrt(D_ch / L_eff)
 //   network sum   est  = 2.8e-6 * sum|w| + k * sqrt(sum_ch w^2 s_ch^2)

@@ -10,7 +10,7 @@
 // regular entry points allocate their working arrays per call from the
 // device's stream-ordered pool; this one does not allocate at all.
 //
-// What it does: the plain FP32 form (the same kernels as fmf_matched_filter),
+// What it does: FP32 on the CUDA cores (the kernels of fmf_matched_filter's small searches),
 // with every working array (per-template lag ranges, window statistics, the
 // template energies when the caller passes none, and for 'full' the centred
 // data and templates) carved out of ONE file-scope device array of

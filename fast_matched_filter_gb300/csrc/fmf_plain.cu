@@ -1,4 +1,5 @@
-// fmf_plain.cu -- plain FP32 CUDA-core matched filter (drop-in form).
+// fmf_plain.cu -- FP32 matched filter on the CUDA cores: small searches, short templates,
+// and what the tensor cores' operands cannot hold.
 //
 // Replaces the reference kernels network_corr + sum_cc
 // (matched_filter.cu:42-168) and the per-lag loop of the CPU library

@@ -248,7 +248,7 @@ __global__ void zero_count_kernel(const float *__restrict__ out, long long row_l
 // through shared memory.  Zeros outside the valid lags and on channels of weight 0; all
 // zeros if the flag leaves the search to the CUDA cores.  (Written in place, 4
 // bytes per 32-byte sector, the coefficients of 8 templates x 36 channels x
-// 119,601 lags took 712 us; now 150 us and 50 us here.)
+// 119,601 lags took 712 us; now 119 us and 75 us here.)
 constexpr int kTurnLags = 64, kTurnChannels = 64;
 __global__ void __launch_bounds__(256) channel_outputs_kernel(
     const float *__restrict__ by_channel, const float *__restrict__ w, const int *__restrict__ k_lo,

@@ -49,7 +49,7 @@
 // What bounds it: the tensor pipe, and with it the power limit, from some 400
 // taps (40 templates x 60 channels x 1.08M lags x 600 taps in 6.3 ms: 1.8
 // PFLOP/s of MMAs, 1.74 is what cuBLAS sustains under the limit); the issuing
-// threads and the epilogue below (60 taps: 3.3 ms).  An issuing thread's code
+// threads and the epilogue below (60 taps: 3.8 ms with the preparation).  An issuing thread's code
 // costs as much as its MMAs: a branchy loop took 500 cycles per MMA of 64.
 //
 // Roles of a persistent CTA (12 warps, one CTA per SM), which takes items (one

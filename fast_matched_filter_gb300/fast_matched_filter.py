@@ -9,9 +9,9 @@ reference's CPU architectures are not part of this package, which reports
 them as not loaded exactly as the reference wrapper does when its CPU
 library is missing (fast_matched_filter.py:164-177).
 
-One keyword is added: ``precision`` -- 'fp32' (plain FP32 CUDA-core form,
-the default and the drop-in), 'split_bf16' (tensor cores, bf16 hi+lo with
-three products), 'auto' (split_bf16 where its error model puts the search's
+One keyword is added: ``precision`` -- 'fp32' (the default and the drop-in:
+fp16 pairs of 22 bits on the tensor cores, the CUDA cores for small searches),
+'split_bf16' (tensor cores, bf16 hi+lo with three products), 'auto' (split_bf16 where its error model puts the search's
 largest error at or below 1e-5, else fp32; ``last_precision()`` tells which)
 or 'bf16' (single bf16 product).
 
@@ -272,7 +272,7 @@ def last_precision():
 def _output_array(out, shape):
     """The flat float32 output: a new array (the library writes every element,
     so it is not zeroed first, and maps its pages on several threads while the
-    GPU computes), or a view of ``out`` after checking that the library may
+    inputs travel or the GPU computes), or a view of ``out`` after checking that the library may
     write it in place."""
     if out is None:
         return np.empty(int(np.prod(shape)), dtype=np.float32)
@@ -287,7 +287,7 @@ def _matched_filter_variable(templates, moveouts, weights, data, step, n_samples
                              check_zeros, normalize, network_sum, precision="fp32", out=None):
     """Per-channel template lengths (the reference's arch 'variable_precise',
     fast_matched_filter.py:216-229, 307-313) on the GPU library; ``precision``
-    selects the plain FP32 or the tensor-core numerators."""
+    selects the numerators."""
     if precision not in _lib.PRECISIONS:
         raise ValueError("precision must be one of %s" % sorted(_lib.PRECISIONS))
     if n_samples_template is None:
@@ -436,8 +436,8 @@ class Batch:
     ``add`` takes canonical, contiguous torch CUDA tensors (as
     ``matched_filter_device``) and keeps references to them; ``run`` launches
     every search asynchronously on ``stream`` -- preprocessing, then one
-    persistent tensor-core launch over a shared tile queue (or the plain
-    kernel per search for precision='fp32').  The graph is captured on the
+    persistent tensor-core launch per mode over a shared tile queue (small
+    searches of precision='fp32' run a CUDA-core kernel each).  The graph is captured on the
     first ``run`` after the last ``add`` and replayed afterwards.
     """
 

@@ -51,7 +51,11 @@ extern "C" {
 #define FMF_ERR_UNSUPPORTED 6 /* option not available in this build/device */
 
 /* numerator precision */
-#define FMF_PREC_FP32 0       /* plain FP32 CUDA-core form */
+/* FP32: on the tensor cores as scaled fp16 pairs (22 bits) in searches large
+ * enough (56 taps at least; per-channel lengths 112), with an error no larger
+ * than that of FP32 multiply-adds; else, and where the amplitudes do not fit
+ * such pairs, on the CUDA cores */
+#define FMF_PREC_FP32 0
 #define FMF_PREC_SPLIT_BF16 1 /* tensor cores, bf16 hi+lo, 3 products, FP32 accumulate */
 #define FMF_PREC_BF16 2       /* tensor cores, single bf16 product (loss demonstration) */
 /* FMF_PREC_SPLIT_BF16 where an error model of that form puts the search's
@@ -84,7 +88,7 @@ extern "C" {
  *                       size_t n_components, size_t n_corr, float* cc_out,
  *                       int normalize, int sum_cc_mode)
  * (fast_matched_filter/src/matched_filter_GPU.h:1-4, matched_filter.cu:171-176).
- * Host pointers; plain FP32 form; synchronous.
+ * Host pointers; FMF_PREC_FP32; synchronous.
  */
 FMF_API int fmf_matched_filter(const float *templates, const float *sum_square_templates,
                        const int *moveouts, const float *data, const float *weights,
@@ -149,7 +153,7 @@ FMF_API int fmf_matched_filter_check_zeros(const float *templates, const float *
  *
  * Same arguments as fmf_matched_filter plus a stream; every array argument is
  * a 4-byte-aligned device pointer (a misaligned one is rejected with
- * FMF_ERR_ARG); plain FP32 form; asynchronous on `stream`.  As in
+ * FMF_ERR_ARG); FP32 on the CUDA cores; asynchronous on `stream`.  As in
  * fmf_matched_filter, sum_square_templates may be NULL and is then computed on
  * the device.  It allocates nothing: its working arrays live in one
  * file-scope device array of FMF_NOALLOC_SCRATCH_BYTES that every GPU loading
@@ -175,9 +179,9 @@ FMF_API int fmf_matched_filter_noalloc(const float *templates, const float *sum_
  * runs one search per call, matched_filter.cu:171-399).  A batch records
  * searches of any sizes -- device pointers, the same 15 arguments as
  * fmf_matched_filter -- and runs them all as one CUDA graph: the searches'
- * preprocessing, then one persistent tensor-core launch per 64 searches over
- * a shared tile queue (FMF_PREC_SPLIT_BF16 / FMF_PREC_BF16) or the plain kernel
- * per search (FMF_PREC_FP32).  The graph is captured by the first
+ * preprocessing, then one persistent tensor-core launch per mode and 64
+ * searches over a shared tile queue; of FMF_PREC_FP32, the small searches run
+ * the CUDA-core kernel each.  The graph is captured by the first
  * fmf_batch_run after the last fmf_batch_add and replayed by later runs,
  * which read the input buffers anew.  fmf_batch_run is asynchronous on
  * `stream` (NULL = legacy default stream).  A batch belongs to the device
@@ -203,8 +207,8 @@ FMF_API int fmf_batch_destroy(fmf_batch *batch);
  * Per-channel template lengths with a Fisher-z network sum: the arguments of
  * the reference's CPU-only matched_filter_variable_precise
  * (fast_matched_filter/src/matched_filter_CPU.h, matched_filter.c:321-325,
- * called from fast_matched_filter.py:307-309), run on the GPU (plain FP32
- * form; the tensor-core form through the flags of the _ex entry point).
+ * called from fast_matched_filter.py:307-309), run on the GPU
+ * (FMF_PREC_FP32; the bf16 forms through the flags of the _ex entry point).
  * n_samples_template (T, S, C) gives each channel's length; templates
  * are (T, S, C, max length), zero-padded; cc_sum is (T, n_corr) with
  * n_corr = (N - max length) / step + 1.  Host pointers, synchronous.
@@ -218,8 +222,8 @@ FMF_API int fmf_matched_filter_variable(const float *templates, const float *sum
                                         size_t n_components, size_t n_corr, float *cc_sum,
                                         int normalize);
 /* Same, with flags and a stream: FMF_FLAG_DEVICE_POINTERS;
- * FMF_FLAG_PRECISION(FMF_PREC_SPLIT_BF16 or FMF_PREC_BF16) runs the numerators
- * on the tensor cores (each channel's K range cut at its own length),
+ * FMF_FLAG_PRECISION (on the tensor cores each channel's K range is cut at its
+ * own length),
  * FMF_FLAG_TILE / FMF_FLAG_TEMPLATE_GROUP as for fmf_matched_filter_ex. */
 FMF_API int fmf_matched_filter_variable_ex(const float *templates, const float *sum_square_templates,
                                            const int *moveouts, const float *data, const float *weights,
@@ -316,8 +320,8 @@ FMF_API int fmf_selftest_wait_timeout(unsigned ms);
 /* Measurement helper (no reference counterpart): the FP32 multiply-add rate
  * of the current device in TFLOP/s (2 flops per FMA), from a kernel of
  * independent FMA chains on every SM, best of three timed runs (about 10 ms
- * in all; synchronizes the device).  The denominator of the plain FP32
- * kernel's roofline. */
+ * in all; synchronizes the device).  The bound of the CUDA-core
+ * kernel. */
 FMF_API int fmf_measure_fp32_fma(double *tflops);
 
 /* Accuracy check of the atanh used by the tensor-core form of the per-channel
