@@ -173,12 +173,15 @@ __device__ __forceinline__ RowSplit split_row(const float *row, long long n)
     return r;
 }
 
-__global__ void det_init_kernel(DetState *__restrict__ st, int T, int n_corr,
-                                const int *__restrict__ begin, const int *__restrict__ end)
+// The rows that need more passes, and how far a pass has come.
+struct DetLists {
+    int *select, *n_select;  // rows selecting over key bits
+    int *peaks, *n_peaks;    // rows whose peaks were not gathered by the counting pass
+    unsigned *blocks;        // blocks of a selection pass that are through
+};
+
+__device__ void init_row(DetState *st, int t, int n_corr, const int *begin, const int *end)
 {
-    const int t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= T)
-        return;
     int b = 0, e = n_corr;
     if (begin) {
         b = min(max(begin[t], 0), n_corr);
@@ -461,8 +464,9 @@ __device__ unsigned last_key(unsigned c, F pred)
 constexpr int kPad = 3 * 64 + 16;
 
 __global__ void __launch_bounds__(kDetSampleThreads, 2)
-det_sample_kernel(const float *__restrict__ cc, size_t ld, DetState *__restrict__ st, int mode,
-                  float n_mad, float *__restrict__ saved)
+det_sample_kernel(const float *__restrict__ cc, size_t ld, DetState *st, int mode, float n_mad,
+                  float *__restrict__ saved, int n_corr, const int *__restrict__ lag_begin,
+                  const int *__restrict__ lag_end, const DetLists lists)
 {
     extern __shared__ unsigned long long sample_smem[];
     unsigned *sk = reinterpret_cast<unsigned *>(sample_smem);  // kDetSample keys
@@ -470,6 +474,13 @@ det_sample_kernel(const float *__restrict__ cc, size_t ld, DetState *__restrict_
     __shared__ int pick[4];
     __shared__ unsigned range[4];
     const int t = blockIdx.x;
+    if (threadIdx.x == 0) {
+        if (mode == 0)
+            init_row(st, t, n_corr, lag_begin, lag_end);
+        if (t == 0)
+            *lists.n_select = *lists.n_peaks = 0, *lists.blocks = 0;
+    }
+    __syncthreads();
     const int begin = st[t].begin;
     const long long n = st[t].end - begin;
     if (n <= 0)
@@ -932,14 +943,17 @@ det_count_kernel(const float *__restrict__ cc, size_t ld, DetState *__restrict__
 // median inside [m_lo, m_hi]) and its hot values; for the MAD, the hot values (the
 // superset may miss some, or have overflowed its list).  One warp per row.
 __global__ void det_pick_kernel(DetState *__restrict__ st, const unsigned *__restrict__ bins, int mode, int pcap,
-                                float n_mad)
+                                float n_mad, const DetLists lists)
 {
     const int t = blockIdx.x, lane = threadIdx.x;
-    if (st[t].src != kSrcCand)
-        return;
     DetState s = st[t];
     __syncwarp();
     const long long n = s.end - s.begin;
+    if (s.src != kSrcCand) {
+        if (s.src == kSrcRow && n > 0 && lane == 0)
+            lists.select[atomicAdd(lists.n_select, 1)] = t;
+        return;
+    }
     const long long a = (n - 1) / 2, b = n / 2;
     if (!s.over_k && s.n_lt <= a && b < (long long)s.n_lt + s.n_in) {
         s.rank[0] = (int)(a - s.n_lt);
@@ -1002,8 +1016,11 @@ __global__ void det_pick_kernel(DetState *__restrict__ st, const unsigned *__res
         s.peaks_ready = 0;
     if (!s.peaks_ready)
         s.n_cand = 0;
-    if (lane == 0)
+    if (lane == 0) {
         st[t] = s;
+        if (s.src == kSrcRow || s.src == kSrcKeys)
+            lists.select[atomicAdd(lists.n_select, 1)] = t;
+    }
 }
 
 // The candidates in the middle ranks' bins, into the row's list (a few dozen of a
@@ -1100,26 +1117,60 @@ __device__ __forceinline__ void hist_add(unsigned *h, float v, bool ok, int mode
     }
 }
 
-// The rows that need more passes, compacted into list[0..*count) (one block):
-// kind 0 those selecting over key bits, kind 1 those whose
-// peaks were not gathered by the counting pass (at least 3 lags).
-__global__ void __launch_bounds__(1024)
-det_collect_kernel(const DetState *__restrict__ st, int T, int kind, int *__restrict__ list,
-                   int *__restrict__ count)
+// Picks each rank's bucket from the pass's histogram of row t (one warp),
+// clears the histogram, and after the last pass turns the two keys into the
+// median (mode 0) or the MAD and the threshold (mode 1).
+__device__ void resolve_row(DetState *st, unsigned *hist, int t, int lane, int pass, int mode, float n_mad)
 {
-    __shared__ int n;
-    if (threadIdx.x == 0)
-        n = 0;
-    __syncthreads();
-    for (int t = threadIdx.x; t < T; t += blockDim.x) {
-        const bool need = kind == 0 ? (st[t].src == kSrcRow || st[t].src == kSrcKeys) && st[t].end > st[t].begin
-                                    : !st[t].peaks_ready && st[t].end - st[t].begin >= 3;
-        if (need)
-            list[atomicAdd(&n, 1)] = t;
+    DetState s = st[t];
+    const int n = s.end - s.begin;
+    int shift, width;
+    pass_digit(s.top, pass, shift, width);
+    if (width == 0)
+        return;  // the key was complete after an earlier pass
+    unsigned *gh = hist + (size_t)t * 2 * kDetBins;
+    const int per = kDetBins / 32;  // bins per lane (digits of fewer bits leave the rest empty)
+    const bool two = s.prefix[0] != s.prefix[1];
+    for (int r = 0; r < 2; r++) {
+        const unsigned *h = gh + (two ? r : 0) * kDetBins;
+        unsigned sum = 0;
+        for (int i = 0; i < per; i++)
+            sum += h[lane * per + i];
+        unsigned inc = sum;
+        for (int o = 1; o < 32; o <<= 1) {
+            const unsigned y = __shfl_up_sync(0xffffffffu, inc, o);
+            if (lane >= o)
+                inc += y;
+        }
+        const unsigned exc = inc - sum;
+        const unsigned rk = (unsigned)s.rank[r];
+        const unsigned found = __ballot_sync(0xffffffffu, rk >= exc && rk < inc);
+        const int src = found ? __ffs(found) - 1 : 0;
+        unsigned bin = 0, before = 0;
+        if (lane == src) {
+            unsigned c = exc;
+            int i = 0;
+            for (; i < per - 1; i++) {
+                const unsigned hv = h[lane * per + i];
+                if (rk < c + hv)
+                    break;
+                c += hv;
+            }
+            bin = (unsigned)(lane * per + i);
+            before = c;
+        }
+        bin = __shfl_sync(0xffffffffu, bin, src);
+        before = __shfl_sync(0xffffffffu, before, src);
+        s.prefix[r] |= bin << shift;
+        s.rank[r] = (int)(rk - before);
     }
-    __syncthreads();
-    if (threadIdx.x == 0)
-        *count = n;
+    __syncwarp();
+    for (int i = lane; i < 2 * kDetBins; i += 32)
+        gh[i] = 0u;
+    if (shift == 0)
+        finish_select(s, mode, middle_value(s.prefix[0], s.prefix[1], n), n_mad);
+    if (lane == 0)
+        st[t] = s;
 }
 
 // One selection pass by key bits: histogram of the current digit over the keys whose
@@ -1129,17 +1180,21 @@ det_collect_kernel(const DetState *__restrict__ st, int T, int kind, int *__rest
 // wrote them).  Every block of a fixed grid takes a slice of each such row in turn, so
 // a row that fell back is read at the rate of the whole GPU, not of its own few
 // blocks.  mode 0 keys the values, mode 1 |x - median|; equal digits are aggregated
-// per warp in the first pass over a row (its keys share their high digits).
+// per warp in the first pass over a row (its keys share their high digits).  The block
+// that is through last picks the rows' buckets.
 __global__ void __launch_bounds__(kDetThreads)
-det_hist_row_kernel(const float *__restrict__ cc, size_t ld, const DetState *__restrict__ st,
-                    const int *__restrict__ list, const int *__restrict__ count,
-                    unsigned *__restrict__ hist, const float *__restrict__ cand, long long cap, Lanes g,
-                    int pass, int mode)
+det_hist_row_kernel(const float *__restrict__ cc, size_t ld, DetState *st, const DetLists lists,
+                    unsigned *hist, const float *__restrict__ cand, long long cap, Lanes g, int pass, int mode,
+                    float n_mad)
 {
     __shared__ unsigned h[2 * kDetBins];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     constexpr int kWarps = kDetThreads / 32;
-    const int nrows = *count;
+    __shared__ bool last;
+    const int *const list = lists.select;
+    const int nrows = *lists.n_select;
+    if (nrows == 0)
+        return;  // every block
     for (int k = 0; k < nrows; k++) {
         const int t = list[k];
         const DetState s = st[t];
@@ -1206,67 +1261,18 @@ det_hist_row_kernel(const float *__restrict__ cc, size_t ld, const DetState *__r
         }
         __syncthreads();  // h is cleared for the next row
     }
-}
-
-// Picks each rank's bucket from the pass's histogram (one warp per template),
-// clears the histogram, and after the last pass turns the two keys into the
-// median (mode 0) or the MAD and the threshold (mode 1).
-__global__ void det_resolve_kernel(DetState *__restrict__ st, unsigned *__restrict__ hist, int pass,
-                                   int mode, float n_mad)
-{
-    const int t = blockIdx.x;
-    const int lane = threadIdx.x;
-    DetState s = st[t];
-    const int n = s.end - s.begin;
-    if (n <= 0 || s.src == kSrcDone)
+    __threadfence();
+    __syncthreads();
+    if (threadIdx.x == 0)
+        last = atomicAdd(lists.blocks, 1u) == gridDim.x - 1;
+    __syncthreads();
+    if (!last)
         return;
-    int shift, width;
-    pass_digit(s.top, pass, shift, width);
-    if (width == 0)
-        return;  // the key was complete after an earlier pass
-    unsigned *gh = hist + (size_t)t * 2 * kDetBins;
-    const int per = kDetBins / 32;  // bins per lane (digits of fewer bits leave the rest empty)
-    const bool two = s.prefix[0] != s.prefix[1];
-    for (int r = 0; r < 2; r++) {
-        const unsigned *h = gh + (two ? r : 0) * kDetBins;
-        unsigned sum = 0;
-        for (int i = 0; i < per; i++)
-            sum += h[lane * per + i];
-        unsigned inc = sum;
-        for (int o = 1; o < 32; o <<= 1) {
-            const unsigned y = __shfl_up_sync(0xffffffffu, inc, o);
-            if (lane >= o)
-                inc += y;
-        }
-        const unsigned exc = inc - sum;
-        const unsigned rk = (unsigned)s.rank[r];
-        const unsigned found = __ballot_sync(0xffffffffu, rk >= exc && rk < inc);
-        const int src = found ? __ffs(found) - 1 : 0;
-        unsigned bin = 0, before = 0;
-        if (lane == src) {
-            unsigned c = exc;
-            int i = 0;
-            for (; i < per - 1; i++) {
-                const unsigned hv = h[lane * per + i];
-                if (rk < c + hv)
-                    break;
-                c += hv;
-            }
-            bin = (unsigned)(lane * per + i);
-            before = c;
-        }
-        bin = __shfl_sync(0xffffffffu, bin, src);
-        before = __shfl_sync(0xffffffffu, before, src);
-        s.prefix[r] |= bin << shift;
-        s.rank[r] = (int)(rk - before);
-    }
-    __syncwarp();
-    for (int i = lane; i < 2 * kDetBins; i += 32)
-        gh[i] = 0u;
-    if (shift == 0)
-        finish_select(s, mode, middle_value(s.prefix[0], s.prefix[1], n), n_mad);
-    if (lane == 0)
-        st[t] = s;
+    __threadfence();
+    for (int k = warp; k < nrows; k += kWarps)
+        resolve_row(st, hist, list[k], lane, pass, mode, n_mad);
+    if (threadIdx.x == 0)
+        *lists.blocks = 0;  // for the next pass
 }
 
 // The local maxima among a row's hot values (at or above thr_lo), one block
@@ -1275,12 +1281,15 @@ __global__ void det_resolve_kernel(DetState *__restrict__ st, unsigned *__restri
 // the list hands the row to det_peaks_kernel (exact threshold).
 __global__ void __launch_bounds__(kDetThreads)
 det_hot_kernel(const float *__restrict__ cc, size_t ld, DetState *__restrict__ st,
-               const int *__restrict__ hot, int hcap, int2 *__restrict__ cand, int cap)
+               const int *__restrict__ hot, int hcap, int2 *__restrict__ cand, int cap, const DetLists lists)
 {
     const int t = blockIdx.x;
-    if (!st[t].peaks_ready)
-        return;  // uniform over the block
     const long long b = st[t].begin, e = st[t].end;
+    if (!st[t].peaks_ready) {  // uniform over the block
+        if (threadIdx.x == 0 && e - b >= 3)
+            lists.peaks[atomicAdd(lists.n_peaks, 1)] = t;
+        return;
+    }
     const float thr_lo = st[t].thr_lo;
     const float *row = cc + (size_t)t * ld;
     const int n = min(st[t].n_hot, hcap);
@@ -1292,6 +1301,7 @@ det_hot_kernel(const float *__restrict__ cc, size_t ld, DetState *__restrict__ s
     if (threadIdx.x == 0 && st[t].n_cand > cap) {
         st[t].peaks_ready = 0;
         st[t].n_cand = 0;
+        lists.peaks[atomicAdd(lists.n_peaks, 1)] = t;  // (at least 3 lags: it has peaks)
     }
 }
 
@@ -1521,7 +1531,7 @@ int detect_device(const float *cc, int T, int n_corr, size_t ld, const int *begi
         (rc = ws.get(&col_cnt, 2 * ((size_t)kDetBlocks + chunk) * kDetThreads, "list column counts")) ||
         (rc = ws.get(&bins, (size_t)chunk * kCandBins, "candidate bins")) ||
         (rc = ws.get(&list, (size_t)chunk * kPickCap, "picked candidates")) ||
-        (rc = ws.get(&row_list, (size_t)chunk + 1, "rows of whole-row passes")))
+        (rc = ws.get(&row_list, 2 * (size_t)chunk + 3, "rows of further passes")))
         return rc;
     cudaError_t e = cudaFuncSetAttribute(det_select_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          (int)select_smem(kDetCap));
@@ -1557,35 +1567,31 @@ int detect_device(const float *cc, int T, int n_corr, size_t ld, const int *begi
         const dim3 pick_grid((unsigned)std::min(per_row, ((long long)kDetPickBlocks + nt - 1) / nt), (unsigned)nt);
         g.cnt_k = col_cnt;
         g.cnt_a = col_cnt + ((size_t)kDetBlocks + chunk) * kDetThreads;
-        det_init_kernel<<<(nt + 127) / 128, 128, 0, s>>>(st, nt, n_corr, begin ? begin + t0 : nullptr,
-                                                         end ? end + t0 : nullptr);
-        int *const rcount = row_list + chunk;
+        const DetLists lists{row_list, row_list + 2 * chunk, row_list + chunk, row_list + 2 * chunk + 1,
+                             reinterpret_cast<unsigned *>(row_list + 2 * chunk + 2)};
         // mode 0, the median: sample, the one read of the rows, selection over the candidates;
         // mode 1, the MAD: the sample about the exact median, the listed values, selection
         for (int mode = 0; mode < 2; mode++) {
-            det_sample_kernel<<<nt, kDetSampleThreads, kDetSample * sizeof(unsigned), s>>>(rows, ld, st, mode, n_mad, saved);
+            det_sample_kernel<<<nt, kDetSampleThreads, kDetSample * sizeof(unsigned), s>>>(
+                rows, ld, st, mode, n_mad, saved, n_corr, begin ? begin + t0 : nullptr, end ? end + t0 : nullptr, lists);
             if ((e = cudaMemsetAsync(bins, 0, (size_t)nt * kCandBins * sizeof(unsigned), s)) != cudaSuccess)
                 return set_error(FMF_ERR_CUDA, "clearing the candidate bins: %s", cudaGetErrorString(e));
             (mode ? det_count_kernel<false> : det_count_kernel<true>)<<<grid, kDetThreads, kCountSmem, s>>>(
                 rows, ld, st, keys, key_cap, amb, amb_cap, g, bins, hot, kDetCap);
-            det_pick_kernel<<<nt, 32, 0, s>>>(st, bins, mode, kDetCap, n_mad);
+            det_pick_kernel<<<nt, 32, 0, s>>>(st, bins, mode, kDetCap, n_mad, lists);
             det_gather_kernel<<<pick_grid, kDetThreads, 0, s>>>(st, keys, key_cap, g, list);
             det_finish_kernel<<<nt, kDetThreads, 0, s>>>(st, list, mode, n_mad);
-            det_collect_kernel<<<1, 1024, 0, s>>>(st, nt, 0, row_list, rcount);
-            for (int pass = 0; pass < 3; pass++) {
-                det_hist_row_kernel<<<kDetRowBlocks, kDetThreads, 0, s>>>(rows, ld, st, row_list, rcount, hist, keys,
-                                                                          key_cap, g, pass, mode);
-                det_resolve_kernel<<<nt, 32, 0, s>>>(st, hist, pass, mode, n_mad);
-            }
+            for (int pass = 0; pass < 3; pass++)
+                det_hist_row_kernel<<<kDetRowBlocks, kDetThreads, 0, s>>>(rows, ld, st, lists, hist, keys, key_cap, g,
+                                                                          pass, mode, n_mad);
         }
-        det_hot_kernel<<<nt, kDetThreads, 0, s>>>(rows, ld, st, hot, kDetCap, cand, kDetCap);
-        det_collect_kernel<<<1, 1024, 0, s>>>(st, nt, 1, row_list, rcount);
-        det_peaks_kernel<<<kDetRowBlocks, kDetThreads, 0, s>>>(rows, ld, st, row_list, rcount, cand, kDetCap);
+        det_hot_kernel<<<nt, kDetThreads, 0, s>>>(rows, ld, st, hot, kDetCap, cand, kDetCap, lists);
+        det_peaks_kernel<<<kDetRowBlocks, kDetThreads, 0, s>>>(rows, ld, st, lists.peaks, lists.n_peaks, cand, kDetCap);
         det_select_kernel<<<nt, kDetSelectThreads, select_smem(kDetCap), s>>>(
             st, cand, kDetCap, min_sep, max_det, med_out ? med_out + t0 : nullptr,
             mad_out ? mad_out + t0 : nullptr, thr_out ? thr_out + t0 : nullptr, count_out + t0,
             lag_out + (size_t)t0 * max_det, val_out + (size_t)t0 * max_det);
-        count_launch(29);
+        count_launch(19);
         if ((rc = check_launch("detection kernels")))
             return rc;
     }
