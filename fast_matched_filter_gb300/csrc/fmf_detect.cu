@@ -68,7 +68,9 @@ namespace {
 
 constexpr int kDetBins = 2048;            // histogram bins of the 11-bit passes
 constexpr int kDetThreads = 256;          // histogram / peak kernels
-constexpr int kDetSampleThreads = 512;    // two sample blocks per SM
+// Threads of a sample block: 1,024 for few rows; 512, two blocks per SM, for more (500
+// rows: 0.48 ms with one block of 1,024 per SM, 0.32 ms).
+constexpr int kDetFewRows = 152;
 constexpr int kDetSelectThreads = 1024;   // per-template filter kernel
 constexpr int kDetChunk = 1024;           // templates per round of scratch
 constexpr int kDetCap = 16384;            // candidate peaks per template row
@@ -255,7 +257,7 @@ __device__ void find_rank(const unsigned *h, unsigned rk, int lane, int *pick)
     const int per = kDetBins / 32;
     unsigned sum = 0;
     for (int i = 0; i < per; i++)
-        sum += h[lane * per + i];
+        sum += h[lane * per + ((i + lane) & (per - 1))];  // each lane in a bank of its own
     unsigned inc = sum;
     for (int o = 1; o < 32; o <<= 1) {
         const unsigned y = __shfl_up_sync(0xffffffffu, inc, o);
@@ -463,7 +465,8 @@ __device__ unsigned last_key(unsigned c, F pred)
 // over the whole row, a few reads of it at the rate of the whole GPU
 constexpr int kPad = 3 * 64 + 16;
 
-__global__ void __launch_bounds__(kDetSampleThreads, 2)
+template <int THREADS>
+__global__ void __launch_bounds__(THREADS, 1024 / THREADS)
 det_sample_kernel(const float *__restrict__ cc, size_t ld, DetState *st, int mode, float n_mad,
                   float *__restrict__ saved, int n_corr, const int *__restrict__ lag_begin,
                   const int *__restrict__ lag_end, const DetLists lists)
@@ -518,11 +521,11 @@ det_sample_kernel(const float *__restrict__ cc, size_t ld, DetState *st, int mod
     // in flight together)
     const unsigned long long stepq = ((unsigned long long)n << 20) / (unsigned long long)m;
     constexpr int kPer = 16;
-    for (int i0 = threadIdx.x; i0 < m; i0 += kPer * kDetSampleThreads) {
+    for (int i0 = threadIdx.x; i0 < m; i0 += kPer * THREADS) {
         float v[kPer];
 #pragma unroll
         for (int j = 0; j < kPer; j++) {
-            const int i = i0 + j * kDetSampleThreads;
+            const int i = i0 + j * THREADS;
             v[j] = 0.0f;
             if (i < m) {
                 if (mode == 0) {
@@ -535,7 +538,7 @@ det_sample_kernel(const float *__restrict__ cc, size_t ld, DetState *st, int mod
         }
 #pragma unroll
         for (int j = 0; j < kPer; j++) {
-            const int i = i0 + j * kDetSampleThreads;
+            const int i = i0 + j * THREADS;
             if (i < m) {
                 if (mode == 0)
                     sv[i] = v[j];
@@ -1536,7 +1539,10 @@ int detect_device(const float *cc, int T, int n_corr, size_t ld, const int *begi
     cudaError_t e = cudaFuncSetAttribute(det_select_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          (int)select_smem(kDetCap));
     if (e == cudaSuccess)
-        e = cudaFuncSetAttribute(det_sample_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+        e = cudaFuncSetAttribute(det_sample_kernel<512>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 (int)(kDetSample * sizeof(unsigned)));
+    if (e == cudaSuccess)
+        e = cudaFuncSetAttribute(det_sample_kernel<1024>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  (int)(kDetSample * sizeof(unsigned)));
     if (e == cudaSuccess)
         e = cudaFuncSetAttribute(det_count_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kCountSmem);
@@ -1567,12 +1573,13 @@ int detect_device(const float *cc, int T, int n_corr, size_t ld, const int *begi
         const dim3 pick_grid((unsigned)std::min(per_row, ((long long)kDetPickBlocks + nt - 1) / nt), (unsigned)nt);
         g.cnt_k = col_cnt;
         g.cnt_a = col_cnt + ((size_t)kDetBlocks + chunk) * kDetThreads;
+        const bool few = nt <= kDetFewRows;
         const DetLists lists{row_list, row_list + 2 * chunk, row_list + chunk, row_list + 2 * chunk + 1,
                              reinterpret_cast<unsigned *>(row_list + 2 * chunk + 2)};
         // mode 0, the median: sample, the one read of the rows, selection over the candidates;
         // mode 1, the MAD: the sample about the exact median, the listed values, selection
         for (int mode = 0; mode < 2; mode++) {
-            det_sample_kernel<<<nt, kDetSampleThreads, kDetSample * sizeof(unsigned), s>>>(
+            (few ? det_sample_kernel<1024> : det_sample_kernel<512>)<<<nt, few ? 1024 : 512, kDetSample * sizeof(unsigned), s>>>(
                 rows, ld, st, mode, n_mad, saved, n_corr, begin ? begin + t0 : nullptr, end ? end + t0 : nullptr, lists);
             if ((e = cudaMemsetAsync(bins, 0, (size_t)nt * kCandBins * sizeof(unsigned), s)) != cudaSuccess)
                 return set_error(FMF_ERR_CUDA, "clearing the candidate bins: %s", cudaGetErrorString(e));
