@@ -398,8 +398,10 @@ int prepare_problem(const Args &a, Scratch &ws, cudaStream_t s, Problem *Pout, i
     }
     unsigned *list = nullptr;
     if (const size_t words = window_list_words(N, SC))
-        if ((rc = ws.get(&list, words, "window statistics")))
-            return rc;
+        if (ws.get(&list, words, "window statistics")) {  // no memory: without it, as small searches
+            clear_error();
+            list = nullptr;
+        }
     unsigned *dc = nullptr;
     if (full && a.precision == FMF_PREC_AUTO)
         if ((rc = ws.get(&dc, (size_t)SC, "precision estimate")) ||
@@ -576,12 +578,12 @@ struct Search {
         }
     }
     TcSearch *search() { return reinterpret_cast<TcSearch *>(tc.data()); }
-    int run(int t0, int nt, Scratch &ws, cudaStream_t s)
+    int run(int t0, int nt, cudaStream_t s)
     {
         int rc;
         Problem Q = problem_subset(P, t0, nt);
         if (!tc.empty()) {
-            if ((rc = tc_run_templates(search(), t0, nt, err, ws, s)) || !fp32)
+            if ((rc = tc_run_templates(search(), t0, nt, err, s)) || !fp32)
                 return rc;
             Q.only_if = tc_flag(search());
         } else if ((rc = clear_outputs(Q, s))) {
@@ -609,7 +611,7 @@ static int run_device_ws(const Args &a, cudaStream_t s, Scratch &ws, Problem *Po
     set_last_precision(precision);
     cudaEvent_t ev_main0 = mark(s);
     Search f(P, precision, tiles, a.flags, P.T, ws, s);
-    rc = f.status ? f.status : f.run(0, P.T, ws, s);
+    rc = f.status ? f.status : f.run(0, P.T, s);
     span(ev_main0, mark(s), kSpanKernel);
     return rc;
 }
@@ -690,7 +692,7 @@ static int run_streamed(const Args &d, float *host_out, HostPages &pages, cudaSt
         for (int c = 0; c < n_chunks && rc == FMF_OK && e == cudaSuccess; c++, launched++) {
             const int t0 = bounds[c], nt = bounds[c + 1] - bounds[c];
             if (nt > 0) {
-                rc = search.run(t0, nt, ws, s);
+                rc = search.run(t0, nt, s);
                 if (!rc && zc)
                     rc = launch_zero_count(d, P.out, t0, nt, zc, s);
             }

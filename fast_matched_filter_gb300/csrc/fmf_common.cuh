@@ -296,7 +296,7 @@ inline int tc_pad(int nb) { return nb ? 128 * nb + 16 : 0; }  // statistics padd
 size_t tc_search_size();
 int tc_begin(const Problem &P, int form, int nb, int tg, int max_templates, Scratch &ws, cudaStream_t s,
              TcSearch *out, bool turn = true);
-int tc_run_templates(TcSearch *full, int t0, int nt, unsigned *err, Scratch &ws, cudaStream_t s);
+int tc_run_templates(TcSearch *full, int t0, int nt, unsigned *err, cudaStream_t s);
 const unsigned *tc_flag(const TcSearch *full);
 size_t tc_prob_size();
 size_t tc_template_bytes(const Problem &P, int nb);  // operand blocks of all templates

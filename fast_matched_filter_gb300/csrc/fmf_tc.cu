@@ -1342,10 +1342,10 @@ static int tc_run_n(const TcProb *probs, int n, int form, int parts, unsigned lo
     const bool var = P0.ntap != nullptr, full = P0.normalize != 0, nsum = P0.network_sum != 0;
     Scratch pws(s);
     float *part_out = nullptr;
-    if (parts > 1 && nsum) {
-        int rc = pws.get(&part_out, (size_t)parts * P0.T * P0.n_corr, "channel-part sums");
-        if (rc)
-            return rc;
+    if (parts > 1 && nsum && pws.get(&part_out, (size_t)parts * P0.T * P0.n_corr, "channel-part sums")) {
+        set_error(FMF_OK, "");  // no memory: in one part
+        part_out = nullptr;
+        parts = 1;
     }
     B.split = form != TC_FORM_BF16;  // operand pairs
     B.mma_types = form == TC_FORM_FP32 ? 0u : (1u << 7) | (1u << 10);
@@ -1442,6 +1442,7 @@ struct TcSearch {
     int form, room, parts;
     TcDataWork data;
     bool data_due;   // the data streams are made with the first templates
+    unsigned long long *queue;
     uint16_t *w;
     size_t w_elems;  // of one half, all room templates
 };
@@ -1533,7 +1534,8 @@ int tc_begin(const Problem &P, int form, int nb, int tg, int max_templates, Scra
     int *exps = nullptr;
     if ((rc = ws.get(&g_hi, halves * g_elems, "tensor-core data streams")) ||
         (rc = ws.get(&out->w, halves * out->w_elems, "tensor-core template blocks")) ||
-        (fp32 && (rc = ws.get(&exps, n_rows + SC, "operand exponents"))))
+        (fp32 && (rc = ws.get(&exps, n_rows + SC, "operand exponents"))) ||
+        (rc = ws.get(&out->queue, 1, "tile queue")))
         return rc;
     if (turned && ws.get(&pr.P.by_channel, room * turned, "per-channel outputs")) {
         set_error(FMF_OK, "");  // no room for them: written in place
@@ -1605,17 +1607,16 @@ static int tc_templates(TcSearch *full, int t0, int nt, unsigned long long *queu
 // those of all its templates, so that its results do not depend on how they are
 // parted (a call with host arrays runs them in parts); the bf16 forms choose them
 // for each launch, which keeps the SMs busier through the last few templates.
-int tc_run_templates(TcSearch *full, int t0, int nt, unsigned *err, Scratch &ws, cudaStream_t s)
+int tc_run_templates(TcSearch *full, int t0, int nt, unsigned *err, cudaStream_t s)
 {
     int rc;
     for (int a = t0; a < t0 + nt; a += full->room) {
         const int n = t0 + nt - a < full->room ? t0 + nt - a : full->room;
         TcProb sub;
-        unsigned long long *queue = nullptr;
-        if ((rc = ws.get(&queue, 1, "tile queue")) || (rc = tc_templates(full, a, n, queue, s, &sub)) ||
+        if ((rc = tc_templates(full, a, n, full->queue, s, &sub)) ||
             (!sub.P.by_channel && (rc = clear_outputs(sub.P, s))) ||
-            (rc = tc_run(&sub, 1, full->form, full->form == TC_FORM_FP32 ? full->parts : tc_choose_parts(&sub), queue,
-                         err, s)) ||
+            (rc = tc_run(&sub, 1, full->form, full->form == TC_FORM_FP32 ? full->parts : tc_choose_parts(&sub),
+                         full->queue, err, s)) ||
             (sub.P.by_channel && (rc = launch_channel_outputs(sub.P, sub.skip, s))))
             return rc;
     }

@@ -719,7 +719,7 @@ static int variable_device(const VArgs &a, int L, cudaStream_t s, float *host_ou
         const int t0 = bounds[c], nt = bounds[c + 1] - bounds[c];
         if (nt > 0) {
             if (!tc.empty() &&
-                (rc = tc_run_templates(reinterpret_cast<TcSearch *>(tc.data()), t0, nt, err, ws, s)))
+                (rc = tc_run_templates(reinterpret_cast<TcSearch *>(tc.data()), t0, nt, err, s)))
                 return rc;
             if (fp32) {  // after the tensor cores: only if the search's flag says so
                 if ((rc = launch_plain_all(var_subset(P, t0, nt), s)))
