@@ -887,14 +887,35 @@ det_count_kernel(const float *__restrict__ cc, size_t ld, DetState *__restrict__
         // this thread's own column of undecided values
         const int m = min(g.cnt_a[col], g.Ca);
         const int mw = __reduce_max_sync(0xffffffffu, m);
-        for (int k = 0; k < mw; k += 8) {
-            float x[8] = {};
-            if (k < m)
-                load_sector(ac, k, x);
+        float next[16] = {};  // two sectors in flight while two are counted
+        const auto load2 = [&](int k) {
+            float a[8], b[8];
+            if (k < m) {
+                load_sector(ac, k, a);
 #pragma unroll
-            for (int j = 0; j < 8; j++)
+                for (int j = 0; j < 8; j++)
+                    next[j] = a[j];
+            }
+            if (k + 8 < m) {
+                load_sector(ac, k + 8, b);
+#pragma unroll
+                for (int j = 0; j < 8; j++)
+                    next[8 + j] = b[j];
+            }
+        };
+        load2(0);
+        for (int k = 0; k < mw; k += 16) {
+            float x[16];
+#pragma unroll
+            for (int j = 0; j < 16; j++)
+                x[j] = next[j];
+            load2(k + 16);
+#pragma unroll
+            for (int j = 0; j < 16; j++) {
                 take(k + j < m ? dev(x[j], med) : none);
-            step_done(false);
+                if (j % 8 == 7)
+                    step_done(false);
+            }
         }
     }
     step_done(true);
@@ -1044,16 +1065,23 @@ det_gather_kernel(DetState *__restrict__ st, const float *__restrict__ cand, lon
         const size_t col = ((size_t)t * g.S + blk) * kDetThreads + threadIdx.x;
         const float *kc = cand + (size_t)t * cap + ((size_t)blk * kWarps + warp) * (size_t)g.Ck * 32 + 8 * lane;
         const int m = g.cnt_k[col];  // <= Ck: no column overflowed
-        for (int k = 0; k < m; k += 8) {
-            float x[8];
-            load_sector(kc, k, x);
+        constexpr int kSectors = 3;  // in flight: a column holds some 20 entries
+        for (int k0 = 0; k0 < m; k0 += 8 * kSectors) {
+            float x[kSectors][8];
 #pragma unroll
-            for (int j = 0; j < 8; j++) {
-                const int b = value_bin<kCandBins>(x[j], lo, scale);
-                if (k + j < m && b >= bin0 && b <= bin1) {  // (the bins between them are empty)
+            for (int q = 0; q < kSectors; q++)
+                if (k0 + 8 * q < m)
+                    load_sector(kc, k0 + 8 * q, x[q]);
+#pragma unroll
+            for (int i = 0; i < 8 * kSectors; i++) {
+                if (k0 + i >= m)
+                    break;
+                const float v = x[i / 8][i % 8];
+                const int b = value_bin<kCandBins>(v, lo, scale);
+                if (b >= bin0 && b <= bin1) {  // (the bins between them are empty)
                     const int at = atomicAdd(&st[t].n_list, 1);
                     if (at < kPickCap)
-                        list[(size_t)t * kPickCap + at] = order_key(__fadd_rn(x[j], 0.0f));
+                        list[(size_t)t * kPickCap + at] = order_key(__fadd_rn(v, 0.0f));
                 }
             }
         }
