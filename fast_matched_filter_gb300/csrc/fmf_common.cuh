@@ -58,7 +58,8 @@ struct Problem {
     // (tanh(x / vp_norm[t]) + vp_bias[t]) * vp_scale[t] for every output x
     const float *vp_norm, *vp_bias, *vp_scale;
     // FP32 on the tensor cores, else null: the channel scan of prepare_problem
-    // [3 SC + 1]: the largest |x| of each data channel; its smallest window energy
+    // [3 SC + 1]: the largest |x| of each data channel (the largest finite one with a
+    // common length); its smallest window energy
     // that can pass the threshold (bits complemented, so that zero means none); the
     // largest template energy on it; the search's flag: the scan or the operands
     // left it to the CUDA-core kernel

@@ -112,8 +112,10 @@ __device__ __forceinline__ int max_exponent(unsigned bits, bool &ok)
 
 __device__ __forceinline__ bool finite_bits(unsigned abs_bits) { return abs_bits < 0x7f800000u; }
 
-// x / s as the pair (h, l); x that is not finite becomes 0: every window that
-// holds it has a NaN energy, and its coefficient is 0 in both kernels.
+// x / s as the pair (h, l); x that is not finite becomes 0.  With a common length every
+// window that holds it has a NaN energy, and its coefficient is 0 in both kernels;
+// with per-channel lengths, whose energies are integers, such a channel raises the
+// search's flag.
 __device__ __forceinline__ void split_fp16(float x, float inv_s, uint16_t &hi, uint16_t &lo)
 {
     const float y = finite_bits(__float_as_uint(x) & 0x7fffffffu) ? x * inv_s : 0.0f;
@@ -178,10 +180,11 @@ struct StatSlot {
     __host__ __device__ constexpr int align() const { return 16 / elem - 1; }  // mask of elements
 };
 
-// The same as a bf16 pair in the data's own units: l is bf16(x - h).
-__device__ __forceinline__ void split_bf16(float x, uint16_t &hi, uint16_t &lo)
+// The same as a bf16 pair in the data's own units: l is bf16(x - h).  keep: x that is not
+// finite stays so.
+__device__ __forceinline__ void split_bf16(float x, bool keep, uint16_t &hi, uint16_t &lo)
 {
-    const float y = finite_bits(__float_as_uint(x) & 0x7fffffffu) ? x : 0.0f;
+    const float y = keep || finite_bits(__float_as_uint(x) & 0x7fffffffu) ? x : 0.0f;
     const __nv_bfloat16 h = __float2bfloat16_rn(y);
     const __nv_bfloat16 l = __float2bfloat16_rn(y - __bfloat162float(h));
     hi = __bfloat16_as_ushort(h);
@@ -189,12 +192,12 @@ __device__ __forceinline__ void split_bf16(float x, uint16_t &hi, uint16_t &lo)
 }
 
 template <bool FP32>
-__device__ __forceinline__ void split_pair(float x, float inv_s, uint16_t &hi, uint16_t &lo)
+__device__ __forceinline__ void split_pair(float x, float inv_s, bool keep, uint16_t &hi, uint16_t &lo)
 {
     if constexpr (FP32)
         split_fp16(x, inv_s, hi, lo);
     else
-        split_bf16(x, hi, lo);
+        split_bf16(x, keep, hi, lo);
 }
 
 // ------------------------------------------------------------------ operands
@@ -247,6 +250,9 @@ struct TcDataWork {
     uint16_t *g_hi, *g_lo;
     int *d_exp;
     unsigned *skip;
+    // bf16 forms: samples that are not finite stay so, and with them the numerators of the
+    // windows round them ('short' with per-channel lengths: no energy tells of them)
+    bool keep;
 };
 
 template <bool FP32>
@@ -283,7 +289,7 @@ __device__ __forceinline__ void tc_data_block(const TcDataWork &d, int block, ui
                 const int at = one ? (i >> 7) * TC_TURN_PITCH + (i & (TC_Q - 1))
                                    : (psi * rows + (q >> 7)) * TC_TURN_PITCH + (q & (TC_Q - 1));
                 uint16_t h, l;
-                split_pair<FP32>(x[j], inv_s, h, l);
+                split_pair<FP32>(x[j], inv_s, d.keep, h, l);
                 hi[at] = h;
                 if (g_lo)
                     lo[at] = l;
@@ -318,7 +324,7 @@ template <bool FP32>
 __global__ void tc_data_sparse_kernel(const float *__restrict__ data, int N, int SC, int step, int rows_total,
                                       int row_front, const unsigned *__restrict__ stat,
                                       uint16_t *__restrict__ g_hi, uint16_t *__restrict__ g_lo,
-                                      int *__restrict__ d_exp, unsigned *skip)
+                                      int *__restrict__ d_exp, unsigned *skip, bool keep)
 {
     const long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     const long long per_ch = (long long)step * TC_CB * rows_total;
@@ -340,7 +346,7 @@ __global__ void tc_data_sparse_kernel(const float *__restrict__ data, int N, int
     for (int i = 0; i < 8; i++) {
         const long long pos = (long long)step * (x0 + i) + psi;
         const float v = (x0 + i >= 0 && pos < N) ? src[pos] : 0.0f;
-        split_pair<FP32>(v, inv_s, h[i], l[i]);
+        split_pair<FP32>(v, inv_s, keep, h[i], l[i]);
     }
     reinterpret_cast<uint4 *>(g_hi)[idx] = pack8(h);
     if (g_lo)
@@ -421,7 +427,7 @@ __device__ __forceinline__ void tc_template_block(const TcTemplateWork &w, long 
 #pragma unroll
         for (int c = 0; c < 8; c++) {
             const int q = q0 + c, j = step * q + phi;
-            split_pair<FP32>(q >= 0 && j < L ? taps[j] : 0.0f, inv_s, h[c], l[c]);
+            split_pair<FP32>(q >= 0 && j < L ? taps[j] : 0.0f, inv_s, false, h[c], l[c]);
         }
         const long long o = row * step * per_phase + i;
         reinterpret_cast<uint4 *>(w_hi)[o] = pack8(h);
@@ -1558,7 +1564,7 @@ int tc_begin(const Problem &P, int form, int nb, int tg, int max_templates, Scra
     pr.chain_cols = fp32 ? (kChain / most > 1 ? kChain / most : 1) : step * (TC_CB / 2);
     TcDataWork &d = out->data;
     d = TcDataWork{P.data, P.N, SC, step, 0, pr.rows_total, pr.row_front, fp32 ? P.scan : nullptr, g_hi, g_lo,
-                   fp32 ? exps + n_rows : nullptr, fp32 ? P.scan + 3 * SC : nullptr};
+                   fp32 ? exps + n_rows : nullptr, fp32 ? P.scan + 3 * SC : nullptr, P.ntap && P.normalize == 0};
     const int rows = tc_turn_rows(step);
     d.tiles = (pr.rows_total + rows - 1) / rows;
     out->data_due = step <= TC_TURN_STEP && (long long)d.tiles * SC < (1ll << 30);
@@ -1567,7 +1573,7 @@ int tc_begin(const Problem &P, int form, int nb, int tg, int max_templates, Scra
     const long long n = (long long)SC * step * TC_CB * pr.rows_total;
     auto kern = fp32 ? tc_data_sparse_kernel<true> : tc_data_sparse_kernel<false>;
     kern<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(P.data, P.N, SC, step, pr.rows_total, pr.row_front, d.stat,
-                                                     g_hi, g_lo, d.d_exp, d.skip);
+                                                     g_hi, g_lo, d.d_exp, d.skip, d.keep);
     count_launch();
     return check_launch("tensor-core data streams");
 }

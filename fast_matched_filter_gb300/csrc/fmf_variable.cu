@@ -223,13 +223,11 @@ __global__ void channel_energy_kernel(const float *__restrict__ data, int N, con
         const float sq = x[e] * x[e];
         pair_add(h, l, sq, fmaf(x[e], x[e], -sq));
     }
-    if (scan) {  // Problem::scan: the channel's largest finite |d|
+    if (scan) {  // Problem::scan: the channel's largest |d|; a value that is not finite above all
         unsigned top = 0;
 #pragma unroll
-        for (int e = 0; e < per; e++) {
-            const unsigned a = __float_as_uint(x[e]) & 0x7fffffffu;
-            top = a < 0x7f800000u ? max(top, a) : top;
-        }
+        for (int e = 0; e < per; e++)
+            top = max(top, __float_as_uint(x[e]) & 0x7fffffffu);
         top = __reduce_max_sync(0xffffffffu, top);
         if ((threadIdx.x & 31) == 0)
             tops[threadIdx.x >> 5] = top;
