@@ -356,8 +356,9 @@ __global__ void tc_data_sparse_kernel(const float *__restrict__ data, int N, int
 // W[t][ch][phi][n][e][c] = pair of tphi[8n + e + c - (Q-1+s)], tphi[q] = tpl[step*q + phi],
 // s = mu mod Q, mu = floor((mo + phi) / step); one block per (template,
 // channel), its taps in shared memory (read once, written 8 times over).
-// FP32: also the channel's exponent.  queue: the tile queue of the persistent launch
-// that follows, cleared here (a memset costs 2 us).
+// FP32: also the channel's exponent, and the search's flag where a tap is not finite; the
+// bf16 forms keep such a tap.  queue: the tile queue of the persistent launch that
+// follows, cleared here (a memset costs 2 us).
 struct TcTemplateWork {
     const float *tpl;
     const int *mo;
@@ -427,7 +428,7 @@ __device__ __forceinline__ void tc_template_block(const TcTemplateWork &w, long 
 #pragma unroll
         for (int c = 0; c < 8; c++) {
             const int q = q0 + c, j = step * q + phi;
-            split_pair<FP32>(q >= 0 && j < L ? taps[j] : 0.0f, inv_s, false, h[c], l[c]);
+            split_pair<FP32>(q >= 0 && j < L ? taps[j] : 0.0f, inv_s, true, h[c], l[c]);
         }
         const long long o = row * step * per_phase + i;
         reinterpret_cast<uint4 *>(w_hi)[o] = pack8(h);

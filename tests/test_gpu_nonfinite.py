@@ -38,3 +38,26 @@ def test_sample_of_a_search_with_per_channel_lengths(monkeypatch, step, bad):
         assert np.isnan(got[holds]).all()
         far = (first > at + 300 * step) | (first + n[:, 1, 0][:, None] < at - 300 * step)
         assert np.isfinite(got[far]).all()
+
+
+@pytest.mark.parametrize("bad", [np.nan, np.inf, -np.inf])
+@pytest.mark.parametrize("normalize", ["short", "full"])
+@pytest.mark.parametrize("given", [True, False])
+def test_template_that_is_not_finite(monkeypatch, normalize, bad, given):
+    """given: with the energies of the templates as they were before."""
+    torch = pytest.importorskip("torch")
+    tp, mo, w, d = random_search(5, 2, 2, 1, 60, 6000, 0, 50)
+    sst = np.sum(tp ** 2, axis=-1) if given else None
+    tp[1, 0, 0, 7] = bad
+    if not given:
+        sst = np.sum(tp ** 2, axis=-1)
+    monkeypatch.setenv("FMF_TC32", "0")
+    dev = [torch.from_numpy(np.ascontiguousarray(x, x.dtype)).cuda() for x in (tp, sst, mo, w, d)]
+    outs = []
+    for precision in ("fp32", "split_bf16", "bf16"):
+        out = torch.empty((2, 5941, 2, 1), device="cuda")
+        fmf.matched_filter_device(*dev, 1, out, normalize, False, precision)
+        outs.append(out.cpu().numpy())
+    assert given <= (not np.isfinite(outs[0]).all())
+    for got in outs[1:]:
+        assert np.array_equal(np.isfinite(got), np.isfinite(outs[0]))
