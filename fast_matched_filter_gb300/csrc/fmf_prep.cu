@@ -60,45 +60,49 @@ __device__ __forceinline__ double block_sum_f64(double v, double *red)
 // per row walked the whole row: 7.6 us for rows of 100 values, against 3 us.)
 constexpr int kEnergyLeaves = 256;  // blocks of one round; a block has at least 57 values
 
-// numpy's recursion over n values as a walk: the leaves in order, and after each
-// how many finished pairs to add (bits of its path).  Calls f(offset, length, adds).
-template <class F>
-__device__ __forceinline__ void pairwise_walk(int n, F f)
-{
+// numpy's recursion over n values as a walk: the leaves in order, and after each how many
+// finished pairs to add (bits of its path).
+struct PairwiseWalk {
     int off[32], len[32];
     bool right[32];  // frame's left half is done
-    int sp = 0;
-    off[0] = 0;
-    len[0] = n;
-    right[0] = false;
-    while (sp >= 0) {
-        if (len[sp] <= 128) {
-            int o = off[sp], m = len[sp], adds = 0;
-            sp--;
-            while (sp >= 0 && right[sp]) {  // this leaf ends the frame's right half
-                adds++;
-                sp--;
-            }
-            f(o, m, adds);
-            if (sp >= 0) {  // the frame's left half is done: its right half
-                right[sp] = true;
-                int m2 = len[sp] / 2;
-                m2 -= m2 % 8;
-                off[sp + 1] = off[sp] + m2;
-                len[sp + 1] = len[sp] - m2;
-                sp++;
-                right[sp] = false;
-            }
-        } else {
-            int m2 = len[sp] / 2;
-            m2 -= m2 % 8;
+    int sp;
+    __device__ explicit PairwiseWalk(int n) : sp(0)
+    {
+        off[0] = 0;
+        len[0] = n;
+        right[0] = false;
+    }
+    // The next leaf; false after the last.
+    __device__ bool next(int &o, int &m, int &adds)
+    {
+        if (sp < 0)
+            return false;
+        while (len[sp] > 128) {
             off[sp + 1] = off[sp];
-            len[sp + 1] = m2;
+            len[sp + 1] = half(len[sp]);
             sp++;
             right[sp] = false;
         }
+        o = off[sp];
+        m = len[sp];
+        adds = 0;
+        sp--;
+        while (sp >= 0 && right[sp]) {  // this leaf ends the frame's right half
+            adds++;
+            sp--;
+        }
+        if (sp >= 0) {  // the frame's left half is done: its right half
+            right[sp] = true;
+            const int m2 = half(len[sp]);
+            off[sp + 1] = off[sp] + m2;
+            len[sp + 1] = len[sp] - m2;
+            sp++;
+            right[sp] = false;
+        }
+        return true;
     }
-}
+    static __device__ int half(int n) { return n / 2 - n / 2 % 8; }
+};
 
 // The squares of a[0:n), n <= 128, by 8 lanes (k = 0..7) of a warp.
 __device__ __forceinline__ float pairwise_leaf_sq(const float *a, int n, int k)
@@ -126,26 +130,27 @@ __device__ __forceinline__ float pairwise_leaf_sq(const float *a, int n, int k)
 __device__ __forceinline__ float row_energy(const float *a, int L)
 {
     __shared__ float leaf[4][kEnergyLeaves];
-    __shared__ int at[4][kEnergyLeaves];              // offset * 256 + length
+    __shared__ int at[4][kEnergyLeaves];              // first value of the block
+    __shared__ unsigned char size[4][kEnergyLeaves];  // and how many: 128 at most
     __shared__ unsigned char ends[4][kEnergyLeaves];  // pairs to add after the block
     const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
     float stack[32];
-    int sp = 0;
-    for (int first = 0, total = 1; first < total; first += kEnergyLeaves) {  // a round of blocks
+    int sp = 0, here;
+    PairwiseWalk walk(L);
+    do {  // a round of blocks
         int n = 0;
-        if (lane == 0)
-            pairwise_walk(L, [&](int o, int m, int adds) {
-                const int j = n++ - first;
-                if (j >= 0 && j < kEnergyLeaves) {
-                    at[w][j] = o * 256 + m;
-                    ends[w][j] = (unsigned char)adds;
-                }
-            });
-        total = __shfl_sync(0xffffffffu, n, 0);
+        if (lane == 0) {
+            int o, m, adds;
+            for (; n < kEnergyLeaves && walk.next(o, m, adds); n++) {
+                at[w][n] = o;
+                size[w][n] = (unsigned char)m;
+                ends[w][n] = (unsigned char)adds;
+            }
+        }
+        here = __shfl_sync(0xffffffffu, n, 0);
         __syncwarp();
-        const int here = min(total - first, kEnergyLeaves);
         for (int j = lane >> 3; j < here; j += 4) {
-            const float v = pairwise_leaf_sq(a + (at[w][j] >> 8), at[w][j] & 255, lane & 7);
+            const float v = pairwise_leaf_sq(a + at[w][j], size[w][j], lane & 7);
             if ((lane & 7) == 0)
                 leaf[w][j] = v;
         }
@@ -158,7 +163,7 @@ __device__ __forceinline__ float row_energy(const float *a, int L)
                 stack[sp++] = v;
             }
         __syncwarp();
-    }
+    } while (here == kEnergyLeaves);
     return stack[0];
 }
 

@@ -70,3 +70,9 @@ def test_search_without_energies_is_unchanged(precision, normalize, network_sum)
     got = fmf.matched_filter(tp, mo, w, d, 1, check_zeros=False, normalize=normalize,
                              network_sum=network_sum, precision=precision)
     assert np.array_equal(got.ravel(), res[0])
+
+
+def test_row_past_eight_million_values():
+    rng = np.random.default_rng(4)
+    t = rng.standard_normal((2, 2 ** 23 + 1003), dtype=np.float32)
+    assert np.array_equal(energies(t), np.sum(t ** 2, axis=-1))
