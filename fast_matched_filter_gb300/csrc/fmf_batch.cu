@@ -4,8 +4,8 @@
 // batch records any number of searches (device pointers, each with its own
 // T, S, C, L, N, step, normalisation and output layout) and runs them as one
 // CUDA graph: every search's preprocessing kernels, then, for the tensor-core
-// form, one persistent launch per normalisation and 64 searches over a
-// shared tile queue (fmf_tc.cu); small FP32 searches run on the CUDA cores.  The graph is
+// form, one persistent launch per mode and up to 64 searches that fit together over
+// a shared tile queue (fmf_tc.cu); small FP32 searches run on the CUDA cores.  The graph is
 // captured on the first run (on a stream the batch owns, joined to the
 // caller's stream with events) and replayed afterwards; its scratch lives in
 // graph memory nodes.  The searches' preprocessing (and the FP32 searches)
@@ -101,10 +101,10 @@ static int batch_record(fmf_batch *b, cudaStream_t s)
             unsigned *err = nullptr;
             if ((status = device_error_word(&err)) == FMF_OK) {
                 // One persistent launch per normalisation and output layout (each runs the
-                // instantiation of its own mode), 64 searches at most per launch, each mode
-                // on a branch of its own: a mode's blocks start as the SMs finish the one
-                // before.  The items of a launch are taken up in order of their work, the
-                // long ones (1.3 ms of 7.4 in the uneven batch of 24) first.
+                // instantiation of its own mode) for the searches whose buffers fit together
+                // (tc_group), each mode on a branch of its own: a mode's blocks start as the SMs
+                // finish the one before.  The items of a launch are taken up in order of their
+                // work, the long ones (1.3 ms of 7.4 in the uneven batch of 24) first.
                 std::vector<size_t> order;
                 for (size_t i = 0; i < n; i++)
                     if (nb[i])
@@ -122,7 +122,14 @@ static int batch_record(fmf_batch *b, cudaStream_t s)
                     const size_t ng = grp.size() / psz;
                     if (ng && (e = cudaStreamWaitEvent(sm, b->ev_main, 0)) != cudaSuccess)
                         status = set_error(FMF_ERR_CUDA, "ordering the batch launches: %s", cudaGetErrorString(e));
-                    for (size_t i0 = 0; i0 < ng && status == FMF_OK; i0 += TC_MAX_PROBS) {
+                    std::vector<unsigned char> taken(ng), shared;
+                    int members[TC_MAX_PROBS];
+                    for (int m; status == FMF_OK && (m = tc_group(reinterpret_cast<const TcProb *>(grp.data()), (int)ng,
+                                                                  form, taken.data(), members)) > 0;) {
+                        shared.clear();
+                        for (int j = 0; j < m; j++)
+                            shared.insert(shared.end(), grp.begin() + psz * members[j],
+                                          grp.begin() + psz * (members[j] + 1));
                         unsigned long long *queue = nullptr;
                         if ((status = bws[mode]->get(&queue, 1, "tile queue")))
                             break;
@@ -130,9 +137,7 @@ static int batch_record(fmf_batch *b, cudaStream_t s)
                             status = set_error(FMF_ERR_CUDA, "clearing the tile queue: %s", cudaGetErrorString(e));
                             break;
                         }
-                        const int m = (int)(ng - i0 < (size_t)TC_MAX_PROBS ? ng - i0 : TC_MAX_PROBS);
-                        status = tc_run(reinterpret_cast<const TcProb *>(grp.data() + psz * i0), m, form, 1,
-                                        queue, err, sm);
+                        status = tc_run(reinterpret_cast<const TcProb *>(shared.data()), m, form, 1, queue, err, sm);
                     }
                     if (ng && ((e = cudaEventRecord(b->ev_join[mode], sm)) != cudaSuccess ||
                                (e = cudaStreamWaitEvent(s, b->ev_join[mode], 0)) != cudaSuccess))

@@ -302,6 +302,7 @@ const unsigned *tc_flag(const TcSearch *full);
 size_t tc_prob_size();
 size_t tc_template_bytes(const Problem &P, int nb);  // operand blocks of all templates
 int tc_prepare(const Problem &P, int form, int nb, int tg, Scratch &ws, cudaStream_t s, TcProb *out);
+int tc_group(const TcProb *probs, int n, int form, unsigned char *taken, int *members);
 int tc_run(const TcProb *probs, int n, int form, int parts, unsigned long long *queue, unsigned *err,
            cudaStream_t s);
 int launch_plain(const Problem &P, cudaStream_t stream);

@@ -1311,6 +1311,41 @@ static size_t tc_layout(TcLaunch *B, int nb, bool var, bool full)
     return 0;
 }
 
+// What a search asks of the shared memory of a launch it is in.
+static void tc_add_needs(TcLaunch *B, int *nb, const TcProb &pr, int form)
+{
+    const int halves = form != TC_FORM_BF16 ? 2 : 1;
+    B->w_bytes = max(B->w_bytes, halves * pr.NW * 128);
+    B->row_bytes = max(B->row_bytes, halves * 4 * pr.R * 16);
+    *nb = max(*nb, pr.nb);
+}
+
+// The members of the next launch among n searches of one mode: the first that is not
+// `taken` yet and those after it, in order, that share a launch with it -- at most
+// TC_MAX_PROBS.  The buffers are as large as the largest member's, so a search stays out
+// that would leave fewer than three data slots (a long template beside a large tile: a
+// bf16 search of 5,600 taps and one of 600 leave none).
+int tc_group(const TcProb *probs, int n, int form, unsigned char *taken, int *members)
+{
+    TcLaunch B = {};
+    int nb = 0, count = 0;
+    for (int i = 0; i < n && count < TC_MAX_PROBS; i++) {
+        if (taken[i])
+            continue;
+        TcLaunch with = B;
+        int with_nb = nb;
+        tc_add_needs(&with, &with_nb, probs[i], form);
+        const Problem &P = probs[i].P;
+        if (count && (tc_layout(&with, with_nb, P.ntap != nullptr, P.normalize != 0) == 0 || with.n_rows < 3))
+            continue;
+        B = with;
+        nb = with_nb;
+        taken[i] = 1;
+        members[count++] = i;
+    }
+    return count;
+}
+
 // Channel parts of a prepared search run by itself (tc_run).  A lone search with
 // fewer (tile, template) items than SMs runs each item as k channel parts
 // (network sum only; with per-channel lengths the parts add raw Fisher-z sums
@@ -1359,7 +1394,6 @@ static int tc_run_n(const TcProb *probs, int n, int form, int parts, unsigned lo
     B.lo_unit = form == TC_FORM_FP32 ? 1.0f / kLoScale : 1.0f;
     B.w_bytes = B.row_bytes = 0;
     int nb = 0;
-    const int halves = B.split ? 2 : 1;
     long long items = 0;
     for (int i = 0; i < n; i++) {
         const Problem &P = probs[i].P;
@@ -1370,9 +1404,7 @@ static int tc_run_n(const TcProb *probs, int n, int form, int parts, unsigned lo
         B.prob[i].parts = parts;
         B.prob[i].part_out = part_out;
         items += (long long)probs[i].n_tiles * P.T * parts;
-        B.w_bytes = max(B.w_bytes, halves * probs[i].NW * 128);
-        B.row_bytes = max(B.row_bytes, halves * 4 * probs[i].R * 16);
-        nb = max(nb, probs[i].nb);
+        tc_add_needs(&B, &nb, probs[i], form);
     }
     B.n_probs = n;
     B.total_items = items;

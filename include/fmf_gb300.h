@@ -179,8 +179,8 @@ FMF_API int fmf_matched_filter_noalloc(const float *templates, const float *sum_
  * runs one search per call, matched_filter.cu:171-399).  A batch records
  * searches of any sizes -- device pointers, the same 15 arguments as
  * fmf_matched_filter -- and runs them all as one CUDA graph: the searches'
- * preprocessing, then one persistent tensor-core launch per mode and 64
- * searches over a shared tile queue; of FMF_PREC_FP32, the small searches run
+ * preprocessing, then one persistent tensor-core launch per mode and up to 64
+ * searches that fit together over a shared tile queue; of FMF_PREC_FP32, the small searches run
  * the CUDA-core kernel each.  The graph is captured by the first
  * fmf_batch_run after the last fmf_batch_add and replayed by later runs,
  * which read the input buffers anew.  fmf_batch_run is asynchronous on

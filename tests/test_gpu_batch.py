@@ -92,3 +92,23 @@ def test_many_searches_span_several_persistent_launches():
         torch.cuda.synchronize()
         assert np.abs(out.cpu().numpy() - single.cpu().numpy()).max() <= TOL
     b.close()
+
+
+@pytest.mark.parametrize("precision,longest", [("bf16", 5602), ("split_bf16", 2386), ("fp32", 2386)])
+def test_batch_of_the_longest_templates_and_others(precision, longest):
+    """The longest templates that a tile holds beside ordinary ones, whose buffers do not
+    fit one launch."""
+    b = fmf.Batch(precision)
+    cases = []
+    for i, L in enumerate((600, longest, 200, longest - 30, 5000 if precision == "bf16" else 2000)):
+        host, g, out = _dev(300 + i, 4, 3, 2, L, 30000, 1, "short", True)
+        b.add(*g, 1, out, "short", True)
+        cases.append((g, out))
+    b.run()
+    torch.cuda.synchronize()
+    for g, out in cases:
+        single = torch.empty_like(out)
+        fmf.matched_filter_device(*g, 1, single, "short", True, precision)
+        torch.cuda.synchronize()
+        assert np.abs(out.cpu().numpy() - single.cpu().numpy()).max() <= TOL
+    b.close()
