@@ -39,12 +39,15 @@
 //     down to 2^-50 of the channel's largest value (below that l runs out of
 //     exponent), and the dropped l l is at most 2^-24 of |t d|.
 //   * single bf16: h alone, one MMA.
-// The tensor core rounds every accumulation toward zero, so a long chain
-// drifts: one accumulator over the 38 steps of a 600-tap template was 2.3e-8
-// RMS off (FP32 FMAs: 1.8e-8), 1.2e-6 at a perfect match.  So the h h products
-// run in chains of at most kChain steps, each in a fresh accumulator that the
-// epilogue adds to its registers in FP32 (rounded to nearest); h l and l h,
-// smaller by the pair's rounding, share one accumulator per channel.
+// The tensor core rounds every accumulation toward zero, so a long chain drifts, most of
+// all at a match, where every product adds: a chain of m steps that add something to the
+// output is some 0.6e-7 m low at a perfect match.  So the h h products run in chains of a
+// few steps (tc_chain_cols), each in a fresh accumulator that the epilogue adds to its
+// registers in FP32 (rounded to nearest); h l and l h, smaller by the pair's rounding,
+// share one accumulator per channel.  RMS error at perfect matches of Hann-tapered noise,
+// FP32 multiply-adds and here: 56 taps 1.34 and 1.36e-7, 112 taps 1.74 and 1.21e-7, 300
+// taps 2.80 and 1.73e-7, 600 taps 4.1 and 3.5e-7, 1,200 taps 6.0 and 3.8e-7 (with chains of
+// 16 steps 2.1, 2.8, 4.7, 7.2, 7.3e-7); away from matches it is further below.
 //
 // What bounds it: the tensor pipe, and with it the power limit, from some 400
 // taps (40 templates x 60 channels x 1.08M lags x 600 taps in 6.3 ms: 1.8
@@ -70,6 +73,7 @@
 // Every wait is bounded (globaltimer); on timeout the CTA raises an error
 // word, stops issuing, waits for its own copies/MMAs (bounded) and frees TMEM.
 #include <cfloat>
+#include <cmath>
 #include <cstdlib>
 
 #include <cuda_bf16.h>
@@ -89,7 +93,6 @@ constexpr int tc_groups(bool var) { return tc_epi_warps(var) / 4; }  // column g
 constexpr int TC_MAX_ROWS = 8;     // data slots, at most
 constexpr int TC_MAX_PARTS = 32;   // channel parts of an item, at most
 constexpr int TC_MAX_STATS = 2;    // statistics slots, at most
-constexpr int kChain = 16;          // K steps of one h h chain
 constexpr float kLoScale = 2048.0f;  // l is kept 2^11 up
 constexpr int kTopExp = 15;          // operands are scaled to below 2^15
 // data and template channels whose largest value lies outside [2^-41, 2^60) go
@@ -518,8 +521,19 @@ __device__ __forceinline__ void tc_issue(const TcBatch<N> &B, const long long *r
             for (; active; active &= active - 1) {
                 const int src = __ffs(active) - 1;
                 const int mo = __shfl_sync(0xffffffffu, mo_l, src), ntap = __shfl_sync(0xffffffffu, n_l, src);
+                const uint32_t parts_log2 = SMALL ? 0 : (uint32_t)tc_pair_chains(L, step, ntap, pr.chain_steps);
                 uint32_t left = 0;  // column-block pairs left to the accumulator
                 uint32_t dt = 0, acc = 0;
+                const auto next_acc = [&]() {
+                    const uint32_t empty = bar + (SMALL ? TcBars::sempty : TcBars::hempty) + 8 * (acc_i & 1);
+                    if (acc_i >= 2 && !wait(empty, ((acc_i >> 1) - 1) & 1, 4u))
+                        return false;
+                    tc_fence_after();
+                    dt = tmem + (SMALL ? 256u : 0u) + 128u * (acc_i & 1);
+                    acc = 0;
+                    left = SMALL ? (uint32_t)step * (TC_CB / 2) : (parts_log2 ? 1u : chain_cols);
+                    return true;
+                };
                 for (int phi = 0; phi < step; phi++, stages++) {
                     const uint32_t wb = stages & 1;
                     int psi;
@@ -531,15 +545,8 @@ __device__ __forceinline__ void tc_issue(const TcBatch<N> &B, const long long *r
                     const uint32_t a0 = a_base + (wb ? a_buf : 0u);
 #pragma unroll 1
                     for (uint32_t j = 0; j < TC_CB / 2; j++) {
-                        if (left == 0) {  // the next accumulator
-                            const uint32_t empty = bar + (SMALL ? TcBars::sempty : TcBars::hempty) + 8 * (acc_i & 1);
-                            if (acc_i >= 2 && !wait(empty, ((acc_i >> 1) - 1) & 1, 4u))
-                                return;
-                            tc_fence_after();
-                            dt = tmem + (SMALL ? 256u : 0u) + 128u * (acc_i & 1);
-                            acc = 0;
-                            left = SMALL ? (uint32_t)step * (TC_CB / 2) : chain_cols;
-                        }
+                        if (left == 0 && !next_acc())
+                            return;
                         // two column-block pairs per slot
                         if ((j & 1) == 0 && !wait(bar + TcBars::dfull + 8 * slot, turn & 1, 8u))
                             return;
@@ -547,23 +554,39 @@ __device__ __forceinline__ void tc_issue(const TcBatch<N> &B, const long long *r
                         // row (16 bytes) per step.  The start-address field (16-byte units) of
                         // an address below 256 KB never carries out of its 14 bits.
                         const uint32_t late = 16 * j < k_first ? 1u : 0u;
-                        const uint32_t n = ((k_end - 16 * j + TC_Q - 1) >> 7) - late;
+                        uint32_t n = ((k_end - 16 * j + TC_Q - 1) >> 7) - late;
                         uint32_t a = a0 + 16 * j + late * TC_Q;
                         uint32_t b = b_base + slot * b_slot + (j & 1 ? b_pair : 0u) + late;
+                        const auto issue = [&](uint32_t steps) {
 #pragma unroll 1
-                        for (uint32_t i = 0; i < n; i++) {
-                            if (one) {
-                                if (SMALL) {
-                                    mma_f16(dt, a, a_hi, b + b_low, b_hi, idesc, acc);
-                                    mma_f16(dt, a + a_low, a_hi, b, b_hi, idesc, 1);
-                                } else {
-                                    mma_f16(dt, a, a_hi, b, b_hi, idesc, acc);
+                            for (uint32_t i = 0; i < steps; i++) {
+                                if (one) {
+                                    if (SMALL) {
+                                        mma_f16(dt, a, a_hi, b + b_low, b_hi, idesc, acc);
+                                        mma_f16(dt, a + a_low, a_hi, b, b_hi, idesc, 1);
+                                    } else {
+                                        mma_f16(dt, a, a_hi, b, b_hi, idesc, acc);
+                                    }
                                 }
+                                acc = 1;
+                                a += TC_Q;
+                                b += 1;
                             }
-                            acc = 1;
-                            a += TC_Q;
-                            b += 1;
+                        };
+                        if (!SMALL && parts_log2) {  // all chains of this pair but the last
+                            const uint32_t all = n;
+                            for (uint32_t part = 1; part >> parts_log2 == 0; part++) {
+                                const uint32_t rest = all - ((all * part) >> parts_log2);
+                                issue(n - rest);
+                                n = rest;
+                                if (one)
+                                    mma_commit(bar + TcBars::hfull + 8 * (acc_i & 1));
+                                acc_i++;
+                                if (!next_acc())
+                                    return;
+                            }
                         }
+                        issue(n);
                         const bool done = --left == 0 || (!SMALL && j == TC_CB / 2 - 1 && phi == step - 1);
                         if (one) {
                             if (j & 1)
@@ -897,8 +920,12 @@ __global__ void __launch_bounds__(tc_threads(VAR), 1) tc_persistent(const __grid
             for (int i = 0; i < NCM; i++)
                 sum[i] = 0.0f;
             const size_t row0 = (size_t)t * SC;
-            const int n_chains = (step * (TC_CB / 2) + pr.chain_cols - 1) / pr.chain_cols;
-            const int n_sums = n_chains + (pairs ? 1 : 0);
+            // h h chains of a channel: of whole pairs, or several of each
+            const auto chains_of = [&](int n) {
+                const int log2 = tc_pair_chains(pr.P.L, step, n, pr.chain_steps);
+                return log2 ? (step * (TC_CB / 2)) << log2 : (step * (TC_CB / 2) + pr.chain_cols - 1) / pr.chain_cols;
+            };
+            const int chains = ONE || VAR ? 1 : chains_of(pr.P.L);
             for (int g0 = c_begin; busy && g0 < c_end; g0 += 32) {
                 // the scalars of 32 channels, one per lane
                 const int cl = min(g0 + lane, c_end - 1);
@@ -909,6 +936,7 @@ __global__ void __launch_bounds__(tc_threads(VAR), 1) tc_persistent(const __grid
                 const int n_l = VAR ? pr.P.ntap[row0 + cl] : 0;
                 const float z_l = VAR ? pr.P.zweight[row0 + cl] : 0.0f, u2_l = VAR ? pr.P.unit2[cl] : 0.0f;
                 const float ts_l = FULL ? pr.P.tsum[row0 + cl] * exp2_int(-unit_l) : 0.0f;
+                const int chains_l = VAR && !ONE ? chains_of(n_l) : 0;
                 uint32_t active = __ballot_sync(0xffffffffu, w_l != 0.0f);
 #pragma unroll 1
                 for (; active; active &= active - 1) {
@@ -929,6 +957,8 @@ __global__ void __launch_bounds__(tc_threads(VAR), 1) tc_persistent(const __grid
                             goto epilogue_done;
                         tc_fence_after();
                     }
+                    const int n_chains = VAR && !ONE ? __shfl_sync(0xffffffffu, chains_l, from) : chains;
+                    const int n_sums = n_chains + (pairs ? 1 : 0);
                     // numerators: the chains' sums, then S (FP32: times 2^-11)
 #pragma unroll 1
                     for (int j = 0; !ONE && j < n_sums; j++) {
@@ -1541,6 +1571,19 @@ int tc_fp32_nb(size_t T, size_t SC, size_t L, size_t step, size_t n_corr)
     return 0;
 }
 
+// Column-block pairs of one h h chain of an FP32 search, and the K steps (least of the pairs')
+// past which a pair is several.  Of a pair's steps, (taps + 15) / 128 add something to an
+// output, and a chain of m such steps is off by some 0.6e-7 m at a perfect match (the
+// header of this file); multiply-adds of L taps in a row by 1.65e-8 sqrt(L), RMS.  m up to
+// 0.22 sqrt(L) keeps the former below the latter.
+static int tc_chain_cols(int L, int step, int *chain_steps)
+{
+    const double most = 0.22 * std::sqrt((double)L), per_pair = ((L + step - 1) / step + 15) / 128.0;
+    const int cols = (int)(most / per_pair);
+    *chain_steps = (int)std::ceil(most);
+    return cols < 1 ? 1 : (cols < step * (TC_CB / 2) ? cols : step * (TC_CB / 2));
+}
+
 // Begins a search: data streams of `form`, and room for the operand blocks of up to
 // max_templates templates at a time.  The statistics of P (running sums, with
 // per-channel lengths) have a tile of padding round them; FP32 needs P.scan.  turn:
@@ -1590,11 +1633,8 @@ int tc_begin(const Problem &P, int form, int nb, int tg, int max_templates, Scra
         pr.d_exp = exps + n_rows;
         pr.skip = P.scan + 3 * SC;
     }
-    // FP32: chains of whole column-block pairs, at most kChain K steps where a pair has no
-    // more; the bf16 pairs' own rounding (4.4e-6 of a product) is far above a channel-long
-    // chain's
-    const int most = (g.k_span + TC_Q - 1) / TC_Q;  // K steps of one pair
-    pr.chain_cols = fp32 ? (kChain / most > 1 ? kChain / most : 1) : step * (TC_CB / 2);
+    // The bf16 pairs' own rounding (4.4e-6 of a product) is far above a channel-long chain's
+    pr.chain_cols = fp32 ? tc_chain_cols(P.L, step, &pr.chain_steps) : step * (TC_CB / 2);
     TcDataWork &d = out->data;
     d = TcDataWork{P.data, P.N, SC, step, 0, pr.rows_total, pr.row_front, fp32 ? P.scan : nullptr, g_hi, g_lo,
                    fp32 ? exps + n_rows : nullptr, fp32 ? P.scan + 3 * SC : nullptr, P.ntap && P.normalize == 0};

@@ -37,6 +37,7 @@ struct TcProb {
     const int *t_exp;             // [T][SC] exponent of each channel's template
     const int *d_exp;             // [SC] exponent of each data channel
     int chain_cols;               // column-block pairs of one h h chain
+    int chain_steps;              // a pair of more K steps than this is several chains (tc_pair_chains); 0: one
     const unsigned *skip;         // nonzero: the FP32 CUDA-core kernel runs this search instead
 };
 
@@ -354,6 +355,18 @@ __host__ __device__ __forceinline__ int tc_phase_taps(int L, int step, int phi, 
 
 // End of the K range of a phase with moveout residual s (its start is s & ~15).
 __host__ __device__ __forceinline__ int tc_k_end(int s, int taps) { return (s + taps + TC_Q - 1 + 15) & ~15; }
+
+// log2 of the chains that the K steps of one column-block pair make, of a channel that uses
+// the first n taps.  A pair has at least ceil(taps / 128) steps of a phase with `taps`
+// taps (the last phase has the fewest), so that none of the chains is empty.
+__host__ __device__ __forceinline__ int tc_pair_chains(int L, int step, int n, int chain_steps)
+{
+    const int least = (tc_phase_taps(L, step, step - 1, n) + TC_Q - 1) / TC_Q;
+    int log2 = 0;
+    while (chain_steps && least > chain_steps << log2)
+        log2++;
+    return log2;
+}
 
 struct TcShape {
     int k_span, R, NW;

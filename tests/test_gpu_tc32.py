@@ -185,3 +185,43 @@ def test_batch_of_fp32_searches(small):
     torch.cuda.synchronize()
     for out, _, ref in want:
         _check(out.cpu().numpy(), ref.reshape(tuple(out.shape)))
+
+
+@pytest.mark.parametrize("L", [56, 80, 112, 160, 257, 300, 600, 800, 1200])
+@pytest.mark.parametrize("step", [1, 3])
+@pytest.mark.parametrize("noise", [0.1, 0.5])
+def test_error_at_matches_is_no_larger_than_on_the_cuda_cores(monkeypatch, L, step, noise):
+    """RMS over 2,000 copies of a template of several amplitudes, in noise; a tenth for the
+    scatter of two such figures (their relative standard deviations are 1 / sqrt(4,000))."""
+    rng = np.random.default_rng(L + step)
+    S, K = 8, 250
+    slot = ((L + 20) // step + 1) * step
+    tp = (rng.standard_normal((1, S, 1, L)) * np.hanning(L + 2)[1:-1]).astype(np.float32)
+    d = rng.standard_normal((S, 1, K * slot + L)) * noise * tp.std()
+    at = np.arange(K) * slot
+    for a in at:
+        d[:, 0, a:a + L] += rng.uniform(0.3, 3.0, (S, 1)) * tp[0, :, 0]
+    d = d.astype(np.float32)
+    mo, w = np.zeros((1, S, 1), np.int32), np.ones((1, S, 1), np.float32)
+    t64 = tp[0, :, 0].astype(np.float64)
+    win = np.stack([d[:, 0, a:a + L] for a in at]).astype(np.float64)
+    ref = (win * t64).sum(-1) / np.sqrt((t64 ** 2).sum(-1) * (win ** 2).sum(-1))
+    plain, tensor = [_search(monkeypatch, tile, tp, mo, w, d, step, network_sum=False)[0, at // step, :, 0] - ref
+                     for tile in (0, 64)]
+    assert np.sqrt((tensor ** 2).mean()) <= 1.1 * np.sqrt((plain ** 2).mean())
+
+
+@pytest.mark.parametrize("normalize", ["short", "full"])
+@pytest.mark.parametrize("step", [1, 2])
+def test_per_channel_lengths_of_one_and_several_chains(monkeypatch, normalize, step):
+    """Long channels, whose column-block pairs are several chains each, beside short ones."""
+    rng = np.random.default_rng(10)
+    tp, mo, w, d = random_search(12, 2, 3, 2, 1300, 9000, -30, 90, dc=2.0, zero_weights=1)
+    n = rng.integers(56, 1301, mo.shape).astype(np.int32)
+    n[0, 0, 0] = 1300
+    for i in np.ndindex(n.shape):
+        tp[i][n[i]:] = 0.0
+    got = _search(monkeypatch, 32, tp, mo, w, d, step, normalize=normalize, n_samples_template=n)
+    ref = fp64.fp64_matched_filter_variable(tp, n, mo, w, d, step, normalize)
+    scale = np.cumsum(w.reshape(2, -1).sum(axis=1))[:, None]
+    assert (np.abs(got - ref) / scale).max() <= 6 * TOL
