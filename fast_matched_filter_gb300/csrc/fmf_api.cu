@@ -258,7 +258,8 @@ int launch_wait_selftest(unsigned *err, unsigned ms, cudaStream_t s);
 int launch_fisher_atanh(const float *y, float *out, long long n, cudaStream_t s);
 
 // ---------------------------------------------------------------- device error word
-// Kernels with bounded waits OR a code into this word when a wait gives up.
+// Kernels with bounded waits OR a code into this word when a wait gives up.  kLeftWord
+// words on, the launches of FP32 searches that the tensor cores left to the CUDA cores.
 constexpr int kMaxDevices = 64;
 static unsigned *g_err_word[kMaxDevices];
 
@@ -282,13 +283,13 @@ int device_error_word(unsigned **out)
     return FMF_OK;
 }
 
-// Reads and clears the error word after the device has finished the work.
 int collect_device_errors();
 
-// The same for the calling thread's own call: nothing to read where it launched
-// no kernel that waits.
+// collect_device_errors for the calling thread's own call: nothing to read where it
+// launched no kernel that waits.
 int collect_own_errors() { return g_bounded_waits ? collect_device_errors() : FMF_OK; }
 
+// Reads and clears the error word after the device has finished the work.
 int collect_device_errors()
 {
     unsigned *w = nullptr;
@@ -444,6 +445,7 @@ int prepare_problem(const Args &a, Scratch &ws, cudaStream_t s, Problem *Pout, i
     P.scan = scan;
     P.dc = dc;
     P.only_if = nullptr;
+    P.left = nullptr;
 
     P.by_channel = nullptr;
     *Pout = P;
@@ -586,6 +588,7 @@ struct Search {
             if ((rc = tc_run_templates(search(), t0, nt, err, s)) || !fp32)
                 return rc;
             Q.only_if = tc_flag(search());
+            Q.left = err + kLeftWord;
         } else if ((rc = clear_outputs(Q, s))) {
             return rc;
         }
@@ -1329,6 +1332,24 @@ int fmf_timing_end(double *prep_ms, double *kernel_ms, int *n_calls)
 }
 
 int fmf_last_precision(void) { return fmf::g_last_precision; }
+
+int fmf_last_tensor_cores(void)
+{
+    using namespace fmf;
+    clear_error();
+    unsigned *w = nullptr, left = 0;
+    int rc = device_error_word(&w);
+    if (rc)
+        return -rc;
+    cudaError_t e = cudaDeviceSynchronize();
+    if (e == cudaSuccess)
+        e = cudaMemcpy(&left, w + kLeftWord, sizeof(left), cudaMemcpyDeviceToHost);
+    if (e == cudaSuccess && left)
+        e = cudaMemset(w + kLeftWord, 0, sizeof(left));
+    if (e != cudaSuccess)
+        return -cuda_status(e, "fmf_last_tensor_cores");
+    return g_bounded_waits ? (left ? 2 : 1) : 0;
+}
 
 int fmf_release_cache(void)
 {

@@ -148,6 +148,7 @@ static int batch_record(fmf_batch *b, cudaStream_t s)
                 for (size_t i = 0; i < n && fp32 && status == FMF_OK; i++)
                     if (nb[i]) {
                         P[i].only_if = P[i].scan + 3 * P[i].SC;
+                        P[i].left = err + kLeftWord;
                         status = launch_plain_all(P[i], s);
                     }
             }

@@ -68,6 +68,7 @@ struct Problem {
     // window of channel ch over every kDcStride-th window, as float bits [SC]
     unsigned *dc;
     const unsigned *only_if;  // plain kernel: run only if this word is nonzero (null: always)
+    unsigned *left;           // counts the plain launches that such a word let run
 };
 
 #ifdef __CUDACC__
@@ -311,6 +312,7 @@ int launch_plain_all(const Problem &P, cudaStream_t stream);
 int choose_auto_precision(const Problem &P, Scratch &ws, cudaStream_t s, int *precision);
 void set_last_precision(int precision);
 int device_error_word(unsigned **out);
+constexpr int kLeftWord = 1;  // and where it counts the searches left to the CUDA cores
 
 // Detection on network-summed rows (fmf_detect.cu).
 int detect_device(const float *cc, int T, int n_corr, size_t ld, const int *begin, const int *end,

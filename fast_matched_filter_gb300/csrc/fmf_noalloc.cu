@@ -236,6 +236,7 @@ extern "C" int fmf_matched_filter_noalloc(const float *templates, const float *s
     P.scan = nullptr;
     P.dc = nullptr;
     P.only_if = nullptr;
+    P.left = nullptr;
     if ((rc = launch_plain_all(P, s)))
         return rc;
     return FMF_OK;

@@ -200,8 +200,12 @@ plain_kernel(const Problem P, const PlainGeom g)
 {
     extern __shared__ __align__(16) float smem[];
     float *net = smem + 2 * g.stage_floats;  // [PL_R][PL_THREADS]
-    if (P.only_if && *P.only_if == 0)  // the tensor cores ran this search
-        return;
+    if (P.only_if) {
+        if (*P.only_if == 0)  // the tensor cores ran this search
+            return;
+        if (blockIdx.x == 0 && threadIdx.x == 0)
+            atomicAdd(P.left, 1u);
+    }
 
     // templates fastest: the CTAs running at any time share a few tiles, so
     // their data windows and window statistics are read from L2

@@ -662,6 +662,7 @@ static int variable_device(const VArgs &a, int L, cudaStream_t s, float *host_ou
     P.scan = scan;
     P.dc = nullptr;
     P.only_if = nullptr;
+    P.left = nullptr;
     if (precision == FMF_PREC_AUTO && (rc = choose_auto_precision(P, ws, s, &precision)))
         return rc;
     set_last_precision(precision);
@@ -707,6 +708,7 @@ static int variable_device(const VArgs &a, int L, cudaStream_t s, float *host_ou
             return rc;
         } else {
             P.only_if = tc_flag(search);
+            P.left = err + kLeftWord;
         }
     }
     CopyStream cs;

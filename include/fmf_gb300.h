@@ -349,6 +349,12 @@ FMF_API int fmf_timing_end_ex(double *ms, int n_kinds, int *n_calls);
  * it chose.  -1 before the first search. */
 FMF_API int fmf_last_precision(void);
 
+/* Whether the calling thread's last search ran on the tensor cores (for tests;
+ * synchronizes the device): 0 no; 1 yes; 2 it was prepared for them, and an FP32
+ * search since the last call of this function was left to the CUDA cores, because
+ * its amplitudes do not fit fp16 pairs.  Negative: a status of this header. */
+FMF_API int fmf_last_tensor_cores(void);
+
 /* Releases device memory cached by the library on the current device. */
 FMF_API int fmf_release_cache(void);
 

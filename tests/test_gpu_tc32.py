@@ -13,6 +13,7 @@ import numpy as np
 import pytest
 
 import fast_matched_filter_gb300 as fmf
+from fast_matched_filter_gb300 import _lib
 from oracle import fp64
 from tests._cases import random_search
 
@@ -225,3 +226,58 @@ def test_per_channel_lengths_of_one_and_several_chains(monkeypatch, normalize, s
     ref = fp64.fp64_matched_filter_variable(tp, n, mo, w, d, step, normalize)
     scale = np.cumsum(w.reshape(2, -1).sum(axis=1))[:, None]
     assert (np.abs(got - ref) / scale).max() <= 6 * TOL
+
+
+def _ran():
+    """0: the CUDA cores; 1: the tensor cores; 2: they left it to the CUDA cores."""
+    return _lib.load().fmf_last_tensor_cores()
+
+
+@pytest.mark.parametrize("normalize", ["short", "full"])
+@pytest.mark.parametrize("network_sum", [True, False])
+@pytest.mark.parametrize("tile", [0, 32, 64, 128])
+@pytest.mark.parametrize("step", [1, 3])
+def test_ordinary_searches_run_where_they_are_sent(monkeypatch, normalize, network_sum, tile, step):
+    """Noise, levels, a gap of zeros, amplitudes a thousand apart."""
+    tp, mo, w, d = random_search(21, 2, 3, 2, 100, 9000, -20, 90, dc=1.0, zero_weights=1)
+    d[1] *= np.float32(1e3)
+    tp[:, 2] *= np.float32(1e-3)
+    d[0, :, 2000:2500] = d[0, :, 2000:2001]
+    _ran()
+    _search(monkeypatch, tile, tp, mo, w, d, step, normalize=normalize, network_sum=network_sum)
+    assert _ran() == (tile != 0)
+
+
+@pytest.mark.parametrize("normalize", ["short", "full"])
+def test_ordinary_searches_with_per_channel_lengths_run_where_they_are_sent(monkeypatch, normalize):
+    rng = np.random.default_rng(22)
+    tp, mo, w, d = random_search(23, 2, 3, 2, 200, 9000, -20, 90, dc=1.0, zero_weights=1)
+    n = rng.integers(100, 201, mo.shape).astype(np.int32)
+    n[0, 0, 0] = 200
+    for i in np.ndindex(n.shape):
+        tp[i][n[i]:] = 0.0
+    for tile in (0, 64):
+        _search(monkeypatch, tile, tp, mo, w, d, normalize=normalize, n_samples_template=n)
+        assert _ran() == (tile != 0)
+    d[2, 0, 5000] = np.nan
+    _search(monkeypatch, 64, tp, mo, w, d, normalize=normalize, n_samples_template=n)
+    assert _ran() == 2
+
+
+@pytest.mark.parametrize("change,ran", [("nan sample", 1), ("nan tap", 2), ("loud data", 2), ("faint template", 2),
+                                        ("transient", 2)])
+def test_what_operand_pairs_cannot_hold_is_left_to_the_cuda_cores(monkeypatch, change, ran):
+    tp, mo, w, d = random_search(24, 2, 2, 1, 60, 6000, 0, 50)
+    if change == "nan sample":
+        d[0, 0, 3000] = np.nan
+    elif change == "nan tap":
+        tp[1, 0, 0, 7] = np.nan
+    elif change == "loud data":
+        d[1] *= np.float32(1e19)
+    elif change == "faint template":
+        tp[0, 1] *= np.float32(1e-13)
+    else:
+        d[1, 0, 100] = 1e8
+    _ran()
+    _search(monkeypatch, 32, tp, mo, w, d)
+    assert _ran() == ran
