@@ -52,9 +52,9 @@ extern "C" {
 
 /* numerator precision */
 /* FP32: on the tensor cores as scaled fp16 pairs (22 bits) in searches large
- * enough (56 taps at least; per-channel lengths 112), with an error no larger
- * than that of FP32 multiply-adds; else, and where the amplitudes do not fit
- * such pairs, on the CUDA cores */
+ * enough (56 taps at least, of every channel of weight where the lengths
+ * differ), with an RMS error no larger than that of FP32 multiply-adds; else,
+ * and where the amplitudes do not fit such pairs, on the CUDA cores */
 #define FMF_PREC_FP32 0
 #define FMF_PREC_SPLIT_BF16 1 /* tensor cores, bf16 hi+lo, 3 products, FP32 accumulate */
 #define FMF_PREC_BF16 2       /* tensor cores, single bf16 product (loss demonstration) */

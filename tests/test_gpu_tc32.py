@@ -281,3 +281,26 @@ def test_what_operand_pairs_cannot_hold_is_left_to_the_cuda_cores(monkeypatch, c
     _ran()
     _search(monkeypatch, 32, tp, mo, w, d)
     assert _ran() == ran
+
+
+@pytest.mark.parametrize("device", [False, True])
+@pytest.mark.parametrize("shortest,weight,ran", [(55, 0.1, 0), (56, 0.1, 1), (10, 0.0, 1), (10, 0.1, 0)])
+def test_per_channel_lengths_by_the_shortest_of_weight(monkeypatch, shortest, weight, ran, device):
+    torch = pytest.importorskip("torch")
+    tp, mo, w, d = random_search(25, 2, 3, 2, 150, 9000, -20, 90)
+    n = np.full(mo.shape, 150, np.int32)
+    n[1, 2, 0] = shortest
+    w[1, 2, 0] = weight
+    tp[1, 2, 0, shortest:] = 0.0
+    if not device:
+        _search(monkeypatch, 64, tp, mo, w, d, n_samples_template=n)
+    else:
+        monkeypatch.setenv("FMF_TC32", "64")
+        lib = _lib.load()
+        g = [torch.from_numpy(x).cuda() for x in (tp, np.sum(tp ** 2, axis=-1), mo, d, w, n)]
+        out = torch.empty((2, 8851), device="cuda")
+        torch.cuda.synchronize()
+        _lib.check(lib.fmf_matched_filter_variable_ex(
+            *[x.data_ptr() for x in g[:5]], 1, g[5].data_ptr(), 9000, 2, 3, 2, 8851, out.data_ptr(), 0,
+            _lib.FLAG_DEVICE_POINTERS, None), lib)
+    assert _ran() == ran
