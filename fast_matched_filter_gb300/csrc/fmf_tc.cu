@@ -440,6 +440,30 @@ __device__ __forceinline__ void tc_template_block(const TcTemplateWork &w, long 
     }
 }
 
+// FP32: raises the flag where pairs cannot hold a template, as tc_template_block does, for
+// searches whose operands are made in parts: the first parts run before the others'
+// operands are made, and the flag is the whole search's.  A block per (template, channel).
+__global__ void __launch_bounds__(128) tc_template_check_kernel(const float *__restrict__ tpl, int L, unsigned *skip)
+{
+    const float *src = tpl + (size_t)blockIdx.x * L;
+    unsigned top = 0;
+    for (int j = threadIdx.x; j < L; j += blockDim.x)
+        top = max(top, __float_as_uint(src[j]) & 0x7fffffffu);
+    top = __reduce_max_sync(0xffffffffu, top);
+    __shared__ unsigned red[4];
+    if ((threadIdx.x & 31) == 0)
+        red[threadIdx.x >> 5] = top;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        for (int i = 1; i < 4; i++)
+            top = max(top, red[i]);
+        bool ok;
+        max_exponent(top, ok);  // (a value that is not finite is above them all)
+        if (!ok)
+            atomicOr(skip, 1u);
+    }
+}
+
 // Both in one launch: blocks [0, n_data) turn data, the others make template blocks.
 template <bool FP32>
 __global__ void __launch_bounds__(256) tc_operand_kernel(const TcDataWork d, unsigned n_data, const TcTemplateWork w)
@@ -1632,6 +1656,12 @@ int tc_begin(const Problem &P, int form, int nb, int tg, int max_templates, Scra
         pr.t_exp = exps;
         pr.d_exp = exps + n_rows;
         pr.skip = P.scan + 3 * SC;
+        if (out->room < P.T) {
+            tc_template_check_kernel<<<(unsigned)n_rows, 128, 0, s>>>(P.tpl, P.L, P.scan + 3 * SC);
+            count_launch();
+            if ((rc = check_launch("tc_template_check_kernel")))
+                return rc;
+        }
     }
     // The bf16 pairs' own rounding (4.4e-6 of a product) is far above a channel-long chain's
     pr.chain_cols = fp32 ? tc_chain_cols(P.L, step, &pr.chain_steps) : step * (TC_CB / 2);
