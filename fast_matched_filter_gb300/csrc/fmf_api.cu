@@ -57,6 +57,11 @@ static int clear_error()
 }
 
 void count_launch(int n) { g_launches += n; }
+size_t &scratch_asked()
+{
+    static thread_local size_t bytes = 0;
+    return bytes;
+}
 static thread_local int g_last_precision = -1;
 void set_last_precision(int precision) { g_last_precision = precision; }
 void reset_launch_count()

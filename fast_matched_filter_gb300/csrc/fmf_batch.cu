@@ -23,7 +23,8 @@
 namespace fmf {
 constexpr int kBatchBranches = 8;  // concurrent graph branches for the per-search work
 // A graph holds the operand blocks of all its searches at once: FP32 searches with
-// more than this stay on the CUDA cores.
+// more than this stay on the CUDA cores, and so do all of a batch whose operands the
+// device has no memory for (batch_fits).
 constexpr size_t kBatchTemplateBytes = (size_t)1 << 30;
 }
 
@@ -42,11 +43,13 @@ struct fmf_batch {
     cudaGraph_t graph = nullptr;
     cudaGraphExec_t exec = nullptr;
     int launches = 0;  // kernel launches in one replay
+    bool operands = false;  // it holds operands of FP32 searches on the tensor cores
 };
 
 namespace fmf {
 
-static int batch_record(fmf_batch *b, cudaStream_t s)
+// cuda_cores: FP32 searches run there without the tensor cores' operands.
+static int batch_record(fmf_batch *b, cudaStream_t s, bool cuda_cores)
 {
     int rc;
     cudaError_t e;
@@ -72,7 +75,7 @@ static int batch_record(fmf_batch *b, cudaStream_t s)
             const int k = (int)(i % kBatchBranches);
             cudaStream_t si = b->branch[k];
             const Args &a = b->searches[i];
-            nb[i] = fp32 ? tc_fp32_nb(a.T, a.S * a.C, a.L, a.step, a.n_corr)
+            nb[i] = fp32 ? (cuda_cores ? 0 : tc_fp32_nb(a.T, a.S * a.C, a.L, a.step, a.n_corr))
                          : tc_choose_nb((int)a.L, (int)a.step, form != TC_FORM_BF16, b->tile);
             if (!fp32 && nb[i] == 0) {
                 status = set_error(FMF_ERR_SMEM, "search %zu: template length %zu with step %zu does not "
@@ -85,6 +88,7 @@ static int batch_record(fmf_batch *b, cudaStream_t s)
                 nb[i] = 0;
             if ((status = clear_outputs(P[i], si)))
                 break;
+            b->operands = b->operands || (fp32 && nb[i]);
             if (nb[i] == 0)
                 status = launch_plain_all(P[i], si);
             else
@@ -178,6 +182,60 @@ static void batch_reset_graph(fmf_batch *b)
         cudaGraphDestroy(b->graph);
     b->exec = nullptr;
     b->graph = nullptr;
+}
+
+// Records the searches into b->graph; *bytes: the scratch it asks for.
+static int batch_capture(fmf_batch *b, bool cuda_cores, size_t *bytes)
+{
+    unsigned *err = nullptr;  // allocated outside the capture
+    int rc = device_error_word(&err);
+    if (rc)
+        return rc;
+    cudaError_t e = cudaStreamBeginCapture(b->stream, cudaStreamCaptureModeThreadLocal);
+    if (e != cudaSuccess)
+        return set_error(FMF_ERR_CUDA, "beginning graph capture: %s", cudaGetErrorString(e));
+    const int before = fmf_last_launch_count();
+    const size_t asked = scratch_asked();
+    b->operands = false;
+    rc = batch_record(b, b->stream, cuda_cores);
+    *bytes = scratch_asked() - asked;
+    b->launches = fmf_last_launch_count() - before;
+    cudaGraph_t g = nullptr;
+    e = cudaStreamEndCapture(b->stream, &g);
+    if (rc) {
+        if (g)
+            cudaGraphDestroy(g);
+        return rc;
+    }
+    if (e != cudaSuccess)
+        return set_error(FMF_ERR_CUDA, "ending graph capture: %s", cudaGetErrorString(e));
+    b->graph = g;
+    return FMF_OK;
+}
+
+// Whether the device has `bytes` for a graph's scratch, given back by the default pool if
+// need be.  A graph takes its memory when it is launched, and what a launch that failed
+// for want of it had taken stays lost to the process, so the batch asks first.  (A
+// sixteenth and 128 MB more: the driver takes memory in large pieces.)
+static bool batch_fits(int device, size_t bytes)
+{
+    const size_t need = bytes + bytes / 16 + ((size_t)128 << 20);
+    unsigned long long used = 0, reserved = 0;
+    size_t free = 0, total = 0;
+    cudaMemPool_t pool;
+    for (int attempt = 0; attempt < 2; attempt++) {
+        if (cudaDeviceGetGraphMemAttribute(device, cudaGraphMemAttrUsedMemCurrent, &used) != cudaSuccess ||
+            cudaDeviceGetGraphMemAttribute(device, cudaGraphMemAttrReservedMemCurrent, &reserved) != cudaSuccess ||
+            cudaMemGetInfo(&free, &total) != cudaSuccess)
+            break;
+        if (need <= free + (reserved - used))
+            return true;
+        if (attempt == 0 && (cudaDeviceGetDefaultMemPool(&pool, device) != cudaSuccess ||
+                             cudaMemPoolTrimTo(pool, 0) != cudaSuccess))
+            break;
+    }
+    cudaGetLastError();
+    return false;
 }
 
 }  // namespace fmf
@@ -286,27 +344,15 @@ int fmf_batch_run(fmf_batch *b, void *stream)
     cudaStream_t user = (cudaStream_t)stream;
     cudaError_t e;
     if (!b->exec) {
-        unsigned *err = nullptr;  // allocated outside the capture
-        int rc = fmf::device_error_word(&err);
+        size_t bytes = 0;
+        int rc = fmf::batch_capture(b, false, &bytes);
+        if (rc == FMF_OK && b->operands && !fmf::batch_fits(dev, bytes)) {
+            fmf::batch_reset_graph(b);
+            rc = fmf::batch_capture(b, true, &bytes);
+        }
         if (rc)
             return rc;
-        e = cudaStreamBeginCapture(b->stream, cudaStreamCaptureModeThreadLocal);
-        if (e != cudaSuccess)
-            return fmf::set_error(FMF_ERR_CUDA, "beginning graph capture: %s", cudaGetErrorString(e));
-        const int before = fmf_last_launch_count();
-        rc = fmf::batch_record(b, b->stream);
-        b->launches = fmf_last_launch_count() - before;
-        cudaGraph_t g = nullptr;
-        e = cudaStreamEndCapture(b->stream, &g);
-        if (rc) {
-            if (g)
-                cudaGraphDestroy(g);
-            return rc;
-        }
-        if (e != cudaSuccess)
-            return fmf::set_error(FMF_ERR_CUDA, "ending graph capture: %s", cudaGetErrorString(e));
-        b->graph = g;
-        e = cudaGraphInstantiate(&b->exec, g, 0);
+        e = cudaGraphInstantiate(&b->exec, b->graph, 0);
         if (e != cudaSuccess) {
             fmf::batch_reset_graph(b);
             return fmf::set_error(FMF_ERR_CUDA, "instantiating the batch graph: %s", cudaGetErrorString(e));

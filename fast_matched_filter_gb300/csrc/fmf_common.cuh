@@ -205,6 +205,7 @@ private:
 // default pool).  The pool keeps freed blocks for reuse by later calls;
 // fmf_release_cache() trims it.  Everything is freed, in stream order, when
 // the Scratch goes out of scope.
+size_t &scratch_asked();  // bytes the calling thread has asked for so far
 struct Scratch {
     cudaStream_t s;
     std::vector<void *> ptr;
@@ -223,6 +224,7 @@ struct Scratch {
                              cudaGetErrorString(e));
         }
         ptr.push_back(p);
+        scratch_asked() += count * sizeof(T) + 16;
         *out = static_cast<T *>(p);
         return FMF_OK;
     }

@@ -1,0 +1,53 @@
+"""FP32 searches with too little memory for the tensor cores' operands run on the CUDA
+cores, whichever call they come through (needs a GB300)."""
+import contextlib
+
+import numpy as np
+import pytest
+
+import fast_matched_filter_gb300 as fmf
+from fast_matched_filter_gb300 import _lib
+
+pytestmark = pytest.mark.gpu
+torch = pytest.importorskip("torch")
+
+
+def _search(T=500, S=20, C=3, L=600, N=20000):
+    """Operands of 950 MB; 5 MB of window statistics and 40 MB of outputs."""
+    g = torch.Generator(device="cuda")
+    g.manual_seed(1)
+    tp = torch.randn((T, S, C, L), device="cuda", generator=g)
+    d = torch.randn((S, C, N), device="cuda", generator=g)
+    mo = torch.zeros((T, S, C), dtype=torch.int32, device="cuda")
+    w = torch.full((T, S, C), 1 / (S * C), device="cuda")
+    return (tp, (tp * tp).sum(-1), mo, w, d), torch.empty((T, N - L + 1), device="cuda")
+
+
+@contextlib.contextmanager
+def _little_memory(megabytes):
+    torch.cuda.synchronize()
+    lib = _lib.load()
+    _lib.check(lib.fmf_release_cache(), lib)
+    hold = torch.empty(torch.cuda.mem_get_info()[0] - (megabytes << 20), dtype=torch.uint8, device="cuda")
+    try:
+        yield
+    finally:
+        del hold
+        torch.cuda.empty_cache()
+
+
+def test_batch(monkeypatch):
+    args, out = _search()
+    monkeypatch.setenv("FMF_TC32", "0")
+    want = torch.empty_like(out)
+    fmf.matched_filter_device(*args, 1, want)
+    monkeypatch.delenv("FMF_TC32")
+    b = fmf.Batch("fp32")
+    b.add(*args, 1, out)
+    with _little_memory(500):
+        for _ in range(2):
+            out.zero_()
+            b.run()
+            torch.cuda.synchronize()
+            assert np.array_equal(out.cpu().numpy(), want.cpu().numpy())
+    b.close()
