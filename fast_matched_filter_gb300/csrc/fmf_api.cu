@@ -601,8 +601,9 @@ struct Search {
     }
 };
 
-// Search on device pointers with its working arrays in `ws` (they stay
-// allocated, and *Pout valid, until ws goes out of scope).
+// Search on device pointers with the arrays of its preparation in `ws` (they stay
+// allocated, and *Pout valid, until ws goes out of scope).  The tensor cores' operands are
+// freed behind it: what follows may need the memory that an FP32 search took for speed.
 static int run_device_ws(const Args &a, cudaStream_t s, Scratch &ws, Problem *Pout)
 {
     int rc;
@@ -618,7 +619,8 @@ static int run_device_ws(const Args &a, cudaStream_t s, Scratch &ws, Problem *Po
         return rc;
     set_last_precision(precision);
     cudaEvent_t ev_main0 = mark(s);
-    Search f(P, precision, tiles, a.flags, P.T, ws, s);
+    Scratch operands(s);
+    Search f(P, precision, tiles, a.flags, P.T, operands, s);
     rc = f.status ? f.status : f.run(0, P.T, s);
     span(ev_main0, mark(s), kSpanKernel);
     return rc;
@@ -678,9 +680,6 @@ static int run_streamed(const Args &d, float *host_out, HostPages &pages, cudaSt
     set_last_precision(precision);
     for (int c = 0; c < n_chunks; c++)
         most = bounds[c + 1] - bounds[c] > most ? bounds[c + 1] - bounds[c] : most;
-    Search search(P, precision, tiles, d.flags, most, ws, s);
-    if ((rc = search.status))
-        return rc;
     unsigned long long *zc = nullptr;  // device zero counts, copied to d.zero_counts (host)
     if (d.zero_counts) {
         if ((rc = ws.get(&zc, (size_t)P.T, "zero counts")) ||
@@ -688,6 +687,9 @@ static int run_streamed(const Args &d, float *host_out, HostPages &pages, cudaSt
                               "clearing the zero counts")))
             return rc;
     }
+    Search search(P, precision, tiles, d.flags, most, ws, s);
+    if ((rc = search.status))
+        return rc;
     cudaStream_t s2 = nullptr;
     cudaEvent_t ev[9] = {};
     cudaError_t e = cudaStreamCreateWithFlags(&s2, cudaStreamNonBlocking);

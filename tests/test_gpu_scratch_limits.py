@@ -51,3 +51,18 @@ def test_batch(monkeypatch):
             torch.cuda.synchronize()
             assert np.array_equal(out.cpu().numpy(), want.cpu().numpy())
     b.close()
+
+
+@pytest.mark.parametrize("megabytes", [500, 1180])
+def test_search_and_detection(megabytes):
+    """1,180 MB hold the operands (945) or what detection needs (220) beside inputs, sums and
+    statistics (120)."""
+    args, _ = _search()
+    tp, _, mo, w, d = [x.cpu().numpy() for x in args]
+    del args
+    torch.cuda.empty_cache()
+    first = fmf.matched_filter_detect(tp, mo, w, d, 1)
+    with _little_memory(megabytes):
+        again = fmf.matched_filter_detect(tp, mo, w, d, 1)
+    assert np.array_equal(first.count, again.count) or megabytes == 500
+    assert np.abs(first.threshold - again.threshold).max() <= 1e-6
