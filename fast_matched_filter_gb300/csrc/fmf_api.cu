@@ -549,6 +549,21 @@ struct Tiles {
     int bad = 0;  // a tile that does not exist
 };
 
+// prepare_problem for these tiles.  FP32 without memory for the padding round the
+// statistics that tiles read: for the CUDA cores, which need none.
+static int prepare_for_tiles(const Args &a, Tiles &tiles, Scratch &ws, cudaStream_t s, Problem *P)
+{
+    const size_t held = ws.ptr.size();
+    int rc = prepare_problem(a, ws, s, P, tiles.pad(), tiles.fp32 != 0);
+    if (rc == FMF_ERR_OOM && a.precision == FMF_PREC_FP32 && tiles.fp32) {
+        clear_error();
+        ws.shrink(held);
+        tiles.fp32 = 0;
+        rc = prepare_problem(a, ws, s, P, 0, false);
+    }
+    return rc;
+}
+
 // A prepared search, run in parts of its templates.  FP32: on the tensor cores
 // where it has a tile and their working arrays can be had, followed by the
 // CUDA-core kernel, which runs only where the operands' flag says so; else on the
@@ -609,8 +624,8 @@ static int run_device_ws(const Args &a, cudaStream_t s, Scratch &ws, Problem *Po
     int rc;
     Problem &P = *Pout;
     cudaEvent_t ev_prep0 = mark(s);
-    const Tiles tiles(a);
-    if ((rc = prepare_problem(a, ws, s, &P, tiles.pad(), tiles.fp32 != 0)))
+    Tiles tiles(a);
+    if ((rc = prepare_for_tiles(a, tiles, ws, s, &P)))
         return rc;
     cudaEvent_t ev_prep1 = mark(s);
     span(ev_prep0, ev_prep1, kSpanPrep);
@@ -649,8 +664,8 @@ static int run_streamed(const Args &d, float *host_out, HostPages &pages, cudaSt
     Scratch ws(s);
     Problem P;
     cudaEvent_t ev_prep0 = mark(s);
-    const Tiles tiles(d);
-    if ((rc = prepare_problem(d, ws, s, &P, tiles.pad(), tiles.fp32 != 0)))
+    Tiles tiles(d);
+    if ((rc = prepare_for_tiles(d, tiles, ws, s, &P)))
         return rc;
     cudaEvent_t ev_kern0 = mark(s);
     span(ev_prep0, ev_kern0, kSpanPrep);

@@ -228,11 +228,13 @@ struct Scratch {
         *out = static_cast<T *>(p);
         return FMF_OK;
     }
-    ~Scratch()
+    // Frees all but the first n allocations.
+    void shrink(size_t n)
     {
-        for (void *p : ptr)
-            cudaFreeAsync(p, s);
+        for (; ptr.size() > n; ptr.pop_back())
+            cudaFreeAsync(ptr.back(), s);
     }
+    ~Scratch() { shrink(0); }
 };
 
 // Preprocessing shared by every form: per-template lag ranges, 'full'

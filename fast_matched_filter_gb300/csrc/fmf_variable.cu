@@ -555,7 +555,7 @@ struct CopyStream {
 // tapering size (8,8,8,8,4,2,1,1 of 40 parts), each chunk's copy on a second
 // stream overlapping the later chunks' kernels (all of which are queued before
 // the first copy, which blocks the host when host_out is pageable).
-static int variable_device(const VArgs &a, int L, int shortest, cudaStream_t s, float *host_out = nullptr, HostPages *pages = nullptr)
+static int variable_device(const VArgs &a, int L, int shortest, cudaStream_t s, float *host_out, HostPages *pages)
 {
     int rc;
     const int T = (int)a.T, SC = (int)(a.S * a.C), N = (int)a.N;
@@ -757,6 +757,18 @@ static int variable_device(const VArgs &a, int L, int shortest, cudaStream_t s, 
     return FMF_OK;
 }
 
+// FP32 without memory for the padding round the running sums that tiles read: on the CUDA
+// cores, which need none.
+static int variable_search(const VArgs &a, int L, int shortest, cudaStream_t s, float *host_out = nullptr,
+                           HostPages *pages = nullptr)
+{
+    const int rc = variable_device(a, L, shortest, s, host_out, pages);
+    if (rc != FMF_ERR_OOM || FMF_FLAG_PRECISION_OF(a.flags) != FMF_PREC_FP32)
+        return rc;
+    set_error(FMF_OK, "");
+    return variable_device(a, L, 0, s, host_out, pages);
+}
+
 static int variable_entry(const VArgs &a, void *stream)
 {
     set_error(FMF_OK, "");
@@ -814,7 +826,7 @@ static int variable_entry(const VArgs &a, void *stream)
     if (a.n_corr > (a.N - L) / a.step + 1)
         return set_error(FMF_ERR_ARG, "n_corr exceeds (N - longest template)/step + 1");
     if (dev)
-        return variable_device(a, L, shortest, s);
+        return variable_search(a, L, shortest, s);
 
     int rc;
     const size_t SC = a.S * a.C;
@@ -840,7 +852,7 @@ static int variable_entry(const VArgs &a, void *stream)
         d.w = buf[4];
         d.ntap = reinterpret_cast<const int *>(buf[5]);
         d.out = buf[6];
-        if ((rc = variable_device(d, L, shortest, s, a.out, &pages)))
+        if ((rc = variable_search(d, L, shortest, s, a.out, &pages)))
             return rc;
     }
     cudaError_t e = cudaStreamSynchronize(s);

@@ -66,3 +66,33 @@ def test_search_and_detection(megabytes):
         again = fmf.matched_filter_detect(tp, mo, w, d, 1)
     assert np.array_equal(first.count, again.count) or megabytes == 500
     assert np.abs(first.threshold - again.threshold).max() <= 1e-6
+
+
+@pytest.mark.parametrize("lengths", [False, True])
+@pytest.mark.parametrize("normalize", ["short", "full"])
+def test_statistics_of_a_large_step(monkeypatch, normalize, lengths):
+    """Tiles of 128 lag blocks have 33,000 statistics of padding round each of the 3,000 rows
+    of 60 channels at step 50: 390 MB and more."""
+    T, S, C, L, N, step = 4, 20, 3, 600, 100000, 50
+    (tp, sst, mo, w, d), _ = _search(T, S, C, L, N)
+    n = torch.full((T, S, C), L, dtype=torch.int32, device="cuda")
+    lib = _lib.load()
+
+    def run():
+        out = torch.zeros((T, (N - L) // step + 1), device="cuda")
+        if lengths:
+            _lib.check(lib.fmf_matched_filter_variable_ex(
+                *[x.data_ptr() for x in (tp, sst, mo, d, w)], step, n.data_ptr(), N, T, S, C, out.shape[1],
+                out.data_ptr(), normalize == "full", _lib.FLAG_DEVICE_POINTERS,
+                torch.cuda.current_stream().cuda_stream), lib)
+        else:
+            fmf.matched_filter_device(tp, sst, mo, w, d, step, out, normalize)
+        return out.cpu().numpy()
+
+    monkeypatch.setenv("FMF_TC32", "0")
+    want = run()
+    monkeypatch.setenv("FMF_TC32", "128")
+    with _little_memory(280):
+        got = run()
+    assert lib.fmf_last_tensor_cores() == 0
+    assert np.array_equal(got, want)
