@@ -63,45 +63,34 @@ constexpr int kEnergyLeaves = 256;  // blocks of one round; a block has at least
 // numpy's recursion over n values as a walk: the leaves in order, and after each how many
 // finished pairs to add (bits of its path).
 struct PairwiseWalk {
-    int off[32], len[32];
-    bool right[32];  // frame's left half is done
-    int sp;
-    __device__ explicit PairwiseWalk(int n) : sp(0)
-    {
-        off[0] = 0;
-        len[0] = n;
-        right[0] = false;
-    }
+    int off[32], len[32];   // right halves still to come, the innermost last
+    int n_off = 0, o, m;    // the next node, none if m is 0
+    unsigned in_right = 0;  // whether it lies in the right half of its parent (bit 0), of that one's, ...
+    __device__ explicit PairwiseWalk(int n) : o(0), m(n) {}
     // The next leaf; false after the last.
-    __device__ bool next(int &o, int &m, int &adds)
+    __device__ bool next(int &leaf, int &size, int &adds)
     {
-        if (sp < 0)
+        if (m == 0)
             return false;
-        while (len[sp] > 128) {
-            off[sp + 1] = off[sp];
-            len[sp + 1] = half(len[sp]);
-            sp++;
-            right[sp] = false;
+        while (m > 128) {
+            const int half = m / 2 - m / 2 % 8;
+            off[n_off] = o + half;
+            len[n_off++] = m - half;
+            m = half;
+            in_right <<= 1;
         }
-        o = off[sp];
-        m = len[sp];
-        adds = 0;
-        sp--;
-        while (sp >= 0 && right[sp]) {  // this leaf ends the frame's right half
-            adds++;
-            sp--;
-        }
-        if (sp >= 0) {  // the frame's left half is done: its right half
-            right[sp] = true;
-            const int m2 = half(len[sp]);
-            off[sp + 1] = off[sp] + m2;
-            len[sp + 1] = len[sp] - m2;
-            sp++;
-            right[sp] = false;
+        leaf = o;
+        size = m;
+        adds = __ffs(~in_right) - 1;  // halves that this leaf ends
+        in_right >>= adds;
+        m = 0;
+        if (n_off) {
+            o = off[--n_off];
+            m = len[n_off];
+            in_right |= 1;
         }
         return true;
     }
-    static __device__ int half(int n) { return n / 2 - n / 2 % 8; }
 };
 
 // The squares of a[0:n), n <= 128, by 8 lanes (k = 0..7) of a warp.
