@@ -537,6 +537,8 @@ __device__ __forceinline__ void tc_issue(const TcBatch<N> &B, const long long *r
         const uint32_t a_base = (uint32_t)sdesc(w_base, 128, 128), b_base = (uint32_t)sdesc(d_base, col_bytes, 128);
         const uint32_t a_buf = (uint32_t)B.w_bytes >> 4, b_slot = (uint32_t)B.row_bytes >> 4;
         const size_t row0 = (size_t)t * SC;
+        const int chain_steps = SMALL ? 0 : pr.chain_steps;
+        uint32_t parts_log2 = (uint32_t)uniform(tc_pair_chains(L, step, L, chain_steps));
         for (int g0 = uniform(c_begin); g0 < c_end; g0 += 32) {
             // the scalars of 32 channels, one per lane
             const int cl = min(g0 + (int)(threadIdx.x & 31), c_end - 1);
@@ -545,7 +547,8 @@ __device__ __forceinline__ void tc_issue(const TcBatch<N> &B, const long long *r
             for (; active; active &= active - 1) {
                 const int src = __ffs(active) - 1;
                 const int mo = __shfl_sync(0xffffffffu, mo_l, src), ntap = __shfl_sync(0xffffffffu, n_l, src);
-                const uint32_t parts_log2 = SMALL ? 0 : (uint32_t)tc_pair_chains(L, step, ntap, pr.chain_steps);
+                if (VAR && chain_steps)
+                    parts_log2 = (uint32_t)tc_pair_chains(L, step, ntap, chain_steps);
                 uint32_t left = 0;  // column-block pairs left to the accumulator
                 uint32_t dt = 0, acc = 0;
                 const auto next_acc = [&]() {

@@ -361,10 +361,12 @@ __host__ __device__ __forceinline__ int tc_k_end(int s, int taps) { return (s + 
 // taps (the last phase has the fewest), so that none of the chains is empty.
 __host__ __device__ __forceinline__ int tc_pair_chains(int L, int step, int n, int chain_steps)
 {
-    const int least = (tc_phase_taps(L, step, step - 1, n) + TC_Q - 1) / TC_Q;
     int log2 = 0;
-    while (chain_steps && least > chain_steps << log2)
-        log2++;
+    if (chain_steps) {
+        const int least = (tc_phase_taps(L, step, step - 1, n) + TC_Q - 1) / TC_Q;
+        while (least > chain_steps << log2)
+            log2++;
+    }
     return log2;
 }
 
