@@ -1,7 +1,8 @@
 """Tile-shape autotuner of the tensor-core forms.
 
-Two shape parameters of ``tc_persistent`` (csrc/fmf_tc.cu) change its speed but
-not its results: the lag blocks per tile (NB = 32, 64 or 128; 128 outputs each)
+Two shape parameters of ``tc_persistent`` (csrc/fmf_tc.cu) change its speed, and of its
+results at most the last bits (the tiles decide into how many channel parts a small search
+is split, whose sums are then added): the lag blocks per tile (NB = 32, 64 or 128; 128 outputs each)
 and the number of templates whose items are interleaved in the tile queue
 (data rows and window statistics they share stay in L2 while the group sweeps
 the tiles).  ``tune`` times candidate shapes on a sample of a real search

@@ -181,8 +181,6 @@ int check_launch(const char *what);
 // that calls from several host threads with different needs cannot lower it
 // under one another's launch.
 constexpr int kMaxDynamicSmem = 227 * 1024;
-// Maps the host pages of a result buffer for writing before a copy into it
-// (parallel; a no-op where the kernel refuses).
 // Host outputs of this size are copied in pieces, each behind the next one's kernels.
 constexpr size_t kPieceBytes = (size_t)64 << 20;
 // Maps the pages of a host output, of a medium size on threads of its own from

@@ -49,11 +49,13 @@
 // taps 2.80 and 1.73e-7, 600 taps 4.1 and 3.5e-7, 1,200 taps 6.0 and 3.8e-7 (with chains of
 // 16 steps 2.1, 2.8, 4.7, 7.2, 7.3e-7); away from matches it is further below.
 //
-// What bounds it: the tensor pipe, and with it the power limit, from some 400
+// What bounds it: the tensor pipe, and with it the power limit, from some 500
 // taps (40 templates x 60 channels x 1.08M lags x 600 taps in 6.3 ms: 1.8
 // PFLOP/s of MMAs, 1.74 is what cuBLAS sustains under the limit); the issuing
-// threads and the epilogue below (60 taps: 3.8 ms with the preparation).  An issuing thread's code
-// costs as much as its MMAs: a branchy loop took 500 cycles per MMA of 64.
+// threads and the epilogue below, which takes some 400 cycles per chain (with the
+// preparation 300 taps 5.8 ms, 60 taps 4.3 ms; in chains of 16 steps 4.7 and 3.5 ms).
+// An issuing thread's code costs as much as its MMAs: a branchy loop took 500 cycles
+// per MMA of 64.
 //
 // Roles of a persistent CTA (12 warps, one CTA per SM), which takes items (one
 // template x NB*Q consecutive outputs, all channels or a part of them) from a
@@ -207,9 +209,10 @@ __device__ __forceinline__ void split_pair(float x, float inv_s, bool keep, uint
 // FP32: the scale of a data channel from the scan of prepare_problem, stat (largest
 // |x|; smallest window energy that can pass the threshold, complemented).  The
 // caller that is `first` also writes the channel's exponent and decides whether
-// the pairs hold its values: the error of a coefficient from them is at most
-// 2^-51 of the largest value over the root of the window's energy, so windows
-// down to 2^-42 of the largest value squared keep it at 1e-9.
+// the pairs hold its values.  A sample is off by 2^-51 of the largest value M at most, a
+// coefficient so by sqrt(L) 2^-51 M over the root of the window's energy (Cauchy-Schwarz):
+// windows down to 2^-42 M^2 keep it at sqrt(L) 2^-30, 2.3e-8 at 600 taps, and near 1e-9
+// where the samples' errors are independent.
 __device__ __forceinline__ float tc_channel_scale(const unsigned *stat, int ch, int SC, bool first, int *d_exp,
                                                   unsigned *skip)
 {
@@ -1570,8 +1573,9 @@ size_t tc_template_bytes(const Problem &P, int nb)
 // channels x 50 taps, 651 outputs: 55, 56, 58 us with 32, 64, 128; 39,984 outputs: 86,
 // 75, 70 us).
 //
-// Below kFp32LeastTaps the pairs' 22 bits show: the error against 64 bits is 1.4 of the
-// FMAs' at 10 taps, 1.08 at 40, 1.00 at 44 to 52 and falls to 0.6 at 300.
+// Below kFp32LeastTaps the pairs' 22 bits show: the RMS error against 64 bits is 1.4 of the
+// FMAs' at 10 taps, 1.08 at 40, 1.00 at 44 to 52 and falls to 0.4 at 300 (random searches; at
+// matches tc_chain_cols keeps it below theirs).
 int tc_fp32_nb(size_t T, size_t SC, size_t L, size_t step, size_t n_corr)
 {
     if (const char *env = getenv("FMF_TC32")) {  // 0: the CUDA cores; 32, 64, 128: this tile
@@ -1715,9 +1719,9 @@ static int tc_templates(TcSearch *full, int t0, int nt, unsigned long long *queu
 }
 
 // Templates [t0, t0 + nt) of a begun search: their operand blocks and the
-// persistent launch, a roomful at a time.  The channel parts of an FP32 search are
-// those of all its templates, so that its results do not depend on how they are
-// parted (a call with host arrays runs them in parts); the bf16 forms choose them
+// persistent launch, a roomful at a time.  The channel parts of an FP32 search and its
+// flag are those of all its templates, so that its results do not depend on how they
+// are parted (a call with host arrays runs them in parts); the bf16 forms choose them
 // for each launch, which keeps the SMs busier through the last few templates.
 int tc_run_templates(TcSearch *full, int t0, int nt, unsigned *err, cudaStream_t s)
 {

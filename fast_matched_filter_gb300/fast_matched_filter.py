@@ -334,7 +334,13 @@ def matched_filter_device(templates, sum_square_templates, moveouts, weights, da
     computed on the GPU as numpy.sum(templates**2, axis=-1) would), moveouts
     (T,S,C) int32, weights (T,S,C) f32, data (S,C,N) f32, out (T,n_corr) or
     (T,n_corr,S,C) f32.  Asynchronous on ``stream`` (a torch.cuda.Stream or
-    raw handle; default: torch's current stream).  Returns the launch count."""
+    raw handle; default: torch's current stream).  Returns the launch count.
+
+    Asynchronous errors: a wait inside the tensor-core kernel that gives up after 2 s
+    (FP32 searches of some size run there, too) leaves ``out`` incomplete, and only
+    ``fmf_device_errors()`` of the C library tells; the calls on host arrays check it.
+    The search's working arrays come from the device's default stream-ordered pool, which
+    keeps them for the next call (``fmf_release_cache()`` gives them back)."""
     import torch  # plumbing only: device memory and streams
 
     lib = _require_lib()

@@ -54,7 +54,11 @@ extern "C" {
 /* FP32: on the tensor cores as scaled fp16 pairs (22 bits) in searches large
  * enough (56 taps at least, of every channel of weight where the lengths
  * differ), with an RMS error no larger than that of FP32 multiply-adds; else,
- * and where the amplitudes do not fit such pairs, on the CUDA cores */
+ * and where the amplitudes do not fit such pairs, on the CUDA cores.  The tensor
+ * cores' operands take 4 bytes per sample of the data, up to 4 GiB of template
+ * blocks and 1 GiB of per-channel outputs from the device's default memory pool,
+ * which keeps them (fmf_release_cache); without memory for them a search runs on
+ * the CUDA cores. */
 #define FMF_PREC_FP32 0
 #define FMF_PREC_SPLIT_BF16 1 /* tensor cores, bf16 hi+lo, 3 products, FP32 accumulate */
 #define FMF_PREC_BF16 2       /* tensor cores, single bf16 product (loss demonstration) */
