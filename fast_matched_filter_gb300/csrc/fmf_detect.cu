@@ -38,12 +38,12 @@
 //   3. the median: if the window holds both middle ranks, the candidates' bins
 //      (counted as the pass ended) give the one or two that hold them; a read of the
 //      candidates gathers those bins' few values, and a block per row selects among
-//      them.  If a bin holds too many (ties), a radix selection over the candidates
-//      (passes of up to 11 bits over the key bits the window's keys do not share);
-//      if the window does not hold -- one that missed (about one row in 800), heavy
-//      ties, an adversarial row -- the same selection over the whole row.  A fixed
-//      grid of blocks takes these passes over the list of such rows, so that a row is
-//      read at the rate of the whole GPU;
+//      them.  If a bin holds too many (ties), the block takes a radix selection over
+//      the candidates (passes of up to 11 bits over the key bits the window's keys do
+//      not share); if the window does not hold -- one that missed (about one row in
+//      800), heavy ties, an adversarial row -- the same selection over the whole row.
+//      A fixed grid of blocks takes these passes over the list of such rows, so that a
+//      row is read at the rate of the whole GPU;
 //   4. the MAD: the sample keyed by |x - med| narrows [a_lo, a_hi]; the listed
 //      values keyed by |x - med| are counted below the window or gathered in
 //      it, and selected as in 3.  A row whose median or MAD window missed, or
@@ -82,6 +82,7 @@ constexpr int kDetPickBlocks = 152 * 8;   // blocks of the pass over the candida
 constexpr int kCandBins = 1024;           // bins of the candidates' window
 constexpr int kPickCap = 2048;            // candidates that share the middle ranks' bins
 constexpr int kDetRowBlocks = 152 * 4;    // the fixed grid of the passes over rows that fell back
+constexpr int kRowGroup = kDetThreads / 32;  // such rows that a block resolves at once
 
 // source of a row's radix selection
 constexpr int kSrcRow = 0;   // the row itself (fallback)
@@ -177,9 +178,9 @@ __device__ __forceinline__ RowSplit split_row(const float *row, long long n)
 
 // The rows that need more passes, and how far a pass has come.
 struct DetLists {
-    int *select, *n_select;  // rows selecting over key bits
+    int *select, *n_select;  // rows selecting over all their values
     int *peaks, *n_peaks;    // rows whose peaks were not gathered by the counting pass
-    unsigned *blocks;        // blocks of a selection pass that are through
+    unsigned *blocks;        // of every kRowGroup rows: blocks of a selection pass that are through
 };
 
 __device__ void init_row(DetState *st, int t, int n_corr, const int *begin, const int *end)
@@ -481,7 +482,9 @@ det_sample_kernel(const float *__restrict__ cc, size_t ld, DetState *st, int mod
         if (mode == 0)
             init_row(st, t, n_corr, lag_begin, lag_end);
         if (t == 0)
-            *lists.n_select = *lists.n_peaks = 0, *lists.blocks = 0;
+            *lists.n_select = *lists.n_peaks = 0;
+        if (t % kRowGroup == 0)
+            lists.blocks[t / kRowGroup] = 0;
     }
     __syncthreads();
     const int begin = st[t].begin;
@@ -1042,7 +1045,7 @@ __global__ void det_pick_kernel(DetState *__restrict__ st, const unsigned *__res
         s.n_cand = 0;
     if (lane == 0) {
         st[t] = s;
-        if (s.src == kSrcRow || s.src == kSrcKeys)
+        if (s.src == kSrcRow)
             lists.select[atomicAdd(lists.n_select, 1)] = t;
     }
 }
@@ -1088,22 +1091,85 @@ det_gather_kernel(DetState *__restrict__ st, const float *__restrict__ cand, lon
     }
 }
 
-// The middle keys of the list: one block per row.
-__global__ void __launch_bounds__(kDetThreads)
-det_finish_kernel(DetState *__restrict__ st, const unsigned *__restrict__ list, int mode, float n_mad)
+// The keys of ranks r[0] <= r[1] among a row's candidates, which share the bits `prefix` from
+// `top` up: radix passes by the block as in block_select2, each a read of the columns as
+// the counting pass wrote them (regions of 32, a warp each; no column overflowed).
+__device__ void columns_select2(const float *cand, const int *cnt, int regions, int Ck, int top, unsigned prefix,
+                                int r0, int r1, unsigned *hist, int *pick, unsigned &k0, unsigned &k1)
+{
+    unsigned pre[2] = {prefix, prefix};
+    int r[2] = {r0, r1};
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    for (int pass = 0; pass < 3; pass++) {
+        int shift, width;
+        pass_digit(top, pass, shift, width);
+        if (width == 0)
+            break;
+        const unsigned dmask = (1u << width) - 1u, high = above_mask(shift + width);
+        const bool two = pre[0] != pre[1];
+        for (int i = threadIdx.x; i < 2 * kDetBins; i += blockDim.x)
+            hist[i] = 0u;
+        __syncthreads();
+        for (int q = warp; q < regions; q += blockDim.x >> 5) {
+            const float *kc = cand + (size_t)q * Ck * 32 + 8 * lane;
+            const int m = cnt[q * 32 + lane], mw = __reduce_max_sync(0xffffffffu, m);
+            for (int k = 0; k < mw; k += 8) {
+                float x[8] = {};
+                if (k < m)
+                    load_sector(kc, k, x);
+#pragma unroll
+                for (int j = 0; j < 8; j++) {
+                    // v + 0: the counting pass compares floats, where -0 and +0 are one value
+                    const unsigned key = order_key(__fadd_rn(x[j], 0.0f)), dig = (key >> shift) & dmask;
+                    for (int s = 0; s < (two ? 2 : 1); s++) {
+                        const bool in = k + j < m && (key & high) == pre[s];
+                        const unsigned g = __match_any_sync(0xffffffffu, in ? dig : 0xffffffffu);  // (ties)
+                        if (in && (__ffs(g) - 1) == lane)
+                            atomicAdd(&hist[s * kDetBins + dig], __popc(g));
+                    }
+                }
+            }
+        }
+        __syncthreads();
+        if (warp < 2)
+            find_rank(hist + (two ? warp : 0) * kDetBins, (unsigned)r[warp], lane, pick + 2 * warp);
+        __syncthreads();
+        for (int s = 0; s < 2; s++) {
+            pre[s] |= (unsigned)pick[2 * s] << shift;
+            r[s] -= pick[2 * s + 1];
+        }
+        __syncthreads();
+    }
+    k0 = pre[0];
+    k1 = pre[1];
+}
+
+// The middle keys of the list, or of all candidates where the middle ranks' bins hold too
+// many (a value that the row holds thousands of times, as the zeros of a gap): one block
+// per row.  (These were passes of the whole GPU over one row after the other: 500 rows of
+// a million values, 1 % of them zeros, took 17.9 ms, 1.01 ms here.)
+__global__ void __launch_bounds__(kDetThreads, 4)
+det_finish_kernel(DetState *__restrict__ st, const unsigned *__restrict__ list, const float *__restrict__ cand,
+                  long long cap, Lanes g, int mode, float n_mad)
 {
     __shared__ unsigned sk[kPickCap];
     __shared__ unsigned hist[2 * kDetBins];
     __shared__ int pick[4];
     const int t = blockIdx.x;
-    if (st[t].src != kSrcPick)
-        return;
-    const int n = min(st[t].n_list, kPickCap), r0 = st[t].rank[0], r1 = st[t].rank[1];
-    for (int i = threadIdx.x; i < n; i += kDetThreads)
-        sk[i] = list[(size_t)t * kPickCap + i];
-    __syncthreads();
+    const int from = st[t].src, r0 = st[t].rank[0], r1 = st[t].rank[1];
     unsigned k0, k1;
-    block_select2(sk, n, r0, r1, hist, pick, k0, k1);
+    if (from == kSrcPick) {
+        const int n = min(st[t].n_list, kPickCap);
+        for (int i = threadIdx.x; i < n; i += blockDim.x)
+            sk[i] = list[(size_t)t * kPickCap + i];
+        __syncthreads();
+        block_select2(sk, n, r0, r1, hist, pick, k0, k1);
+    } else if (from == kSrcKeys) {
+        columns_select2(cand + (size_t)t * cap, g.cnt_k + (size_t)t * g.S * kDetThreads, g.S * (kDetThreads / 32), g.Ck,
+                        st[t].top, st[t].prefix[0], r0, r1, hist, pick, k0, k1);
+    } else {
+        return;
+    }
     if (threadIdx.x == 0) {
         DetState s = st[t];
         finish_select(s, mode, middle_value(k0, k1, s.end - s.begin), n_mad);
@@ -1121,9 +1187,7 @@ __device__ __forceinline__ void hist_add(unsigned *h, float v, bool ok, int mode
                                          unsigned dmask, unsigned high, unsigned p0, unsigned p1,
                                          bool two, int lane, bool aggregate)
 {
-    // mode 2: a candidate, keyed as v + 0 (the counting pass compares floats, where
-    // -0 and +0 are one value)
-    const unsigned key = mode == 2 ? order_key(__fadd_rn(v, 0.0f)) : sel_key(v, mode, med);
+    const unsigned key = sel_key(v, mode, med);
     const unsigned dig = (key >> shift) & dmask;
     const bool m0 = ok && (key & high) == p0;
     const bool m1 = two && ok && (key & high) == p1;
@@ -1151,7 +1215,7 @@ __device__ __forceinline__ void hist_add(unsigned *h, float v, bool ok, int mode
 // Picks each rank's bucket from the pass's histogram of row t (one warp),
 // clears the histogram, and after the last pass turns the two keys into the
 // median (mode 0) or the MAD and the threshold (mode 1).
-__device__ void resolve_row(DetState *st, unsigned *hist, int t, int lane, int pass, int mode, float n_mad)
+__device__ __noinline__ void resolve_row(DetState *st, unsigned *hist, int t, int lane, int pass, int mode, float n_mad)
 {
     DetState s = st[t];
     const int n = s.end - s.begin;
@@ -1160,44 +1224,54 @@ __device__ void resolve_row(DetState *st, unsigned *hist, int t, int lane, int p
     if (width == 0)
         return;  // the key was complete after an earlier pass
     unsigned *gh = hist + (size_t)t * 2 * kDetBins;
-    const int per = kDetBins / 32;  // bins per lane (digits of fewer bits leave the rest empty)
     const bool two = s.prefix[0] != s.prefix[1];
+    constexpr int kParts = kDetBins / 128;  // of four bins a lane
     for (int r = 0; r < 2; r++) {
-        const unsigned *h = gh + (two ? r : 0) * kDetBins;
-        unsigned sum = 0;
-        for (int i = 0; i < per; i++)
-            sum += h[lane * per + i];
+        const uint4 *h = reinterpret_cast<const uint4 *>(gh + (two ? r : 0) * kDetBins) + lane;
+        const unsigned rk = (unsigned)s.rank[r];
+        unsigned before = 0;
+        int part = kParts - 1;  // the part that holds the rank, `before` below it
+        unsigned run = 0;
+        for (int q0 = 0; q0 < kParts; q0 += 4) {
+            uint4 v[4];
+#pragma unroll
+            for (int q = 0; q < 4; q++)
+                v[q] = __ldcg(h + 32 * (q0 + q));
+#pragma unroll
+            for (int q = 0; q < 4; q++) {
+                const unsigned sum = __reduce_add_sync(0xffffffffu, v[q].x + v[q].y + v[q].z + v[q].w);
+                if (rk >= run && rk < run + sum) {
+                    part = q0 + q;
+                    before = run;
+                }
+                run += sum;
+            }
+        }
+        const uint4 v = __ldcg(h + 32 * part);
+        const unsigned bins[4] = {v.x, v.y, v.z, v.w}, sum = v.x + v.y + v.z + v.w;
         unsigned inc = sum;
         for (int o = 1; o < 32; o <<= 1) {
             const unsigned y = __shfl_up_sync(0xffffffffu, inc, o);
             if (lane >= o)
                 inc += y;
         }
-        const unsigned exc = inc - sum;
-        const unsigned rk = (unsigned)s.rank[r];
-        const unsigned found = __ballot_sync(0xffffffffu, rk >= exc && rk < inc);
+        unsigned c = before + inc - sum;
+        const unsigned found = __ballot_sync(0xffffffffu, rk >= c && rk < c + sum);
         const int src = found ? __ffs(found) - 1 : 0;
-        unsigned bin = 0, before = 0;
-        if (lane == src) {
-            unsigned c = exc;
-            int i = 0;
-            for (; i < per - 1; i++) {
-                const unsigned hv = h[lane * per + i];
-                if (rk < c + hv)
-                    break;
-                c += hv;
+        int i = 0;
+#pragma unroll
+        for (int j = 0; j < 3; j++)
+            if (i == j && rk >= c + bins[j]) {
+                c += bins[j];
+                i = j + 1;
             }
-            bin = (unsigned)(lane * per + i);
-            before = c;
-        }
-        bin = __shfl_sync(0xffffffffu, bin, src);
-        before = __shfl_sync(0xffffffffu, before, src);
+        const unsigned bin = __shfl_sync(0xffffffffu, (unsigned)(part * 128 + 4 * lane + i), src);
         s.prefix[r] |= bin << shift;
-        s.rank[r] = (int)(rk - before);
+        s.rank[r] = (int)(rk - __shfl_sync(0xffffffffu, c, src));
     }
     __syncwarp();
-    for (int i = lane; i < 2 * kDetBins; i += 32)
-        gh[i] = 0u;
+    for (int i = lane; i < 2 * kDetBins / 4; i += 32)
+        reinterpret_cast<uint4 *>(gh)[i] = make_uint4(0u, 0u, 0u, 0u);
     if (shift == 0)
         finish_select(s, mode, middle_value(s.prefix[0], s.prefix[1], n), n_mad);
     if (lane == 0)
@@ -1205,62 +1279,55 @@ __device__ void resolve_row(DetState *st, unsigned *hist, int t, int lane, int p
 }
 
 // One selection pass by key bits: histogram of the current digit over the keys whose
-// higher bits equal a rank's prefix, for the rows that fell back to selection over the
-// whole row (a sample window that missed, a column that overflowed) and those with too
-// many candidates in one bin (each thread then reads columns as the counting pass
-// wrote them).  Every block of a fixed grid takes a slice of each such row in turn, so
-// a row that fell back is read at the rate of the whole GPU, not of its own few
-// blocks.  mode 0 keys the values, mode 1 |x - median|; equal digits are aggregated
-// per warp in the first pass over a row (its keys share their high digits).  The block
-// that is through last picks the rows' buckets.
-__global__ void __launch_bounds__(kDetThreads)
+// higher bits equal a rank's prefix, for the rows that fell back to selection over all
+// their values (a sample window that missed, a column that overflowed).  Every block of a
+// fixed grid takes a slice of each such row in turn, so a row that fell back is read at
+// the rate of the whole GPU, not of its own few blocks.  mode 0 keys the values, mode 1
+// |x - median|; equal digits are aggregated per warp in the first pass (a row's keys share
+// their high digits).  The block that is through with a group of rows last picks their
+// buckets, a warp per row; the blocks begin at different groups, so that different blocks
+// are the last ones, side by side.  (64 rows of a million values, 30 % of them zeros: 2.52
+// ms with one last block for all rows, 1.75 ms here.)
+__global__ void __launch_bounds__(kDetThreads, 4)  // the whole grid at once
 det_hist_row_kernel(const float *__restrict__ cc, size_t ld, DetState *st, const DetLists lists,
-                    unsigned *hist, const float *__restrict__ cand, long long cap, Lanes g, int pass, int mode,
-                    float n_mad)
+                    unsigned *hist, int pass, int mode, float n_mad)
 {
     __shared__ unsigned h[2 * kDetBins];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     constexpr int kWarps = kDetThreads / 32;
     __shared__ bool last;
     const int *const list = lists.select;
-    const int nrows = *lists.n_select;
-    if (nrows == 0)
-        return;  // every block
-    for (int k = 0; k < nrows; k++) {
-        const int t = list[k];
-        const DetState s = st[t];
-        const long long n = s.end - s.begin;
-        if (n <= 0)
-            continue;
-        int shift, width;
-        pass_digit(s.top, pass, shift, width);
-        if (width == 0)
-            continue;
-        const unsigned dmask = (1u << width) - 1u;
-        const unsigned high = above_mask(shift + width);
-        const unsigned p0 = s.prefix[0], p1 = s.prefix[1];
-        const bool two = p0 != p1;
-        const bool agg = pass == 0;
-        for (int i = threadIdx.x; i < 2 * kDetBins; i += kDetThreads)
-            h[i] = 0u;
-        __syncthreads();
-        if (s.src == kSrcKeys) {
-            for (int r = (int)blockIdx.x * kWarps + warp; r < g.S * kWarps; r += (int)gridDim.x * kWarps) {
-                const float *kc = cand + (size_t)t * cap + (size_t)r * g.Ck * 32 + 8 * lane;
-                const int m = g.cnt_k[((size_t)t * g.S * kWarps + r) * 32 + lane];  // <= Ck: no column overflowed
-                const int mw = __reduce_max_sync(0xffffffffu, m);
-                for (int j = 0; j < mw; j++)
-                    hist_add(h, j < m ? kc[(j & ~7) * 32 + (j & 7)] : 0.0f, j < m, 2, s.med, shift, dmask, high, p0, p1, two,
-                             lane, true);
-            }
-        } else {
-            const float *row = cc + (size_t)t * ld + s.begin;
+    const int nrows = *lists.n_select, groups = (nrows + kRowGroup - 1) / kRowGroup;
+    int group = (int)((long long)blockIdx.x * groups / gridDim.x);
+    for (int turn = 0; turn < groups; turn++) {
+        const int k0 = group * kRowGroup, k1 = min(k0 + kRowGroup, nrows);
+        for (int k = k0; k < k1; k++) {
+            const int t = list[k];
+            // (all of the row's fields on their way at once)
+            const int begin = __ldcg(&st[t].begin), end = __ldcg(&st[t].end), top = __ldcg(&st[t].top);
+            const unsigned p0 = __ldcg(&st[t].prefix[0]), p1 = __ldcg(&st[t].prefix[1]);
+            const float med = __ldcg(&st[t].med);
+            const long long n = end - begin;
+            if (n <= 0)
+                continue;
+            int shift, width;
+            pass_digit(top, pass, shift, width);
+            if (width == 0)
+                continue;
+            const unsigned dmask = (1u << width) - 1u;
+            const unsigned high = above_mask(shift + width);
+            const bool two = p0 != p1;
+            const bool agg = pass == 0;
+            for (int i = threadIdx.x; i < 2 * kDetBins; i += kDetThreads)
+                h[i] = 0u;
+            __syncthreads();
+            const float *row = cc + (size_t)t * ld + begin;
             const RowSplit rs = split_row(row, n);
             if (blockIdx.x == 0 && warp == 0) {  // the unaligned ends, at most 3 + 3 values
                 const long long i = lane < rs.head ? lane : rs.head + 4 * rs.nvec + (lane - rs.head);
                 const bool ok = lane < rs.head + rs.tail;
                 const float v = ok ? row[i] : 0.f;
-                hist_add(h, v, ok, mode, s.med, shift, dmask, high, p0, p1, two, lane, agg);
+                hist_add(h, v, ok, mode, med, shift, dmask, high, p0, p1, two, lane, agg);
             }
             const float4 *vrow = reinterpret_cast<const float4 *>(row + rs.head);
             const long long steps = (rs.nvec + 63) / 64;  // 64 float4s per warp step
@@ -1276,34 +1343,36 @@ det_hist_row_kernel(const float *__restrict__ cc, size_t ld, DetState *st, const
                 }
 #pragma unroll
                 for (int u = 0; u < 2; u++) {
-                    hist_add(h, v[u].x, ok[u], mode, s.med, shift, dmask, high, p0, p1, two, lane, agg);
-                    hist_add(h, v[u].y, ok[u], mode, s.med, shift, dmask, high, p0, p1, two, lane, agg);
-                    hist_add(h, v[u].z, ok[u], mode, s.med, shift, dmask, high, p0, p1, two, lane, agg);
-                    hist_add(h, v[u].w, ok[u], mode, s.med, shift, dmask, high, p0, p1, two, lane, agg);
+                    hist_add(h, v[u].x, ok[u], mode, med, shift, dmask, high, p0, p1, two, lane, agg);
+                    hist_add(h, v[u].y, ok[u], mode, med, shift, dmask, high, p0, p1, two, lane, agg);
+                    hist_add(h, v[u].z, ok[u], mode, med, shift, dmask, high, p0, p1, two, lane, agg);
+                    hist_add(h, v[u].w, ok[u], mode, med, shift, dmask, high, p0, p1, two, lane, agg);
                 }
             }
+            __syncthreads();
+            unsigned *gh = hist + (size_t)t * 2 * kDetBins;
+            for (int i = threadIdx.x; i < (two ? 2 : 1) * kDetBins; i += kDetThreads) {
+                const unsigned c = h[i];
+                if (c)
+                    atomicAdd(gh + i, c);
+            }
+            __syncthreads();  // h is cleared for the next row
         }
+        __threadfence();
         __syncthreads();
-        unsigned *gh = hist + (size_t)t * 2 * kDetBins;
-        for (int i = threadIdx.x; i < (two ? 2 : 1) * kDetBins; i += kDetThreads) {
-            const unsigned c = h[i];
-            if (c)
-                atomicAdd(gh + i, c);
+        if (threadIdx.x == 0)
+            last = atomicAdd(lists.blocks + group, 1u) == gridDim.x - 1;
+        __syncthreads();
+        if (last) {
+            __threadfence();
+            if (k0 + warp < k1)
+                resolve_row(st, hist, list[k0 + warp], lane, pass, mode, n_mad);
+            if (threadIdx.x == 0)
+                lists.blocks[group] = 0;  // for the next pass
         }
-        __syncthreads();  // h is cleared for the next row
+        if (++group == groups)
+            group = 0;
     }
-    __threadfence();
-    __syncthreads();
-    if (threadIdx.x == 0)
-        last = atomicAdd(lists.blocks, 1u) == gridDim.x - 1;
-    __syncthreads();
-    if (!last)
-        return;
-    __threadfence();
-    for (int k = warp; k < nrows; k += kWarps)
-        resolve_row(st, hist, list[k], lane, pass, mode, n_mad);
-    if (threadIdx.x == 0)
-        *lists.blocks = 0;  // for the next pass
 }
 
 // The local maxima among a row's hot values (at or above thr_lo), one block
@@ -1562,7 +1631,7 @@ int detect_device(const float *cc, int T, int n_corr, size_t ld, const int *begi
         (rc = ws.get(&col_cnt, 2 * ((size_t)kDetBlocks + chunk) * kDetThreads, "list column counts")) ||
         (rc = ws.get(&bins, (size_t)chunk * kCandBins, "candidate bins")) ||
         (rc = ws.get(&list, (size_t)chunk * kPickCap, "picked candidates")) ||
-        (rc = ws.get(&row_list, 2 * (size_t)chunk + 3, "rows of further passes")))
+        (rc = ws.get(&row_list, 3 * (size_t)chunk + 2, "rows of further passes")))
         return rc;
     cudaError_t e = cudaFuncSetAttribute(det_select_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          (int)select_smem(kDetCap));
@@ -1603,7 +1672,7 @@ int detect_device(const float *cc, int T, int n_corr, size_t ld, const int *begi
         g.cnt_a = col_cnt + ((size_t)kDetBlocks + chunk) * kDetThreads;
         const bool few = nt <= kDetFewRows;
         const DetLists lists{row_list, row_list + 2 * chunk, row_list + chunk, row_list + 2 * chunk + 1,
-                             reinterpret_cast<unsigned *>(row_list + 2 * chunk + 2)};
+                             reinterpret_cast<unsigned *>(row_list + 2 * chunk + 2)};  // (one per kRowGroup rows)
         // mode 0, the median: sample, the one read of the rows, selection over the candidates;
         // mode 1, the MAD: the sample about the exact median, the listed values, selection
         for (int mode = 0; mode < 2; mode++) {
@@ -1615,10 +1684,9 @@ int detect_device(const float *cc, int T, int n_corr, size_t ld, const int *begi
                 rows, ld, st, keys, key_cap, amb, amb_cap, g, bins, hot, kDetCap);
             det_pick_kernel<<<nt, 32, 0, s>>>(st, bins, mode, kDetCap, n_mad, lists);
             det_gather_kernel<<<pick_grid, kDetThreads, 0, s>>>(st, keys, key_cap, g, list);
-            det_finish_kernel<<<nt, kDetThreads, 0, s>>>(st, list, mode, n_mad);
+            det_finish_kernel<<<nt, kDetThreads, 0, s>>>(st, list, keys, key_cap, g, mode, n_mad);
             for (int pass = 0; pass < 3; pass++)
-                det_hist_row_kernel<<<kDetRowBlocks, kDetThreads, 0, s>>>(rows, ld, st, lists, hist, keys, key_cap, g,
-                                                                          pass, mode, n_mad);
+                det_hist_row_kernel<<<kDetRowBlocks, kDetThreads, 0, s>>>(rows, ld, st, lists, hist, pass, mode, n_mad);
         }
         det_hot_kernel<<<nt, kDetThreads, 0, s>>>(rows, ld, st, hot, kDetCap, cand, kDetCap, lists);
         det_peaks_kernel<<<kDetRowBlocks, kDetThreads, 0, s>>>(rows, ld, st, lists.peaks, lists.n_peaks, cand, kDetCap);

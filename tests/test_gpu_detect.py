@@ -210,3 +210,18 @@ def test_detect_equal_values_at_the_median(n, share):
     cc[1] += np.float32(0.25)
     cc[2, ::1000] = np.float32(3.0)
     assert_matches(fmf.detect(cc, n_mad=8.0, min_separation=25, max_detections=512), cc, 8.0, 25, 512)
+
+
+@pytest.mark.parametrize("share", [0.004, 0.03, 0.3])
+@pytest.mark.parametrize("T", [8, 9, 70])
+def test_detect_many_rows_with_a_gap(T, share):
+    """Rows that all select among their candidates by key bits, or all over their values, in
+    groups of eight: one group, one more row, several."""
+    rng = np.random.default_rng(T)
+    n = 70001
+    cc = (rng.standard_normal((T, n)) * 0.01).astype(np.float32)
+    cc[:, 3000:3000 + int(n * share)] = 0.0
+    cc[:, ::5000] += np.float32(1.0)
+    cc[T // 2] = np.float32(0.5)
+    cc[T - 1] = (rng.standard_normal(n) * 0.01).astype(np.float32)
+    assert_matches(fmf.detect(cc, n_mad=8.0, min_separation=25, max_detections=64), cc, 8.0, 25, 64)
