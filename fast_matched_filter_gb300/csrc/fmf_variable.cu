@@ -797,29 +797,45 @@ static int variable_entry(const VArgs &a, void *stream)
     // the longest template (stride of the template array), and the shortest of weight
     int L = 0, shortest = INT_MAX;
     std::vector<int> lengths;
-    std::vector<float> weights;
     const int *ntap = a.ntap;
-    const float *w = a.w;
     if (dev) {
         try {
             lengths.resize(n_meta);
-            weights.resize(n_meta);
         } catch (const std::bad_alloc &) {
             return set_error(FMF_ERR_OOM, "host memory for the template lengths");
         }
         cudaError_t e = cudaMemcpyAsync(lengths.data(), a.ntap, n_meta * sizeof(int), cudaMemcpyDeviceToHost, s);
         if (e == cudaSuccess)
-            e = cudaMemcpyAsync(weights.data(), a.w, n_meta * sizeof(float), cudaMemcpyDeviceToHost, s);
-        if (e == cudaSuccess)
             e = cudaStreamSynchronize(s);
         if (e != cudaSuccess)
             return set_error(FMF_ERR_CUDA, "reading the template lengths: %s", cudaGetErrorString(e));
         ntap = lengths.data();
-        w = weights.data();
     }
     for (size_t i = 0; i < n_meta; i++) {
         L = ntap[i] > L ? ntap[i] : L;
-        shortest = w[i] != 0.0f && ntap[i] < shortest ? ntap[i] : shortest;
+        shortest = ntap[i] < shortest ? ntap[i] : shortest;
+    }
+    const int precision = FMF_FLAG_PRECISION_OF(a.flags);
+    if (shortest < (int)kFp32LeastTaps && L >= (int)kFp32LeastTaps &&
+        (precision == FMF_PREC_FP32 || precision == FMF_PREC_AUTO)) {  // its weight may be 0
+        std::vector<float> weights;
+        const float *w = a.w;
+        if (dev) {
+            try {
+                weights.resize(n_meta);
+            } catch (const std::bad_alloc &) {
+                return set_error(FMF_ERR_OOM, "host memory for the weights");
+            }
+            cudaError_t e = cudaMemcpyAsync(weights.data(), a.w, n_meta * sizeof(float), cudaMemcpyDeviceToHost, s);
+            if (e == cudaSuccess)
+                e = cudaStreamSynchronize(s);
+            if (e != cudaSuccess)
+                return set_error(FMF_ERR_CUDA, "reading the weights: %s", cudaGetErrorString(e));
+            w = weights.data();
+        }
+        shortest = INT_MAX;
+        for (size_t i = 0; i < n_meta; i++)
+            shortest = w[i] != 0.0f && ntap[i] < shortest ? ntap[i] : shortest;
     }
     if (L < 1 || (size_t)L > a.N)
         return set_error(FMF_ERR_ARG, "longest template %d not in [1, N]", L);
