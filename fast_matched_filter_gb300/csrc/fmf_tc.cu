@@ -74,6 +74,7 @@
 // TMEM: H0, H1, S0, S1 of 128 columns each: all 512.
 // Every wait is bounded (globaltimer); on timeout the CTA raises an error
 // word, stops issuing, waits for its own copies/MMAs (bounded) and frees TMEM.
+#include <algorithm>
 #include <cfloat>
 #include <cmath>
 #include <cstdlib>
@@ -1589,17 +1590,28 @@ int tc_fp32_nb(size_t T, size_t SC, size_t L, size_t step, size_t n_corr)
     // a tile of 4,096 outputs per block, two blocks per SM, groups of 20 taps per phase
     const double taps = (double)step * (double)((((L + step - 1) / step + 19) / 20) * 20);
     const double tiles = (double)T * (double)((n_corr + 4095) / 4096) / 304.0;
-    const double plain_us = (double)SC * ((taps * 0.0165 + (double)step * 1.45 + 1.9) * (tiles < 1.0 ? 1.0 : tiles) +
-                                          taps * 0.03 * tiles);
+    const double outputs = (double)T * (double)n_corr / (304.0 * 4096.0);
+    const double phases = std::min((double)step * 1.45 + 1.9, (double)step * 1.14 + 3.6);
+    const double plain_us = (double)SC * ((taps * 0.0165 + phases) * (tiles < 1.0 ? 1.0 : tiles) +
+                                          taps * 0.03 * (step > 3 ? outputs : tiles));
     if (plain_us < 50.0)
         return 0;
     const int want = n_corr > 8192 ? 128 : (n_corr > 4096 ? 64 : 32);
-    for (int nb = want; nb >= 32; nb >>= 1) {
-        const int fit = tc_choose_nb((int)L, (int)step, 1, nb);
-        if (fit)
-            return fit;
-    }
-    return 0;
+    int nb = 0;
+    for (int i = want; i >= 32 && !nb; i >>= 1)
+        nb = tc_choose_nb((int)L, (int)step, 1, i);
+    if (!nb)
+        return 0;
+    // Many templates of few lags: a tile holds little, and each costs 2.7 us and more per
+    // channel and phase.  (100 templates x 9 channels x 300 lags, step 20, 300 taps: 319 us
+    // on the CUDA cores, 397 here; 10 templates x 3 channels 128 and 114; the line is within
+    // 10 % of the faster side in 240 searches of steps 3 to 200.)
+    const long long items = (long long)T * (long long)((n_corr + 128 * (size_t)nb - 1) / (128 * (size_t)nb));
+    double rounds = 1e300;  // of whole items on the busiest SM, in the best number of channel parts
+    for (long long k = 1; k <= TC_MAX_PARTS && k <= (long long)SC; k++)
+        rounds = std::min(rounds, (double)((k * items + 151) / 152) / (double)k);
+    const double used = (double)std::min(step, L), tc_us = 50.0 + rounds * (double)SC * used * (2.7 + 0.0066 * (double)L / used);
+    return plain_us + 21.0 < tc_us ? 0 : nb;
 }
 
 // Column-block pairs of one h h chain of an FP32 search, and the K steps (least of the pairs')

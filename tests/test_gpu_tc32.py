@@ -304,3 +304,12 @@ def test_per_channel_lengths_by_the_shortest_of_weight(monkeypatch, shortest, we
             *[x.data_ptr() for x in g[:5]], 1, g[5].data_ptr(), 9000, 2, 3, 2, 8851, out.data_ptr(), 0,
             _lib.FLAG_DEVICE_POINTERS, None), lib)
     assert _ran() == ran
+
+
+@pytest.mark.parametrize("T,SC,L,step,n_corr,ran", [(100, 9, 300, 20, 300, 0), (10, 9, 300, 20, 300, 1),
+                                                    (100, 9, 300, 20, 5000, 1), (100, 9, 1600, 20, 300, 1)])
+def test_many_templates_of_few_lags_stay_on_the_cuda_cores(T, SC, L, step, n_corr, ran):
+    """A search on either side of the line by each of its sizes."""
+    tp, mo, w, d = random_search(41, T, SC, 1, L, n_corr * step + L - 1, 0, 50, plant=False)
+    fmf.matched_filter(tp, mo, w, d, step, check_zeros=False)
+    assert _ran() == ran
