@@ -425,8 +425,8 @@ __device__ __forceinline__ void tc_template_block(const TcTemplateWork &w, long 
         __syncthreads();
     }
     const int m0 = w.mo[row];
-    const int per_phase = NW * 8;
-    for (int i = threadIdx.x; i < step * per_phase; i += blockDim.x) {
+    const int per_phase = NW * 8, used = tc_phases(step, L) * per_phase;
+    for (int i = threadIdx.x; i < used; i += blockDim.x) {
         const int phi = i / per_phase, ne = i - phi * per_phase;
         int psi;
         const int s = tc_phase(m0 + phi, step, psi) & (TC_Q - 1);
@@ -542,6 +542,7 @@ __device__ __forceinline__ void tc_issue(const TcBatch<N> &B, const long long *r
         const uint32_t a_buf = (uint32_t)B.w_bytes >> 4, b_slot = (uint32_t)B.row_bytes >> 4;
         const size_t row0 = (size_t)t * SC;
         const int chain_steps = SMALL ? 0 : pr.chain_steps;
+        int phases = uniform(tc_phases(step, L));
         uint32_t parts_log2 = (uint32_t)uniform(tc_pair_chains(L, step, L, chain_steps));
         for (int g0 = uniform(c_begin); g0 < c_end; g0 += 32) {
             // the scalars of 32 channels, one per lane
@@ -551,6 +552,8 @@ __device__ __forceinline__ void tc_issue(const TcBatch<N> &B, const long long *r
             for (; active; active &= active - 1) {
                 const int src = __ffs(active) - 1;
                 const int mo = __shfl_sync(0xffffffffu, mo_l, src), ntap = __shfl_sync(0xffffffffu, n_l, src);
+                if (VAR)
+                    phases = tc_phases(step, ntap);
                 if (VAR && chain_steps)
                     parts_log2 = (uint32_t)tc_pair_chains(L, step, ntap, chain_steps);
                 uint32_t left = 0;  // column-block pairs left to the accumulator
@@ -562,10 +565,10 @@ __device__ __forceinline__ void tc_issue(const TcBatch<N> &B, const long long *r
                     tc_fence_after();
                     dt = tmem + (SMALL ? 256u : 0u) + 128u * (acc_i & 1);
                     acc = 0;
-                    left = SMALL ? (uint32_t)step * (TC_CB / 2) : (parts_log2 ? 1u : chain_cols);
+                    left = SMALL ? (uint32_t)phases * (TC_CB / 2) : (parts_log2 ? 1u : chain_cols);
                     return true;
                 };
-                for (int phi = 0; phi < step; phi++, stages++) {
+                for (int phi = 0; phi < phases; phi++, stages++) {
                     const uint32_t wb = stages & 1;
                     int psi;
                     const uint32_t sres = (uint32_t)tc_phase(mo + phi, step, psi) & (TC_Q - 1);
@@ -618,7 +621,7 @@ __device__ __forceinline__ void tc_issue(const TcBatch<N> &B, const long long *r
                             }
                         }
                         issue(n);
-                        const bool done = --left == 0 || (!SMALL && j == TC_CB / 2 - 1 && phi == step - 1);
+                        const bool done = --left == 0 || (!SMALL && j == TC_CB / 2 - 1 && phi == phases - 1);
                         if (one) {
                             if (j & 1)
                                 mma_commit(bar + TcBars::dempty + 8 * slot);
@@ -745,18 +748,19 @@ __global__ void __launch_bounds__(tc_threads(VAR), 1) tc_persistent(const __grid
             const long long I0 = (long long)tile * TC_Q * pr.nb;
             if (!tc_busy(pr, I0, t))
                 continue;
-            const int SC = P.SC, step = P.step;
+            const int SC = P.SC, step = P.step, all_phases = tc_phases(P.step, P.L);
             const uint32_t col_bytes = (uint32_t)pr.R * 16, wbytes = (uint32_t)pr.NW * 128;
             const size_t row0 = (size_t)t * SC;
             for (int g0 = c_begin; ok && g0 < c_end; g0 += 32) {
                 // the scalars of 32 channels, one per lane
                 const int cl = min(g0 + lane, c_end - 1);
-                const int mo_l = P.mo[row0 + cl];
+                const int mo_l = P.mo[row0 + cl], n_l = VAR ? P.ntap[row0 + cl] : 0;
                 uint32_t active = __ballot_sync(0xffffffffu, g0 + lane < c_end && P.w[row0 + cl] != 0.0f);
                 for (; ok && active; active &= active - 1) {
                     const int from = __ffs(active) - 1, ch = g0 + from;
                     const int mo = __shfl_sync(0xffffffffu, mo_l, from);
-                    for (int phi = 0; ok && phi < step; phi++, stages++) {
+                    const int phases = VAR ? tc_phases(step, __shfl_sync(0xffffffffu, n_l, from)) : all_phases;
+                    for (int phi = 0; ok && phi < phases; phi++, stages++) {
                         const int wb = stages & 1;
                         int psi;
                         const int mu = tc_phase(mo + phi, step, psi);
@@ -953,8 +957,8 @@ __global__ void __launch_bounds__(tc_threads(VAR), 1) tc_persistent(const __grid
             const size_t row0 = (size_t)t * SC;
             // h h chains of a channel: of whole pairs, or several of each
             const auto chains_of = [&](int n) {
-                const int log2 = tc_pair_chains(pr.P.L, step, n, pr.chain_steps);
-                return log2 ? (step * (TC_CB / 2)) << log2 : (step * (TC_CB / 2) + pr.chain_cols - 1) / pr.chain_cols;
+                const int log2 = tc_pair_chains(pr.P.L, step, n, pr.chain_steps), cols = tc_phases(step, n) * (TC_CB / 2);
+                return log2 ? cols << log2 : (cols + pr.chain_cols - 1) / pr.chain_cols;
             };
             const int chains = ONE || VAR ? 1 : chains_of(pr.P.L);
             for (int g0 = c_begin; busy && g0 < c_end; g0 += 32) {

@@ -353,6 +353,9 @@ __host__ __device__ __forceinline__ int tc_phase_taps(int L, int step, int phi, 
     return own < all ? own : all;
 }
 
+// Phases of a channel that uses the first n taps: those past its taps hold none.
+__host__ __device__ __forceinline__ int tc_phases(int step, int n) { return n < step ? (n < 1 ? 1 : n) : step; }
+
 // End of the K range of a phase with moveout residual s (its start is s & ~15).
 __host__ __device__ __forceinline__ int tc_k_end(int s, int taps) { return (s + taps + TC_Q - 1 + 15) & ~15; }
 

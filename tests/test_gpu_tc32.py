@@ -313,3 +313,27 @@ def test_many_templates_of_few_lags_stay_on_the_cuda_cores(T, SC, L, step, n_cor
     tp, mo, w, d = random_search(41, T, SC, 1, L, n_corr * step + L - 1, 0, 50, plant=False)
     fmf.matched_filter(tp, mo, w, d, step, check_zeros=False)
     assert _ran() == ran
+
+
+@pytest.mark.parametrize("step,L", [(60, 59), (60, 60), (60, 61), (200, 56), (300, 1)])
+@pytest.mark.parametrize("network_sum", [True, False])
+def test_steps_around_and_past_the_template(monkeypatch, step, L, network_sum):
+    """Phases past the last tap are left out."""
+    tp, mo, w, d = random_search(step + L, 3, 2, 2, L, 40 * step + L, -200, 300, zero_weights=1)
+    got = _search(monkeypatch, 32, tp, mo, w, d, step, network_sum=network_sum)
+    ref = fp64.fp64_matched_filter(tp, mo, w, d, step, "short", network_sum)
+    _check(got, ref.reshape(got.shape))
+
+
+@pytest.mark.parametrize("precision", ["fp32", "split_bf16"])
+def test_per_channel_lengths_past_the_step_and_below(monkeypatch, precision):
+    rng = np.random.default_rng(31)
+    tp, mo, w, d = random_search(32, 2, 3, 2, 150, 16000, -30, 90, zero_weights=1)
+    n = rng.integers(56, 151, mo.shape).astype(np.int32)
+    n[0, 0, 0] = 150
+    for i in np.ndindex(n.shape):
+        tp[i][n[i]:] = 0.0
+    got = _search(monkeypatch, 32, tp, mo, w, d, 100, n_samples_template=n, precision=precision)
+    ref = fp64.fp64_matched_filter_variable(tp, n, mo, w, d, 100, "short")
+    scale = np.cumsum(w.reshape(2, -1).sum(axis=1))[:, None]
+    assert (np.abs(got - ref) / scale).max() <= (6 * TOL if precision == "fp32" else 1e-4)
