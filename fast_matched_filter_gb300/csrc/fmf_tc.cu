@@ -1595,7 +1595,9 @@ int tc_fp32_nb(size_t T, size_t SC, size_t L, size_t step, size_t n_corr)
     const double taps = (double)step * (double)((((L + step - 1) / step + 19) / 20) * 20);
     const double tiles = (double)T * (double)((n_corr + 4095) / 4096) / 304.0;
     const double outputs = (double)T * (double)n_corr / (304.0 * 4096.0);
-    const double phases = std::min((double)step * 1.45 + 1.9, (double)step * 1.14 + 3.6);
+    // a phase's loads and barriers: 1.45 us in full tiles, 1.14 in nearly empty ones
+    const double fill = std::min(1.0, (double)n_corr / 4096.0), full = (double)step * 1.45 + 1.9;
+    const double phases = fill * full + (1.0 - fill) * std::min(full, (double)step * 1.14 + 3.6);
     const double plain_us = (double)SC * ((taps * 0.0165 + phases) * (tiles < 1.0 ? 1.0 : tiles) +
                                           taps * 0.03 * (step > 3 ? outputs : tiles));
     if (plain_us < 50.0)
