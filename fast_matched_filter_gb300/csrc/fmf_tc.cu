@@ -362,7 +362,9 @@ __global__ void tc_data_sparse_kernel(const float *__restrict__ data, int N, int
 
 // W[t][ch][phi][n][e][c] = pair of tphi[8n + e + c - (Q-1+s)], tphi[q] = tpl[step*q + phi],
 // s = mu mod Q, mu = floor((mo + phi) / step); one block per (template,
-// channel), its taps in shared memory (read once, written 8 times over).
+// channel), its taps in shared memory (read once, written 8 times over), or several where
+// that would leave SMs idle over the phases of a large step (4 templates x 3 channels,
+// step 439: 256 us with one block each, 20 us here).
 // FP32: also the channel's exponent, and the search's flag where a tap is not finite; the
 // bf16 forms keep such a tap.  queue: the tile queue of the persistent launch that
 // follows, cleared here (a memset costs 2 us).
@@ -374,17 +376,20 @@ struct TcTemplateWork {
     int *t_exp;
     unsigned *skip;
     unsigned long long *queue;
+    int parts;  // blocks per (template, channel)
 };
 
 template <bool FP32>
-__device__ __forceinline__ void tc_template_block(const TcTemplateWork &w, long long row /* t*SC + ch */, float *taps)
+__device__ __forceinline__ void tc_template_block(const TcTemplateWork &w, unsigned block, float *taps)
 {
+    const unsigned part = block % (unsigned)w.parts;
+    const long long row = block / (unsigned)w.parts;  // t*SC + ch
     const float *__restrict__ tpl = w.tpl;
     uint16_t *__restrict__ w_hi = w.w_hi, *__restrict__ w_lo = w.w_lo;
     const int L = w.L, step = w.step, NW = w.NW;
     int *t_exp = w.t_exp;
     unsigned *skip = w.skip;
-    if (w.queue && row == 0 && threadIdx.x == 0)
+    if (w.queue && block == 0 && threadIdx.x == 0)
         *w.queue = 0;
     const float *src = tpl + row * L;
     float inv_s = 1.0f;
@@ -426,7 +431,8 @@ __device__ __forceinline__ void tc_template_block(const TcTemplateWork &w, long 
     }
     const int m0 = w.mo[row];
     const int per_phase = NW * 8, used = tc_phases(step, L) * per_phase;
-    for (int i = threadIdx.x; i < used; i += blockDim.x) {
+    const int end = (int)((long long)used * (part + 1) / w.parts);
+    for (int i = (int)((long long)used * part / w.parts) + threadIdx.x; i < end; i += blockDim.x) {
         const int phi = i / per_phase, ne = i - phi * per_phase;
         int psi;
         const int s = tc_phase(m0 + phi, step, psi) & (TC_Q - 1);
@@ -476,7 +482,7 @@ __global__ void __launch_bounds__(256) tc_operand_kernel(const TcDataWork d, uns
     if (blockIdx.x < n_data)
         tc_data_block<FP32>(d, (int)blockIdx.x, operand_smem);
     else
-        tc_template_block<FP32>(w, (long long)(blockIdx.x - n_data), reinterpret_cast<float *>(operand_smem));
+        tc_template_block<FP32>(w, blockIdx.x - n_data, reinterpret_cast<float *>(operand_smem));
 }
 
 // ------------------------------------------------------------------ persistent kernel
@@ -1725,11 +1731,14 @@ static int tc_templates(TcSearch *full, int t0, int nt, unsigned long long *queu
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxDynamicSmem - 1024);
     if (e != cudaSuccess)
         return set_error(FMF_ERR_CUDA, "tc_operand_kernel shared memory: %s", cudaGetErrorString(e));
+    // blocks of 2,048 16-byte pairs at least, until there are eight per SM
+    const size_t rows = (size_t)nt * P.SC, most = (size_t)tc_phases(P.step, P.L) * sub->NW * 8 / 2048;
+    const unsigned parts = rows >= 1216 || most < 2 ? 1u : (unsigned)std::min(most, (1216 + rows - 1) / rows);
     const TcTemplateWork w{sub->P.tpl, sub->P.mo, P.L, P.step, sub->NW, full->w,
                            const_cast<uint16_t *>(full->pr.w_lo), const_cast<int *>(sub->t_exp),
-                           const_cast<unsigned *>(full->pr.skip), queue};
+                           const_cast<unsigned *>(full->pr.skip), queue, (int)parts};
     unsigned n_data = full->data_due ? (unsigned)full->data.tiles * full->data.SC : 0;
-    const unsigned n_templates = (unsigned)((size_t)nt * P.SC);
+    const unsigned n_templates = (unsigned)rows * parts;
     const size_t turn = tc_turn_bytes(P.step, full->pr.g_lo != nullptr), taps = (size_t)P.L * sizeof(float);
     // one launch (4 us less than two in a search of 50 us), unless the templates' shared
     // memory would leave room for fewer of the data's blocks
