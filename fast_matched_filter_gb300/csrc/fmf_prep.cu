@@ -765,6 +765,9 @@ constexpr int kFixThreads = 512;
 constexpr int kFixChunk = 16;
 constexpr int kFixBits = 40, kFixDigit = 20;
 constexpr int kFixLongest = 2048;
+// Windows of fewer samples are too quiet now and then by themselves, and every block of
+// noise would go on the list: 1 to 3 samples ('full': 4) in a block of 4,096 windows.
+constexpr int kFixShortest = 8;
 // Fewer blocks than this are one or two rounds of the SMs either way, and the second
 // launch would cost more than it saves.
 constexpr int kFixLeastBlocks = 608;
@@ -993,7 +996,7 @@ int launch_window_stats(const float *data, int N, int L, int SC, const float *mu
     unsigned grid = (unsigned)per_ch * SC;
     cudaError_t e;
     const size_t fixed = FixLayout(L, full).bytes();
-    if (fixed > (size_t)kMaxDynamicSmem - 1024 || L > kFixLongest || SC > 65535)
+    if (fixed > (size_t)kMaxDynamicSmem - 1024 || L > kFixLongest || L < kFixShortest || SC > 65535)
         list = nullptr;
     if (list) {
         auto kern = scan ? (full ? window_fixed_kernel<true, true> : window_fixed_kernel<false, true>)

@@ -47,3 +47,9 @@ def test_blocks_of_either_kind(monkeypatch, L, step, normalize):
         assert np.array_equal(a == 0, b == 0)
         a, b = np.nan_to_num(a, posinf=0, neginf=0), np.nan_to_num(b, posinf=0, neginf=0)
         assert np.abs(a - b).max() <= 2.0 ** -20, (s, c)
+
+
+@pytest.mark.parametrize("normalize", ["short", "full"])
+@pytest.mark.parametrize("L", [7, 8, 9])
+def test_windows_around_the_shortest_of_the_usual_blocks(monkeypatch, L, normalize):
+    test_blocks_of_either_kind(monkeypatch, L, 1, normalize)
