@@ -1614,11 +1614,12 @@ int detect_device(const float *cc, int T, int n_corr, size_t ld, const int *begi
     unsigned *bins = nullptr, *list = nullptr;
     float *saved = nullptr, *amb = nullptr, *keys = nullptr;
     // candidates per row: a sample window holds about 2.5 % of a row; the values whose
-    // MAD class waits for the median, about 7 % of a Gaussian row (at least two sectors
-    // of each of a block's columns; whole sectors)
+    // MAD class waits for the median, about 7 % of a Gaussian row.  A short row, which has a
+    // block to itself, may list all its values: a column gets 16 per step of its warp and a
+    // few of the row's ends, in whole sectors.
     const auto list_cap = [&](int part) {
-        const long long n = n_corr < 65536 ? n_corr : std::max(65536, n_corr / part);
-        return (std::max(2LL * kStep * kDetThreads, n) + 7) & ~7LL;
+        const long long all = ((n_corr + 4095LL) / 4096 * 16 + kStep) * kDetThreads;
+        return n_corr < 65536 ? all : (std::max(65536LL, (long long)n_corr / part) + 7) & ~7LL;
     };
     const long long key_cap = list_cap(8), amb_cap = list_cap(4);
     if ((rc = ws.get(&st, (size_t)chunk, "detection state")) ||

@@ -225,3 +225,15 @@ def test_detect_many_rows_with_a_gap(T, share):
     cc[T // 2] = np.float32(0.5)
     cc[T - 1] = (rng.standard_normal(n) * 0.01).astype(np.float32)
     assert_matches(fmf.detect(cc, n_mad=8.0, min_separation=25, max_detections=64), cc, 8.0, 25, 64)
+
+
+@pytest.mark.parametrize("n", [16385, 20480, 20481, 65535, 65536])
+def test_detect_short_rows_of_one_value(n):
+    """Rows of up to 65,535 lags list all their values; longer ones overflow their columns."""
+    cc = np.full((3, n), 0.25, np.float32)
+    cc[1, 7000:7010] = 1.0
+    cc[2] += np.arange(n, dtype=np.float32) % 3
+    for begin in (0, 3):
+        b, e = np.full(3, begin, np.int32), np.full(3, n - begin, np.int32)
+        assert_matches(fmf.detect(cc, n_mad=8.0, min_separation=25, max_detections=64, lag_begin=b, lag_end=e), cc, 8.0,
+                       25, 64, b, e)
