@@ -1618,10 +1618,13 @@ int tc_fp32_nb(size_t T, size_t SC, size_t L, size_t step, size_t n_corr)
     // channel and phase.  (100 templates x 9 channels x 300 lags, step 20, 300 taps: 319 us
     // on the CUDA cores, 397 here; 10 templates x 3 channels 128 and 114; the line is within
     // 10 % of the faster side in 240 searches of steps 3 to 200.)
-    const long long items = (long long)T * (long long)((n_corr + 128 * (size_t)nb - 1) / (128 * (size_t)nb));
-    double rounds = 1e300;  // of whole items on the busiest SM, in the best number of channel parts
-    for (long long k = 1; k <= TC_MAX_PARTS && k <= (long long)SC; k++)
-        rounds = std::min(rounds, (double)((k * items + 151) / 152) / (double)k);
+    // Rounds of whole items on the busiest SM, in the channel parts of all templates, a
+    // roomful of templates at a time (few at large steps, whose operand blocks are large).
+    const size_t per_template = SC * step * (size_t)tc_shape((int)L, (int)step, 1, nb).NW * 256;
+    const long long room = std::min((long long)T, std::max(1ll, (long long)(kMaxTemplateBytes / per_template)));
+    const long long n_tiles = (long long)((n_corr + 128 * (size_t)nb - 1) / (128 * (size_t)nb));
+    const long long k = choose_parts((long long)T * n_tiles, (int)SC);
+    const double rounds = (double)((T + room - 1) / room) * (double)((k * room * n_tiles + 151) / 152) / (double)k;
     const double used = (double)std::min(step, L), tc_us = 50.0 + rounds * (double)SC * used * (2.7 + 0.0066 * (double)L / used);
     return plain_us + 21.0 < tc_us ? 0 : nb;
 }
