@@ -42,18 +42,18 @@
 // The tensor core rounds every accumulation toward zero, so a long chain drifts, most of
 // all at a match, where every product adds: a chain of m steps that add something to the
 // output is some 0.6e-7 m low at a perfect match.  So the h h products run in chains of a
-// few steps (tc_chain_cols), each in a fresh accumulator that the epilogue adds to its
+// few steps (tc_chains), each in a fresh accumulator that the epilogue adds to its
 // registers in FP32 (rounded to nearest); h l and l h, smaller by the pair's rounding,
 // share one accumulator per channel.  RMS error at perfect matches of Hann-tapered noise,
 // FP32 multiply-adds and here: 56 taps 1.34 and 1.36e-7, 112 taps 1.74 and 1.21e-7, 300
-// taps 2.80 and 1.73e-7, 600 taps 4.1 and 3.5e-7, 1,200 taps 6.0 and 3.8e-7 (with chains of
+// taps 2.80 and 2.50e-7, 600 taps 4.1 and 3.5e-7, 1,200 taps 6.0 and 3.8e-7 (with chains of
 // 16 steps 2.1, 2.8, 4.7, 7.2, 7.3e-7); away from matches it is further below.
 //
 // What bounds it: the tensor pipe, and with it the power limit, from some 500
 // taps (40 templates x 60 channels x 1.08M lags x 600 taps in 6.3 ms: 1.8
 // PFLOP/s of MMAs, 1.74 is what cuBLAS sustains under the limit); the issuing
 // threads and the epilogue below, which takes some 400 cycles per chain (with the
-// preparation 300 taps 5.8 ms, 60 taps 4.3 ms; in chains of 16 steps 4.7 and 3.5 ms).
+// preparation 300 taps 5.2 ms, 60 taps 4.3 ms; in chains of 16 steps 4.7 and 3.5 ms).
 // An issuing thread's code costs as much as its MMAs: a branchy loop took 500 cycles
 // per MMA of 64.
 //
@@ -538,7 +538,8 @@ __device__ __forceinline__ void tc_issue(const TcBatch<N> &B, const long long *r
         // kind::f16 descriptor: F32 accumulate, A and B both FP16 or both BF16, K-major, N = cols, M = 128
         const uint32_t idesc = (1u << 4) | B.mma_types | ((uint32_t)(cols >> 3) << 17) | ((uint32_t)(TC_Q >> 4) << 24);
         const int SC = pr.P.SC, step = pr.P.step, L = pr.P.L;
-        const uint32_t chain_cols = (uint32_t)pr.chain_cols;
+        const uint32_t all_pairs = (uint32_t)uniform(tc_phases(step, L)) * (TC_CB / 2);
+        const uint32_t chains = SMALL ? 0u : (uint32_t)pr.chains;
         const uint32_t col_bytes = (uint32_t)pr.R * 16;
         // 16-byte units from a high half to its low half, and of a column-block pair
         const uint32_t a_low = (uint32_t)pr.NW * 8, b_low = 4u * (uint32_t)pr.R, b_pair = 2u * (uint32_t)pr.R;
@@ -562,7 +563,9 @@ __device__ __forceinline__ void tc_issue(const TcBatch<N> &B, const long long *r
                     phases = tc_phases(step, ntap);
                 if (VAR && chain_steps)
                     parts_log2 = (uint32_t)tc_pair_chains(L, step, ntap, chain_steps);
-                uint32_t left = 0;  // column-block pairs left to the accumulator
+                // a chain ends where `chains` of them spread over all pairs do, and at the last pair
+                uint32_t credit = 0;
+                bool fresh = true;
                 uint32_t dt = 0, acc = 0;
                 const auto next_acc = [&]() {
                     const uint32_t empty = bar + (SMALL ? TcBars::sempty : TcBars::hempty) + 8 * (acc_i & 1);
@@ -571,7 +574,6 @@ __device__ __forceinline__ void tc_issue(const TcBatch<N> &B, const long long *r
                     tc_fence_after();
                     dt = tmem + (SMALL ? 256u : 0u) + 128u * (acc_i & 1);
                     acc = 0;
-                    left = SMALL ? (uint32_t)phases * (TC_CB / 2) : (parts_log2 ? 1u : chain_cols);
                     return true;
                 };
                 for (int phi = 0; phi < phases; phi++, stages++) {
@@ -585,7 +587,7 @@ __device__ __forceinline__ void tc_issue(const TcBatch<N> &B, const long long *r
                     const uint32_t a0 = a_base + (wb ? a_buf : 0u);
 #pragma unroll 1
                     for (uint32_t j = 0; j < TC_CB / 2; j++) {
-                        if (left == 0 && !next_acc())
+                        if (fresh && !next_acc())
                             return;
                         // two column-block pairs per slot
                         if ((j & 1) == 0 && !wait(bar + TcBars::dfull + 8 * slot, turn & 1, 8u))
@@ -627,7 +629,11 @@ __device__ __forceinline__ void tc_issue(const TcBatch<N> &B, const long long *r
                             }
                         }
                         issue(n);
-                        const bool done = --left == 0 || (!SMALL && j == TC_CB / 2 - 1 && phi == phases - 1);
+                        credit += chains;
+                        const bool done = credit >= all_pairs || (!SMALL && parts_log2) ||
+                                          (j == TC_CB / 2 - 1 && phi == phases - 1);
+                        if (credit >= all_pairs)
+                            credit -= all_pairs;
                         if (one) {
                             if (j & 1)
                                 mma_commit(bar + TcBars::dempty + 8 * slot);
@@ -638,10 +644,9 @@ __device__ __forceinline__ void tc_issue(const TcBatch<N> &B, const long long *r
                             slot = 0;
                             turn++;
                         }
-                        if (done) {
+                        fresh = done;
+                        if (done)
                             acc_i++;
-                            left = 0;
-                        }
                     }
                     if (one)
                         mma_commit(bar + TcBars::wempty + 8 * wb);
@@ -964,7 +969,9 @@ __global__ void __launch_bounds__(tc_threads(VAR), 1) tc_persistent(const __grid
             // h h chains of a channel: of whole pairs, or several of each
             const auto chains_of = [&](int n) {
                 const int log2 = tc_pair_chains(pr.P.L, step, n, pr.chain_steps), cols = tc_phases(step, n) * (TC_CB / 2);
-                return log2 ? cols << log2 : (cols + pr.chain_cols - 1) / pr.chain_cols;
+                const long long all = tc_phases(step, pr.P.L) * (TC_CB / 2);
+                // (the last pair ends one, whether or not the chains before it come out even)
+                return log2 ? cols << log2 : (int)((cols - 1) * (long long)pr.chains / all) + 1;
             };
             const int chains = ONE || VAR ? 1 : chains_of(pr.P.L);
             for (int g0 = c_begin; busy && g0 < c_end; g0 += 32) {
@@ -1586,7 +1593,7 @@ size_t tc_template_bytes(const Problem &P, int nb)
 //
 // Below kFp32LeastTaps the pairs' 22 bits show: the RMS error against 64 bits is 1.4 of the
 // FMAs' at 10 taps, 1.08 at 40, 1.00 at 44 to 52 and falls to 0.4 at 300 (random searches; at
-// matches tc_chain_cols keeps it below theirs).
+// matches tc_chains keeps it below theirs).
 int tc_fp32_nb(size_t T, size_t SC, size_t L, size_t step, size_t n_corr)
 {
     if (const char *env = getenv("FMF_TC32")) {  // 0: the CUDA cores; 32, 64, 128: this tile
@@ -1629,17 +1636,24 @@ int tc_fp32_nb(size_t T, size_t SC, size_t L, size_t step, size_t n_corr)
     return plain_us + 21.0 < tc_us ? 0 : nb;
 }
 
-// Column-block pairs of one h h chain of an FP32 search, and the K steps (least of the pairs')
-// past which a pair is several.  Of a pair's steps, (taps + 15) / 128 add something to an
-// output, and a chain of m such steps is off by some 0.6e-7 m at a perfect match (the
-// header of this file); multiply-adds of L taps in a row by 1.65e-8 sqrt(L), RMS.  m up to
-// 0.22 sqrt(L) keeps the former below the latter.
-static int tc_chain_cols(int L, int step, int *chain_steps)
+// h h chains of a channel of an FP32 search, and the K steps (least of the pairs') past
+// which a column-block pair is several.  Of a pair's steps, (taps + 15) / 128 add something
+// to an output, and chains of m such steps are off by some 0.6e-7 m at a perfect match (the
+// header of this file; of unequal ones m is the mean over the steps); multiply-adds of L
+// taps in a row by 1.65e-8 sqrt(L), RMS.  m up to 0.24 sqrt(L) - 0.35 keeps the former below
+// the latter.
+static int tc_chains(int L, int step, int *chain_steps)
 {
-    const double most = 0.22 * std::sqrt((double)L), per_pair = ((L + step - 1) / step + 15) / 128.0;
-    const int cols = (int)(most / per_pair);
-    *chain_steps = (int)std::ceil(most);
-    return cols < 1 ? 1 : (cols < step * (TC_CB / 2) ? cols : step * (TC_CB / 2));
+    const double most = 0.24 * std::sqrt((double)L) - 0.35, per_pair = ((L + step - 1) / step + 15) / 128.0;
+    *chain_steps = (int)std::ceil(most < 1.0 ? 1.0 : most);
+    const long long pairs = (long long)tc_phases(step, L) * (TC_CB / 2);
+    for (long long n = 1; n < pairs; n++) {  // n chains: `longer` of them have a pair more
+        const long long each = pairs / n, longer = pairs - each * n;
+        const double mean = (double)(longer * (each + 1) * (each + 1) + (n - longer) * each * each) / (double)pairs;
+        if (mean * per_pair <= most)
+            return (int)n;
+    }
+    return (int)pairs;
 }
 
 // Per-channel outputs of at least so many channels go through an array of their own and
@@ -1706,7 +1720,7 @@ int tc_begin(const Problem &P, int form, int nb, int tg, int max_templates, Scra
         }
     }
     // The bf16 pairs' own rounding (4.4e-6 of a product) is far above a channel-long chain's
-    pr.chain_cols = fp32 ? tc_chain_cols(P.L, step, &pr.chain_steps) : step * (TC_CB / 2);
+    pr.chains = fp32 ? tc_chains(P.L, step, &pr.chain_steps) : 0;
     TcDataWork &d = out->data;
     d = TcDataWork{P.data, P.N, SC, step, 0, pr.rows_total, pr.row_front, fp32 ? P.scan : nullptr, g_hi, g_lo,
                    fp32 ? exps + n_rows : nullptr, fp32 ? P.scan + 3 * SC : nullptr, P.ntap && P.normalize == 0};

@@ -36,7 +36,8 @@ struct TcProb {
     // FP32 form (fmf_tc.cu): operands are fp16 pairs in units of powers of two
     const int *t_exp;             // [T][SC] exponent of each channel's template
     const int *d_exp;             // [SC] exponent of each data channel
-    int chain_cols;               // column-block pairs of one h h chain
+    int chains;                   // h h chains of a channel that uses all phases, of as many
+                                  // column-block pairs each as it goes; 0: one, whatever its phases
     int chain_steps;              // a pair of more K steps than this is several chains (tc_pair_chains); 0: one
     const unsigned *skip;         // nonzero: the FP32 CUDA-core kernel runs this search instead
 };

@@ -337,3 +337,17 @@ def test_per_channel_lengths_past_the_step_and_below(monkeypatch, precision):
     ref = fp64.fp64_matched_filter_variable(tp, n, mo, w, d, 100, "short")
     scale = np.cumsum(w.reshape(2, -1).sum(axis=1))[:, None]
     assert (np.abs(got - ref) / scale).max() <= (6 * TOL if precision == "fp32" else 1e-4)
+
+
+@pytest.mark.parametrize("step", [1, 5, 100])
+@pytest.mark.parametrize("n", [56, 58, 62, 79, 81, 99, 100, 149])
+def test_chains_of_channels_shorter_than_the_longest(monkeypatch, n, step):
+    """The issuer and the epilogue count a channel's chains apart."""
+    tp, mo, w, d = random_search(n, 2, 2, 1, 150, 6000 + 10 * step, -30, 90)
+    lengths = np.full(mo.shape, 150, np.int32)
+    lengths[:, 1] = n
+    tp[:, 1, :, n:] = 0.0
+    got = _search(monkeypatch, 32, tp, mo, w, d, step, n_samples_template=lengths)
+    ref = fp64.fp64_matched_filter_variable(tp, lengths, mo, w, d, step, "short")
+    scale = np.cumsum(w.reshape(2, -1).sum(axis=1))[:, None]
+    assert (np.abs(got - ref) / scale).max() <= 6 * TOL
